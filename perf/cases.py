@@ -4,7 +4,8 @@
 makes what a program holds before the call (tensors, rotation tables, block masks, the traced
 function), `run(state)` is one call through the public entry points, `work(case)` counts the bytes
 and floating-point operations that call cannot do without, and `tolerance(case)` bounds the
-difference between two correct implementations at the same precision.
+difference between two correct implementations at the same precision, and `exact(case, seed)` is the
+result in 64 bits.
 
 Kinds: "prefill" (square forward), "chunk" (rows of a prompt against a cache), "train" (forward and
 backward of one layer), "blocks" (block-sparse forward and backward) and "decode" (one query row per
@@ -252,3 +253,83 @@ def tolerance(case):
     if case["dtype"] == "f16":
         return {"rel": 2e-3 if grad else 1.5e-3}
     return {"rel": 1.5e-2 if grad else 1.2e-2}
+
+
+def _slopes(n):
+    """ALiBi slopes of n heads (Press et al.): geometric for a power of two, else the closest lower
+    power of two followed by every other slope of the doubled sequence."""
+    def geometric(m):
+        return [2.0 ** (-8.0 * (i + 1) / m) for i in range(m)]
+    if n & (n - 1) == 0:
+        return geometric(n)
+    low = 1 << (n.bit_length() - 1)
+    return geometric(low) + geometric(2 * low)[0::2][:n - low]
+
+
+def _rotated(x, cos, sin):
+    half = x.shape[-1] // 2
+    return x * cos + torch.cat([-x[..., half:], x[..., :half]], dim=-1) * sin
+
+
+def exact(case, seed):
+    """What `run` returns, in 64 bits, one (batch, KV head) group after the other; gradients are
+    written out: P and dP of one head, then the four products."""
+    state = prepare(case, seed)
+    q, k, v = (state[t].detach() for t in ("q", "k", "v"))
+    dev, kw, kind = q.device, state["kw"], state["kind"]
+    B, H_q, n_q, D = q.shape
+    H_kv, n_kv = k.shape[1], k.shape[2]
+    group, scale, train = H_q // H_kv, D ** -0.5, kind in ("train", "blocks")
+    first = kw.get("q_offset", 0)
+    first = first.tolist() if torch.is_tensor(first) else [first] * B
+    lens = kw["kv_lens"].tolist() if "kv_lens" in kw else [n_kv] * B
+    cols = torch.arange(n_kv, device=dev)
+    rope = "cos" in kw
+    if rope:
+        cos, sin = (kw[t].double().reshape(-1, D) for t in ("cos", "sin"))
+    # the slope table is created in the type of the operands
+    slopes = torch.tensor(_slopes(H_q), dtype=DTYPES[case["dtype"]]).double().tolist() if case.get("alibi") else None
+    grids = torch.from_numpy(_bigbird(case, seed)).to(dev) if kind == "blocks" else None
+    out = torch.empty(q.shape, dtype=torch.float64, device=dev)
+    if train:
+        dq, dk, dv = (torch.zeros(t.shape, dtype=torch.float64, device=dev) for t in (q, k, v))
+    for b in range(B):
+        rows = torch.arange(n_q, device=dev) + first[b]
+        rel = rows[:, None] - cols[None, :]
+        keep = None
+        if kind == "chunk" or (kind != "decode" and case.get("mask") == "causal"):
+            keep = rel >= 0
+        elif case.get("mask") == "window":
+            keep = rel.abs() < case["window"]
+        elif kind == "decode":
+            keep = (cols < lens[b])[None, :]
+        for h in range(H_q):
+            g = h // group
+            qh, kh, vh = q[b, h].double(), k[b, g].double(), v[b, g].double()
+            if rope:
+                qh = _rotated(qh, cos[rows], sin[rows])
+                if not case.get("rotated"):
+                    kh = _rotated(kh, cos[:n_kv], sin[:n_kv])
+            s = (qh @ kh.T).mul_(scale)
+            if slopes:
+                s -= slopes[h] * rel.abs()
+            if kind == "blocks":
+                keep = grids[h].repeat_interleave(case["block"], 0).repeat_interleave(case["block"], 1)[:n_q, :n_kv]
+            if keep is not None:
+                s.masked_fill_(~keep, float("-inf"))
+            p = torch.softmax(s, dim=-1)
+            del s
+            out[b, h] = p @ vh
+            if train:
+                do = state["do"][b, h].double()
+                dv[b, g] += p.T @ do
+                ds = do @ vh.T
+                ds.sub_((do * out[b, h]).sum(-1, keepdim=True)).mul_(p).mul_(scale)
+                gq, gk = ds @ kh, ds.T @ qh
+                if rope:          # the transpose of the rotation is the one with -sin
+                    gq, gk = _rotated(gq, cos[rows], -sin[rows]), _rotated(gk, cos[:n_kv], -sin[:n_kv])
+                dq[b, h] += gq
+                dk[b, g] += gk
+                del ds
+            del p
+    return (out, dq, dk, dv) if train else out

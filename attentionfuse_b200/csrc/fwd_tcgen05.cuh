@@ -48,6 +48,11 @@ enum { ROPE_NONE = 0, ROPE_FUSED = 1 };   // a pre-pass rotation runs the ROPE_N
 enum { EMASK_NONE = 0, EMASK_CAUSAL = 1, EMASK_WINDOW = 2, EMASK_BITS = 3 };  // element-level mask of the instantiation
 // (EMASK_BITS: block lists in which some tiles carry a bit matrix of their active elements)
 
+// What an item's key tiles are: all that its query tile visits; the share of a split-K decode call; one of
+// TcArgs::key_shares shares of a query tile (instances of their own: the extra item arithmetic and
+// epilogue cost the plain ones 3 - 5 %).
+enum { SPLIT_NONE = 0, SPLIT_DECODE = 1, SPLIT_SHARES = 2 };
+
 constexpr int BM = 128;
 constexpr int BN = 128;
 constexpr int PANEL_BYTES = 128 * 128;   // 128 rows x 64 elements x 2 bytes
@@ -142,6 +147,12 @@ struct TcArgs {
   // combine kernel instead of O.  Row index of the partials: (split * B + b) * H_total + head.
   int num_splits;
   const int32_t* kv_lens;   // optional per-batch valid key count
+  // Shares of the key tiles of a query tile (dense, causal and window masks; otherwise 1): with more
+  // than one, an item is (query tile, share), its epilogue writes the un-normalised partials, and
+  // the merge kernel of the host file makes O of them.  Row index of the partials:
+  // ((share * B + b) * H_q + h) * N_q + row.
+  int key_shares;
+  FastDiv div_shares;
   float* ws_m;
   float* ws_l;
   float* ws_acc;
@@ -161,6 +172,21 @@ struct TileWalk {
   }
 };
 
+// Key tiles [first, first + n) that the query rows [m_blk * BM, ...) visit under a dense, causal or
+// window mask.
+__host__ __device__ __forceinline__ void tile_range(const AfProblem& p, int m_blk, int& first, int& n) {
+  const int m0 = m_blk * BM + p.q_offset;                 // first / one-past-last position of the tile
+  const int rows_end = m_blk * BM + BM, m_end = (rows_end < p.N_q ? rows_end : p.N_q) + p.q_offset;
+  int lo = 0, hi = p.N_kv;
+  if (p.mask_kind == AF_MASK_CAUSAL) hi = m_end < hi ? m_end : hi;
+  if (p.mask_kind == AF_MASK_WINDOW) {
+    lo = m0 - p.window + 1 > 0 ? m0 - p.window + 1 : 0;
+    hi = m_end + p.window - 1 < hi ? m_end + p.window - 1 : hi;
+  }
+  first = lo / BN;
+  n = hi > lo ? (hi + BN - 1) / BN - first : 0;
+}
+
 __device__ __forceinline__ TileWalk make_walk(const AfProblem& p, const TcArgs& args, int m_blk, int h) {
   TileWalk w;
   w.list = nullptr;
@@ -171,23 +197,14 @@ __device__ __forceinline__ TileWalk make_walk(const AfProblem& p, const TcArgs& 
   // would raise the row maximum (and rescale the accumulator) at every tile; walking down from
   // the diagonal sets the reference in the first tile and every later tile stays below it.
   w.step = (p.mask_kind == AF_MASK_CAUSAL && p.bias_kind == AF_BIAS_ALIBI) ? -1 : 1;
-  const int m0 = m_blk * BM + p.q_offset;                 // first / one-past-last position of the tile
-  const int m_end = min(m_blk * BM + BM, p.N_q) + p.q_offset;
   if (p.mask_kind == AF_MASK_BLOCKS) {
     const int qb = m_blk / args.q_tiles_per_block;
     w.per_block = args.kv_tiles_per_block;
     w.list = p.kv_idx + (int64_t)h * p.kv_idx_stride_h + (int64_t)qb * p.kv_idx_stride_q;
     if (p.kv_slot != nullptr) w.slots = p.kv_slot + (int64_t)h * p.kv_idx_stride_h + (int64_t)qb * p.kv_idx_stride_q;
     w.n_tiles = p.kv_num[(int64_t)h * p.kv_num_stride_h + qb] * w.per_block;
-  } else if (p.mask_kind == AF_MASK_CAUSAL) {
-    w.n_tiles = (min(m_end, p.N_kv) + BN - 1) / BN;
-  } else if (p.mask_kind == AF_MASK_WINDOW) {
-    const int lo = max(0, m0 - p.window + 1);
-    const int hi = min(p.N_kv, m_end + p.window - 1);
-    w.first_tile = lo / BN;
-    w.n_tiles = hi > lo ? (hi + BN - 1) / BN - w.first_tile : 0;
   } else {
-    w.n_tiles = (p.N_kv + BN - 1) / BN;
+    tile_range(p, m_blk, w.first_tile, w.n_tiles);
   }
   if (w.n_tiles < 0) w.n_tiles = 0;
   return w;
@@ -213,7 +230,7 @@ struct Item {
 // r*G + c in even rounds r and r*G + (G-1-c) in odd rounds (c = blockIdx.x, G = gridDim.x): with
 // item weights that fall monotonically the zig-zag evens out the key tiles per CTA to within a
 // fraction of a percent.  With G = number of items every CTA runs exactly one item.
-template <int EMASK, bool SPLIT>
+template <int EMASK, int SPLIT>
 __device__ __forceinline__ bool get_item(const TcArgs& args, int round, Item& it) {
   const int G = (int)gridDim.x, c = (int)blockIdx.x;
   const int64_t w64 = (int64_t)round * G + ((round & 1) ? G - 1 - c : c);
@@ -221,13 +238,14 @@ __device__ __forceinline__ bool get_item(const TcArgs& args, int round, Item& it
   const int w = (int)w64;
   const AfProblem& p = args.a.p;
   int w_over_bh, bh;   // row of query tiles in visiting order (split mode: the split), (batch, head) unit
-  split_item(args, w, SPLIT ? args.num_splits : args.num_m_blocks, w_over_bh, bh);
+  split_item(args, w, SPLIT == SPLIT_DECODE ? args.num_splits : SPLIT == SPLIT_SHARES ? args.num_m_blocks * args.key_shares
+                                                                                       : args.num_m_blocks, w_over_bh, bh);
   it.b = args.div_hq.div(bh);
   it.h = bh - it.b * p.H_q;
   it.h_kv = args.div_group.div(it.h);
   it.split = 0;
   it.n_kv = p.N_kv;
-  if (SPLIT) {
+  if (SPLIT == SPLIT_DECODE) {
     // split-K decode: one query tile per (batch, pseudo-head); the 128-key tiles of the valid
     // length are dealt out evenly to the splits
     it.split = w_over_bh;
@@ -240,9 +258,19 @@ __device__ __forceinline__ bool get_item(const TcArgs& args, int round, Item& it
     wk.n_tiles = (int)((int64_t)(it.split + 1) * tiles / args.num_splits) - wk.first_tile;
     return true;
   }
+  if (SPLIT == SPLIT_SHARES) {
+    const int m_idx = args.div_shares.div(w_over_bh);
+    it.split = w_over_bh - m_idx * args.key_shares;
+    w_over_bh = m_idx;
+  }
   const int m_blk = (EMASK == EMASK_CAUSAL) ? (args.num_m_blocks - 1 - w_over_bh) : w_over_bh;
   it.m0 = m_blk * BM;
   it.walk = make_walk(p, args, m_blk, it.h);
+  if (SPLIT == SPLIT_SHARES) {
+    const int lo = args.div_shares.div(it.split * it.walk.n_tiles);
+    it.walk.n_tiles = args.div_shares.div((it.split + 1) * it.walk.n_tiles) - lo;
+    it.walk.first_tile += lo;
+  }
   return true;
 }
 
@@ -256,7 +284,7 @@ __device__ __forceinline__ void cursor_init(TileCursor& c) {
   c.round = -1; c.j = 0; c.gg = -1; c.qi = -1;
   c.it.walk.n_tiles = 0;
 }
-template <int EMASK, bool SPLIT>
+template <int EMASK, int SPLIT>
 __device__ __forceinline__ bool cursor_next(const TcArgs& args, TileCursor& c) {
   if (c.j + 1 < c.it.walk.n_tiles) { ++c.j; ++c.gg; return true; }
   for (;;) {
@@ -450,7 +478,7 @@ __device__ __forceinline__ void exp_pass(const uint32_t (&xr)[NC], uint32_t (&pk
 // One instantiation per composition: element type, head_dim, RoPE mode, element-level mask and
 // ALiBi are compile-time, so the per-element code of the softmax group carries no run-time
 // branches on the composition.
-template <typename T, int D, int ROPE, int EMASK, bool ALIBI, bool SPLIT>
+template <typename T, int D, int ROPE, int EMASK, bool ALIBI, int SPLIT>
 __global__ void __launch_bounds__(ROPE == ROPE_FUSED ? 384 : 352, 1)
 fwd_tcgen05_kernel(const TcArgs args, const __grid_constant__ CUtensorMap tmap_q,
                    const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
@@ -530,7 +558,7 @@ fwd_tcgen05_kernel(const TcArgs args, const __grid_constant__ CUtensorMap tmap_q
       // Two cursors over the same tile sequence: K runs one tile ahead of V, so that a wait for
       // a V slot (free only after the P.V product two tiles back) never holds up a K load.
       // split-K decode reads every cache tile exactly once: nothing to keep there
-      const uint64_t stream = l2_policy_evict_first(), keep = SPLIT ? stream : l2_policy_evict_last();
+      const uint64_t stream = l2_policy_evict_first(), keep = SPLIT == SPLIT_DECODE ? stream : l2_policy_evict_last();
       TileCursor ck, cv;
       cursor_init(ck);
       cursor_init(cv);
@@ -715,7 +743,7 @@ fwd_tcgen05_kernel(const TcArgs args, const __grid_constant__ CUtensorMap tmap_q
         tmem_wait_ld();
 
         // Tile-level decision: only edge / diagonal tiles pay for element masking.
-        const int n_kv = SPLIT ? it.n_kv : p.N_kv;
+        const int n_kv = SPLIT == SPLIT_DECODE ? it.n_kv : p.N_kv;
         bool need_mask = key0 + BN > n_kv;
         const int pos0 = m0 + p.q_offset;           // position of the tile's first row on the key axis
         if (EMASK == EMASK_CAUSAL) need_mask = need_mask || (key0 + BN - 1 > pos0);
@@ -803,7 +831,7 @@ fwd_tcgen05_kernel(const TcArgs args, const __grid_constant__ CUtensorMap tmap_q
           exp_pass<T, ALIBI ? EXP_PRESCALED : EXP_SCALE>(xr, pk, scale2, neg_m, 0.f, rsum);
         }
         l_part = l_part * alpha + rsum;
-        if (SPLIT && key0 + BN > n_kv) {
+        if (SPLIT == SPLIT_DECODE && key0 + BN > n_kv) {
           // Split-K decode: cache rows past the valid length hold whatever the allocation held
           // (TMA zero-fills only past the tensor's extent) and 0 * NaN would poison O, so the
           // softmax threads clear those V rows of the stage before they release P.
@@ -832,7 +860,8 @@ fwd_tcgen05_kernel(const TcArgs args, const __grid_constant__ CUtensorMap tmap_q
       // through the same words (two hand-shakes; the next item's words are written only after
       // this item's have been read).
       if (!alive) break;
-      if (!SPLIT && lane == 0) bulk_wait_read_all();   // previous item's staged rows: long gone by now
+      constexpr bool partial = SPLIT != SPLIT_NONE;
+      if (!partial && lane == 0) bulk_wait_read_all();   // previous item's staged rows: long gone by now
       float c0 = 0.f, c1 = 0.f, m_all = 0.f, l_sum = 0.f;
       if (half == 1) {
         bars->xchg[rtid] = m_ref;
@@ -845,8 +874,8 @@ fwd_tcgen05_kernel(const TcArgs args, const __grid_constant__ CUtensorMap tmap_q
         const float w_mine = (m_ref == -INFINITY) ? 0.f : ex2_approx(m_ref - m_all);
         const float w_other = (m_other == -INFINITY) ? 0.f : ex2_approx(m_other - m_all);
         l_sum = l_part * w_mine + l_other * w_other;
-        // split-K decode keeps the partial un-normalised for the combine kernel
-        const float inv = SPLIT ? 1.f : 1.f / ((l_sum == 0.f) ? 1.f : l_sum);
+        // a share of the keys keeps its partial un-normalised for the merge
+        const float inv = partial ? 1.f : 1.f / ((l_sum == 0.f) ? 1.f : l_sum);
         c0 = w_mine * inv;
         c1 = w_other * inv;
         bars->xchg[rtid] = c0;
@@ -880,8 +909,8 @@ fwd_tcgen05_kernel(const TcArgs args, const __grid_constant__ CUtensorMap tmap_q
 #pragma unroll
         for (int i = 0; i < D / 2; ++i) o[i] = 0.f;
       }
-      if (SPLIT) {
-        // split-K decode: un-normalised partial of this (split, batch, head) for the combine kernel
+      if (partial) {
+        // un-normalised partial of this (split, batch, head) for the merge
         // The fp32 rows go through the warp's staging region too, 32 columns at a time, and leave
         // as whole 128-byte lines (four rows per store instruction) instead of 32 lines per
         // instruction: rows of the partials are D floats apart and consecutive in the workspace.
@@ -988,7 +1017,7 @@ fwd_tcgen05_kernel(const TcArgs args, const __grid_constant__ CUtensorMap tmap_q
 // ---------------------------------------------------------------------------------------
 // Launch of one instantiation (tensor maps are encoded by the host file)
 // ---------------------------------------------------------------------------------------
-template <typename T, int D, int ROPE, int EMASK, bool ALIBI, bool SPLIT = false>
+template <typename T, int D, int ROPE, int EMASK, bool ALIBI, int SPLIT = SPLIT_NONE>
 int launch_instance(const TcArgs& args, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
                     const CUtensorMap& mo, cudaStream_t st) {
   auto kern = fwd_tcgen05_kernel<T, D, ROPE, EMASK, ALIBI, SPLIT>;
@@ -1010,7 +1039,7 @@ int launch_composition(const TcArgs& args, const CUtensorMap& mq, const CUtensor
                        const CUtensorMap& mo, cudaStream_t st) {
   const AfProblem& p = args.a.p;
   if (args.num_splits > 0) {   // split-K decode: dense, no bias, no rotation (one extra instantiation)
-    if constexpr (ROPE == ROPE_NONE) return launch_instance<T, D, ROPE_NONE, EMASK_NONE, false, true>(args, mq, mk, mv, mo, st);
+    if constexpr (ROPE == ROPE_NONE) return launch_instance<T, D, ROPE_NONE, EMASK_NONE, false, SPLIT_DECODE>(args, mq, mk, mv, mo, st);
     else return fail(AF_ERR_UNSUPPORTED, "split-K decode takes no rotation");
   }
   int em = p.mask_kind == AF_MASK_CAUSAL ? EMASK_CAUSAL : p.mask_kind == AF_MASK_WINDOW ? EMASK_WINDOW : EMASK_NONE;
@@ -1023,6 +1052,20 @@ int launch_composition(const TcArgs& args, const CUtensorMap& mq, const CUtensor
                    : launch_instance<T, D, ROPE_NONE, EMASK_BITS, false>(args, mq, mk, mv, mo, st);
     } else {
       return fail(AF_ERR_UNSUPPORTED, "block lists with element bit matrices take no rotation");
+    }
+  }
+  if (args.key_shares > 1) {
+    if constexpr (ROPE == ROPE_NONE && D == 128) {
+      switch (em * 2 + (alibi ? 1 : 0)) {
+        case 0: return launch_instance<T, D, ROPE, EMASK_NONE, false, SPLIT_SHARES>(args, mq, mk, mv, mo, st);
+        case 1: return launch_instance<T, D, ROPE, EMASK_NONE, true, SPLIT_SHARES>(args, mq, mk, mv, mo, st);
+        case 2: return launch_instance<T, D, ROPE, EMASK_CAUSAL, false, SPLIT_SHARES>(args, mq, mk, mv, mo, st);
+        case 3: return launch_instance<T, D, ROPE, EMASK_CAUSAL, true, SPLIT_SHARES>(args, mq, mk, mv, mo, st);
+        case 4: return launch_instance<T, D, ROPE, EMASK_WINDOW, false, SPLIT_SHARES>(args, mq, mk, mv, mo, st);
+        default: return launch_instance<T, D, ROPE, EMASK_WINDOW, true, SPLIT_SHARES>(args, mq, mk, mv, mo, st);
+      }
+    } else {
+      return fail(AF_ERR_UNSUPPORTED, "shares of the keys exist for head_dim 128 and rotated operands");
     }
   }
   switch (em * 2 + (alibi ? 1 : 0)) {

@@ -205,6 +205,47 @@ int launch_prepass(const AfProblem& p, void* q_out, void* k_out, cudaStream_t st
 
 }  // namespace
 
+// O of the rows whose keys were dealt out to several shares (TcArgs::key_shares): D / 4 lanes per row,
+// one 16-byte load per share and lane.  Bound by latency at the sizes it runs at (a few MB).
+namespace {
+template <typename T>
+__global__ void merge_shares_kernel(const AfFwdParams a, const int shares, const float* __restrict__ ws_m,
+                                    const float* __restrict__ ws_l, const float* __restrict__ ws_acc) {
+  constexpr int D = 128, LANES = D / 4;
+  const AfProblem& p = a.p;
+  const int rows = p.B * p.H_q * p.N_q;
+  const int row = (int)((blockIdx.x * blockDim.x + threadIdx.x) / LANES), lane = (int)(threadIdx.x % LANES);
+  if (row >= rows) return;
+  float m = -INFINITY;
+  for (int s = 0; s < shares; ++s) m = fmaxf(m, ws_m[(int64_t)s * rows + row]);
+  const float m_use = (m == -INFINITY) ? 0.f : m;
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  float l = 0.f;
+#pragma unroll 4
+  for (int s = 0; s < shares; ++s) {
+    const int64_t r = (int64_t)s * rows + row;
+    const float4 v = *reinterpret_cast<const float4*>(ws_acc + r * D + lane * 4);
+    const float w = expf(ws_m[r] - m_use);
+    l += w * ws_l[r];
+    acc.x += w * v.x; acc.y += w * v.y; acc.z += w * v.z; acc.w += w * v.w;
+  }
+  const float inv = 1.f / ((l == 0.f) ? 1.f : l);
+  const int n = row % p.N_q, bh = row / p.N_q, h = bh % p.H_q, b = bh / p.H_q;
+  T* dst = reinterpret_cast<T*>(a.o) + (int64_t)b * a.o_stride[0] + (int64_t)h * a.o_stride[1] + (int64_t)n * a.o_stride[2];
+  *reinterpret_cast<uint2*>(dst + lane * 4) = make_uint2(Pack2<T>::run(acc.x * inv, acc.y * inv), Pack2<T>::run(acc.z * inv, acc.w * inv));
+}
+
+template <typename T>
+int launch_merge_shares(const AfFwdParams& a, const TcArgs& args, cudaStream_t st) {
+  const AfProblem& p = a.p;
+  const int64_t threads = (int64_t)p.B * p.H_q * p.N_q * (p.D / 4);
+  const unsigned blocks = (unsigned)((threads + 127) / 128);
+  merge_shares_kernel<T><<<blocks, 128, 0, st>>>(a, args.key_shares, args.ws_m, args.ws_l, args.ws_acc);
+  count_launch();
+  return check_cuda(cudaGetLastError(), "merge_shares launch");
+}
+}  // namespace
+
 // Multiprocessor count of the current device, looked up once per device.
 int tc_sm_count(int* sms) {
   static int cached[64] = {};
@@ -238,7 +279,7 @@ int tc_launch_prepass(const AfProblem& p, void* q_out, void* k_out, cudaStream_t
 // tile it visits: O(N_q/128 * group) rotations per key against one.
 static int64_t align256(int64_t x) { return (x + 255) & ~(int64_t)255; }
 
-int64_t fwd_tcgen05_workspace_bytes(const AfProblem& p) {
+static int64_t rope_workspace_bytes(const AfProblem& p) {
   if (!p.rope) return 0;
   const int64_t q_tiles_per_kv_head = (int64_t)((p.N_q + tc::BM - 1) / tc::BM) * (p.H_q / p.H_kv);
   if (q_tiles_per_kv_head < 4) return 0;   // short sequences: rotate in shared memory, one launch
@@ -300,13 +341,76 @@ static void set_item_order(tc::TcArgs& args, int units, int unit_chunk, int rows
 }
 
 // The two-heads-per-CTA schedule (fwd_pair_tcgen05.cuh): head dim 128, an even number of query
-// heads per KV head, element masks only, operands already rotated.  ATTNFUSE_FWD_PAIR=0 in the
-// environment (read at every call) keeps the one-head schedule, for comparisons between the two.
-static bool pair_schedule_applies(const AfProblem& p, int rope_mode) {
+// heads per KV head, element masks only, operands already rotated.  ATTNFUSE_FWD_PAIR in the
+// environment (read at every call) keeps to the one-head schedule (0) or to this one wherever it
+// exists (1), for comparisons between the two.
+static bool pair_schedule_exists(const AfProblem& p, int rope_mode) {
   if (p.D != 128 || rope_mode != tc::ROPE_NONE || p.mask_kind == AF_MASK_BLOCKS) return false;
-  if (p.H_kv < 1 || p.H_q % p.H_kv != 0 || ((p.H_q / p.H_kv) & 1) != 0) return false;
+  return p.H_kv >= 1 && p.H_q % p.H_kv == 0 && ((p.H_q / p.H_kv) & 1) == 0;
+}
+
+// How a forward problem is laid over the SMs: one or two heads per CTA, and the number of shares the
+// keys of a query tile are dealt out to.
+struct FwdPlan { bool pair; int shares; };
+
+// Longest chain of work on one SM, in key tiles of the one-head schedule (about 1800 cycles), for each layout, and the shortest wins.  An item costs its key tiles plus about
+// two tiles at its boundary; two heads per CTA do a tile of both in 1.95 tiles but halve the number of
+// items, which leaves SMs without work when there are few: 500 rows against 8011 keys, 32 heads,
+// are 64 pair items (0.121 ms) or 128 one-head items (0.074 ms) on 148 SMs.  Shares cost the partials' way
+// through memory and the merge launch, about six tiles.  They exist at head dim 128, for calls that keep no
+// log-sum-exp: an autograd forward holds its workspace until the backward.
+static FwdPlan plan_forward(const AfFwdParams& a, int rope_mode, int sms) {
+  const AfProblem& p = a.p;
+  FwdPlan best{false, 1};
+  const bool pair_ok = pair_schedule_exists(p, rope_mode);
   const char* e = std::getenv("ATTNFUSE_FWD_PAIR");
-  return !(e != nullptr && e[0] == '0');
+  if (pair_ok && e != nullptr && e[0] == '1') return FwdPlan{true, 1};
+  if (p.mask_kind == AF_MASK_BLOCKS || sms < 1) return best;
+  const int m_blocks = (p.N_q + tc::BM - 1) / tc::BM;
+  const int64_t items = (int64_t)m_blocks * p.B * p.H_q;
+  const bool shares_ok = p.D == 128 && rope_mode == tc::ROPE_NONE && a.lse == nullptr && items < 2 * (int64_t)sms;
+  if (!pair_ok && !shares_ok) return best;                 // nothing to choose from
+  int64_t sum = 0;
+  int longest = 0;
+  for (int m = 0; m < m_blocks; ++m) {
+    int first, n;
+    tc::tile_range(p, m, first, n);
+    sum += n;
+    longest = n > longest ? n : longest;
+  }
+  const double mean = (double)sum / m_blocks;
+  auto chain = [&](int64_t n_items, double tiles_per_item, double tiles_longest, double boundary) {
+    const double dealt = (double)((n_items + sms - 1) / sms) * (tiles_per_item + boundary);
+    return dealt > tiles_longest + boundary ? dealt : tiles_longest + boundary;
+  };
+  double best_cost = chain(items, mean, longest, 2.0);
+  if (pair_ok && !(e != nullptr && e[0] == '0')) {
+    const double c = chain(items / 2, 1.95 * mean, 1.95 * longest, 2.5);
+    if (c <= best_cost) { best_cost = c; best.pair = true; }
+  }
+  if (shares_ok) {
+    for (int s = 2; s <= 16 && longest >= 4 * s; ++s) {
+      const double c = chain(items * s, mean / s, (double)(longest + s - 1) / s, 2.0) + 6.0;
+      if (c < 0.95 * best_cost) { best_cost = c; best = FwdPlan{false, s}; }
+    }
+  }
+  return best;
+}
+
+// Workspace: the rotated Q and K, then the partials of a problem whose keys are dealt out to shares
+// (m and l, each padded to 256 bytes, and the accumulators).
+static int64_t share_workspace_bytes(const AfProblem& p, int shares) {
+  if (shares < 2) return 0;
+  const int64_t rows = (int64_t)shares * p.B * p.H_q * p.N_q;
+  return 2 * align256(rows * 4) + rows * p.D * 4;
+}
+
+int64_t fwd_tcgen05_workspace_bytes(const AfFwdParams& a) {
+  const int64_t rotated = rope_workspace_bytes(a.p);
+  const int mode = (a.p.rope && rotated == 0) ? tc::ROPE_FUSED : tc::ROPE_NONE;
+  int sms = 0;
+  if (a.p.N_q < 1 || tc_sm_count(&sms) != AF_OK) return rotated;
+  return rotated + share_workspace_bytes(a.p, plan_forward(a, mode, sms).shares);
 }
 
 int launch_fwd_tcgen05(const AfFwdParams& a, cudaStream_t st) {
@@ -328,13 +432,15 @@ int launch_fwd_tcgen05(const AfFwdParams& a, cudaStream_t st) {
     const double kv_bytes = 2.0 * 2.0 * (double)p.N_kv * p.D / group;   // K and V of a query head's share
     set_item_order(args, p.B * p.H_q, choose_unit_chunk(p.B * p.H_q, group, kv_bytes), args.num_m_blocks);
   }
+  int sms = 0;
+  { const int rc_sm = tc_sm_count(&sms); if (rc_sm != AF_OK) return rc_sm; }
+  auto set_grid = [&]() { args.grid_ctas = (sms > 0 && sms < args.total_items) ? sms : args.total_items; };
+  args.key_shares = 1;
   {
     // One CTA fits per SM (shared memory), so the kernel runs persistently: one CTA per SM walks
     // its share of the query tiles with the pipeline kept full across tile boundaries (measured
     // faster than one CTA per query tile at every size, 951 vs 851 TFLOP/s on causal 4x32x4096x128).
-    int sms = 0;
-    { const int rc_sm = tc_sm_count(&sms); if (rc_sm != AF_OK) return rc_sm; }
-    args.grid_ctas = (sms > 0 && sms < args.total_items) ? sms : args.total_items;
+    set_grid();
   }
 
   int mode = p.rope ? tc::ROPE_FUSED : tc::ROPE_NONE;
@@ -342,7 +448,7 @@ int launch_fwd_tcgen05(const AfFwdParams& a, cudaStream_t st) {
   const void* k_ptr = p.k;
   int64_t q_stride[4] = {p.q_stride[0], p.q_stride[1], p.q_stride[2], p.q_stride[3]};
   int64_t k_stride[4] = {p.k_stride[0], p.k_stride[1], p.k_stride[2], p.k_stride[3]};
-  const int64_t need = fwd_tcgen05_workspace_bytes(p);
+  const int64_t need = rope_workspace_bytes(p);
   if (p.rope && need > 0 && a.workspace != nullptr && a.workspace_bytes >= need &&
       ((uintptr_t)a.workspace & 255) == 0) {
     void* q_rot = a.workspace;
@@ -362,7 +468,16 @@ int launch_fwd_tcgen05(const AfFwdParams& a, cudaStream_t st) {
   if ((rc = make_map(&mv, p.dtype, p.v, p.B, p.H_kv, p.N_kv, p.D, p.v_stride)) != AF_OK) return rc;
   // output rows leave through a TMA store: one box = the 32 rows of a warp x half of the head dim
   if ((rc = make_map(&mo, p.dtype, a.o, p.B, p.H_q, p.N_q, p.D, a.o_stride, 32, p.D / 2)) != AF_OK) return rc;
-  if (pair_schedule_applies(p, mode)) {
+  FwdPlan plan = plan_forward(a, mode, sms);
+  if (plan.shares > 1) {
+    const int64_t rotated = p.rope && mode == tc::ROPE_NONE ? need : 0;
+    if (a.workspace == nullptr || ((uintptr_t)a.workspace & 255) != 0 ||
+        a.workspace_bytes < rotated + share_workspace_bytes(p, plan.shares))
+      plan.shares = 1;                                     // no room for partials: whole rows per item
+    else
+      args.ws_m = reinterpret_cast<float*>(static_cast<char*>(a.workspace) + rotated);
+  }
+  if (plan.pair) {
     // two query heads of a KV group per CTA: one K / V load feeds two S products
     const int pairs = p.H_q / 2;
     args.total_items = args.num_m_blocks * p.B * pairs;
@@ -373,17 +488,27 @@ int launch_fwd_tcgen05(const AfFwdParams& a, cudaStream_t st) {
       const double kv_bytes = 2.0 * 2.0 * (double)p.N_kv * p.D / group_pairs;
       set_item_order(args, p.B * pairs, choose_unit_chunk(p.B * pairs, group_pairs, kv_bytes), args.num_m_blocks);
     }
-    int sms = 0;
-    { const int rc_sm = tc_sm_count(&sms); if (rc_sm != AF_OK) return rc_sm; }
-    args.grid_ctas = (sms > 0 && sms < args.total_items) ? sms : args.total_items;
+    set_grid();
     return tc::launch_pair_d128(p.dtype, args, mq, mk, mv, mo, st);
   }
-  if (p.D == 64) {
-    if (mode == tc::ROPE_NONE) return tc::launch_d64_norope(p.dtype, args, mq, mk, mv, mo, st);
-    return tc::launch_d64_fused(p.dtype, args, mq, mk, mv, mo, st);
+  if (plan.shares > 1) {
+    const int64_t rows = (int64_t)plan.shares * p.B * p.H_q * p.N_q;
+    args.ws_l = args.ws_m + align256(rows * 4) / 4;
+    args.ws_acc = args.ws_l + align256(rows * 4) / 4;
+    args.key_shares = plan.shares;
+    args.div_shares = tc::FastDiv::make((uint32_t)plan.shares);
+    args.total_items *= plan.shares;                       // < 2 SMs worth of items before
+    set_item_order(args, p.B * p.H_q, args.unit_chunk, args.num_m_blocks * plan.shares);
+    set_grid();
   }
-  if (mode == tc::ROPE_NONE) return tc::launch_d128_norope(p.dtype, args, mq, mk, mv, mo, st);
-  return tc::launch_d128_fused(p.dtype, args, mq, mk, mv, mo, st);
+  if (p.D == 64)
+    rc = mode == tc::ROPE_NONE ? tc::launch_d64_norope(p.dtype, args, mq, mk, mv, mo, st)
+                               : tc::launch_d64_fused(p.dtype, args, mq, mk, mv, mo, st);
+  else
+    rc = mode == tc::ROPE_NONE ? tc::launch_d128_norope(p.dtype, args, mq, mk, mv, mo, st)
+                               : tc::launch_d128_fused(p.dtype, args, mq, mk, mv, mo, st);
+  if (rc != AF_OK || plan.shares == 1) return rc;
+  return p.dtype == AF_F16 ? launch_merge_shares<__half>(a, args, st) : launch_merge_shares<__nv_bfloat16>(a, args, st);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -427,6 +552,7 @@ int launch_decode_split_tc(const AfDecodeParams& a, cudaStream_t st) {
   args.num_m_blocks = 1;
   args.kv_tiles_per_block = args.q_tiles_per_block = 1;
   args.num_splits = a.num_splits;
+  args.key_shares = 1;
   args.kv_lens = a.kv_lens;
   args.ws_m = a.ws_m; args.ws_l = a.ws_l; args.ws_acc = a.ws_acc;
   AF_REQUIRE((int64_t)a.num_splits * a.B * a.H_kv <= 0x7fffffff, "too many items for one launch");

@@ -181,6 +181,10 @@ def launch_forward(Q, K, V, out, *, sm_scale, mask_kind, window=0, bias_kind=0, 
         if keep_workspace is not None:
             workspace = torch.empty(need, dtype=torch.uint8, device=Q.device)
             keep_workspace.append(workspace)
+        elif cos is None:
+            # partials of a problem whose keys are dealt out to several shares: the allocator's
+            # stream order (and a graph capture's own pool) covers their lifetime
+            workspace = torch.empty(need, dtype=torch.uint8, device=Q.device)
         else:
             workspace = _inference_workspace(Q.device, stream, need)
         params.workspace, params.workspace_bytes = workspace.data_ptr(), need

@@ -186,12 +186,13 @@ int launch_bwd_mma(const AfBwdParams& a, cudaStream_t st) {
   dkv.a = a;
   dkv.tiles = (p.N_kv + 127) / 128;
   dkv.stat_per_block = blocks ? p.block_n / 128 : 1;
-  dkv.steps_per_block = blocks ? p.block_m / 64 : 1;
+  const int strm_rows = p.D == 64 ? tcb::BCfg<64>::BT : tcb::BCfg<128>::BT;
+  dkv.steps_per_block = blocks ? p.block_m / strm_rows : 1;
   tcb::BwdArgs dq{};
   dq.a = a;
   dq.tiles = (p.N_q + 127) / 128;
   dq.stat_per_block = blocks ? p.block_m / 128 : 1;
-  dq.steps_per_block = blocks ? p.block_n / 64 : 1;
+  dq.steps_per_block = blocks ? p.block_n / strm_rows : 1;
   AF_REQUIRE((int64_t)dq.tiles * p.B * p.H_q <= 0x7fffffff, "too many tiles for one launch");
   // Persistent launches: one CTA per SM walks its share of the stationary tiles, so that the loads
   // and first products of the next tile overlap the epilogue of the previous one.
@@ -210,8 +211,9 @@ int launch_bwd_mma(const AfBwdParams& a, cudaStream_t st) {
   }
 
   if (p.D == 64) {
-    if ((rc = tcb::launch_dkv_d64(p.dtype, dkv, k128, v128, q64, do64, st)) != AF_OK) return rc;
-    return tcb::launch_dq_d64(p.dtype, dq, q128, do128, k64, v64, st);
+    // streamed tiles of 128 rows too
+    if ((rc = tcb::launch_dkv_d64(p.dtype, dkv, k128, v128, q128, do128, st)) != AF_OK) return rc;
+    return tcb::launch_dq_d64(p.dtype, dq, q128, do128, k128, v128, st);
   }
   if ((rc = tcb::launch_dkv_d128(p.dtype, dkv, k128, v128, q64, do64, st)) != AF_OK) return rc;
   return tcb::launch_dq_d128(p.dtype, dq, q128, do128, k64, v64, st);

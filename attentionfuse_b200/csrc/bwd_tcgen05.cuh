@@ -18,15 +18,15 @@
 // dS = P * (dP - delta), delta = rowsum(dO * O); dK and dQ are multiplied by the scale at the
 // end (codegen_backward.py:161-191).  With RoPE the operands are the pre-rotated Q', K' and the
 // epilogue applies the transpose of the rotation to dQ', dK' while they are still fp32.
-// S^T/dP^T (or S/dP) are double-buffered in TMEM so that the products of step i+1 run while the
-// 128 element-wise threads work on step i; the products and the accumulations are issued by two
+// S^T (or S) is double-buffered in TMEM so that the products of step i+1 run while the element-wise
+// threads work on step i; the products and the accumulations are issued by two
 // different threads.  All waits are bounded.
 //
 //   MODE_FUSED  (head_dim 128) the key-stationary pass also produces dQ, so that S and dP are
-//             computed once: 5 products per step instead of 7 over the two passes.  dS^T goes to
-//             shared memory (128 keys x 64 queries, query-contiguous, 128-byte swizzle) instead
-//             of TMEM and is read twice from there: as the K-major A operand of dK_j += dS^T Q_i
-//             and as the N-major B operand of  dQ_i^T = K_j^T dS^T  (A = the stationary K tile
+//             computed once: 5 products per step instead of 7 over the two passes.  dS^T goes
+//             both to TMEM, next to P^T in the step's S^T columns, as the A operand of
+//             dK_j += dS^T Q_i, and to shared memory (128 keys x 64 queries, query-contiguous,
+//             128-byte swizzle) as the N-major B operand of  dQ_i^T = K_j^T dS^T  (A = the stationary K tile
 //             read M-major).  dQ_i^T (TMEM lane = d, column = query) is not kept: the element-wise
 //             threads read it back and add it to an fp32 (B, H_q, N_q, D) accumulator in global
 //             memory with red.global.add.f32 (32 lanes = 32 consecutive d = one 128-byte line);
@@ -55,34 +55,69 @@ enum { EMASK_NONE = 0, EMASK_CAUSAL = 1, EMASK_WINDOW = 2, EMASK_BITS = 3 };   /
 // (EMASK_BITS: block lists in which some blocks carry a bit matrix of their active elements)
 
 constexpr int BS = 128;   // rows of the stationary operands (TMEM lanes)
-constexpr int BT = 64;    // rows of a streamed tile (columns of S per step)
 
 template <int D, int MODE = MODE_DKV> struct BCfg {
   static constexpr bool FUSED = MODE == MODE_FUSED;
   static constexpr int PANELS = D / 64;
   static constexpr int STAT_PANEL = BS * 128;               // bytes of a 128-row, 64-element panel
-  static constexpr int STRM_PANEL = BT * 128;
   static constexpr int STAT_TILE = PANELS * STAT_PANEL;
-  static constexpr int STRM_TILE = PANELS * STRM_PANEL;
+  // Rows of a streamed tile = columns of S per step.  What bounds a step is as much the two issuing
+  // threads as the tensor pipe: every barrier wait that is already over costs them 130 - 180 clocks, an
+  // MMA about 60, a commit 70 (timeline of a head dim 64 dQ step of 64 columns: 1030 clocks, all of it
+  // the first issuing thread's, for 512 clocks of products).  Head dim 64 takes 128 columns a step --
+  // N = 128 products also read the stationary operand half as often -- head dim 128 has no TMEM
+  // columns left for that.
+  static constexpr int BT = (D == 64) ? 128 : 64;
+  static constexpr int COLS = 64;                           // columns of a step per element-wise thread
+  static constexpr int SHARES = BT / COLS;                  // element-wise threads per stationary row
+  static constexpr int EW_THREADS = BS * SHARES;
+  static constexpr int DRAIN_THREADS = FUSED ? BS : 0;      // fused: threads that add dQ^T to its accumulator
+  static constexpr int THREADS = EW_THREADS + DRAIN_THREADS + 96;   // and the producer and two MMA issuers
   static constexpr int STAGES = FUSED ? 3 : 4;
-  static constexpr int STATS_BYTES = 2 * BT * 4;            // L*log2e and delta of a streamed tile
+  static constexpr int STRM_PANEL = BT * 128;
+  static constexpr int STRM_TILE = PANELS * STRM_PANEL;
+  // Key-stationary modes: -L / scale and -delta of the streamed query rows enter S^T and dP^T as one more
+  // 16-wide product step, ones(128 x 16) * stats(64 x 16)^T, each value as three bf16 terms (24 bits,
+  // fp32's range; the operands of that one product are bf16 whatever T is).  As shared-memory loads
+  // of the element-wise threads -- every lane needs both numbers of every column -- they took 64 KB
+  // of the 304 KB a fused step moves through the shared-memory port, which bounds it; the product
+  // steps read 12 KB.  A tile of 64 rows x 128 bytes holds the steps of two ring stages: 32 bytes
+  // of L terms and 32 bytes of delta terms each.
+  static constexpr bool KEY_STAT = MODE != MODE_DQ;
+  static constexpr int ONES_BYTES = KEY_STAT ? BS * 128 : 0;
+  static constexpr int STATS_TILE = BT * 128;
+  static constexpr int STATS_BYTES = KEY_STAT ? (STAGES + 1) / 2 * STATS_TILE : 0;
   static constexpr int DS_TILE = BS * BT * 2;               // dS^T of one step (fused mode): 128 keys x 64 queries
   static constexpr int DS_BYTES = FUSED ? 2 * DS_TILE : 0;  // two buffers, right after the stationary tiles
-  static constexpr int SMEM_BYTES = 2 * STAT_TILE + DS_BYTES + STAGES * (2 * STRM_TILE + STATS_BYTES) + 1024 + 512;
+  static constexpr int ONES_OFF = 2 * STAT_TILE + DS_BYTES, STATS_OFF = ONES_OFF + ONES_BYTES;
+  static constexpr int STAGE0_OFF = STATS_OFF + STATS_BYTES, STAGE_BYTES = 2 * STRM_TILE;
+  static constexpr int SMEM_BYTES = STAGE0_OFF + STAGES * STAGE_BYTES + 1024 + 512;
+  static_assert(SMEM_BYTES <= 232448, "shared memory of one CTA");
   static constexpr int TMEM_COLS = 512;
-  // two-pass: X0 Y0 X1 Y1; fused: X0 X1 Y Z (Y = dP^T, single; Z = dQ^T, single)
-  static constexpr int COL_X0 = 0, COL_Y0 = FUSED ? 128 : 64, COL_X1 = FUSED ? 64 : 128, COL_Y1 = FUSED ? 128 : 192;
-  static constexpr int COL_Z = 192, COL_ACC1 = 256, COL_ACC2 = 256 + D;
-  // MODE_DQ has one accumulator only: dS gets columns of its own (two buffers of 32), so the next
-  // S / dP product does not have to wait until dQ += dS K has consumed the previous dS.
-  static constexpr int COL_DS0 = 384, COL_DS1 = 416;
+  // X = S, Y = dP of a step, BT columns each; P and dS as half-precision A operands take half the columns.
+  // fused:            X0 X1 Y Z (Z = dQ^T): P^T and dS^T of a step share its X columns; Y and Z are single,
+  //                   free again as soon as the threads that want them have loaded them.
+  // head dim 64:      X0 X1 Y: the same, a share's P and dS over the share's own 64 columns of X.
+  // head dim 128:     X0 Y0 X1 Y1: P^T over X, dS^T over Y; MODE_DQ has one accumulator only, dS gets
+  //                   columns of its own there (two buffers of 32), so that the next S / dP product does
+  //                   not have to wait until dQ += dS K has consumed the previous dS.
+  static constexpr bool DS_IN_X = FUSED || D == 64;
+  static constexpr bool Y_SINGLE = FUSED || D == 64;
+  __host__ __device__ static constexpr int col_x(int t) { return DS_IN_X ? t * BT : t * 128; }
+  __host__ __device__ static constexpr int col_y(int t) { return FUSED ? 128 : D == 64 ? 256 : 64 + t * 128; }
+  static constexpr int COL_Z = 192, COL_ACC1 = (D == 64) ? 384 : 256, COL_ACC2 = COL_ACC1 + D;
+  // k-step kk (16 columns of the step) of the A operands
+  __host__ __device__ static constexpr int col_p(int t, int kk) { return col_x(t) + (kk >> 2) * COLS + (kk & 3) * 8; }
+  __host__ __device__ static constexpr int col_ds(int t, int kk) {
+    return DS_IN_X ? col_p(t, kk) + (MODE == MODE_DQ ? 0 : 32) : MODE == MODE_DQ ? 384 + t * 32 + kk * 8 : col_y(t) + kk * 8;
+  }
 };
 
 struct BBarriers {
   uint64_t stat_full, stat_empty, acc_free;
   uint64_t strm_full[4], strm_empty[4];
   uint64_t xy_full[2], p_full[2], acc_done[2];
-  uint64_t y_free, z_free;                      // fused mode: dP^T loaded / dQ^T loaded by the element-wise threads
+  uint64_t y_free, z_free;                      // single dP / dQ^T columns: loaded by the threads that want them
   uint64_t sched_full[4], sched_empty[4];       // fused mode: ring of dynamically fetched item numbers
   int32_t sched_item[4];
   uint32_t tmem_base;
@@ -92,7 +127,7 @@ struct BBarriers {
 struct BwdArgs {
   AfBwdParams a;
   int tiles;            // stationary tiles along the sequence
-  int steps_per_block;  // block lists: streamed 64-row steps per listed block
+  int steps_per_block;  // block lists: streamed steps (BCfg::BT rows) per listed block
   int stat_per_block;   // block lists: stationary 128-row tiles per block
   int total_items;      // tiles * B * heads: stationary tiles to process
   int grid_ctas;        // one persistent CTA per SM (or one per item when there are fewer)
@@ -103,6 +138,7 @@ struct BwdArgs {
 };
 
 // The streamed steps one stationary tile visits for one head.
+template <int BT>
 struct StepWalk {
   int cnt, first;
   const int32_t* list;
@@ -114,9 +150,9 @@ struct StepWalk {
   }
 };
 
-template <int MODE>
-__device__ __forceinline__ StepWalk make_steps(const AfProblem& p, const BwdArgs& args, int tile, int h) {
-  StepWalk w;
+template <int MODE, int BT>
+__device__ __forceinline__ StepWalk<BT> make_steps(const AfProblem& p, const BwdArgs& args, int tile, int h) {
+  StepWalk<BT> w;
   w.list = nullptr; w.slots = nullptr; w.per = 1; w.block = BT; w.first = 0;
   const int t0 = tile * BS;
   if (p.mask_kind == AF_MASK_BLOCKS) {
@@ -158,7 +194,7 @@ struct BItem {
   int tile, b, hx, h_kv, t0, total_steps;
 };
 
-template <int MODE, int EMASK>
+template <int MODE, int EMASK, int BT>
 __device__ __forceinline__ void decode_bitem(const AfProblem& p, const BwdArgs& args, int w, BItem& bi) {
   const int grp = p.H_q / p.H_kv;
   const int heads = (MODE != MODE_DQ) ? p.H_kv : p.H_q;
@@ -186,14 +222,14 @@ __device__ __forceinline__ void decode_bitem(const AfProblem& p, const BwdArgs& 
   const int heads_per_item = (MODE != MODE_DQ) ? grp : 1;
   bi.total_steps = 0;                                    // all heads of the group in DKV mode
   for (int g = 0; g < heads_per_item; ++g)
-    bi.total_steps += make_steps<MODE>(p, args, bi.tile, (MODE != MODE_DQ) ? bi.h_kv * grp + g : bi.hx).cnt;
+    bi.total_steps += make_steps<MODE, BT>(p, args, bi.tile, (MODE != MODE_DQ) ? bi.h_kv * grp + g : bi.hx).cnt;
 }
 
 // Item number k of this CTA.  Two-pass modes: static zig-zag.  Fused mode: the producer warp draws
 // the numbers from a global counter and publishes them through a 4-deep ring; every other role
-// (two issuing threads, 128 element-wise threads) reads slot k % 4 and releases it.
+// (two issuing threads, the element-wise and dQ-adding threads) reads slot k % 4 and releases it.
 // Returns 1 (item), 0 (no more items) or -1 (aborted wait).
-template <int MODE, int EMASK, bool IS_PRODUCER>
+template <int MODE, int EMASK, int BT, bool IS_PRODUCER>
 __device__ __forceinline__ int next_bitem(const AfProblem& p, const BwdArgs& args, BBarriers* bars, int k, int lane,
                                           volatile int* abort_flag, BItem& bi) {
   int w;
@@ -224,12 +260,12 @@ __device__ __forceinline__ int next_bitem(const AfProblem& p, const BwdArgs& arg
     if (w64 >= args.total_items) return 0;
     w = (int)w64;
   }
-  decode_bitem<MODE, EMASK>(p, args, w, bi);
+  decode_bitem<MODE, EMASK, BT>(p, args, w, bi);
   return 1;
 }
 
 template <typename T, int D, int MODE, int EMASK, bool ALIBI, bool ROPE>
-__global__ void __launch_bounds__(224, 1)
+__global__ void __launch_bounds__(BCfg<D, MODE>::THREADS, 1)
 bwd_tcgen05_kernel(const BwdArgs args, const __grid_constant__ CUtensorMap map_a1,
                    const __grid_constant__ CUtensorMap map_a2, const __grid_constant__ CUtensorMap map_b1,
                    const __grid_constant__ CUtensorMap map_b2) {
@@ -237,13 +273,14 @@ bwd_tcgen05_kernel(const BwdArgs args, const __grid_constant__ CUtensorMap map_a
   constexpr bool FUSED = MODE == MODE_FUSED;
   constexpr bool KVS = MODE != MODE_DQ;          // key-stationary: MODE_DKV and MODE_FUSED
   static_assert(!FUSED || D == 128, "the fused pass computes dQ^T with M = head_dim = 128");
-  constexpr int STAGES = C::STAGES;
+  constexpr int STAGES = C::STAGES, BT = C::BT, COLS = C::COLS, SHARES = C::SHARES;
+  constexpr int WARP_LOAD = (C::EW_THREADS + C::DRAIN_THREADS) / 32, WARP_MMA1 = WARP_LOAD + 1, WARP_MMA2 = WARP_LOAD + 2;
   constexpr int AB_FMT = (Elem<T>::code == AF_BF16) ? 1 : 0;
   constexpr uint32_t IDESC_XY = umma_idesc_f16(AB_FMT, BS, BT, 0, 0);
   constexpr uint32_t IDESC_ACC = umma_idesc_f16(AB_FMT, BS, D, 0, 1);
   constexpr uint32_t IDESC_DQT = umma_idesc_f16(AB_FMT, D, BT, 1, 1);   // dQ^T = K^T dS^T: A M-major, B N-major
-  constexpr int STAGE_BYTES = 2 * C::STRM_TILE + C::STATS_BYTES;
-  constexpr int STAGE0_OFF = 2 * C::STAT_TILE + C::DS_BYTES;
+  constexpr int STAGE_BYTES = C::STAGE_BYTES, STAGE0_OFF = C::STAGE0_OFF;
+  constexpr uint32_t IDESC_STATS = umma_idesc_f16(1, BS, BT, 0, 0);      // bf16 terms, whatever T is
 
   const AfBwdParams& a = args.a;
   const AfProblem& p = a.p;
@@ -264,24 +301,33 @@ bwd_tcgen05_kernel(const BwdArgs args, const __grid_constant__ CUtensorMap map_a
   if (tid == 0) {
     mbar_init(&bars->stat_full, 1);
     mbar_init(&bars->stat_empty, FUSED ? 2 : 1);   // fused: both issuing threads read the stationary K tile
-    mbar_init(&bars->acc_free, 128);
-    mbar_init(&bars->y_free, 128);
+    mbar_init(&bars->acc_free, C::EW_THREADS);
+    mbar_init(&bars->y_free, C::EW_THREADS);
     mbar_init(&bars->z_free, 128);
     for (int s = 0; s < 4; ++s) {
       mbar_init(&bars->strm_full[s], 1);
       mbar_init(&bars->strm_empty[s], 1);
       mbar_init(&bars->sched_full[s], 1);
-      mbar_init(&bars->sched_empty[s], 130);       // two issuing threads + 128 element-wise threads
+      mbar_init(&bars->sched_empty[s], 2 + C::EW_THREADS + C::DRAIN_THREADS);   // every role but the producer
     }
     for (int t = 0; t < 2; ++t) {
       mbar_init(&bars->xy_full[t], 1);
-      mbar_init(&bars->p_full[t], 128);
+      mbar_init(&bars->p_full[t], C::EW_THREADS);
       mbar_init(&bars->acc_done[t], 1);
     }
     bars->abort_flag = 0;
     mbar_fence_init();
   }
-  if (warp == 4) {
+  if (KVS) {
+    // the ones (bf16 1.0 in the first three of 16 columns), and zeros behind the terms of the statistics
+    for (int i = tid; i < (C::ONES_BYTES + C::STATS_BYTES) / 16; i += C::THREADS) {
+      const int r = (i >> 3) & 7, c = (i & 7) ^ r;       // row within its 8-row group, logical 16-byte chunk
+      const bool ones = i < C::ONES_BYTES / 16 && c == 0;
+      tc::sts128(smem_base + C::ONES_OFF + i * 16, ones ? make_uint4(0x3f803f80u, 0x00003f80u, 0u, 0u) : make_uint4(0u, 0u, 0u, 0u));
+    }
+    fence_proxy_async_smem();
+  }
+  if (warp == WARP_LOAD) {
     tmem_alloc(&bars->tmem_base, C::TMEM_COLS);
     tmem_relinquish();
   }
@@ -295,7 +341,7 @@ bwd_tcgen05_kernel(const BwdArgs args, const __grid_constant__ CUtensorMap map_a
   // loads and the first products of the next item overlap the previous item's epilogue; `qi`
   // counts the items with at least one step (phases of the stationary-tile and accumulator
   // hand-overs).
-  if (warp == 4) {
+  if (warp == WARP_LOAD) {
     // ============================== producer (TMA + per-step statistics) ==============================
     if (lane == 0) {
       tma_prefetch_desc(&map_a1); tma_prefetch_desc(&map_a2); tma_prefetch_desc(&map_b1); tma_prefetch_desc(&map_b2);
@@ -303,10 +349,11 @@ bwd_tcgen05_kernel(const BwdArgs args, const __grid_constant__ CUtensorMap map_a
     // L2 hints: the stationary tiles are read once per item, the streamed rows once per stationary
     // tile of their unit
     const uint64_t pol_once = l2_policy_evict_first(), pol_keep = l2_policy_evict_last();
+    const float inv_scale = 1.f / p.sm_scale;
     BItem bi;
     int it0 = 0, qi = 0;
     bool ok = true;
-    for (int k = 0; ok && next_bitem<MODE, EMASK, true>(p, args, bars, k, lane, abort_flag, bi) > 0; ++k) {
+    for (int k = 0; ok && next_bitem<MODE, EMASK, BT, true>(p, args, bars, k, lane, abort_flag, bi) > 0; ++k) {
       if (bi.total_steps == 0) continue;
       const int tile = bi.tile, b = bi.b, hx = bi.hx, h_kv = bi.h_kv, t0 = bi.t0;
       // the stationary tiles are free once the last product of the previous item that reads them has run
@@ -321,50 +368,85 @@ bwd_tcgen05_kernel(const BwdArgs args, const __grid_constant__ CUtensorMap map_a
         }
       }
       int it = it0;                                                   // running step count
-      for (int g = 0; g < n_heads && ok; ++g) {
-        const int h = KVS ? h_kv * group + g : hx;
-        const int hb = KVS ? h : h_kv;                                // head of the streamed tensors
-        const StepWalk w = make_steps<MODE>(p, args, tile, h);
-        for (int s = 0; s < w.cnt; ++s, ++it) {
-          const int st = it % STAGES;
-          if (it >= STAGES && !mbar_wait(&bars->strm_empty[st], ((it / STAGES) & 1) ^ 1, abort_flag)) { ok = false; break; }
-          const int r0 = w.row0(s);
-          unsigned char* stage = smem + STAGE0_OFF + st * STAGE_BYTES;
-          // The TMA loads go out first; the statistics of the streamed rows (two global loads per
-          // lane) are fetched while they fly, and the warp's arrival completes the stage.
-          if (lane == 0) {
-            mbar_expect_tx(&bars->strm_full[st], 2 * C::STRM_TILE);
-#pragma unroll
-            for (int pn = 0; pn < C::PANELS; ++pn) {
-              tma_load_4d_hint(stage + pn * C::STRM_PANEL, &map_b1, &bars->strm_full[st], pn * 64, r0, hb, b, pol_keep);
-              tma_load_4d_hint(stage + C::STRM_TILE + pn * C::STRM_PANEL, &map_b2, &bars->strm_full[st], pn * 64, r0, hb, b, pol_keep);
-            }
+      // The statistics of a step are fetched one step ahead, into the other of two register sets: two
+      // dependent trips to memory per step otherwise set the pace of the ring (a head dim 64 step of
+      // 128 columns took 3000 - 4000 clocks, 2500 of them the product thread's wait for this warp).
+      struct Stats { float l[BT / 32], d[BT / 32]; } st_a, st_b;
+      int g = -1, s = -1, h = 0, r0 = 0;
+      StepWalk<BT> w;
+      w.cnt = 0;
+      auto advance = [&](Stats& x) -> bool {           // next step of the item, and its statistics on their way
+        if (++s >= w.cnt) {
+          for (;;) {
+            if (++g >= n_heads) return false;
+            w = make_steps<MODE, BT>(p, args, tile, KVS ? h_kv * group + g : hx);
+            if (w.cnt > 0) break;
           }
-          if (KVS) {
-            // L*log2e and delta of the 64 streamed query rows; rows past N_q get (+inf, 0) so that
-            // their probabilities are exactly zero.
-            float* stats = reinterpret_cast<float*>(stage + 2 * C::STRM_TILE);
-#pragma unroll
-            for (int k2 = 0; k2 < 2; ++k2) {
-              const int q = r0 + lane + 32 * k2;
-              float l2 = INFINITY, dl = 0.f;
-              if (q < p.N_q) {
-                const float l = a.lse[(int64_t)b * a.lse_stride[0] + (int64_t)h * a.lse_stride[1] + (int64_t)q * a.lse_stride[2]];
-                l2 = (l == -INFINITY) ? INFINITY : l * kLog2e;
-                dl = a.delta[((int64_t)b * p.H_q + h) * p.N_q + q];
-              }
-              stats[lane + 32 * k2] = l2;
-              stats[BT + lane + 32 * k2] = dl;
-            }
-            __syncwarp();
-          }
-          if (lane == 0) mbar_arrive(&bars->strm_full[st]);
+          s = 0;
+          h = KVS ? h_kv * group + g : hx;
         }
+        r0 = w.row0(s);
+        if (KVS) {
+#pragma unroll
+          for (int k2 = 0; k2 < BT / 32; ++k2) {
+            const int q = r0 + lane + 32 * k2;
+            x.l[k2] = -INFINITY; x.d[k2] = 0.f;        // rows past N_q: their probabilities are exactly zero
+            if (q < p.N_q) {
+              x.l[k2] = __ldg(a.lse + (int64_t)b * a.lse_stride[0] + (int64_t)h * a.lse_stride[1] + (int64_t)q * a.lse_stride[2]);
+              x.d[k2] = __ldg(a.delta + ((int64_t)b * p.H_q + h) * p.N_q + q);
+            }
+          }
+        }
+        return true;
+      };
+      // One step: TMA loads of the tiles, the next step's statistics under way, this step's as operand
+      // terms.  Returns whether another step follows.
+      auto load_step = [&](const Stats& cur, Stats& nxt) -> bool {
+        const int st = it % STAGES;
+        const int hb = KVS ? h : h_kv;                                // head of the streamed tensors
+        if (it >= STAGES && !mbar_wait(&bars->strm_empty[st], ((it / STAGES) & 1) ^ 1, abort_flag)) { ok = false; return false; }
+        unsigned char* stage = smem + STAGE0_OFF + st * STAGE_BYTES;
+        if (lane == 0) {
+          mbar_expect_tx(&bars->strm_full[st], 2 * C::STRM_TILE);
+#pragma unroll
+          for (int pn = 0; pn < C::PANELS; ++pn) {
+            tma_load_4d_hint(stage + pn * C::STRM_PANEL, &map_b1, &bars->strm_full[st], pn * 64, r0, hb, b, pol_keep);
+            tma_load_4d_hint(stage + C::STRM_TILE + pn * C::STRM_PANEL, &map_b2, &bars->strm_full[st], pn * 64, r0, hb, b, pol_keep);
+          }
+        }
+        ++it;
+        const bool more = advance(nxt);
+        if (KVS) {
+          // -L / scale and -delta of the streamed query rows, (-inf, 0) where a row sees no key
+          const uint32_t stats_tile = smem_base + C::STATS_OFF + (st >> 1) * C::STATS_TILE;
+          const int chunk = (st & 1) * 4;            // L terms; the delta terms are two chunks further
+          // v as the sum of three bf16 numbers (-inf: the first one alone)
+          auto terms = [](float v) {
+            const float hi = __bfloat162float(__float2bfloat16_rn(v));
+            const float r1 = hi == v ? 0.f : v - hi;
+            const float mid = __bfloat162float(__float2bfloat16_rn(r1));
+            return make_uint4(Pack2<__nv_bfloat16>::run(hi, mid), Pack2<__nv_bfloat16>::run(r1 - mid, 0.f), 0u, 0u);
+          };
+#pragma unroll
+          for (int k2 = 0; k2 < BT / 32; ++k2) {
+            const int row = lane + 32 * k2;
+            tc::sts128(stats_tile + row * 128 + ((chunk ^ (row & 7)) << 4),
+                       terms(cur.l[k2] == -INFINITY ? -INFINITY : -cur.l[k2] * inv_scale));
+            tc::sts128(stats_tile + row * 128 + (((chunk + 2) ^ (row & 7)) << 4), terms(-cur.d[k2]));
+          }
+          fence_proxy_async_smem();
+          __syncwarp();
+        }
+        if (lane == 0) mbar_arrive(&bars->strm_full[st]);
+        return more;
+      };
+      if (advance(st_a)) {
+        while (load_step(st_a, st_b) && load_step(st_b, st_a)) {}
       }
       it0 += bi.total_steps;
       ++qi;
     }
-  } else if (warp == 5) {
+  } else if (warp == WARP_MMA1) {
     // ============================== MMA issuer 1: S / dP products ==============================
     // Two issuing threads feed the tensor pipe: a tcgen05.mma issue blocks while the pipe's short
     // queue is full, so one thread issuing both kinds leaves the pipe idle during its own barrier
@@ -372,39 +454,44 @@ bwd_tcgen05_kernel(const BwdArgs args, const __grid_constant__ CUtensorMap map_a
     if (lane == 0) {
       const uint64_t desc_a1 = umma_desc_sw128(sA1, 16, 1024), desc_a2 = umma_desc_sw128(sA2, 16, 1024);
       const uint64_t desc_b1k = umma_desc_sw128(sStage0, 16, 1024);              // streamed tile, K-major
+      const uint64_t desc_ones = umma_desc_sw128(smem_base + C::ONES_OFF, 16, 1024);
+      const uint64_t desc_stats = umma_desc_sw128(smem_base + C::STATS_OFF, 16, 1024);
       BItem bi;
       int it0 = 0, qi = 0;
       bool ok = true;
-      for (int k = 0; ok && next_bitem<MODE, EMASK, false>(p, args, bars, k, lane, abort_flag, bi) > 0; ++k) {
+      for (int k = 0; ok && next_bitem<MODE, EMASK, BT, false>(p, args, bars, k, lane, abort_flag, bi) > 0; ++k) {
       if (bi.total_steps == 0) continue;
       ok = mbar_wait(&bars->stat_full, qi & 1, abort_flag);
       for (int it = it0; ok && it < it0 + bi.total_steps; ++it) {     // `it`: running step count
         const int st = it % STAGES, t = it & 1;
         if (!mbar_wait(&bars->strm_full[st], (it / STAGES) & 1, abort_flag)) { ok = false; break; }
-        // X/Y[t] were last used by step it-2.  Key-stationary modes: P^T (and dS^T) overwrite X/Y,
-        // so the accumulate MMAs of that step must have run.  MODE_DQ: the element-wise group must
-        // have read them (its arrival on p_full).
+        // The step's X columns were last used by step it-2.  Where P and dS overwrite them (or Y), the
+        // accumulate MMAs of that step must have run; otherwise the element-wise group must have read
+        // them (its arrival on p_full).
         if (it >= 2) {
-          uint64_t* free_bar = KVS ? &bars->acc_done[t] : &bars->p_full[t];
+          uint64_t* free_bar = (KVS || C::DS_IN_X) ? &bars->acc_done[t] : &bars->p_full[t];
           if (!mbar_wait(free_bar, ((it >> 1) - 1) & 1, abort_flag)) { ok = false; break; }
         }
         tc_fence_after_sync();
         // Descriptors are built once; k-steps and ring stages only move the start-address field.
         const uint64_t b1 = desc_b1k + (uint64_t)((st * STAGE_BYTES) >> 4), b2 = b1 + (uint64_t)(C::STRM_TILE >> 4);
-        const uint32_t xt = tmem + (t ? C::COL_X1 : C::COL_X0), yt = tmem + (t ? C::COL_Y1 : C::COL_Y0);
+        const uint32_t xt = tmem + C::col_x(t), yt = tmem + C::col_y(t);
+        const uint64_t bs = desc_stats + (uint64_t)(((st >> 1) * C::STATS_TILE + (st & 1) * 64) >> 4);   // L terms; delta: 32 bytes on
+        if (KVS) umma_ss(xt, desc_ones, bs, IDESC_STATS, 0u);
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk)
           umma_ss(xt, desc_a1 + (uint64_t)(((kk >> 2) * C::STAT_PANEL + (kk & 3) * 32) >> 4),
-                  b1 + (uint64_t)(((kk >> 2) * C::STRM_PANEL + (kk & 3) * 32) >> 4), IDESC_XY, kk > 0 ? 1u : 0u);
-        if (FUSED && it >= 1) {
-          // the single dP^T buffer: the element-wise threads have loaded the previous step's values
+                  b1 + (uint64_t)(((kk >> 2) * C::STRM_PANEL + (kk & 3) * 32) >> 4), IDESC_XY, (KVS || kk > 0) ? 1u : 0u);
+        if (C::Y_SINGLE && it >= 1) {
+          // the single dP buffer: the element-wise threads have loaded the previous step's values
           if (!mbar_wait(&bars->y_free, (it - 1) & 1, abort_flag)) { ok = false; break; }
           tc_fence_after_sync();
         }
+        if (KVS) umma_ss(yt, desc_ones, bs + 2, IDESC_STATS, 0u);
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk)
           umma_ss(yt, desc_a2 + (uint64_t)(((kk >> 2) * C::STAT_PANEL + (kk & 3) * 32) >> 4),
-                  b2 + (uint64_t)(((kk >> 2) * C::STRM_PANEL + (kk & 3) * 32) >> 4), IDESC_XY, kk > 0 ? 1u : 0u);
+                  b2 + (uint64_t)(((kk >> 2) * C::STRM_PANEL + (kk & 3) * 32) >> 4), IDESC_XY, (KVS || kk > 0) ? 1u : 0u);
         umma_commit(&bars->xy_full[t]);
       }
       if (ok) umma_commit(&bars->stat_empty);   // the item's last products: the stationary tiles may be refilled
@@ -412,43 +499,42 @@ bwd_tcgen05_kernel(const BwdArgs args, const __grid_constant__ CUtensorMap map_a
       ++qi;
       }
     }
-  } else if (warp == 6) {
+  } else if (warp == WARP_MMA2) {
     // ============================== MMA issuer 2: gradient accumulation ==============================
     if (lane == 0) {
       const uint64_t desc_b1n = umma_desc_sw128(sStage0, C::STRM_PANEL, 1024);   // streamed tile, N-major
-      // fused mode: dS^T (128 keys x 64 queries, query-contiguous) as K-major A and as N-major B;
+      // fused mode: dS^T (128 keys x 64 queries, query-contiguous) as N-major B;
       // the stationary K tile (128 keys x D) as M-major A (M = d: 64-element panels LBO apart)
-      const uint64_t desc_ds_k = umma_desc_sw128(sDS0, 16, 1024);
       const uint64_t desc_ds_n = umma_desc_sw128(sDS0, C::DS_TILE, 1024);
       const uint64_t desc_k_m = umma_desc_sw128(sA1, C::STAT_PANEL, 1024);
       BItem bi;
       int it0 = 0, qi = 0;
       bool ok = true;
-      for (int k = 0; ok && next_bitem<MODE, EMASK, false>(p, args, bars, k, lane, abort_flag, bi) > 0; ++k) {
+      for (int k = 0; ok && next_bitem<MODE, EMASK, BT, false>(p, args, bars, k, lane, abort_flag, bi) > 0; ++k) {
       if (bi.total_steps == 0) continue;
       for (int it = it0; it < it0 + bi.total_steps; ++it) {            // `it`: running step count
         const int st = it % STAGES, t = it & 1;
         const bool first = it == it0;                                  // overwrites the accumulators
-        if (!mbar_wait(&bars->strm_full[st], (it / STAGES) & 1, abort_flag)) { ok = false; break; }
+        // P and dS come from products that had waited for the step's tiles (strm_full): no second wait
         if (!mbar_wait(&bars->p_full[t], (it >> 1) & 1, abort_flag)) { ok = false; break; }
         // the previous item's epilogue must have read the accumulators out
         if (first && qi > 0 && !mbar_wait(&bars->acc_free, (qi - 1) & 1, abort_flag)) { ok = false; break; }
         tc_fence_after_sync();
         const uint64_t b1 = desc_b1n + (uint64_t)((st * STAGE_BYTES) >> 4), b2 = b1 + (uint64_t)(C::STRM_TILE >> 4);
-        const uint32_t xt = tmem + (t ? C::COL_X1 : C::COL_X0), yt = tmem + (t ? C::COL_Y1 : C::COL_Y0);
         // streamed tiles as N-major B operands: 16 rows per k-step (2048 B), panels LBO apart
-        if (FUSED) {
-          const uint64_t ds_k = desc_ds_k + (uint64_t)((t * C::DS_TILE) >> 4);
-          const uint64_t ds_n = desc_ds_n + (uint64_t)((t * C::DS_TILE) >> 4);
+        if (KVS) {
 #pragma unroll
           for (int kk = 0; kk < BT / 16; ++kk)      // dV += P^T dO
-            umma_ts(tmem + C::COL_ACC1, xt + kk * 8, b2 + (uint64_t)((kk * 2048) >> 4), IDESC_ACC,
+            umma_ts(tmem + C::COL_ACC1, tmem + C::col_p(t, kk), b2 + (uint64_t)((kk * 2048) >> 4), IDESC_ACC,
                     (!first || kk > 0) ? 1u : 0u);
+        }
 #pragma unroll
-          for (int kk = 0; kk < BT / 16; ++kk)      // dK += dS^T Q, dS^T from shared memory
-            umma_ss(tmem + C::COL_ACC2, ds_k + (uint64_t)((kk * 32) >> 4), b1 + (uint64_t)((kk * 2048) >> 4), IDESC_ACC,
-                    (!first || kk > 0) ? 1u : 0u);
-          // the single dQ^T buffer: the element-wise threads have loaded the previous step's tile
+        for (int kk = 0; kk < BT / 16; ++kk)        // dK += dS^T Q, or dQ += dS K
+          umma_ts(tmem + (KVS ? C::COL_ACC2 : C::COL_ACC1), tmem + C::col_ds(t, kk), b1 + (uint64_t)((kk * 2048) >> 4),
+                  IDESC_ACC, (!first || kk > 0) ? 1u : 0u);
+        if (FUSED) {
+          const uint64_t ds_n = desc_ds_n + (uint64_t)((t * C::DS_TILE) >> 4);
+          // the single dQ^T buffer: the previous step's tile has been loaded
           if (it >= 1) {
             if (!mbar_wait(&bars->z_free, (it - 1) & 1, abort_flag)) { ok = false; break; }
             tc_fence_after_sync();
@@ -457,104 +543,106 @@ bwd_tcgen05_kernel(const BwdArgs args, const __grid_constant__ CUtensorMap map_a
           for (int kk = 0; kk < BS / 16; ++kk)      // dQ^T = K^T dS^T over the 128 keys
             umma_ss(tmem + C::COL_Z, desc_k_m + (uint64_t)((kk * 2048) >> 4), ds_n + (uint64_t)((kk * 2048) >> 4),
                     IDESC_DQT, kk > 0 ? 1u : 0u);
-        } else if (MODE == MODE_DKV) {
-#pragma unroll
-          for (int kk = 0; kk < BT / 16; ++kk)      // dV += P^T dO
-            umma_ts(tmem + C::COL_ACC1, xt + kk * 8, b2 + (uint64_t)((kk * 2048) >> 4), IDESC_ACC,
-                    (!first || kk > 0) ? 1u : 0u);
-#pragma unroll
-          for (int kk = 0; kk < BT / 16; ++kk)      // dK += dS^T Q
-            umma_ts(tmem + C::COL_ACC2, yt + kk * 8, b1 + (uint64_t)((kk * 2048) >> 4), IDESC_ACC,
-                    (!first || kk > 0) ? 1u : 0u);
-        } else {
-          const uint32_t dst = tmem + (t ? C::COL_DS1 : C::COL_DS0);
-#pragma unroll
-          for (int kk = 0; kk < BT / 16; ++kk)      // dQ += dS K
-            umma_ts(tmem + C::COL_ACC1, dst + kk * 8, b1 + (uint64_t)((kk * 2048) >> 4), IDESC_ACC,
-                    (!first || kk > 0) ? 1u : 0u);
         }
-        umma_commit(&bars->strm_empty[st]);
         umma_commit(&bars->acc_done[t]);
+        umma_commit(&bars->strm_empty[st]);
       }
       if (FUSED && ok) umma_commit(&bars->stat_empty);   // dQ^T reads the stationary K tile too
       it0 += bi.total_steps;
       ++qi;
       }
     }
-  } else if (warp < 4) {
+  } else if (FUSED && warp >= C::EW_THREADS / 32) {
+    // ============================== dQ: TMEM -> fp32 accumulator ==============================
+    // 128 threads of their own: a step's 64 reductions per thread take about 1400 clocks of waiting on
+    // the load / store pipe, which the element-wise threads spent between two steps (2700 clocks a step,
+    // half of them here) while the products waited.  TMEM lane = d, column = query; a warp's 32 lanes
+    // cover 32 consecutive d of one query row.
+    const uint32_t z_tmem = tmem + ((uint32_t)((warp & 3) * 32) << 16) + C::COL_Z;
+    const int d = tid & (BS - 1);
+    BItem bi;
+    int it = 0;                                      // running step count
+    bool alive = true;
+    for (int k = 0; alive && next_bitem<MODE, EMASK, BT, false>(p, args, bars, k, lane, abort_flag, bi) > 0; ++k) {
+      for (int g = 0; g < n_heads && alive; ++g) {
+        const int h = bi.h_kv * group + g;
+        const StepWalk<BT> w = make_steps<MODE, BT>(p, args, bi.tile, h);
+        float* head_rows = args.dq_acc + ((int64_t)bi.b * p.H_q + h) * p.N_q * D + d;
+        for (int s = 0; s < w.cnt; ++s, ++it) {
+          const int r0 = w.row0(s), n_valid = p.N_q - r0;
+          if (!mbar_wait(&bars->acc_done[it & 1], (it >> 1) & 1, abort_flag)) { alive = false; break; }
+          tc_fence_after_sync();
+          uint32_t zr[64];
+          tmem_ld32(z_tmem, &zr[0]);
+          tmem_ld32(z_tmem + 32, &zr[32]);
+          tmem_wait_ld();
+          tc_fence_before_sync();
+          mbar_arrive(&bars->z_free);
+          float* acc_rows = head_rows + (int64_t)r0 * D;
+          if (n_valid >= 64) {
+#pragma unroll
+            for (int c = 0; c < 64; ++c) atomicAdd(acc_rows + c * D, __uint_as_float(zr[c]));
+          } else {
+#pragma unroll
+            for (int c = 0; c < 64; ++c)
+              if (c < n_valid) atomicAdd(acc_rows + c * D, __uint_as_float(zr[c]));
+          }
+        }
+      }
+    }
+  } else {
     // ============================== element-wise group / epilogue ==============================
-    const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
+    const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
+    const int lrow = tid & (BS - 1), share = tid / BS, col_first = share * COLS;   // row of the stationary tile, first column of a step
     const float scale2 = p.sm_scale * kLog2e;
     BItem bi;
     int it0 = 0;
     bool alive = true;
-    // Fused mode: read the dQ^T tile of step `k` (TMEM lane = d = tid, column = query) and add it to
-    // the fp32 accumulator rows; a warp's 32 lanes cover 32 consecutive d of one query row.
-    auto drain_dq = [&](int k, float* acc_rows, int n_valid) -> bool {
-      if (!mbar_wait(&bars->acc_done[k & 1], (k >> 1) & 1, abort_flag)) return false;
-      tc_fence_after_sync();
-      uint32_t zr[BT];
-      tmem_ld32(tmem + lane_base + C::COL_Z, &zr[0]);
-      tmem_ld32(tmem + lane_base + C::COL_Z + 32, &zr[32]);
-      tmem_wait_ld();
-      tc_fence_before_sync();
-      mbar_arrive(&bars->z_free);
-      if (n_valid >= BT) {
-#pragma unroll
-        for (int c = 0; c < BT; ++c) atomicAdd(acc_rows + c * D, __uint_as_float(zr[c]));
-      } else {
-#pragma unroll
-        for (int c = 0; c < BT; ++c)
-          if (c < n_valid) atomicAdd(acc_rows + c * D, __uint_as_float(zr[c]));
-      }
-      return true;
-    };
-    float* pend_rows = nullptr;                      // fused: accumulator rows of the step not yet drained
-    int pend_valid = 0, pend_it = -1;
     for (int kitem = 0; alive; ++kitem) {
-    const int got = next_bitem<MODE, EMASK, false>(p, args, bars, kitem, lane, abort_flag, bi);
+    const int got = next_bitem<MODE, EMASK, BT, false>(p, args, bars, kitem, lane, abort_flag, bi);
     if (got <= 0) break;
     const int tile = bi.tile, b = bi.b, hx = bi.hx, h_kv = bi.h_kv, t0 = bi.t0, total_steps = bi.total_steps;
-    const int srow = t0 + tid;                       // key (DKV) or query row (DQ) of this thread
-    float l2_row = INFINITY, dl_row = 0.f;           // DQ mode: statistics of this thread's query row
+    const int srow = t0 + lrow;                      // key (DKV) or query row (DQ) of this thread
+    float nl_one = -INFINITY, nd_one = 0.f;          // DQ mode: statistics of this thread's query row
     if (MODE == MODE_DQ && srow < p.N_q) {
       const float l = a.lse[(int64_t)b * a.lse_stride[0] + (int64_t)hx * a.lse_stride[1] + (int64_t)srow * a.lse_stride[2]];
-      l2_row = (l == -INFINITY) ? INFINITY : l * kLog2e;
-      dl_row = a.delta[((int64_t)b * p.H_q + hx) * p.N_q + srow];
+      nl_one = (l == -INFINITY) ? -INFINITY : -l * kLog2e;
+      nd_one = -a.delta[((int64_t)b * p.H_q + hx) * p.N_q + srow];
     }
+    const uint64_t nl_row = tc::f32x2_pack(nl_one, nl_one), nd_row = tc::f32x2_pack(nd_one, nd_one);
+    const uint64_t sc2 = tc::f32x2_pack(scale2, scale2);
     int it = it0;                                    // running step count
     for (int g = 0; g < n_heads && alive; ++g) {
       const int h = KVS ? h_kv * group + g : hx;
-      const StepWalk w = make_steps<MODE>(p, args, tile, h);
+      const StepWalk<BT> w = make_steps<MODE, BT>(p, args, tile, h);
       const float slope2 = ALIBI ? load_slope<T>(p.slopes, h) * kLog2e : 0.f;
       for (int s = 0; s < w.cnt; ++s, ++it) {
-        const int st = it % STAGES, t = it & 1;
+        const int t = it & 1;
         const int r0 = w.row0(s);
-        if (KVS && !mbar_wait(&bars->strm_full[st], (it / STAGES) & 1, abort_flag)) { alive = false; break; }
         if (!mbar_wait(&bars->xy_full[t], (it >> 1) & 1, abort_flag)) { alive = false; break; }
         tc_fence_after_sync();
-        const uint32_t xt = tmem + lane_base + (t ? C::COL_X1 : C::COL_X0);
-        const uint32_t yt = tmem + lane_base + (t ? C::COL_Y1 : C::COL_Y0);
-        uint32_t xr[BT], yr[BT];
+        const uint32_t xt = tmem + lane_base + C::col_x(t) + col_first;
+        const uint32_t yt = tmem + lane_base + C::col_y(t) + col_first;
+        uint32_t xr[COLS], yr[COLS];
         tmem_ld32(xt, &xr[0]); tmem_ld32(xt + 32, &xr[32]);
         tmem_ld32(yt, &yr[0]); tmem_ld32(yt + 32, &yr[32]);
         tmem_wait_ld();
-        if (FUSED) {
-          // dP^T is in registers: the next step's dP^T product may overwrite the buffer
+        if (C::Y_SINGLE) {
+          // dP is in registers: the next step's dP product may overwrite the buffer
           tc_fence_before_sync();
           mbar_arrive(&bars->y_free);
         }
-        const float* stats = reinterpret_cast<const float*>(smem + STAGE0_OFF + st * STAGE_BYTES + 2 * C::STRM_TILE);
 
-        // Tile-level: does any element of this 128 x 64 tile need masking?
-        //   key-stationary: lane = key srow, column c = query r0 + c;  DQ: lane = query srow, column c = key r0 + c.
-        const int col_limit = (KVS ? p.N_q : p.N_kv) - r0;     // columns c < col_limit exist
-        bool need_mask = col_limit < BT;
+        // Does any element of these 128 x 64 columns need masking?
+        //   key-stationary: lane = key srow, column c = query c0 + c;  DQ: lane = query srow, column c = key c0 + c.
+        const int c0 = r0 + col_first;
+        const int col_limit = (KVS ? p.N_q : p.N_kv) - c0;     // columns c < col_limit exist
+        bool need_mask = col_limit < COLS;
         if (EMASK == EMASK_CAUSAL)
-          need_mask = need_mask || (KVS ? (r0 < t0 + BS - 1) : (r0 + BT - 1 > t0));
+          need_mask = need_mask || (KVS ? (c0 < t0 + BS - 1) : (c0 + COLS - 1 > t0));
         if (EMASK == EMASK_WINDOW)
-          need_mask = need_mask || (r0 + BT - 1 - t0 >= p.window) || (t0 + BS - 1 - r0 >= p.window);
-        const int rel = srow - r0;   // key-stationary: query c kept iff c >= rel;  DQ: key c kept iff c <= rel
+          need_mask = need_mask || (c0 + COLS - 1 - t0 >= p.window) || (t0 + BS - 1 - c0 >= p.window);
+        const int rel = srow - c0;   // key-stationary: query c kept iff c >= rel;  DQ: key c kept iff c <= rel
         uint64_t tile_bits = ~0ull;  // EMASK_BITS: this lane's 64 columns of the block's bit matrix
         if (EMASK == EMASK_BITS && w.slots != nullptr) {
           const int bs = w.slots[s / w.per];
@@ -562,83 +650,68 @@ bwd_tcgen05_kernel(const BwdArgs args, const __grid_constant__ CUtensorMap map_a
             // key-stationary: rows of q_bits are keys, bits are queries; DQ: rows of kv_bits are queries
             const int stat_block = KVS ? p.block_n : p.block_m;
             const uint64_t* bits = KVS ? p.q_bits : p.kv_bits;
-            tile_bits = bits[((int64_t)bs * stat_block + (t0 % stat_block) + tid) * (w.block >> 6) + (s % w.per)];
+            tile_bits = bits[((int64_t)bs * stat_block + (t0 % stat_block) + lrow) * (w.block >> 6) + (s % w.per) * SHARES + share];
             need_mask = true;
           }
         }
 
-        uint32_t pk[BT / 2], dk[BT / 2];
+        uint32_t pk[COLS / 2], dk[COLS / 2];
         const float relf = (float)rel;
         // The masking decision is taken once per tile: the element loop exists in a masked and an
-        // unmasked copy, and the per-column statistics come in float4 shared-memory loads.
+        // unmasked copy.  The arithmetic runs on packed fp32 pairs (half the issue slots).
         auto element_pass = [&](auto masked_tag) {
           constexpr bool MASKED = decltype(masked_tag)::value;
 #pragma unroll
-          for (int c = 0; c < BT; c += 4) {
-            float l2v[4], dlv[4];
-            if (KVS) {
-              const float4 a4 = *reinterpret_cast<const float4*>(stats + c);
-              const float4 b4 = *reinterpret_cast<const float4*>(stats + BT + c);
-              l2v[0] = a4.x; l2v[1] = a4.y; l2v[2] = a4.z; l2v[3] = a4.w;
-              dlv[0] = b4.x; dlv[1] = b4.y; dlv[2] = b4.z; dlv[3] = b4.w;
-            } else {
-#pragma unroll
-              for (int u = 0; u < 4; ++u) { l2v[u] = l2_row; dlv[u] = dl_row; }
-            }
-            float pe[4], de[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-              const int cc = c + u;
-              float e = fmaf(__uint_as_float(xr[cc]), scale2, -l2v[u]);
-              if (ALIBI) e -= slope2 * fabsf(relf - (float)cc);
-              float pr = ex2_approx(e);
-              if (MASKED) {
-                bool keep = cc < col_limit;
-                if (EMASK == EMASK_CAUSAL) keep = keep && (KVS ? (cc >= rel) : (cc <= rel));
-                if (EMASK == EMASK_WINDOW) keep = keep && (cc - rel < p.window) && (rel - cc < p.window);
-                if (EMASK == EMASK_BITS) keep = keep && ((tile_bits >> cc) & 1ull);
-                pr = keep ? pr : 0.f;
+          for (int cc = 0; cc < COLS; cc += 2) {
+            {
+              float e0, e1, d0, d1;
+              // key-stationary: S^T and dP^T come with -L / scale and -delta in them
+              const uint64_t x2 = tc::f32x2_pack(__uint_as_float(xr[cc]), __uint_as_float(xr[cc + 1]));
+              const uint64_t y2 = tc::f32x2_pack(__uint_as_float(yr[cc]), __uint_as_float(yr[cc + 1]));
+              tc::f32x2_unpack(KVS ? tc::f32x2_mul(x2, sc2) : tc::f32x2_fma(x2, sc2, nl_row), e0, e1);
+              if (ALIBI) {
+                e0 -= slope2 * fabsf(relf - (float)cc);
+                e1 -= slope2 * fabsf(relf - (float)(cc + 1));
               }
-              pe[u] = pr;
-              de[u] = pr * (__uint_as_float(yr[cc]) - dlv[u]);
+              float p0 = ex2_approx(e0), p1 = ex2_approx(e1);
+              if (MASKED) {
+                auto kept = [&](int x) {
+                  bool keep = x < col_limit;
+                  if (EMASK == EMASK_CAUSAL) keep = keep && (KVS ? (x >= rel) : (x <= rel));
+                  if (EMASK == EMASK_WINDOW) keep = keep && (x - rel < p.window) && (rel - x < p.window);
+                  if (EMASK == EMASK_BITS) keep = keep && ((tile_bits >> x) & 1ull);
+                  return keep;
+                };
+                p0 = kept(cc) ? p0 : 0.f;
+                p1 = kept(cc + 1) ? p1 : 0.f;
+              }
+              const uint64_t dp2 = KVS ? y2 : tc::f32x2_add(y2, nd_row);
+              tc::f32x2_unpack(tc::f32x2_mul(tc::f32x2_pack(p0, p1), dp2), d0, d1);
+              pk[cc >> 1] = Pack2<T>::run(p0, p1);
+              dk[cc >> 1] = Pack2<T>::run(d0, d1);
             }
-            pk[c >> 1] = Pack2<T>::run(pe[0], pe[1]);
-            pk[(c >> 1) + 1] = Pack2<T>::run(pe[2], pe[3]);
-            dk[c >> 1] = Pack2<T>::run(de[0], de[1]);
-            dk[(c >> 1) + 1] = Pack2<T>::run(de[2], de[3]);
           }
         };
         if (need_mask) element_pass(std::true_type{});
         else element_pass(std::false_type{});
         if (FUSED) {
-          tmem_st32(xt, pk);
           // dS^T row of this key: 64 queries = 128 bytes = eight 16-byte chunks, chunk c stored at
-          // c ^ (row & 7) (the 128-byte swizzle both MMA descriptors expect).  Buffer t was last read
+          // c ^ (row & 7) (the 128-byte swizzle the MMA descriptor expects).  Buffer t was last read
           // by the products of step it-2, which ran before this step's S^T was issued.
-          const uint32_t row_addr = sDS0 + t * C::DS_TILE + tid * 128;
+          const uint32_t row_addr = sDS0 + t * C::DS_TILE + lrow * 128;
 #pragma unroll
           for (int c8 = 0; c8 < 8; ++c8)
-            tc::sts128(row_addr + ((c8 ^ (tid & 7)) << 4),
+            tc::sts128(row_addr + ((c8 ^ (lrow & 7)) << 4),
                        make_uint4(dk[c8 * 4], dk[c8 * 4 + 1], dk[c8 * 4 + 2], dk[c8 * 4 + 3]));
           fence_proxy_async_smem();
-        } else if (MODE == MODE_DKV) {
-          tmem_st32(xt, pk);
-          tmem_st32(yt, dk);
-        } else {
-          // dS buffer t was last read by the accumulate MMAs of step it-2
-          if (it >= 2 && !mbar_wait(&bars->acc_done[t], ((it >> 1) - 1) & 1, abort_flag)) { alive = false; break; }
-          tmem_st32(tmem + lane_base + (t ? C::COL_DS1 : C::COL_DS0), dk);
         }
+        // two-pass dQ at head dim 128: the dS buffer was last read by the accumulate MMAs of step it-2
+        if (MODE == MODE_DQ && !C::DS_IN_X && it >= 2 && !mbar_wait(&bars->acc_done[t], ((it >> 1) - 1) & 1, abort_flag)) { alive = false; break; }
+        if (KVS) tmem_st32(xt, pk);
+        tmem_st32(tmem + lane_base + C::col_ds(t, share * (COLS / 16)), dk);
         tmem_wait_st();
         tc_fence_before_sync();
         mbar_arrive(&bars->p_full[t]);
-        if (FUSED) {
-          // the previous step's dQ^T tile is complete (or about to be): add it to the accumulator
-          if (pend_it >= 0 && !drain_dq(pend_it, pend_rows, pend_valid)) { alive = false; break; }
-          pend_it = it;
-          pend_rows = args.dq_acc + (((int64_t)b * p.H_q + h) * p.N_q + r0) * D + tid;
-          pend_valid = min(BT, p.N_q - r0);
-        }
       }
     }
 
@@ -648,16 +721,12 @@ bwd_tcgen05_kernel(const BwdArgs args, const __grid_constant__ CUtensorMap map_a
       alive = mbar_wait(&bars->acc_done[last & 1], (last >> 1) & 1, abort_flag);
       tc_fence_after_sync();
     }
-    if (FUSED && alive && pend_it >= 0) {
-      // the item's last dQ^T tile first: the next item's first step needs the buffer
-      alive = drain_dq(pend_it, pend_rows, pend_valid);
-      pend_it = -1;
-    }
     if (alive) {
       const int n_rows = KVS ? p.N_kv : p.N_q;
       const bool store = srow < n_rows;
-      // gradient of the stationary operand that carries the scale (dK or dQ), with the rotation undone
-      {
+      // gradient of the stationary operand that carries the scale (dK or dQ), with the rotation undone;
+      // two threads per row: the first takes dK and the second dV, or each half of the columns of dQ
+      if (!KVS || share == 0) {
         const uint32_t acc = tmem + lane_base + (KVS ? C::COL_ACC2 : C::COL_ACC1);
         T* dst = KVS
                      ? reinterpret_cast<T*>(a.dk) + (int64_t)b * a.dk_stride[0] + (int64_t)h_kv * a.dk_stride[1] + (int64_t)srow * a.dk_stride[2]
@@ -679,6 +748,7 @@ bwd_tcgen05_kernel(const BwdArgs args, const __grid_constant__ CUtensorMap map_a
           if (store) {
 #pragma unroll
             for (int q4 = 0; q4 < 4; ++q4) {
+              if (SHARES == 2 && !KVS && (q4 >> 1) != share) continue;
               float gl[8], gh[8];
 #pragma unroll
               for (int i = 0; i < 8; ++i) {
@@ -714,7 +784,7 @@ bwd_tcgen05_kernel(const BwdArgs args, const __grid_constant__ CUtensorMap map_a
           }
         }
       }
-      if (KVS) {
+      if (KVS && share == SHARES - 1) {
         T* dst = reinterpret_cast<T*>(a.dv) + (int64_t)b * a.dv_stride[0] + (int64_t)h_kv * a.dv_stride[1] + (int64_t)srow * a.dv_stride[2];
 #pragma unroll
         for (int c = 0; c < D / 32; ++c) {
@@ -752,7 +822,7 @@ bwd_tcgen05_kernel(const BwdArgs args, const __grid_constant__ CUtensorMap map_a
   tc_fence_before_sync();
   __syncthreads();
   if (tid == 0 && *abort_flag && p.status != nullptr) atomicExch(p.status, AF_STATUS_WAIT_TIMEOUT);
-  if (warp == 4) {
+  if (warp == WARP_LOAD) {
     __syncwarp();
     tc_fence_after_sync();
     tmem_dealloc(tmem, C::TMEM_COLS);
@@ -770,7 +840,7 @@ int launch_instance(const BwdArgs& args, const CUtensorMap& a1, const CUtensorMa
     configured = true;
   }
   if (args.total_items <= 0) return AF_OK;
-  kern<<<(unsigned)args.grid_ctas, 224, smem, st>>>(args, a1, a2, b1, b2);
+  kern<<<(unsigned)args.grid_ctas, (BCfg<D, MODE>::THREADS), smem, st>>>(args, a1, a2, b1, b2);
   count_launch();
   return check_cuda(cudaGetLastError(), "bwd_tcgen05 launch");
 }

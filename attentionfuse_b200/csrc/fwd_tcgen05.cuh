@@ -434,6 +434,12 @@ __device__ __forceinline__ uint64_t f32x2_add(uint64_t a, uint64_t b) {
   return r;
 }
 
+__device__ __forceinline__ uint64_t f32x2_mul(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
 template <typename T, int KIND, int NC>
 __device__ __forceinline__ void exp_pass(const uint32_t (&xr)[NC], uint32_t (&pk)[NC / 2], float scale2, float shift,
                                          float slope_c, float& rsum) {

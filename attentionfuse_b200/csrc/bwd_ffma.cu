@@ -85,30 +85,37 @@ __global__ void bwd_delta_kernel(const AfBwdParams a) {
 }
 
 // Vector form for 2-byte element types with unit inner strides and 16-byte-aligned rows: LPR
-// lanes per row, each with one 16-byte load of O and of dO (8 elements), so that the launch is
-// bound by HBM bandwidth rather than by load instructions.
+// lanes per row, each with one 16-byte load of O and of dO (8 elements) of DELTA_ROWS rows, so that
+// eight loads are in flight per thread and the launch is bound by HBM bandwidth (268 MB of O and dO:
+// 63 us = 4.3 TB/s with one row per thread and 64-bit divisions for its coordinates).
+constexpr int DELTA_ROWS = 4;
 template <typename T, int LPR>
 __global__ void bwd_delta_vec_kernel(const AfBwdParams a) {
   const AfProblem& p = a.p;
-  const int64_t gthread = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t r = gthread / LPR;
-  const int sub = (int)(gthread % LPR);
-  const int64_t total = (int64_t)p.B * p.H_q * p.N_q;
-  float s = 0.f;
-  if (r < total) {
-    const int row = (int)(r % p.N_q), h = (int)((r / p.N_q) % p.H_q);
-    const int64_t b = r / ((int64_t)p.N_q * p.H_q);
-    const T* o = reinterpret_cast<const T*>(a.o) + b * a.o_stride[0] + (int64_t)h * a.o_stride[1] + (int64_t)row * a.o_stride[2] + sub * 8;
-    const T* g = reinterpret_cast<const T*>(a.d_o) + b * a.do_stride[0] + (int64_t)h * a.do_stride[1] + (int64_t)row * a.do_stride[2] + sub * 8;
-    const uint4 ov = *reinterpret_cast<const uint4*>(o), gv = *reinterpret_cast<const uint4*>(g);
-    const T* oe = reinterpret_cast<const T*>(&ov);
-    const T* ge = reinterpret_cast<const T*>(&gv);
+  const uint32_t gthread = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t r0 = gthread / LPR * DELTA_ROWS, sub = gthread % LPR;
+  const uint32_t total = (uint32_t)p.B * p.H_q * p.N_q;
+  uint4 ov[DELTA_ROWS], gv[DELTA_ROWS];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) s += Elem<T>::to_f32(oe[i]) * Elem<T>::to_f32(ge[i]);
+  for (int i = 0; i < DELTA_ROWS; ++i) {
+    const uint32_t r = r0 + i < total ? r0 + i : total - 1;
+    const uint32_t bh = r / (uint32_t)p.N_q, row = r - bh * p.N_q, b = bh / (uint32_t)p.H_q, h = bh - b * p.H_q;
+    ov[i] = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(a.o) + (int64_t)b * a.o_stride[0] +
+                                                 (int64_t)h * a.o_stride[1] + (int64_t)row * a.o_stride[2] + sub * 8));
+    gv[i] = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(a.d_o) + (int64_t)b * a.do_stride[0] +
+                                                 (int64_t)h * a.do_stride[1] + (int64_t)row * a.do_stride[2] + sub * 8));
   }
 #pragma unroll
-  for (int off = LPR / 2; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-  if (sub == 0 && r < total) a.delta[r] = s;
+  for (int i = 0; i < DELTA_ROWS; ++i) {
+    const T* oe = reinterpret_cast<const T*>(&ov[i]);
+    const T* ge = reinterpret_cast<const T*>(&gv[i]);
+    float s = 0.f;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) s += Elem<T>::to_f32(oe[e]) * Elem<T>::to_f32(ge[e]);
+#pragma unroll
+    for (int off = LPR / 2; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+    if (sub == 0 && r0 + i < total) a.delta[r0 + i] = s;
+  }
 }
 
 // Recompute one 32x32 tile of P and dS into shared memory.  Thread (ty, tx) owns query rows
@@ -486,9 +493,9 @@ int launch_bwd_delta(const AfBwdParams& a, cudaStream_t st) {
   const bool aligned = a.o_stride[3] == 1 && a.do_stride[3] == 1 && ((uintptr_t)a.o & 15) == 0 && ((uintptr_t)a.d_o & 15) == 0 &&
                        a.o_stride[0] % 8 == 0 && a.o_stride[1] % 8 == 0 && a.o_stride[2] % 8 == 0 &&
                        a.do_stride[0] % 8 == 0 && a.do_stride[1] % 8 == 0 && a.do_stride[2] % 8 == 0;
-  if (aligned && p.dtype != AF_F32 && (p.D == 64 || p.D == 128 || p.D == 256)) {
+  if (aligned && p.dtype != AF_F32 && (p.D == 64 || p.D == 128 || p.D == 256) && rows * (p.D / 8) < (1ll << 31)) {
     const int lpr = p.D / 8;
-    const unsigned vblocks = (unsigned)((rows * lpr + 255) / 256);
+    const unsigned vblocks = (unsigned)(((rows + DELTA_ROWS - 1) / DELTA_ROWS * lpr + 255) / 256);
 #define AF_DELTA_VEC(TYPE)                                                                  \
     if (lpr == 8) bwd_delta_vec_kernel<TYPE, 8><<<vblocks, 256, 0, st>>>(a);                \
     else if (lpr == 16) bwd_delta_vec_kernel<TYPE, 16><<<vblocks, 256, 0, st>>>(a);         \

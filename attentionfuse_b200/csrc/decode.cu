@@ -438,10 +438,16 @@ __device__ __forceinline__ KeyRange key_range(const AfDecodeParams& a, int b) {
 // next, so a unit is covered by a run of consecutive CTAs, and the partial of (unit u, CTA c)
 // lives in slot u + c (unique, because both only grow along the run).
 __device__ __forceinline__ int unit_tiles(const KeyRange& r) { return max(1, (r.span + DEC_BN - 1) / DEC_BN); }
-__device__ __forceinline__ int64_t total_tiles(const AfDecodeParams& a, int units_per_batch) {
-  int64_t T = 0;
-  for (int b = 0; b < a.B; ++b) T += (int64_t)unit_tiles(key_range(a, b)) * units_per_batch;
-  return T;
+// Tiles of a unit of every batch entry, looked up by all threads at once: one after the other they are
+// a chain of dependent trips to the L2 at the head of every CTA.  Beyond the table the entries are
+// looked up where they are needed.
+constexpr int MAX_TILE_TABLE = 512;
+__device__ __forceinline__ void fill_tile_table(const AfDecodeParams& a, int* table) {
+  for (int b = threadIdx.x; b < min(a.B, MAX_TILE_TABLE); b += blockDim.x) table[b] = unit_tiles(key_range(a, b));
+  __syncthreads();
+}
+__device__ __forceinline__ int tiles_of(const AfDecodeParams& a, const int* table, int b) {
+  return b < MAX_TILE_TABLE ? table[b] : unit_tiles(key_range(a, b));
 }
 // CTA that holds tile index `tile` (0 <= tile < T): the c with  c T / C <= tile < (c + 1) T / C.
 __device__ __forceinline__ int cta_of_tile(int64_t tile, int64_t T, int C) {
@@ -479,12 +485,16 @@ template <int D>
 __device__ __forceinline__ void merge_partials(const AfDecodeParams& a, const PartialRows& pr, int lane, float (&acc)[D / 32],
                                                float& lse) {
   constexpr int VEC = D / 32;
+  // the partials of a row are looked at over the lanes first (one trip to memory for up to 32 of them)
   float mstar = -INFINITY;
-  for (int i = 0; i < pr.count; ++i) mstar = fmaxf(mstar, a.ws_m[pr.base + i * pr.stride]);
+  for (int i = lane; i < pr.count; i += 32) mstar = fmaxf(mstar, a.ws_m[pr.base + i * pr.stride]);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) mstar = fmaxf(mstar, __shfl_xor_sync(0xffffffffu, mstar, o));
   const float m_use = (mstar == -INFINITY) ? 0.f : mstar;
 #pragma unroll
   for (int i = 0; i < VEC; ++i) acc[i] = 0.f;
   float lsum = 0.f;
+#pragma unroll 4
   for (int i = 0; i < pr.count; ++i) {
     const int64_t r = pr.base + i * pr.stride;
     const float w = expf(a.ws_m[r] - m_use);
@@ -519,7 +529,11 @@ __global__ void __launch_bounds__(DEC_THREADS) decode_split_kernel(const AfDecod
   constexpr int VEC = D / 32;
   constexpr int MAX_MINE = 64;
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  __shared__ int s_last, s_failed, s_mine[FUSED ? MAX_MINE : 1];
+  __shared__ int s_last, s_failed, s_mine[FUSED ? MAX_MINE : 1], s_tiles[MAX_TILE_TABLE];
+
+  // The combine may be set up as soon as every CTA is running (it waits for the end of this grid
+  // before it reads a partial).
+  if (!FUSED) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int group = a.H_q / a.H_kv;
@@ -615,15 +629,17 @@ __global__ void __launch_bounds__(DEC_THREADS) decode_split_kernel(const AfDecod
     if (FUSED) after_unit(unit, a.num_splits, split == 0, 0, 0, 0);
   } else {
     const int C = (int)gridDim.x, c = (int)blockIdx.x;
-    const int64_t T_all = total_tiles(a, units_per_batch);
+    fill_tile_table(a, s_tiles);
+    int64_t T_all = 0;
+    for (int b = 0; b < a.B; ++b) T_all += (int64_t)tiles_of(a, s_tiles, b) * units_per_batch;
     const int64_t t_lo = ((int64_t)c * T_all) / C, t_hi = ((int64_t)(c + 1) * T_all) / C;
     const int unit_rows_max = min(group, 64);
     int64_t base = 0;
     for (int b = 0; b < a.B && base < t_hi; ++b) {
-      const KeyRange kr = key_range(a, b);
-      const int tiles_u = unit_tiles(kr);
+      const int tiles_u = tiles_of(a, s_tiles, b);
       const int64_t b_end = base + (int64_t)tiles_u * units_per_batch;
       if (b_end > t_lo) {
+        const KeyRange kr = key_range(a, b);
         const int uu_first = (int)(max(t_lo - base, (int64_t)0) / tiles_u);
         for (int uu = uu_first; uu < units_per_batch; ++uu) {
           const int64_t unit_start = base + (int64_t)uu * tiles_u;
@@ -714,18 +730,30 @@ __global__ void decode_combine_kernel(const AfDecodeParams a, const int head_chu
   int64_t T_all = 0, unit_start = 0;
   int tiles_u = 0, unit = 0;
   if (a.balanced_ctas > 0) {
-    // the row's unit and its place in the tile sequence (the same walk the split kernel does)
+    // the row's unit and its place in the tile sequence (the same walk the split kernel does, the batch
+    // entries over the lanes)
     const int group = a.H_q / a.H_kv, units_per_batch = a.H_kv * head_chunks;
     const int uu = (h / group) * head_chunks + (h % group) / 64;
     unit = b * units_per_batch + uu;
-    for (int bb = 0; bb < a.B; ++bb) {
-      const int tb = unit_tiles(key_range(a, bb));
-      if (bb < b) unit_start += (int64_t)tb * units_per_batch;
-      if (bb == b) { tiles_u = tb; unit_start += (int64_t)uu * tb; }
-      T_all += (int64_t)tb * units_per_batch;
+    long long before = 0, all = 0;
+    for (int bb = lane; bb < a.B; bb += 32) {
+      const long long tb = (long long)unit_tiles(key_range(a, bb)) * units_per_batch;
+      all += tb;
+      if (bb < b) before += tb;
     }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      all += __shfl_xor_sync(0xffffffffu, all, o);
+      before += __shfl_xor_sync(0xffffffffu, before, o);
+    }
+    tiles_u = unit_tiles(key_range(a, b));
+    T_all = all;
+    unit_start = before + (int64_t)uu * tiles_u;
   }
   const PartialRows pr = partial_rows(a, head_chunks, row, T_all, unit_start, tiles_u, unit);
+  // everything above depends on the call's inputs alone; the partials are there once the grid before
+  // this one is over
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   float acc[VEC], lse;
   merge_partials<D>(a, pr, lane, acc, lse);
   if (a.o != nullptr) {
@@ -792,7 +820,18 @@ int launch_split_impl(const AfDecodeParams& a, cudaStream_t st) {
 template <typename T, int D>
 int launch_combine_impl(const AfDecodeParams& a, cudaStream_t st) {
   const int rows = a.B * a.H_q;
-  decode_combine_kernel<T, D><<<(rows + 3) / 4, 128, 0, st>>>(a, (a.H_q / a.H_kv + 63) / 64);
+  // Launched early (programmatic dependent launch): its CTAs find their units while the split grid
+  // drains.
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((rows + 3) / 4);
+  cfg.blockDim = dim3(128);
+  cfg.stream = st;
+  cudaLaunchAttribute early{};
+  early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  early.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &early;
+  cfg.numAttrs = 1;
+  AF_CUDA_OK(cudaLaunchKernelEx(&cfg, decode_combine_kernel<T, D>, a, (a.H_q / a.H_kv + 63) / 64));
   count_launch();
   return check_cuda(cudaGetLastError(), "decode_combine launch");
 }

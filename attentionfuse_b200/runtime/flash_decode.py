@@ -16,7 +16,11 @@ import torch
 
 from ..ir.high_level import Graph, BiasKind, MaskKind
 from . import _lib
+from .kernel_cache import get_or_compile
 
+_PLAIN_MASKS = frozenset({MaskKind.FULL})
+_POSITIONED_MASKS = frozenset({MaskKind.FULL, MaskKind.CAUSAL, MaskKind.SLIDING_WINDOW})
+_DECODE_BIASES = frozenset({BiasKind.ALIBI})
 _DECODE_TEMPLATES: dict = {}
 DECODE_HEAD_DIMS = (64, 128)
 DECODE_DTYPES = (torch.float16, torch.bfloat16)
@@ -27,24 +31,24 @@ def can_use_flash_decode(graph: Graph, Q: torch.Tensor, K: torch.Tensor, positio
     attnfuse/runtime/flash_decode.py:46-65).  With ``positioned`` -- the caller said where the
     query row sits on the key axis -- causal and sliding-window masks and RoPE are taken too:
     for a single row a mask is a range of keys, and the kernel rotates the row and the key tiles."""
-    if Q.shape[2] != 1 or K.shape[2] < 256:
+    q_shape, k_shape = Q.shape, K.shape
+    if q_shape[2] != 1 or k_shape[2] < 256:
         return False
-    allowed_masks = {MaskKind.FULL, MaskKind.CAUSAL, MaskKind.SLIDING_WINDOW} if positioned else {MaskKind.FULL}
-    if {m.kind for m in graph.collect_masks()} - allowed_masks:
+    facts = get_or_compile(graph)
+    if not facts.mask_kinds <= (_POSITIONED_MASKS if positioned else _PLAIN_MASKS):
         return False
-    if {b.kind for b in graph.collect_biases()} - {BiasKind.ALIBI}:
+    if not facts.bias_kinds <= _DECODE_BIASES:
         return False
-    if graph.has_rope() and not positioned:
+    if facts.has_rope and not positioned:
         return False
     # The mma.sync decode kernels are instantiated for these types and head dims; anything
     # else takes the general forward kernel (N_q = 1 is a legal dense problem there).
-    if Q.dtype not in DECODE_DTYPES or Q.shape[3] not in DECODE_HEAD_DIMS:
+    if Q.dtype not in DECODE_DTYPES or q_shape[3] not in DECODE_HEAD_DIMS:
         return False
-    if K.stride(3) != 1 or Q.stride(3) != 1:
+    s0, s1, s2, s3 = K.stride()
+    if s3 != 1 or Q.stride(3) != 1:
         return False
-    if any(s % 8 for s in K.stride()[:3]) or K.data_ptr() % 16:
-        return False
-    return True
+    return (s0 | s1 | s2) % 8 == 0 and K.data_ptr() % 16 == 0
 
 
 @functools.lru_cache(maxsize=8)
@@ -103,7 +107,8 @@ def run_flash_decode(graph: Optional[Graph], Q: torch.Tensor, K: torch.Tensor, V
     lib = _lib.load()
     B, H_q, _, D = Q.shape
     _, H_kv, N_kv, _ = K.shape
-    if V.stride() != K.stride() and (V.stride(3) != 1 or any(s % 8 for s in V.stride()[:3])):
+    q_stride, k_stride = Q.stride(), K.stride()
+    if V.stride() != k_stride and (V.stride(3) != 1 or any(s % 8 for s in V.stride()[:3])):
         V = V.contiguous()
     # A rotated row (cos / sin given) is bound by the rotation of the K tiles, not by bandwidth, and
     # wants the higher occupancy of the split grid (0.60 against 1.2 ms at B16 H32/8 L32768) --
@@ -116,8 +121,15 @@ def run_flash_decode(graph: Optional[Graph], Q: torch.Tensor, K: torch.Tensor, V
     elif num_splits is None:
         dev_index = Q.device.index if Q.device.index is not None else torch.cuda.current_device()
         num_splits = _pick_num_splits(B, H_q, H_kv, N_kv, dev_index, kv_lens is not None)
-    ws_m, ws_l, ws_acc = workspace if workspace is not None else decode_workspace(
-        num_splits, B, H_q, D, Q.device, rows=balanced_rows(B, H_q, H_kv, balanced_ctas) if balanced_ctas else None)
+    if workspace is not None:
+        m_ptr, l_ptr, acc_ptr = (t.data_ptr() for t in workspace)
+    else:
+        # the layout of decode_workspace, addressed without making tensors of its parts
+        rows = balanced_rows(B, H_q, H_kv, balanced_ctas) if balanced_ctas else num_splits * B * H_q
+        rows_pad = (rows + 3) & ~3
+        partials = torch.empty(2 * rows_pad + rows * D, dtype=torch.float32, device=Q.device)
+        m_ptr = partials.data_ptr()
+        l_ptr, acc_ptr = m_ptr + 4 * rows_pad, m_ptr + 8 * rows_pad
 
     slopes = None
     if bias_kind == 1:
@@ -134,7 +146,7 @@ def run_flash_decode(graph: Optional[Graph], Q: torch.Tensor, K: torch.Tensor, V
 
     # the shape / stride / flag part of the parameter block is filled once per distinct problem and
     # copied afterwards: a decode step at short caches is bound by this call path
-    key = (Q.dtype, Q.shape, Q.stride(), K.shape, K.stride(), V.stride(), None if out is None else out.stride(),
+    key = (Q.dtype, Q.shape, q_stride, K.shape, k_stride, V.stride(), None if out is None else out.stride(),
            float(sm_scale), int(bias_kind), int(num_splits), int(kv_offset), int(mask_kind), int(window or 0),
            q_position, cos is not None and cos.stride(0), int(balanced_ctas), bool(kv_rotated),
            int(kv_pos_block), int(kv_pos_stride))
@@ -163,7 +175,7 @@ def run_flash_decode(graph: Optional[Graph], Q: torch.Tensor, K: torch.Tensor, V
     p.slopes, p.kv_lens, p.q_positions = _lib.ptr(slopes), _lib.ptr(kv_lens), _lib.ptr(q_positions)
     if cos is not None:
         p.cos, p.sin = cos.data_ptr(), sin.data_ptr()
-    p.ws_m, p.ws_l, p.ws_acc = ws_m.data_ptr(), ws_l.data_ptr(), ws_acc.data_ptr()
+    p.ws_m, p.ws_l, p.ws_acc = m_ptr, l_ptr, acc_ptr
     if out is not None:
         p.o = out.data_ptr()
     if partial is not None:

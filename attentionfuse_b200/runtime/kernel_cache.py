@@ -30,10 +30,15 @@ class LaunchBundle:
     has_additive_bias: bool
     has_rope: bool
     block_m: int
+    mask_kinds: frozenset      # kinds of the graph's mask and bias nodes: what the routing asks on every call
+    bias_kinds: frozenset
 
 
 def get_or_compile(graph: Graph) -> LaunchBundle:
     key = graph.signature()
+    hit = _cache.get(key)
+    if hit is not None:
+        return hit
     with _lock:
         hit = _cache.get(key)
         if hit is not None:
@@ -49,7 +54,9 @@ def get_or_compile(graph: Graph) -> LaunchBundle:
             mask_kind=MASK_CODE[kernel.mask_kind], window=int(kernel.mask_window or 0),
             bias_kind=BIAS_CODE[kernel.bias_kind], norm_kind=NORM_CODE[kernel.norm_kind],
             has_additive_bias=BIAS_CODE[kernel.bias_kind] == 2, has_rope=kernel.rope_kind == 1,
-            block_m=kernel.config.BLOCK_M)
+            block_m=kernel.config.BLOCK_M,
+            mask_kinds=frozenset(m.kind for m in graph.collect_masks()),
+            bias_kinds=frozenset(b.kind for b in graph.collect_biases()))
         _cache[key] = bundle
         return bundle
 

@@ -16,7 +16,7 @@
 //                   does before its dot (codegen.py:332-341) -- then hand it to the MMA warp.
 //                   The Q tile is rotated once by the softmax group (codegen.py:126-135).
 //   MMA warps       one thread issues  S = Q K^T  (tcgen05.mma, operands from shared memory,
-//                   fp32 accumulator in TMEM, two or three S buffers), a thread of another warp issues
+//                   fp32 accumulator in TMEM, two S buffers), a thread of another warp issues
 //                   O += P V  (P read from TMEM, V from shared memory, N-major); both commit to
 //                   mbarriers.
 //   softmax group   256 threads, two per query row (TMEM lane = row, so row max / row sum need
@@ -80,12 +80,7 @@ template <int D> struct Cfg {
   static constexpr int SMEM_BYTES = TILE_BYTES * (1 + STAGES + STAGES_V) + O_STAGE_BYTES + 1024 /*align*/ +
                                     1536 /*barriers, exchange*/;
   static constexpr int TMEM_COLS = 512;
-  // S buffers: the chain S product -> softmax -> P.V product -> next S product into the same columns is
-  // about 2800 clocks long, half of it barrier and issue latency, so the number of tiles in flight sets
-  // the pace; head dim 64 has the TMEM columns for a third.
-  static constexpr int NS = (D == 64) ? 3 : 2;
-  __host__ __device__ static constexpr int col_s(int t) { return t * 128; }
-  static constexpr int COL_O0 = NS * 128, COL_O1 = COL_O0 + D;   // one O per half of the key columns
+  static constexpr int COL_S0 = 0, COL_S1 = 128, COL_O0 = 256, COL_O1 = 256 + D;   // one O per half of the key columns
 };
 
 // Warp roles.  The softmax group has two threads per query row: warps 0-3 take key columns
@@ -98,7 +93,7 @@ struct Barriers {
   uint64_t q_full, q_ready, q_empty;
   uint64_t k_full[4], k_ready[4], k_empty[4];
   uint64_t v_full[4], v_empty[4];
-  uint64_t s_full[3][2], p_full[3][2], pv_done[3][2];   // [S buffer][half of the key columns]; head dim 128 uses [.][0] of s_full / pv_done
+  uint64_t s_full[2][2], p_full[2][2], pv_done[2][2];   // [S buffer][half of the key columns]; head dim 128 uses [.][0] of s_full / pv_done
   uint64_t o_free;
   uint32_t tmem_base;
   int abort_flag;
@@ -495,7 +490,7 @@ fwd_tcgen05_kernel(const TcArgs args, const __grid_constant__ CUtensorMap tmap_q
                    const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
                    const __grid_constant__ CUtensorMap tmap_o) {
   using C = Cfg<D>;
-  constexpr int STAGES = C::STAGES, STAGES_V = C::STAGES_V, NS = C::NS;
+  constexpr int STAGES = C::STAGES, STAGES_V = C::STAGES_V;
   constexpr bool ROT_K = (ROPE == ROPE_FUSED);
   constexpr int AB_FMT = (Elem<T>::code == AF_BF16) ? 1 : 0;
   // Head dim 64: one S product per half of the key columns, each with barriers of its own, so the
@@ -539,7 +534,7 @@ fwd_tcgen05_kernel(const TcArgs args, const __grid_constant__ CUtensorMap tmap_q
       mbar_init(&bars->v_full[s], 1);
       mbar_init(&bars->v_empty[s], 1);
     }
-    for (int t = 0; t < 3; ++t) {
+    for (int t = 0; t < 2; ++t) {
       for (int hh = 0; hh < 2; ++hh) {
         mbar_init(&bars->s_full[t][hh], 1);
         mbar_init(&bars->p_full[t][hh], SOFTMAX_THREADS / 2);
@@ -638,16 +633,16 @@ fwd_tcgen05_kernel(const TcArgs args, const __grid_constant__ CUtensorMap tmap_q
         ok = mbar_wait(ROPE != ROPE_NONE ? &bars->q_ready : &bars->q_full, qi & 1, abort_flag);
         for (int j = 0; ok && j < n_tiles; ++j) {
           const int gg = g + j;                       // the CTA's running key-tile count
-          const int s = gg % STAGES, t = gg % NS;
+          const int s = gg % STAGES, t = gg & 1;
           if (!mbar_wait(ROT_K ? &bars->k_ready[s] : &bars->k_full[s], (gg / STAGES) & 1, abort_flag)) { ok = false; break; }
           // Descriptors are built once; a k-step, a ring stage or a half only moves the
           // start-address field (address >> 4), so the issuing thread spends one add per operand.
           const uint64_t kdesc = desc_k0 + (uint64_t)((s * C::TILE_BYTES) >> 4);
           for (int hh = 0; hh < S_PARTS && ok; ++hh) {
-            // S buffer t (the half's columns of it) still holds P of tile gg-NS until its P.V product has run
-            if (gg >= NS && !mbar_wait(&bars->pv_done[t][hh], (gg / NS - 1) & 1, abort_flag)) { ok = false; break; }
+            // S buffer t (the half's columns of it) still holds P of tile gg-2 until its P.V product has run
+            if (gg >= 2 && !mbar_wait(&bars->pv_done[t][hh], ((gg >> 1) - 1) & 1, abort_flag)) { ok = false; break; }
             tc_fence_after_sync();
-            const uint32_t d_tmem = tmem + C::col_s(t) + hh * HALF_COLS;
+            const uint32_t d_tmem = tmem + (t ? C::COL_S1 : C::COL_S0) + hh * HALF_COLS;
             const uint64_t kh = kdesc + (uint64_t)((hh * HALF_COLS * 128) >> 4);   // keys 64 hh .. : rows of the K tile
 #pragma unroll
             for (int kk = 0; kk < D / 16; ++kk) {
@@ -677,7 +672,7 @@ fwd_tcgen05_kernel(const TcArgs args, const __grid_constant__ CUtensorMap tmap_q
         if (n_tiles == 0) continue;
         for (int j = 0; j < n_tiles; ++j) {
           const int gg = g + j;
-          const int s = gg % STAGES_V, t = gg % NS;
+          const int s = gg % STAGES_V, t = gg & 1;
           if (!mbar_wait(&bars->v_full[s], (gg / STAGES_V) & 1, abort_flag)) { ok = false; break; }
           // the first P.V product of an item overwrites O: the previous item's rows must be read out
           if (j == 0 && qi > 0 && !mbar_wait(&bars->o_free, (qi - 1) & 1, abort_flag)) { ok = false; break; }
@@ -686,9 +681,9 @@ fwd_tcgen05_kernel(const TcArgs args, const __grid_constant__ CUtensorMap tmap_q
           // their own: O_h += P_h V[64h .. 64h+64), issued as soon as that half's P is there.
           // P_h sits in the first 32 columns of the half's own 64 S columns.
           for (int hh = 0; hh < 2 && ok; ++hh) {
-            if (!mbar_wait(&bars->p_full[t][hh], (gg / NS) & 1, abort_flag)) { ok = false; break; }
+            if (!mbar_wait(&bars->p_full[t][hh], (gg >> 1) & 1, abort_flag)) { ok = false; break; }
             tc_fence_after_sync();
-            const uint32_t p_tmem = tmem + C::col_s(t) + hh * HALF_COLS;
+            const uint32_t p_tmem = tmem + (t ? C::COL_S1 : C::COL_S0) + hh * HALF_COLS;
             const uint32_t o_tmem = tmem + (hh ? C::COL_O1 : C::COL_O0);
 #pragma unroll
             for (int kk = 0; kk < HALF_COLS / 16; ++kk) {
@@ -742,11 +737,11 @@ fwd_tcgen05_kernel(const TcArgs args, const __grid_constant__ CUtensorMap tmap_q
 
       for (int j = 0; j < n_tiles; ++j) {
         const int gg = g + j;                       // the CTA's running key-tile count
-        const int t = gg % NS;
+        const int t = gg & 1;
         const int key0 = walk.key0(j);
-        if (!mbar_wait(&bars->s_full[t][SPLIT_S ? half : 0], (gg / NS) & 1, abort_flag)) { alive = false; break; }
+        if (!mbar_wait(&bars->s_full[t][SPLIT_S ? half : 0], (gg >> 1) & 1, abort_flag)) { alive = false; break; }
         tc_fence_after_sync();
-        const uint32_t s_tmem = tmem + lane_base + C::col_s(t);
+        const uint32_t s_tmem = tmem + lane_base + (t ? C::COL_S1 : C::COL_S0);
         const uint32_t o_tmem = tmem + lane_base + (half ? C::COL_O1 : C::COL_O0);
         uint32_t xr[HALF_COLS];   // fp32 bit patterns of this thread's raw scores
         tmem_ld32(s_tmem + half * HALF_COLS, &xr[0]);
@@ -826,7 +821,7 @@ fwd_tcgen05_kernel(const TcArgs args, const __grid_constant__ CUtensorMap tmap_q
           if (j > 0 && __any_sync(0xffffffffu, bump)) {
             // The accumulator is expressed relative to the old reference: rescale it in TMEM once
             // the previous P.V product has landed.
-            if (!mbar_wait(&bars->pv_done[(gg - 1) % NS][SPLIT_S ? half : 0], ((gg - 1) / NS) & 1, abort_flag)) { alive = false; break; }
+            if (!mbar_wait(&bars->pv_done[(gg - 1) & 1][SPLIT_S ? half : 0], ((gg - 1) >> 1) & 1, abort_flag)) { alive = false; break; }
             tc_fence_after_sync();
 #pragma unroll
             for (int c = 0; c < D / 32; ++c) {
@@ -899,8 +894,8 @@ fwd_tcgen05_kernel(const TcArgs args, const __grid_constant__ CUtensorMap tmap_q
       }
       if (n_tiles > 0) {
         const int gl = g + n_tiles - 1;
-        if (!mbar_wait(&bars->pv_done[gl % NS][0], (gl / NS) & 1, abort_flag) ||
-            (SPLIT_S && !mbar_wait(&bars->pv_done[gl % NS][1], (gl / NS) & 1, abort_flag))) { alive = false; break; }
+        if (!mbar_wait(&bars->pv_done[gl & 1][0], (gl >> 1) & 1, abort_flag) ||
+            (SPLIT_S && !mbar_wait(&bars->pv_done[gl & 1][1], (gl >> 1) & 1, abort_flag))) { alive = false; break; }
         tc_fence_after_sync();
       }
       float o[D / 2];

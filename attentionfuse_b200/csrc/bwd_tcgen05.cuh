@@ -6,12 +6,12 @@
 // group are summed inside the CTA that owns the key tile -- with the recompute on tensor cores:
 //
 //   MODE_DKV  one CTA owns 128 keys of one (batch, kv head): K_j, V_j stay in shared memory,
-//             64-row tiles of Q_i and dO_i stream through a TMA ring, for every query head of
-//             the group.  Scores are computed TRANSPOSED, S^T = K_j Q_i^T and dP^T = V_j dO_i^T
+//             tiles of Q_i and dO_i (BCfg::BT rows) stream through a TMA ring, for every query
+//             head of the group.  Scores are computed TRANSPOSED, S^T = K_j Q_i^T and dP^T = V_j dO_i^T
 //             (TMEM lane = key), so that P^T and dS^T, written back to TMEM as f16/bf16, are
 //             directly the A operands of  dV_j += P^T dO_i  and  dK_j += dS^T Q_i.
-//   MODE_DQ   one CTA owns 128 query rows of one (batch, query head): Q_i, dO_i stay, 64-key
-//             tiles of K_j, V_j stream;  S = Q_i K_j^T, dP = dO_i V_j^T (TMEM lane = query row),
+//   MODE_DQ   one CTA owns 128 query rows of one (batch, query head): Q_i, dO_i stay, tiles of
+//             K_j, V_j stream;  S = Q_i K_j^T, dP = dO_i V_j^T (TMEM lane = query row),
 //             dS goes back to TMEM and feeds  dQ_i += dS K_j.
 //
 // P = exp2(S*scale*log2e - L*log2e) with L the log-sum-exp saved by the forward;
@@ -27,11 +27,11 @@
 //             both to TMEM, next to P^T in the step's S^T columns, as the A operand of
 //             dK_j += dS^T Q_i, and to shared memory (128 keys x 64 queries, query-contiguous,
 //             128-byte swizzle) as the N-major B operand of  dQ_i^T = K_j^T dS^T  (A = the stationary K tile
-//             read M-major).  dQ_i^T (TMEM lane = d, column = query) is not kept: the element-wise
-//             threads read it back and add it to an fp32 (B, H_q, N_q, D) accumulator in global
+//             read M-major).  dQ_i^T (TMEM lane = d, column = query) is not kept: 128
+//             threads of their own read it back and add it to an fp32 (B, H_q, N_q, D) accumulator in global
 //             memory with red.global.add.f32 (32 lanes = 32 consecutive d = one 128-byte line);
 //             a small kernel afterwards applies the scale and the transpose of the rotation and
-//             rounds to the output type.  TMEM: S^T/P^T double-buffered, dP^T single (free again
+//             rounds to the output type.  TMEM: S^T/P^T/dS^T double-buffered, dP^T single (free again
 //             as soon as the element-wise threads have loaded it), dQ^T single, dV, dK = 512
 //             columns.  Summation order of dQ over key tiles depends on scheduling, so dQ is
 //             reproducible only to fp32 rounding; the two-pass kernels remain the deterministic

@@ -18,7 +18,7 @@
 // read 16 bytes at a time and products run on packed fp32 pairs (fma.rn.f32x2: even and odd d, or two
 // output columns).  [2,12,512,64] causal + RoPE + ALiBi, 0.82 GFLOP: 150 us with 4-byte reads and
 // scalar FMAs, 70 us with 16-byte reads (30 % of the issue slots: 1.9 warps per scheduler on average,
-// the longest CTA's eight tiles one after the other).
+// the longest CTA's eight tiles one after the other), 47 us with two groups and packed FMAs.
 #include "common.cuh"
 
 namespace af {

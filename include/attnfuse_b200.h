@@ -192,7 +192,10 @@ AF_API int af_fwd(const AfFwdParams* params, af_stream_t stream);
  * problems with many query tiles per KV head use scratch: K is then rotated once into it
  * instead of once per query tile.  Without (enough) workspace af_fwd rotates K inside the
  * kernel, in shared memory, and gives the same result.  No counterpart in the reference, whose
- * kernel always re-rotates each K tile (attnfuse/compiler/codegen.py:332-341).  Host only. */
+ * kernel always re-rotates each K tile (attnfuse/compiler/codegen.py:332-341).  Host only.
+ * It also asks for room for partials where a call with few query tiles and a long key axis
+ * (head_dim 128, lse NULL) deals the keys of a tile out to several CTAs; without it the rows are
+ * computed whole. */
 AF_API int64_t af_fwd_workspace_bytes(const AfFwdParams* params);
 
 /* Replaces the three launches of run_backward (attnfuse/runtime/backward.py:131-190:

@@ -188,7 +188,7 @@ typedef struct AfDecodeParams {
  * (attnfuse/runtime/block_mask.py:246-270). */
 AF_API int af_fwd(const AfFwdParams* params, af_stream_t stream);
 
-/* Scratch bytes with which af_fwd runs fastest for this problem (0: none needed).  Only RoPE
+/* Scratch bytes with which af_fwd runs fastest for this problem (0: none needed).  RoPE
  * problems with many query tiles per KV head use scratch: K is then rotated once into it
  * instead of once per query tile.  Without (enough) workspace af_fwd rotates K inside the
  * kernel, in shared memory, and gives the same result.  No counterpart in the reference, whose

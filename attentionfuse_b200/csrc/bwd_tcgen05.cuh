@@ -636,8 +636,12 @@ bwd_tcgen05_kernel(const BwdArgs args, const __grid_constant__ CUtensorMap map_a
         // Does any element of these 128 x 64 columns need masking?
         //   key-stationary: lane = key srow, column c = query c0 + c;  DQ: lane = query srow, column c = key c0 + c.
         const int c0 = r0 + col_first;
-        const int col_limit = (KVS ? p.N_q : p.N_kv) - c0;     // columns c < col_limit exist
-        bool need_mask = col_limit < COLS;
+        // Single pass: the lanes of the last key tile past N_kv see no column.  Their S^T is 0, so that
+        // P = exp(-L) can be anything up to inf, and dQ^T sums dS^T over all 128 lanes, where the zero
+        // K row does not cancel an inf.  (A causal mask drops them; the other modes only store rows that exist.)
+        constexpr bool DROP_KEYS = FUSED && EMASK != EMASK_CAUSAL;
+        const int col_limit = (DROP_KEYS && srow >= p.N_kv) ? 0 : (KVS ? p.N_q : p.N_kv) - c0;   // columns c < col_limit exist
+        bool need_mask = (KVS ? p.N_q : p.N_kv) - c0 < COLS || (DROP_KEYS && t0 + BS > p.N_kv);
         if (EMASK == EMASK_CAUSAL)
           need_mask = need_mask || (KVS ? (c0 < t0 + BS - 1) : (c0 + COLS - 1 > t0));
         if (EMASK == EMASK_WINDOW)

@@ -78,3 +78,36 @@ def test_rows_without_a_visible_key():
     assert (q.grad[:, :, 128:256] == 0).all() and (q.grad[:, :, 384:] == 0).all()
     assert_close(k.grad, dk, dtype, grad=True, what="dK with unseen rows")
     assert_close(v.grad, dv, dtype, grad=True, what="dV with unseen rows")
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("dtype,logit", [(torch.float16, -26.0), (torch.bfloat16, -126.0)])
+@pytest.mark.parametrize("mask,window", [("none", 0), ("window", 90), ("blocks", 0), ("causal", 0)])
+@pytest.mark.parametrize("N", [1, 130, 200, 257])
+def test_negative_logits_at_a_ragged_key_axis(N, mask, window, dtype, logit, D):
+    """Every logit is clearly negative, so that exp(-L) leaves the type: the lanes of the last key tile past
+    N_kv have S = 0 and must not reach dQ.  The mean of the logits sits in one column of Q and K, whose
+    gradients are sums of dS that cancel: rounding only, compared on the other columns."""
+    Q, K, V = qkv(8300 + N, 1, 4, 2, N, N, D, dtype)
+    side = (-logit * D ** 0.5) ** 0.5
+    Q[..., 0], K[..., 0] = side, -side
+    dO = orc.randn(8400 + N, Q.shape, dtype)
+    kw = dict(causal=mask == "causal", window=window or None)
+    if mask == "blocks":
+        nb = (N + 127) // 128
+        bm = af.BlockMask.from_dense(torch.ones(nb, nb, dtype=torch.bool), 128, 128, device=DEV)
+        fn = af.attention(lambda q, k, v: af.softmax(af.block_sparse(af.scaled_dot_product(q, k))) @ v)
+        q, k, v = (t.to(DEV).requires_grad_(True) for t in (Q, K, V))
+        fn(q, k, v, block_mask=bm).backward(dO.to(DEV))
+        got = q.grad, k.grad, v.grad
+    else:
+        got = grads(Q, K, V, dO, D ** -0.5, {"none": 0, "causal": 1, "window": 2}[mask], window)
+    _, *want = orc.attention_grads(Q, K, V, dO, **kw)
+    for name, g, w in zip(("dQ", "dK", "dV"), got, want):
+        assert torch.isfinite(g.float()).all(), name
+        if N == 1 and name != "dV":            # one key: P = 1, dQ = dK = 0 up to the rounding of O in delta
+            assert g[..., 1:].float().abs().max().item() < 2e-2
+        elif name == "dV":
+            assert_close(g, w, dtype, grad=True, what=f"negative logits {mask} N{N} D{D} dV")
+        else:
+            assert_close(g[..., 1:], w[..., 1:], dtype, grad=True, what=f"negative logits {mask} N{N} D{D} {name}")

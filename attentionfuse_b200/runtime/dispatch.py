@@ -118,17 +118,6 @@ def validate_qkv(Q, K, V):
 # (about 40 arguments through the Triton launcher: attnfuse/runtime/dispatch.py:196-214).
 _FWD_TEMPLATES: dict = {}
 _FWD_TEMPLATES_MAX = 256
-# Workspace of forward calls outside autograd (the rotated Q and K of a RoPE problem), kept per
-# (device, stream) and grown on demand: calls on one stream are ordered, so they can share it.
-_INFER_WORKSPACE: dict = {}
-
-
-def _inference_workspace(device, stream: int, need: int) -> torch.Tensor:
-    key = (device.index, stream)
-    ws = _INFER_WORKSPACE.get(key)
-    if ws is None or ws.numel() < need:
-        ws = _INFER_WORKSPACE[key] = torch.empty(need, dtype=torch.uint8, device=device)
-    return ws
 
 
 def launch_forward(Q, K, V, out, *, sm_scale, mask_kind, window=0, bias_kind=0, norm_kind=0,
@@ -178,15 +167,12 @@ def launch_forward(Q, K, V, out, *, sm_scale, mask_kind, window=0, bias_kind=0, 
             _FWD_TEMPLATES[key] = (_lib.AfFwdParams.from_buffer_copy(params), need)
     stream = _lib.current_stream(Q.device)
     if need > 0 and not in_kernel_rope:
+        # Allocated per call, never kept for the next one: the allocator's stream order covers its lifetime
+        # outside a capture, the graph's own pool inside one, and calls of several threads, whose
+        # launches (rotation, attention, merge) may interleave on one stream, have one each.
+        workspace = torch.empty(need, dtype=torch.uint8, device=Q.device)
         if keep_workspace is not None:
-            workspace = torch.empty(need, dtype=torch.uint8, device=Q.device)
             keep_workspace.append(workspace)
-        elif cos is None:
-            # partials of a problem whose keys are dealt out to several shares: the allocator's
-            # stream order (and a graph capture's own pool) covers their lifetime
-            workspace = torch.empty(need, dtype=torch.uint8, device=Q.device)
-        else:
-            workspace = _inference_workspace(Q.device, stream, need)
         params.workspace, params.workspace_bytes = workspace.data_ptr(), need
     with _lib.on_device(Q.device):
         rc = lib.af_fwd(C.byref(params), stream)

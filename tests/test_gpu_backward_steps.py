@@ -43,10 +43,10 @@ def test_step_edges(N, D, mask, window, deterministic, monkeypatch):
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("D", [64, 128])
-@pytest.mark.parametrize("scale", [1e-8, 1e-3, 1.0, 4.0])
+@pytest.mark.parametrize("scale", [1e-40, 1e-38, 1e-33, 1e-8, 1e-3, 1.0, 4.0])
 def test_scale_range(scale, D, dtype):
-    """L / scale from 1e9 (flat rows) down to a few (one-hot rows), where a term that was dropped
-    would show as a factor on every probability."""
+    """L / scale from beyond fp32 (scales whose reciprocal overflows) and 1e9 (flat rows) down to a few
+    (one-hot rows), where a term that was dropped would show as a factor on every probability."""
     N = 200
     Q, K, V = qkv(7700, 1, 2, 1, N, N, D, dtype)
     if scale >= 1.0:

@@ -140,11 +140,13 @@ int launch_bwd_mma(const AfBwdParams& a, cudaStream_t st) {
     ks[3] = 1; ks[2] = p.D; ks[1] = (int64_t)p.N_kv * p.D; ks[0] = ks[1] * p.H_kv;
   }
 
-  CUtensorMap k128, v128, q64, do64, q128, do128, k64, v64;
-  if ((rc = tc_make_map(&k128, p.dtype, k_ptr, p.B, p.H_kv, p.N_kv, p.D, ks, 128)) != AF_OK) return rc;
-  if ((rc = tc_make_map(&v128, p.dtype, p.v, p.B, p.H_kv, p.N_kv, p.D, p.v_stride, 128)) != AF_OK) return rc;
-  if ((rc = tc_make_map(&q64, p.dtype, q_ptr, p.B, p.H_q, p.N_q, p.D, qs, 64)) != AF_OK) return rc;
-  if ((rc = tc_make_map(&do64, p.dtype, a.d_o, p.B, p.H_q, p.N_q, p.D, a.do_stride, 64)) != AF_OK) return rc;
+  // boxes of 128 rows for the operands that stay, of a step's rows for those that stream
+  const int strm_rows = p.D == 64 ? tcb::BCfg<64>::BT : tcb::BCfg<128>::BT;
+  CUtensorMap k_stat, v_stat, q_strm, do_strm;
+  if ((rc = tc_make_map(&k_stat, p.dtype, k_ptr, p.B, p.H_kv, p.N_kv, p.D, ks, tcb::BS)) != AF_OK) return rc;
+  if ((rc = tc_make_map(&v_stat, p.dtype, p.v, p.B, p.H_kv, p.N_kv, p.D, p.v_stride, tcb::BS)) != AF_OK) return rc;
+  if ((rc = tc_make_map(&q_strm, p.dtype, q_ptr, p.B, p.H_q, p.N_q, p.D, qs, strm_rows)) != AF_OK) return rc;
+  if ((rc = tc_make_map(&do_strm, p.dtype, a.d_o, p.B, p.H_q, p.N_q, p.D, a.do_stride, strm_rows)) != AF_OK) return rc;
 
   const int64_t acc_bytes = bwd_mma_dq_accum_bytes(a);
   if (acc_bytes > 0 && a.dq_accum != nullptr && a.dq_accum_bytes >= acc_bytes && ((uintptr_t)a.dq_accum & 255) == 0) {
@@ -154,7 +156,7 @@ int launch_bwd_mma(const AfBwdParams& a, cudaStream_t st) {
     const bool blk = p.mask_kind == AF_MASK_BLOCKS;
     f.tiles = (p.N_kv + 127) / 128;
     f.stat_per_block = blk ? p.block_n / 128 : 1;
-    f.steps_per_block = blk ? p.block_m / 64 : 1;
+    f.steps_per_block = blk ? p.block_m / strm_rows : 1;
     const int64_t units = (int64_t)p.B * p.H_kv;
     AF_REQUIRE((int64_t)f.tiles * units <= 0x7fffffff - 1024, "too many tiles for one launch");
     f.total_items = (int)(f.tiles * units);
@@ -173,20 +175,23 @@ int launch_bwd_mma(const AfBwdParams& a, cudaStream_t st) {
     f.dq_acc = static_cast<float*>(a.dq_accum);
     f.sched_counter = reinterpret_cast<int32_t*>(static_cast<char*>(a.dq_accum) + align256(dq_accum_floats(p) * 4));
     AF_CUDA_OK(cudaMemsetAsync(a.dq_accum, 0, (size_t)acc_bytes, st));
-    if ((rc = tcb::launch_fused_d128(p.dtype, f, k128, v128, q64, do64, st)) != AF_OK) return rc;
+    if ((rc = tcb::launch_fused_d128(p.dtype, f, k_stat, v_stat, q_strm, do_strm, st)) != AF_OK) return rc;
     return p.dtype == AF_F16 ? launch_dq_finish<__half>(f.dq_acc, a, st) : launch_dq_finish<__nv_bfloat16>(f.dq_acc, a, st);
   }
-  if ((rc = tc_make_map(&q128, p.dtype, q_ptr, p.B, p.H_q, p.N_q, p.D, qs, 128)) != AF_OK) return rc;
-  if ((rc = tc_make_map(&do128, p.dtype, a.d_o, p.B, p.H_q, p.N_q, p.D, a.do_stride, 128)) != AF_OK) return rc;
-  if ((rc = tc_make_map(&k64, p.dtype, k_ptr, p.B, p.H_kv, p.N_kv, p.D, ks, 64)) != AF_OK) return rc;
-  if ((rc = tc_make_map(&v64, p.dtype, p.v, p.B, p.H_kv, p.N_kv, p.D, p.v_stride, 64)) != AF_OK) return rc;
+  // the dQ pass keeps what streamed and streams what stayed: the same maps where a step has 128 rows
+  CUtensorMap q_stat = q_strm, do_stat = do_strm, k_strm = k_stat, v_strm = v_stat;
+  if (strm_rows != tcb::BS) {
+    if ((rc = tc_make_map(&q_stat, p.dtype, q_ptr, p.B, p.H_q, p.N_q, p.D, qs, tcb::BS)) != AF_OK) return rc;
+    if ((rc = tc_make_map(&do_stat, p.dtype, a.d_o, p.B, p.H_q, p.N_q, p.D, a.do_stride, tcb::BS)) != AF_OK) return rc;
+    if ((rc = tc_make_map(&k_strm, p.dtype, k_ptr, p.B, p.H_kv, p.N_kv, p.D, ks, strm_rows)) != AF_OK) return rc;
+    if ((rc = tc_make_map(&v_strm, p.dtype, p.v, p.B, p.H_kv, p.N_kv, p.D, p.v_stride, strm_rows)) != AF_OK) return rc;
+  }
 
   const bool blocks = p.mask_kind == AF_MASK_BLOCKS;
   tcb::BwdArgs dkv{};
   dkv.a = a;
   dkv.tiles = (p.N_kv + 127) / 128;
   dkv.stat_per_block = blocks ? p.block_n / 128 : 1;
-  const int strm_rows = p.D == 64 ? tcb::BCfg<64>::BT : tcb::BCfg<128>::BT;
   dkv.steps_per_block = blocks ? p.block_m / strm_rows : 1;
   tcb::BwdArgs dq{};
   dq.a = a;
@@ -211,12 +216,11 @@ int launch_bwd_mma(const AfBwdParams& a, cudaStream_t st) {
   }
 
   if (p.D == 64) {
-    // streamed tiles of 128 rows too
-    if ((rc = tcb::launch_dkv_d64(p.dtype, dkv, k128, v128, q128, do128, st)) != AF_OK) return rc;
-    return tcb::launch_dq_d64(p.dtype, dq, q128, do128, k128, v128, st);
+    if ((rc = tcb::launch_dkv_d64(p.dtype, dkv, k_stat, v_stat, q_strm, do_strm, st)) != AF_OK) return rc;
+    return tcb::launch_dq_d64(p.dtype, dq, q_stat, do_stat, k_strm, v_strm, st);
   }
-  if ((rc = tcb::launch_dkv_d128(p.dtype, dkv, k128, v128, q64, do64, st)) != AF_OK) return rc;
-  return tcb::launch_dq_d128(p.dtype, dq, q128, do128, k64, v64, st);
+  if ((rc = tcb::launch_dkv_d128(p.dtype, dkv, k_stat, v_stat, q_strm, do_strm, st)) != AF_OK) return rc;
+  return tcb::launch_dq_d128(p.dtype, dq, q_stat, do_stat, k_strm, v_strm, st);
 }
 
 }  // namespace af

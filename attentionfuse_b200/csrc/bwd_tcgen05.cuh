@@ -82,11 +82,11 @@ template <int D, int MODE = MODE_DKV> struct BCfg {
   static constexpr int STRM_PANEL = BT * 128;
   static constexpr int STRM_TILE = PANELS * STRM_PANEL;
   // Key-stationary modes: -L / scale and -delta of the streamed query rows enter S^T and dP^T as one more
-  // 16-wide product step, ones(128 x 16) * stats(64 x 16)^T, each value as three bf16 terms (24 bits,
+  // 16-wide product step, ones(128 x 16) * stats(BT x 16)^T, each value as three bf16 terms (24 bits,
   // fp32's range; the operands of that one product are bf16 whatever T is).  As shared-memory loads
   // of the element-wise threads -- every lane needs both numbers of every column -- they took 64 KB
   // of the 304 KB a fused step moves through the shared-memory port, which bounds it; the product
-  // steps read 12 KB.  A tile of 64 rows x 128 bytes holds the steps of two ring stages: 32 bytes
+  // steps read 12 KB (BT = 64).  A tile of BT rows x 128 bytes holds the steps of two ring stages: 32 bytes
   // of L terms and 32 bytes of delta terms each.
   static constexpr bool KEY_STAT = MODE != MODE_DQ;
   static constexpr int ONES_BYTES = KEY_STAT ? BS * 128 : 0;

@@ -751,8 +751,9 @@ __global__ void decode_combine_kernel(const AfDecodeParams a, const int head_chu
     unit_start = before + (int64_t)uu * tiles_u;
   }
   const PartialRows pr = partial_rows(a, head_chunks, row, T_all, unit_start, tiles_u, unit);
-  // everything above depends on the call's inputs alone; the partials are there once the grid before
-  // this one is over
+  // Everything above reads kv_lens and q_positions, which were final before the split grid started (the header
+  // says so to callers that put a kernel of their own in between); the partials are there once the
+  // grid before this one is over.
   asm volatile("griddepcontrol.wait;" ::: "memory");
   float acc[VEC], lse;
   merge_partials<D>(a, pr, lane, acc, lse);

@@ -218,7 +218,12 @@ AF_API int64_t af_bwd_dq_accum_bytes(const AfBwdParams* params);
 AF_API int af_decode_split(const AfDecodeParams* params, af_stream_t stream);
 
 /* Replaces the combine launch of run_flash_decode (attnfuse/runtime/flash_decode.py:173-186).
- * Writes o (if non-NULL) and partial (if non-NULL). */
+ * Writes o (if non-NULL) and partial (if non-NULL).  It is set up while the grid ahead of it in the
+ * stream drains (programmatic stream serialization) and reads kv_lens and q_positions then; only the
+ * partials (ws_m, ws_l, ws_acc) are read after that grid's end.  Behind af_decode_split, which reads the
+ * same two arrays, nothing follows from that.  A caller that puts a kernel of its own between the two, or
+ * makes the partials itself, and lets that kernel trigger its dependents early
+ * (griddepcontrol.launch_dependents) must have both arrays final before that kernel starts. */
 AF_API int af_decode_combine(const AfDecodeParams* params, af_stream_t stream);
 
 /* Decode (split + combine) for callers that cannot allocate device memory.  No counterpart in

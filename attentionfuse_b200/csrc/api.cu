@@ -84,6 +84,17 @@ int64_t af_fwd_workspace_bytes(const AfFwdParams* params) {
   return fwd_tcgen05_workspace_bytes(a);
 }
 
+int af_fwd_layout(const AfFwdParams* params, int32_t sm_count, int32_t* heads_per_cta, int32_t* key_shares) {
+  if (params == nullptr || heads_per_cta == nullptr || key_shares == nullptr) return fail(AF_ERR_INVALID, "NULL argument");
+  const AfFwdParams& a = *params;
+  const int rc = validate_problem(a.p);
+  if (rc != AF_OK) return rc;
+  const char* why = "the exact kernels were asked for";
+  if (a.p.family == AF_FAMILY_FFMA || !fwd_tcgen05_supports(a.p, a.o, a.o_stride, &why))
+    return fail(AF_ERR_UNSUPPORTED, "tcgen05 forward: %s", why);
+  return fwd_tcgen05_layout(a, sm_count, heads_per_cta, key_shares);
+}
+
 int af_bwd(const AfBwdParams* params, af_stream_t stream) {
   if (params == nullptr) return fail(AF_ERR_INVALID, "params is NULL");
   const AfBwdParams& a = *params;

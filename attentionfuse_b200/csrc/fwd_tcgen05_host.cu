@@ -1,6 +1,8 @@
 // Host side of the tcgen05 forward: support predicate, TMA descriptor encoding, RoPE mode
 // selection (fused in shared memory vs. a one-off K pre-rotation into caller workspace) and
 // dispatch to the per-(head_dim, RoPE mode) instantiation units.
+#include <algorithm>
+#include <array>
 #include <cstdlib>
 #include <mutex>
 
@@ -341,59 +343,112 @@ static void set_item_order(tc::TcArgs& args, int units, int unit_chunk, int rows
 }
 
 // The two-heads-per-CTA schedule (fwd_pair_tcgen05.cuh): head dim 128, an even number of query
-// heads per KV head, element masks only, operands already rotated.  ATTNFUSE_FWD_PAIR in the
-// environment (read at every call) keeps to the one-head schedule (0) or to this one wherever it
-// exists (1), for comparisons between the two.
+// heads per KV head, element masks only, operands already rotated.
 static bool pair_schedule_exists(const AfProblem& p, int rope_mode) {
   if (p.D != 128 || rope_mode != tc::ROPE_NONE || p.mask_kind == AF_MASK_BLOCKS) return false;
   return p.H_kv >= 1 && p.H_q % p.H_kv == 0 && ((p.H_q / p.H_kv) & 1) == 0;
 }
 
-// How a forward problem is laid over the SMs: one or two heads per CTA, and the number of shares the
+// (batch, head) units per chunk of the item order; heads = query heads of a unit (1 or 2).
+static int unit_chunk(const AfProblem& p, int heads) {
+  const int units = p.B * p.H_q / heads, group_units = p.H_q / p.H_kv / heads;
+  return choose_unit_chunk(units, group_units, 2.0 * 2.0 * (double)p.N_kv * p.D / group_units);
+}
+
+// How a forward problem is laid over the SMs: one or two query heads per CTA, and the number of shares the
 // keys of a query tile are dealt out to.
 struct FwdPlan { bool pair; int shares; };
 
-// Longest chain of work on one SM, in key tiles of the one-head schedule (about 1800 cycles), for each layout, and the shortest wins.  An item costs its key tiles plus about
-// two tiles at its boundary; two heads per CTA do a tile of both in 1.95 tiles but halve the number of
-// items, which leaves SMs without work when there are few: 500 rows against 8011 keys, 32 heads,
-// are 64 pair items (0.121 ms) or 128 one-head items (0.074 ms) on 148 SMs.  Shares cost the partials' way
-// through memory and the merge launch, about six tiles.  They exist at head dim 128, for calls that keep no
-// log-sum-exp: an autograd forward holds its workspace until the backward.
-static FwdPlan plan_forward(const AfFwdParams& a, int rope_mode, int sms) {
-  const AfProblem& p = a.p;
-  FwdPlan best{false, 1};
+// Load of the SM that gets the most when the items -- one per unit and row of query tiles, row i in visiting
+// order costs cost[i] -- are dealt out as get_item and split_item do: chunk after chunk of units,
+// rows slowest within a chunk (reversed in odd ones), in zig-zag rounds over the CTAs.
+constexpr int kMaxPlanSms = 256;
+static float heaviest_sm(const float* cost, int rows, int units, int chunk, int sms) {
+  const int64_t items = (int64_t)rows * units;
+  const int G = (int)(items < sms ? items : sms);
+  float load[kMaxPlanSms] = {};
+  int at = 0, dir = 1;
+  for (int c = 0; c * chunk < units; ++c)
+    for (int i = 0; i < rows; ++i) {
+      const float x = cost[(c & 1) ? rows - 1 - i : i];
+      for (int u = 0; u < chunk; ++u) {
+        load[at] += x;
+        at += dir;
+        if (at == G) { at = G - 1; dir = -1; }
+        else if (at < 0) { at = 0; dir = 1; }
+      }
+    }
+  return *std::max_element(load, load + G);
+}
+
+// Megabytes of partials of a problem in `shares` shares (accumulators; m and l are a hundredth of them).
+static double partial_mb(const AfProblem& p, int shares) { return 4e-6 * shares * p.B * p.H_q * p.N_q * p.D; }
+
+// The layout whose heaviest SM is done first, in key tiles of the one-head schedule (0.86 us).  Measured over 161
+// problems (square causal, window and dense of 512 - 4096 rows, chunks of 16 - 1024 rows against 1k - 16k
+// keys; 1 - 4 sequences, 8 - 64 heads):
+//  * one head per CTA: an item costs its tiles and two at its boundary; two heads: a tile of both costs 2.0 and
+//    the boundary 2.5.  One head has to win by 3 % (near a tie the two-head schedule draws less power, which
+//    counts once every SM is busy: 541 against 581 us at [4,32/8,4096] causal).  The times of the layout
+//    so chosen are 0.04 % above the faster one's on average, 2.4 % at most; a rule on the mean tiles
+//    per item lost up to 19 % ([1,64/8,3584] causal: 183 us with two heads, 215 with one).  Two heads
+//    halve the number of items, which is what few query tiles cannot afford: 500 rows against 8011 keys,
+//    32 heads: 118 us as 64 items, 63 us as 128.  From eight rounds of pair items on the deal is even.
+//  * shares of the keys (head dim 128): the partials' way through memory and the merge launch cost 4 tiles and
+//    0.45 per MB of partials (1 MB: 3 - 6 tiles; 8 MB: 7 - 8; 38 MB: 21), and have to win by 5 %.  32 heads, us with /
+//    without: 64 rows x 2048 keys 14 / 20, x 8011 25 / 61, x 16384 40 / 118; 250 x 8011 42 / 62.  Calls that
+//    keep a log-sum-exp have none: an autograd forward holds its workspace until the backward.
+// ATTNFUSE_FWD_PAIR in the environment (read at every call) fixes the layout to what depends on head_dim, group, mask
+// and rotation alone: two heads per CTA wherever that exists (1), or one (0), and no shares.
+constexpr int kPairRounds = 8, kShareRounds = 4;
+static FwdPlan plan_forward(const AfProblem& p, bool has_lse, int rope_mode, int sms, bool room_for_shares) {
   const bool pair_ok = pair_schedule_exists(p, rope_mode);
-  const char* e = std::getenv("ATTNFUSE_FWD_PAIR");
-  if (pair_ok && e != nullptr && e[0] == '1') return FwdPlan{true, 1};
-  if (p.mask_kind == AF_MASK_BLOCKS || sms < 1) return best;
-  const int m_blocks = (p.N_q + tc::BM - 1) / tc::BM;
-  const int64_t items = (int64_t)m_blocks * p.B * p.H_q;
-  const bool shares_ok = p.D == 128 && rope_mode == tc::ROPE_NONE && a.lse == nullptr && items < 2 * (int64_t)sms;
-  if (!pair_ok && !shares_ok) return best;                 // nothing to choose from
-  int64_t sum = 0;
+  if (const char* e = std::getenv("ATTNFUSE_FWD_PAIR"))
+    if (e[0] == '0' || e[0] == '1') return FwdPlan{pair_ok && e[0] == '1', 1};
+  if (p.mask_kind == AF_MASK_BLOCKS || p.N_q < 1 || sms < 1 || sms > kMaxPlanSms) return FwdPlan{pair_ok, 1};
+  const int m_blocks = (p.N_q + tc::BM - 1) / tc::BM, heads = p.B * p.H_q;
+  const int64_t items = (int64_t)m_blocks * heads;
+  const bool shares_ok = room_for_shares && p.D == 128 && rope_mode == tc::ROPE_NONE && !has_lse && items < 2 * (int64_t)sms;
+  if (!pair_ok && !shares_ok) return FwdPlan{false, 1};    // nothing to choose from
+  if (pair_ok && items / 2 >= kPairRounds * (int64_t)sms) return FwdPlan{true, 1};
+
+  // A program lays the same problem out once per layer: the last few are remembered (plain values, per thread).
+  const int chunk1 = unit_chunk(p, 1), chunk2 = pair_ok ? unit_chunk(p, 2) : 0;
+  const std::array<int, 12> key{p.mask_kind, p.window, p.N_q, p.N_kv, p.q_offset, p.B, p.H_q, p.H_kv, sms, chunk1, chunk2, shares_ok};
+  struct Known { std::array<int, 12> key; FwdPlan plan; };
+  static thread_local std::array<Known, 4> known{};
+  static thread_local unsigned next = 0;
+  for (const Known& k : known)
+    if (k.key == key && k.plan.shares > 0) return k.plan;
+
+  float tiles[kPairRounds * 2 * kMaxPlanSms], cost[kPairRounds * 2 * kMaxPlanSms];   // one per row of items, fewer than items
   int longest = 0;
-  for (int m = 0; m < m_blocks; ++m) {
+  for (int i = 0; i < m_blocks; ++i) {
     int first, n;
-    tc::tile_range(p, m, first, n);
-    sum += n;
+    tc::tile_range(p, p.mask_kind == AF_MASK_CAUSAL ? m_blocks - 1 - i : i, first, n);
+    tiles[i] = (float)n;
     longest = n > longest ? n : longest;
   }
-  const double mean = (double)sum / m_blocks;
-  auto chain = [&](int64_t n_items, double tiles_per_item, double tiles_longest, double boundary) {
-    const double dealt = (double)((n_items + sms - 1) / sms) * (tiles_per_item + boundary);
-    return dealt > tiles_longest + boundary ? dealt : tiles_longest + boundary;
+  auto rows_cost = [&](float per_tile, float boundary) {
+    for (int i = 0; i < m_blocks; ++i) cost[i] = per_tile * tiles[i] + boundary;
   };
-  double best_cost = chain(items, mean, longest, 2.0);
-  if (pair_ok && !(e != nullptr && e[0] == '0')) {
-    const double c = chain(items / 2, 1.95 * mean, 1.95 * longest, 2.5);
-    if (c <= best_cost) { best_cost = c; best.pair = true; }
+  rows_cost(1.f, 2.f);
+  FwdPlan best{false, 1};
+  double best_cost = heaviest_sm(cost, m_blocks, heads, chunk1, sms);
+  if (pair_ok) {
+    rows_cost(2.f, 2.5f);
+    const double c = heaviest_sm(cost, m_blocks, heads / 2, chunk2, sms);
+    if (0.97 * c <= best_cost) { best.pair = true; best_cost = c; }
   }
   if (shares_ok) {
-    for (int s = 2; s <= 16 && longest >= 4 * s; ++s) {
-      const double c = chain(items * s, mean / s, (double)(longest + s - 1) / s, 2.0) + 6.0;
-      if (c < 0.95 * best_cost) { best_cost = c; best = FwdPlan{false, s}; }
+    for (int s = 2; s <= 16 && longest >= 4 * s && items * s <= kShareRounds * (int64_t)sms; ++s) {
+      for (int i = 0; i < m_blocks; ++i)
+        for (int j = 0; j < s; ++j) cost[i * s + j] = (float)((j + 1) * (int)tiles[i] / s - j * (int)tiles[i] / s) + 2.f;
+      const double c = heaviest_sm(cost, m_blocks * s, heads, chunk1, sms) + 4.0 + 0.45 * partial_mb(p, s);
+      if (c < 0.95 * best_cost) { best = FwdPlan{false, s}; best_cost = c / 0.95; }
     }
   }
+  known[next++ % known.size()] = Known{key, best};
   return best;
 }
 
@@ -409,8 +464,36 @@ int64_t fwd_tcgen05_workspace_bytes(const AfFwdParams& a) {
   const int64_t rotated = rope_workspace_bytes(a.p);
   const int mode = (a.p.rope && rotated == 0) ? tc::ROPE_FUSED : tc::ROPE_NONE;
   int sms = 0;
-  if (a.p.N_q < 1 || tc_sm_count(&sms) != AF_OK) return rotated;
-  return rotated + share_workspace_bytes(a.p, plan_forward(a, mode, sms).shares);
+  if (tc_sm_count(&sms) != AF_OK) return rotated;
+  return rotated + share_workspace_bytes(a.p, plan_forward(a.p, a.lse != nullptr, mode, sms, true).shares);
+}
+
+// The layout of a call with the workspace that it has, whether Q and K are rotated up front, and the bytes
+// of that workspace in front of the partials.
+struct FwdSetup { FwdPlan plan; bool rotate; int64_t rotated_bytes; };
+static FwdSetup set_up(const AfFwdParams& a, int sms) {
+  const AfProblem& p = a.p;
+  const bool usable = a.workspace != nullptr && ((uintptr_t)a.workspace & 255) == 0;
+  const int64_t need = rope_workspace_bytes(p);
+  FwdSetup s;
+  s.rotate = p.rope && need > 0 && usable && a.workspace_bytes >= need;
+  s.rotated_bytes = s.rotate ? need : 0;
+  const int mode = p.rope && !s.rotate ? tc::ROPE_FUSED : tc::ROPE_NONE;
+  s.plan = plan_forward(p, a.lse != nullptr, mode, sms, true);
+  if (s.plan.shares > 1 && (!usable || a.workspace_bytes < s.rotated_bytes + share_workspace_bytes(p, s.plan.shares)))
+    s.plan.shares = 1;                                     // no room for partials: whole rows per item
+  return s;
+}
+
+int fwd_tcgen05_layout(const AfFwdParams& a, int sms, int* heads_per_cta, int* key_shares) {
+  if (sms <= 0) {
+    const int rc = tc_sm_count(&sms);
+    if (rc != AF_OK) return rc;
+  }
+  const FwdPlan plan = set_up(a, sms).plan;
+  *heads_per_cta = plan.pair ? 2 : 1;
+  *key_shares = plan.shares;
+  return AF_OK;
 }
 
 int launch_fwd_tcgen05(const AfFwdParams& a, cudaStream_t st) {
@@ -427,13 +510,11 @@ int launch_fwd_tcgen05(const AfFwdParams& a, cudaStream_t st) {
   args.total_items = args.num_m_blocks * p.B * p.H_q;
   args.div_hq = tc::FastDiv::make((uint32_t)p.H_q);
   args.div_group = tc::FastDiv::make((uint32_t)(p.H_q / p.H_kv));
-  {
-    const int group = p.H_q / p.H_kv;
-    const double kv_bytes = 2.0 * 2.0 * (double)p.N_kv * p.D / group;   // K and V of a query head's share
-    set_item_order(args, p.B * p.H_q, choose_unit_chunk(p.B * p.H_q, group, kv_bytes), args.num_m_blocks);
-  }
+  set_item_order(args, p.B * p.H_q, unit_chunk(p, 1), args.num_m_blocks);
   int sms = 0;
   { const int rc_sm = tc_sm_count(&sms); if (rc_sm != AF_OK) return rc_sm; }
+  const FwdSetup setup = set_up(a, sms);
+  const FwdPlan& plan = setup.plan;
   auto set_grid = [&]() { args.grid_ctas = (sms > 0 && sms < args.total_items) ? sms : args.total_items; };
   args.key_shares = 1;
   {
@@ -448,9 +529,7 @@ int launch_fwd_tcgen05(const AfFwdParams& a, cudaStream_t st) {
   const void* k_ptr = p.k;
   int64_t q_stride[4] = {p.q_stride[0], p.q_stride[1], p.q_stride[2], p.q_stride[3]};
   int64_t k_stride[4] = {p.k_stride[0], p.k_stride[1], p.k_stride[2], p.k_stride[3]};
-  const int64_t need = rope_workspace_bytes(p);
-  if (p.rope && need > 0 && a.workspace != nullptr && a.workspace_bytes >= need &&
-      ((uintptr_t)a.workspace & 255) == 0) {
+  if (setup.rotate) {
     void* q_rot = a.workspace;
     void* k_rot = static_cast<char*>(a.workspace) + align256((int64_t)p.B * p.H_q * p.N_q * p.D * 2);
     const int rc = tc_launch_prepass(p, q_rot, k_rot, st);
@@ -468,31 +547,19 @@ int launch_fwd_tcgen05(const AfFwdParams& a, cudaStream_t st) {
   if ((rc = make_map(&mv, p.dtype, p.v, p.B, p.H_kv, p.N_kv, p.D, p.v_stride)) != AF_OK) return rc;
   // output rows leave through a TMA store: one box = the 32 rows of a warp x half of the head dim
   if ((rc = make_map(&mo, p.dtype, a.o, p.B, p.H_q, p.N_q, p.D, a.o_stride, 32, p.D / 2)) != AF_OK) return rc;
-  FwdPlan plan = plan_forward(a, mode, sms);
-  if (plan.shares > 1) {
-    const int64_t rotated = p.rope && mode == tc::ROPE_NONE ? need : 0;
-    if (a.workspace == nullptr || ((uintptr_t)a.workspace & 255) != 0 ||
-        a.workspace_bytes < rotated + share_workspace_bytes(p, plan.shares))
-      plan.shares = 1;                                     // no room for partials: whole rows per item
-    else
-      args.ws_m = reinterpret_cast<float*>(static_cast<char*>(a.workspace) + rotated);
-  }
   if (plan.pair) {
     // two query heads of a KV group per CTA: one K / V load feeds two S products
     const int pairs = p.H_q / 2;
     args.total_items = args.num_m_blocks * p.B * pairs;
     args.div_hq = tc::FastDiv::make((uint32_t)pairs);
     args.div_group = tc::FastDiv::make((uint32_t)(p.H_q / p.H_kv / 2));
-    {
-      const int group_pairs = p.H_q / p.H_kv / 2;
-      const double kv_bytes = 2.0 * 2.0 * (double)p.N_kv * p.D / group_pairs;
-      set_item_order(args, p.B * pairs, choose_unit_chunk(p.B * pairs, group_pairs, kv_bytes), args.num_m_blocks);
-    }
+    set_item_order(args, p.B * pairs, unit_chunk(p, 2), args.num_m_blocks);
     set_grid();
     return tc::launch_pair_d128(p.dtype, args, mq, mk, mv, mo, st);
   }
   if (plan.shares > 1) {
     const int64_t rows = (int64_t)plan.shares * p.B * p.H_q * p.N_q;
+    args.ws_m = reinterpret_cast<float*>(static_cast<char*>(a.workspace) + setup.rotated_bytes);
     args.ws_l = args.ws_m + align256(rows * 4) / 4;
     args.ws_acc = args.ws_l + align256(rows * 4) / 4;
     args.key_shares = plan.shares;

@@ -96,7 +96,7 @@ class AfPeerExchange(C.Structure):
                 ("wait_cycles", I64)]
 
 
-EXPORTS = ("af_fwd", "af_fwd_workspace_bytes", "af_bwd", "af_bwd_workspace_bytes", "af_bwd_dq_accum_bytes", "af_decode_split", "af_decode_combine", "af_decode_static", "af_decode_exchange_bytes", "af_decode_combine_push", "af_decode_wait_merge", "af_decode_sharded_step",
+EXPORTS = ("af_fwd", "af_fwd_workspace_bytes", "af_fwd_layout", "af_bwd", "af_bwd_workspace_bytes", "af_bwd_dq_accum_bytes", "af_decode_split", "af_decode_combine", "af_decode_static", "af_decode_exchange_bytes", "af_decode_combine_push", "af_decode_wait_merge", "af_decode_sharded_step",
            "af_decode_combine_gathered", "af_decode_num_splits", "af_query_family",
            "af_launch_count", "af_last_error", "af_abi_version")
 
@@ -124,6 +124,8 @@ def load() -> C.CDLL:
         lib.af_fwd.argtypes = [C.POINTER(AfFwdParams), PTR]
         lib.af_fwd_workspace_bytes.argtypes = [C.POINTER(AfFwdParams)]
         lib.af_fwd_workspace_bytes.restype = I64
+        lib.af_fwd_layout.argtypes = [C.POINTER(AfFwdParams), I32, C.POINTER(I32), C.POINTER(I32)]
+        lib.af_fwd_layout.restype = I32
         lib.af_bwd.argtypes = [C.POINTER(AfBwdParams), PTR]
         lib.af_bwd_workspace_bytes.argtypes = [C.POINTER(AfBwdParams)]
         lib.af_bwd_workspace_bytes.restype = I64

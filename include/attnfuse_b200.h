@@ -198,6 +198,18 @@ AF_API int af_fwd(const AfFwdParams* params, af_stream_t stream);
  * computed whole. */
 AF_API int64_t af_fwd_workspace_bytes(const AfFwdParams* params);
 
+/* How af_fwd lays this tensor-core problem over sm_count multiprocessors (<= 0: those of the current
+ * device) with the workspace that params carries: query heads per CTA (1 or 2) and shares that the keys
+ * of a query tile are dealt out to (1: none).  Host only, reads no operand.  At head_dim 64 this
+ * is always 1 and 1.  At head_dim 128 it follows from the whole call: batch, heads, query and key
+ * lengths, mask, lse, workspace and the GPU's multiprocessor count.  Layouts add the same terms in
+ * another order, so a row's last bits depend on the call that it is part of: alone, in a
+ * batch, on a shard of the heads or with a log-sum-exp it may differ by the rounding of the output
+ * type.  Calls of one layout give the same bits.  ATTNFUSE_FWD_PAIR=1 or 0 in the
+ * environment keeps to one layout per (head_dim, group, mask, rotation up front or not): two heads per CTA where the
+ * group is even and the mask no block list, or one, and no shares. */
+AF_API int32_t af_fwd_layout(const AfFwdParams* params, int32_t sm_count, int32_t* heads_per_cta, int32_t* key_shares);
+
 /* Replaces the three launches of run_backward (attnfuse/runtime/backward.py:131-190:
  * preproc, dK/dV, dQ) and of run_block_sparse_backward
  * (attnfuse/runtime/block_mask.py:302-362).  dq/dk/dv are fully overwritten. */

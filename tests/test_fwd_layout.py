@@ -1,0 +1,97 @@
+"""How the head-dim-128 forward is laid over the SMs (af_fwd_layout; host only): one or two query heads per
+CTA, shares of the keys.  Expected are the layouts that ran faster on a 148-SM B200."""
+import ctypes as C
+
+import pytest
+
+from attentionfuse_b200.runtime import _lib
+
+MASKS = {"none": 0, "causal": 1, "window": 2}
+SMS = 148
+
+
+def problem(B, H_q, H_kv, N_q, N_kv, mask, lse=False, workspace=True, window=256):
+    a = _lib.AfFwdParams()
+    p = a.p
+    p.dtype, p.B, p.H_q, p.H_kv, p.N_q, p.N_kv, p.D = _lib.AF_BF16, B, H_q, H_kv, N_q, N_kv, 128
+    p.sm_scale, p.mask_kind, p.window, p.q_offset = 128 ** -0.5, MASKS[mask], window, N_kv - N_q
+    base = 1 << 20                                     # never read: the layout is a matter of sizes
+    for name, heads, rows in (("q", H_q, N_q), ("k", H_kv, N_kv), ("v", H_kv, N_kv)):
+        setattr(p, name, base)
+        setattr(p, name + "_stride", (C.c_int64 * 4)(heads * rows * 128, rows * 128, 128, 1))
+    a.o, a.o_stride = base, (C.c_int64 * 4)(H_q * N_q * 128, N_q * 128, 128, 1)
+    if lse:
+        a.lse = base
+    if workspace:
+        a.workspace, a.workspace_bytes = base, 1 << 40
+    return a
+
+
+def layout(*shape, sms=SMS, **kw):
+    heads, shares = C.c_int32(), C.c_int32()
+    a = problem(*shape, **kw)
+    assert _lib.load().af_fwd_layout(C.byref(a), sms, C.byref(heads), C.byref(shares)) == 0, _lib.last_error()
+    return heads.value, shares.value
+
+
+# (B, H_q, H_kv, N_q, N_kv, mask): us with two heads per CTA, with one (whole rows), at least 4 % apart
+MEASURED = [
+    ((1, 32, 8, 512, 512, "causal"), 14.8, 10.7), ((1, 32, 8, 1024, 1024, "causal"), 23.0, 17.9),
+    ((1, 32, 8, 2432, 2432, "causal"), 50.7, 52.9), ((1, 64, 8, 2048, 2048, "causal"), 72.1, 74.9),
+    ((1, 64, 8, 3584, 3584, "causal"), 182.8, 214.9), ((1, 8, 2, 4096, 4096, "causal"), 64.7, 35.5),
+    ((2, 32, 8, 768, 768, "causal"), 19.9, 21.1), ((2, 32, 8, 2432, 2432, "causal"), 93.3, 99.4),
+    ((2, 32, 8, 3072, 3072, "causal"), 144.6, 156.3), ((2, 32, 8, 3584, 3584, "causal"), 183.2, 194.0),
+    ((2, 64, 8, 3584, 3584, "causal"), 364.0, 412.1), ((2, 8, 2, 3072, 3072, "causal"), 51.2, 43.8),
+    ((4, 32, 8, 3072, 3072, "causal"), 290.7, 312.0), ((4, 32, 8, 4096, 4096, "causal"), 541.2, 581.2),
+    ((4, 64, 8, 1536, 1536, "causal"), 158.6, 177.0), ((4, 8, 2, 512, 512, "causal"), 17.6, 12.7),
+    ((4, 8, 2, 4096, 4096, "causal"), 123.1, 128.9), ((1, 32, 8, 2432, 2432, "window"), 38.1, 42.9),
+    ((1, 32, 8, 2432, 2432, "none"), 112.9, 97.3), ((1, 32, 8, 4096, 4096, "none"), 248.1, 227.9),
+    ((2, 32, 8, 2048, 2048, "none"), 131.5, 118.9), ((2, 32, 8, 4096, 4096, "none"), 435.1, 510.9),
+    ((1, 32, 8, 500, 8011, "causal"), 117.6, 63.0), ((1, 32, 8, 768, 4096, "causal"), 64.4, 59.5),
+    ((1, 32, 8, 1024, 8011, "causal"), 124.0, 118.0), ((2, 32, 8, 500, 4096, "causal"), 66.1, 72.6),
+    ((2, 32, 8, 768, 8011, "causal"), 221.4, 178.0), ((2, 32, 8, 1024, 8011, "causal"), 231.6, 254.5),
+]
+
+
+@pytest.mark.parametrize("shape,two,one", MEASURED, ids=lambda x: "x".join(map(str, x)) if isinstance(x, tuple) else str(x))
+def test_whole_rows_take_the_layout_that_ran_faster(shape, two, one):
+    heads, shares = layout(*shape, lse=True)            # calls that keep a log-sum-exp have no shares
+    assert shares == 1
+    assert heads == (2 if two < one else 1)
+
+
+# the same, and us in the shares that the layout has: whole rows of one or two heads, shares
+@pytest.mark.parametrize("shape,whole,shared", [
+    ((1, 32, 8, 64, 2048, "causal"), 20.1, 14.0), ((1, 32, 8, 64, 8011, "causal"), 61.1, 24.6),
+    ((1, 32, 8, 250, 8011, "causal"), 62.3, 42.2), ((2, 32, 8, 128, 8011, "causal"), 62.3, 42.3),
+    ((1, 8, 2, 1024, 8011, "causal"), 61.6, 41.1), ((1, 8, 2, 500, 4096, "causal"), 34.8, 19.2),
+    ((1, 32, 8, 64, 16384, "none"), 115.7, 40.3), ((1, 32, 8, 768, 4096, "causal"), 59.5, 67.3),
+    ((1, 32, 8, 1024, 16384, "causal"), 236.3, 260.1), ((2, 32, 8, 500, 16384, "causal"), 251.8, 264.4),
+], ids=str)
+def test_shares_where_they_ran_faster(shape, whole, shared):
+    assert (layout(*shape)[1] > 1) == (shared < whole)
+
+
+def test_the_deal_of_many_rounds_is_even():
+    """From eight rounds of two-head items on nothing is gained by smaller ones, whatever the remainder."""
+    for B in (3, 4, 5, 8, 16):
+        for N in (4096, 5000, 8192):
+            assert layout(B, 32, 8, N, N, "causal") == (2, 1)
+
+
+def test_a_problem_is_laid_out_the_same_again_and_on_other_sm_counts():
+    """The last few layouts are remembered: more problems in turn than that, twice over."""
+    shapes = [(1, 32, 8, n, 8011, "causal") for n in (1, 64, 250, 500, 768, 1024, 2048)]
+    first = [layout(*s) for s in shapes]
+    assert [layout(*s) for s in shapes] == first
+    assert layout(1, 32, 8, 500, 8011, "causal", sms=1)[0] == 2           # no SM is without work
+    assert layout(1, 32, 8, 500, 8011, "causal", sms=4000) == (2, 1)      # beyond any GPU: no deal is made
+    assert [layout(*s) for s in shapes] == first
+
+
+@pytest.mark.parametrize("switch,heads", [("0", 1), ("1", 2)])
+def test_the_environment_fixes_the_layout(switch, heads, monkeypatch):
+    monkeypatch.setenv("ATTNFUSE_FWD_PAIR", switch)
+    for shape in [s for s, *_ in MEASURED] + [(1, 32, 8, 64, 16384, "none")]:
+        assert layout(*shape) == (heads, 1)
+    assert layout(1, 6, 6, 64, 16384, "none") == (1, 1)                   # no pair in a group of one

@@ -479,9 +479,10 @@ static FwdSetup set_up(const AfFwdParams& a, int sms) {
   s.rotate = p.rope && need > 0 && usable && a.workspace_bytes >= need;
   s.rotated_bytes = s.rotate ? need : 0;
   const int mode = p.rope && !s.rotate ? tc::ROPE_FUSED : tc::ROPE_NONE;
-  s.plan = plan_forward(p, a.lse != nullptr, mode, sms, true);
-  if (s.plan.shares > 1 && (!usable || a.workspace_bytes < s.rotated_bytes + share_workspace_bytes(p, s.plan.shares)))
-    s.plan.shares = 1;                                     // no room for partials: whole rows per item
+  s.plan = plan_forward(p, a.lse != nullptr, mode, sms, usable);
+  // no room for the partials: the better layout of whole rows
+  if (s.plan.shares > 1 && a.workspace_bytes < s.rotated_bytes + share_workspace_bytes(p, s.plan.shares))
+    s.plan = plan_forward(p, a.lse != nullptr, mode, sms, false);
   return s;
 }
 

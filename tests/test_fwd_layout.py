@@ -95,3 +95,17 @@ def test_the_environment_fixes_the_layout(switch, heads, monkeypatch):
     for shape in [s for s, *_ in MEASURED] + [(1, 32, 8, 64, 16384, "none")]:
         assert layout(*shape) == (heads, 1)
     assert layout(1, 6, 6, 64, 16384, "none") == (1, 1)                   # no pair in a group of one
+
+
+@pytest.mark.parametrize("shape", [(1, 32, 8, 640, 16384, "causal"), (1, 32, 8, 64, 8011, "causal"), (2, 32, 8, 500, 16384, "none"),
+                                   (1, 8, 2, 1024, 8011, "causal")], ids=str)
+def test_without_room_for_partials_the_better_layout_of_whole_rows(shape):
+    """What a call without workspace, or with too little, takes is what a call that has no shares takes."""
+    want = layout(*shape, lse=True)
+    assert layout(*shape, workspace=False) == want
+    if layout(*shape)[1] > 1:
+        a = problem(*shape)
+        a.workspace_bytes = 4096
+        heads, shares = C.c_int32(), C.c_int32()
+        assert _lib.load().af_fwd_layout(C.byref(a), SMS, C.byref(heads), C.byref(shares)) == 0
+        assert (heads.value, shares.value) == want

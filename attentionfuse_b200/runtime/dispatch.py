@@ -120,6 +120,11 @@ _FWD_TEMPLATES: dict = {}
 _FWD_TEMPLATES_MAX = 256
 
 
+def _workspace_bytes(lib, params, device) -> int:
+    with _lib.on_device(device):                       # the answer depends on the SM count of the current one
+        return int(lib.af_fwd_workspace_bytes(C.byref(params)))
+
+
 def launch_forward(Q, K, V, out, *, sm_scale, mask_kind, window=0, bias_kind=0, norm_kind=0,
                    slopes=None, bias=None, cos=None, sin=None, save_lse=None,
                    block_lists=None, family=None, q_offset=0, keep_workspace=None):
@@ -149,6 +154,9 @@ def launch_forward(Q, K, V, out, *, sm_scale, mask_kind, window=0, bias_kind=0, 
             p.cos, p.sin = cos.data_ptr(), sin.data_ptr()
         if save_lse is not None:
             params.lse = save_lse.data_ptr()
+        elif Q.shape[3] == 128:
+            # partials of shared keys: whether a call has them follows from the device and the environment too
+            need = _workspace_bytes(lib, params, Q.device)
     else:
         params = _lib.AfFwdParams()
         keep: list = []
@@ -160,13 +168,13 @@ def launch_forward(Q, K, V, out, *, sm_scale, mask_kind, window=0, bias_kind=0, 
         params.o, params.o_stride = out.data_ptr(), _lib.strides(out)
         if save_lse is not None:
             params.lse, params.lse_stride = save_lse.data_ptr(), _lib.strides(save_lse, 3)
-        need = int(lib.af_fwd_workspace_bytes(C.byref(params)))
+        need = _workspace_bytes(lib, params, Q.device)
         if key is not None and not keep:
             if len(_FWD_TEMPLATES) >= _FWD_TEMPLATES_MAX:
                 _FWD_TEMPLATES.clear()
             _FWD_TEMPLATES[key] = (_lib.AfFwdParams.from_buffer_copy(params), need)
     stream = _lib.current_stream(Q.device)
-    if need > 0 and not in_kernel_rope:
+    if need > 0 and not (in_kernel_rope and cos is not None):
         # Allocated per call, never kept for the next one: the allocator's stream order covers its lifetime
         # outside a capture, the graph's own pool inside one, and calls of several threads, whose
         # launches (rotation, attention, merge) may interleave on one stream, have one each.

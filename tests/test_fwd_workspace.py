@@ -78,3 +78,23 @@ def test_a_captured_rope_call_owns_its_workspace(N_q, N_kv):
     torch.cuda.synchronize()
     assert_close(out, orc.attention(Q, K, V, causal=True, cos=cos, sin=sin, q_offset=N_kv - N_q), dtype, what="replayed")
     assert all(bool((f == 3).all()) for f in filled)
+
+
+@pytest.mark.gpu
+def test_the_workspace_follows_the_environment_and_the_rotation_switch(monkeypatch):
+    """A call that could share its keys, first with the layout fixed by the environment, then free; and with
+    rotation kept in the kernel, which is no concern of a call without RoPE."""
+    q, k, v = (t.cuda() for t in qkv(8700, 1, 8, 2, 64, 4096, 128, torch.bfloat16))
+    out = torch.empty_like(q)
+
+    def launches():
+        before = _lib.launch_count()
+        dispatch.launch_forward(q, k, v, out, sm_scale=0.088, mask_kind=0)
+        return _lib.launch_count() - before
+
+    monkeypatch.setenv("ATTNFUSE_FWD_PAIR", "1")
+    assert launches() == 1
+    monkeypatch.delenv("ATTNFUSE_FWD_PAIR")
+    assert launches() == 2                             # shares and their merge
+    monkeypatch.setenv("ATTNFUSE_ROPE_IN_KERNEL", "1")
+    assert launches() == 2

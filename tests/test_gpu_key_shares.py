@@ -17,14 +17,14 @@ DEV, D = "cuda", 128
 MASKS = {"none": 0, "causal": 1, "window": 2}
 
 
-def call(q, k, v, mask, off, slopes, workspace):
+def call(q, k, v, mask, off, slopes, workspace, window=700):
     """af_fwd with or without the workspace it asks for; returns (output, launches, bytes asked for)."""
     lib, params, out = _lib.load(), _lib.AfFwdParams(), torch.full_like(q, float("nan"))
-    fill_problem(params.p, q, k, v, sm_scale=D ** -0.5, mask_kind=MASKS[mask], window=700, bias_kind=1 if slopes is not None else 0,
+    fill_problem(params.p, q, k, v, sm_scale=D ** -0.5, mask_kind=MASKS[mask], window=window, bias_kind=1 if slopes is not None else 0,
                  slopes=slopes, q_offset=off)
     params.o, params.o_stride = out.data_ptr(), _lib.strides(out)
     need = int(lib.af_fwd_workspace_bytes(C.byref(params)))
-    ws = torch.empty(max(need, 1), dtype=torch.uint8, device=DEV)
+    ws = torch.full((max(need, 1),), 0xff, dtype=torch.uint8, device=DEV)      # NaN in every word
     if workspace:
         params.workspace, params.workspace_bytes = ws.data_ptr(), need
     before = _lib.launch_count()
@@ -45,13 +45,38 @@ def test_shares_match_oracle_and_whole_rows(shape, mask, alibi, dtype):
     got, launches, need = call(q, k, v, mask, off, slopes, True)
     whole, one, _ = call(q, k, v, mask, off, slopes, False)
     assert one == 1
-    if mask != "window":                       # a window leaves too few tiles to share
+    if mask != "window":                       # this one leaves too few tiles to share: see below
         assert launches == 2 and need > 0
     want = orc.attention(Q, K, V, causal=mask == "causal", window=700 if mask == "window" else None, q_offset=off,
                          slopes=None if slopes is None else slopes.cpu(),
                          **(dict(q_positions=torch.full((B,), off)) if N_q == 1 else {}))
     assert_close(got, want, dtype, what=f"key shares {mask} {shape}")
     assert_close(whole, want, dtype, what=f"whole rows {mask} {shape}")
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("mask,alibi,shape,off,window", [
+    ("window", False, (1, 8, 2, 200, 9000), 4000, 1500), ("window", True, (1, 8, 2, 200, 9000), 4000, 1500),
+    ("window", False, (1, 4, 2, 130, 3000), 0, 2500), ("none", True, (1, 8, 2, 250, 4011), 3000, 0),
+    ("causal", False, (1, 2, 1, 4096, 4096), 0, 0), ("causal", True, (1, 2, 1, 4096, 4096), 0, 0),
+    ("causal", False, (1, 8, 2, 300, 8000), 100, 0)],
+    ids=lambda x: "x".join(map(str, x)) if isinstance(x, tuple) else str(x))
+def test_shares_of_every_mask(mask, alibi, shape, off, window, dtype):
+    """Calls that must share: windows whose first key tile is not tile 0, ALiBi on a dense score, and causal rows
+    from the first key on, whose first query tiles have fewer key tiles than shares (partials of
+    nothing) -- or, 100 rows in, so few that no call of the length would share."""
+    B, Hq, Hkv, N_q, N_kv = shape
+    Q, K, V = qkv(7450 + N_q, B, Hq, Hkv, N_q, N_kv, D, dtype)
+    q, k, v = Q.to(DEV), K.to(DEV), V.to(DEV)
+    slopes = _alibi_slopes(Hq, DEV, str(dtype)) if alibi else None
+    got, launches, need = call(q, k, v, mask, off, slopes, True, window or 1)
+    if off == 100:
+        assert launches == 1 and need == 0     # 4 key tiles at most, of 63
+    else:
+        assert launches == 2 and need > 0
+    want = orc.attention(Q, K, V, causal=mask == "causal", window=window or None, q_offset=off,
+                         slopes=None if slopes is None else slopes.cpu())
+    assert_close(got, want, dtype, what=f"must share {mask} {shape}")
 
 
 def test_rotated_chunk_and_training_call():

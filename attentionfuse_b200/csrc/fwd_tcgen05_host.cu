@@ -384,19 +384,19 @@ static float heaviest_sm(const float* cost, int rows, int units, int chunk, int 
 // Megabytes of partials of a problem in `shares` shares (accumulators; m and l are a hundredth of them).
 static double partial_mb(const AfProblem& p, int shares) { return 4e-6 * shares * p.B * p.H_q * p.N_q * p.D; }
 
-// The layout whose heaviest SM is done first, in key tiles of the one-head schedule (0.86 us).  Measured over 161
+// The layout whose heaviest SM is done first, in key tiles of the one-head schedule (0.86 us).  Measured over 217
 // problems (square causal, window and dense of 512 - 4096 rows, chunks of 16 - 1024 rows against 1k - 16k
-// keys; 1 - 4 sequences, 8 - 64 heads):
+// keys; 1 - 4 sequences, 8 - 64 heads), each layout in turn:
 //  * one head per CTA: an item costs its tiles and two at its boundary; two heads: a tile of both costs 2.0 and
 //    the boundary 2.5.  One head has to win by 3 % (near a tie the two-head schedule draws less power, which
-//    counts once every SM is busy: 541 against 581 us at [4,32/8,4096] causal).  The times of the layout
-//    so chosen are 0.04 % above the faster one's on average, 2.4 % at most; a rule on the mean tiles
-//    per item lost up to 19 % ([1,64/8,3584] causal: 183 us with two heads, 215 with one).  Two heads
-//    halve the number of items, which is what few query tiles cannot afford: 500 rows against 8011 keys,
-//    32 heads: 118 us as 64 items, 63 us as 128.  From eight rounds of pair items on the deal is even.
+//    counts once every SM is busy: 477 against 505 us at [4,32/8,4096] causal).  The layout so chosen is
+//    within the timer's noise (2 %) of the faster one everywhere; a rule on the mean tiles per item lost up to
+//    12 % ([1,32/8,2432] window 256: 38.7 us with two heads, 43.4 with one).  Two heads halve the number of
+//    items, which is what few query tiles cannot afford: 500 rows against 8011 keys, 32 heads: 119 us as
+//    64 items, 67 us as 128.  From eight rounds of pair items on the deal is even.
 //  * shares of the keys (head dim 128): the partials' way through memory and the merge launch cost 4 tiles and
 //    0.45 per MB of partials (1 MB: 3 - 6 tiles; 8 MB: 7 - 8; 38 MB: 21), and have to win by 5 %.  32 heads, us with /
-//    without: 64 rows x 2048 keys 14 / 20, x 8011 25 / 61, x 16384 40 / 118; 250 x 8011 42 / 62.  Calls that
+//    without: 64 rows x 2048 keys 14 / 21, x 8011 25 / 62, x 16384 40 / 118; 250 x 8011 44 / 64.  Calls that
 //    keep a log-sum-exp have none: an autograd forward holds its workspace until the backward.
 // ATTNFUSE_FWD_PAIR in the environment (read at every call) fixes the layout to what depends on head_dim, group, mask
 // and rotation alone: two heads per CTA wherever that exists (1), or one (0), and no shares.

@@ -1,5 +1,5 @@
 """How the head-dim-128 forward is laid over the SMs (af_fwd_layout; host only): one or two query heads per
-CTA, shares of the keys.  Expected are the layouts that ran faster on a 148-SM B200."""
+CTA, shares of the keys.  Expected are the layouts that ran faster on a 148-SM B200, timed in turn."""
 import ctypes as C
 
 import pytest
@@ -36,20 +36,21 @@ def layout(*shape, sms=SMS, **kw):
 
 # (B, H_q, H_kv, N_q, N_kv, mask): us with two heads per CTA, with one (whole rows), at least 4 % apart
 MEASURED = [
-    ((1, 32, 8, 512, 512, "causal"), 14.8, 10.7), ((1, 32, 8, 1024, 1024, "causal"), 23.0, 17.9),
-    ((1, 32, 8, 2432, 2432, "causal"), 50.7, 52.9), ((1, 64, 8, 2048, 2048, "causal"), 72.1, 74.9),
-    ((1, 64, 8, 3584, 3584, "causal"), 182.8, 214.9), ((1, 8, 2, 4096, 4096, "causal"), 64.7, 35.5),
-    ((2, 32, 8, 768, 768, "causal"), 19.9, 21.1), ((2, 32, 8, 2432, 2432, "causal"), 93.3, 99.4),
-    ((2, 32, 8, 3072, 3072, "causal"), 144.6, 156.3), ((2, 32, 8, 3584, 3584, "causal"), 183.2, 194.0),
-    ((2, 64, 8, 3584, 3584, "causal"), 364.0, 412.1), ((2, 8, 2, 3072, 3072, "causal"), 51.2, 43.8),
-    ((4, 32, 8, 3072, 3072, "causal"), 290.7, 312.0), ((4, 32, 8, 4096, 4096, "causal"), 541.2, 581.2),
-    ((4, 64, 8, 1536, 1536, "causal"), 158.6, 177.0), ((4, 8, 2, 512, 512, "causal"), 17.6, 12.7),
-    ((4, 8, 2, 4096, 4096, "causal"), 123.1, 128.9), ((1, 32, 8, 2432, 2432, "window"), 38.1, 42.9),
-    ((1, 32, 8, 2432, 2432, "none"), 112.9, 97.3), ((1, 32, 8, 4096, 4096, "none"), 248.1, 227.9),
-    ((2, 32, 8, 2048, 2048, "none"), 131.5, 118.9), ((2, 32, 8, 4096, 4096, "none"), 435.1, 510.9),
-    ((1, 32, 8, 500, 8011, "causal"), 117.6, 63.0), ((1, 32, 8, 768, 4096, "causal"), 64.4, 59.5),
-    ((1, 32, 8, 1024, 8011, "causal"), 124.0, 118.0), ((2, 32, 8, 500, 4096, "causal"), 66.1, 72.6),
-    ((2, 32, 8, 768, 8011, "causal"), 221.4, 178.0), ((2, 32, 8, 1024, 8011, "causal"), 231.6, 254.5),
+    ((1, 32, 8, 512, 512, "causal"), 15.0, 10.9), ((1, 32, 8, 1024, 1024, "causal"), 23.3, 17.9),
+    ((1, 32, 8, 2432, 2432, "causal"), 52.7, 55.0), ((1, 64, 8, 2048, 2048, "causal"), 74.5, 78.5),
+    ((1, 64, 8, 3584, 3584, "causal"), 183.7, 195.3), ((1, 8, 2, 4096, 4096, "causal"), 66.2, 37.8),
+    ((2, 32, 8, 768, 768, "causal"), 20.5, 21.8), ((2, 32, 8, 2432, 2432, "causal"), 96.1, 102.0),
+    ((2, 32, 8, 3072, 3072, "causal"), 141.1, 151.4), ((2, 32, 8, 3584, 3584, "causal"), 184.1, 195.8),
+    ((2, 64, 8, 3584, 3584, "causal"), 364.7, 390.2), ((2, 8, 2, 3072, 3072, "causal"), 53.1, 46.0),
+    ((4, 32, 8, 3072, 3072, "causal"), 277.1, 297.0), ((4, 32, 8, 4096, 4096, "causal"), 476.7, 505.3),
+    ((4, 64, 8, 1536, 1536, "causal"), 160.3, 178.2), ((4, 8, 2, 512, 512, "causal"), 15.2, 11.1),
+    ((4, 8, 2, 4096, 4096, "causal"), 122.1, 128.4), ((1, 32, 8, 2432, 2432, "window"), 38.7, 43.4),
+    ((1, 32, 8, 2432, 2432, "none"), 113.5, 98.9), ((1, 32, 8, 4096, 4096, "none"), 240.6, 226.1),
+    ((2, 32, 8, 2048, 2048, "none"), 129.6, 120.9), ((1, 32, 8, 500, 8011, "causal"), 118.7, 66.6),
+    ((1, 32, 8, 768, 4096, "causal"), 66.4, 62.1), ((2, 32, 8, 768, 8011, "causal"), 222.6, 180.7),
+    ((2, 32, 8, 4096, 4096, "causal"), 236.6, 251.6), ((4, 32, 8, 2048, 2048, "causal"), 135.9, 147.7),
+    ((2, 8, 2, 2048, 2048, "causal"), 38.0, 24.7), ((4, 64, 8, 768, 768, "causal"), 60.0, 66.8),
+    ((1, 32, 8, 1024, 1024, "window"), 21.8, 24.6), ((2, 32, 8, 640, 4096, "causal"), 112.6, 92.2),
 ]
 
 
@@ -60,13 +61,13 @@ def test_whole_rows_take_the_layout_that_ran_faster(shape, two, one):
     assert heads == (2 if two < one else 1)
 
 
-# the same, and us in the shares that the layout has: whole rows of one or two heads, shares
+# us of the faster layout of whole rows, and in shares (the last two in 3 and 4: no shares were found to win)
 @pytest.mark.parametrize("shape,whole,shared", [
-    ((1, 32, 8, 64, 2048, "causal"), 20.1, 14.0), ((1, 32, 8, 64, 8011, "causal"), 61.1, 24.6),
-    ((1, 32, 8, 250, 8011, "causal"), 62.3, 42.2), ((2, 32, 8, 128, 8011, "causal"), 62.3, 42.3),
-    ((1, 8, 2, 1024, 8011, "causal"), 61.6, 41.1), ((1, 8, 2, 500, 4096, "causal"), 34.8, 19.2),
-    ((1, 32, 8, 64, 16384, "none"), 115.7, 40.3), ((1, 32, 8, 768, 4096, "causal"), 59.5, 67.3),
-    ((1, 32, 8, 1024, 16384, "causal"), 236.3, 260.1), ((2, 32, 8, 500, 16384, "causal"), 251.8, 264.4),
+    ((1, 32, 8, 64, 2048, "causal"), 20.6, 14.1), ((1, 32, 8, 64, 8011, "causal"), 62.0, 25.2),
+    ((1, 32, 8, 250, 8011, "causal"), 63.7, 43.9), ((2, 32, 8, 128, 8011, "causal"), 64.4, 43.5),
+    ((1, 8, 2, 1024, 8011, "causal"), 63.4, 43.0), ((1, 8, 2, 500, 4096, "causal"), 35.3, 19.7),
+    ((1, 32, 8, 640, 16384, "causal"), 230.8, 184.7), ((1, 32, 8, 64, 16384, "none"), 116.2, 39.9),
+    ((1, 32, 8, 768, 4096, "causal"), 62.1, 67.3), ((1, 32, 8, 1024, 16384, "causal"), 232.4, 260.1),
 ], ids=str)
 def test_shares_where_they_ran_faster(shape, whole, shared):
     assert (layout(*shape)[1] > 1) == (shared < whole)

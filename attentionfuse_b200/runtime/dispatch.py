@@ -134,12 +134,12 @@ def launch_forward(Q, K, V, out, *, sm_scale, mask_kind, window=0, bias_kind=0, 
     lib = _lib.load()
     if family is None:
         family = int(os.environ.get("ATTNFUSE_FAMILY", "0"))
-    in_kernel_rope = os.environ.get("ATTNFUSE_ROPE_IN_KERNEL", "0") == "1"
+    q_ptr, k_ptr, v_ptr, o_ptr = Q.data_ptr(), K.data_ptr(), V.data_ptr(), out.data_ptr()
     key = None
     if block_lists is None and bias is None:
         key = (Q.dtype, Q.shape, Q.stride(), K.shape, K.stride(), V.stride(), out.stride(), float(sm_scale), mask_kind,
                window, bias_kind, norm_kind, family, q_offset, cos is not None and (cos.stride(0), sin.stride(0)),
-               save_lse is not None and save_lse.stride(), (Q.data_ptr() | K.data_ptr() | V.data_ptr() | out.data_ptr()) & 15)
+               save_lse is not None and save_lse.stride(), (q_ptr | k_ptr | v_ptr | o_ptr) & 15)
         hit = _FWD_TEMPLATES.get(key)
     else:
         hit = None
@@ -147,7 +147,7 @@ def launch_forward(Q, K, V, out, *, sm_scale, mask_kind, window=0, bias_kind=0, 
         template, need = hit
         params = _lib.AfFwdParams.from_buffer_copy(template)
         p = params.p
-        p.q, p.k, p.v, params.o = Q.data_ptr(), K.data_ptr(), V.data_ptr(), out.data_ptr()
+        p.q, p.k, p.v, params.o = q_ptr, k_ptr, v_ptr, o_ptr
         if slopes is not None:
             p.slopes = slopes.data_ptr()
         if cos is not None:
@@ -165,7 +165,7 @@ def launch_forward(Q, K, V, out, *, sm_scale, mask_kind, window=0, bias_kind=0, 
                      cos=cos, sin=sin, family=family, keep=keep, q_offset=q_offset)
         if block_lists is not None:
             block_lists.fill(params.p, Q.shape[1])
-        params.o, params.o_stride = out.data_ptr(), _lib.strides(out)
+        params.o, params.o_stride = o_ptr, _lib.strides(out)
         if save_lse is not None:
             params.lse, params.lse_stride = save_lse.data_ptr(), _lib.strides(save_lse, 3)
         need = _workspace_bytes(lib, params, Q.device)
@@ -174,7 +174,7 @@ def launch_forward(Q, K, V, out, *, sm_scale, mask_kind, window=0, bias_kind=0, 
                 _FWD_TEMPLATES.clear()
             _FWD_TEMPLATES[key] = (_lib.AfFwdParams.from_buffer_copy(params), need)
     stream = _lib.current_stream(Q.device)
-    if need > 0 and not (in_kernel_rope and cos is not None):
+    if need > 0 and not (cos is not None and os.environ.get("ATTNFUSE_ROPE_IN_KERNEL", "0") == "1"):
         # Allocated per call, never kept for the next one: the allocator's stream order covers its lifetime
         # outside a capture, the graph's own pool inside one, and calls of several threads, whose
         # launches (rotation, attention, merge) may interleave on one stream, have one each.

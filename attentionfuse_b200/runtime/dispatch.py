@@ -12,12 +12,14 @@ import ctypes as C
 import functools
 import math
 import os
+import threading
 from typing import Optional
 
 import torch
 
 from ..ir.high_level import Graph, MaskKind
 from . import _lib
+from .flash_decode import can_use_flash_decode, run_flash_decode
 from .kernel_cache import get_or_compile
 
 
@@ -120,6 +122,33 @@ _FWD_TEMPLATES: dict = {}
 _FWD_TEMPLATES_MAX = 256
 
 
+class _KeptWorkspaces(threading.local):
+    def __init__(self):
+        self.by_stream = {}
+
+
+_KEPT = _KeptWorkspaces()
+_KEPT_MAX_BYTES, _KEPT_MAX_STREAMS = 16 << 20, 4
+
+
+def _inference_workspace(device, stream: int, need: int) -> torch.Tensor:
+    """Workspace of a call that nobody takes over afterwards.  Small ones are kept for the next call of the
+    same thread on the same stream, whose kernels come after this one's: an allocation costs a short
+    prefill 2 of its 23 us ([4,12,512,64] with RoPE, bound by the host).  Of a thread's own, because calls of
+    two threads may interleave their launches on one stream; not while a graph is captured, which keeps
+    the addresses and replays when it likes; not above 16 MB, where the kernels take longer than the
+    call.  At most four per thread; they go back when a fifth stream comes or the thread ends."""
+    if need > _KEPT_MAX_BYTES or torch.cuda.is_current_stream_capturing():
+        return torch.empty(need, dtype=torch.uint8, device=device)
+    kept = _KEPT.by_stream
+    workspace = kept.get((device.index, stream))
+    if workspace is None or workspace.numel() < need:
+        if len(kept) >= _KEPT_MAX_STREAMS:
+            kept.clear()
+        workspace = kept[device.index, stream] = torch.empty(need, dtype=torch.uint8, device=device)
+    return workspace
+
+
 def _workspace_bytes(lib, params, device) -> int:
     with _lib.on_device(device):                       # the answer depends on the SM count of the current one
         return int(lib.af_fwd_workspace_bytes(C.byref(params)))
@@ -174,15 +203,14 @@ def launch_forward(Q, K, V, out, *, sm_scale, mask_kind, window=0, bias_kind=0, 
                 _FWD_TEMPLATES.clear()
             _FWD_TEMPLATES[key] = (_lib.AfFwdParams.from_buffer_copy(params), need)
     stream = _lib.current_stream(Q.device)
-    if need > 0 and not (cos is not None and os.environ.get("ATTNFUSE_ROPE_IN_KERNEL", "0") == "1"):
-        # Allocated per call, never kept for the next one: the allocator's stream order covers its lifetime
-        # outside a capture, the graph's own pool inside one, and calls of several threads, whose
-        # launches (rotation, attention, merge) may interleave on one stream, have one each.
-        workspace = torch.empty(need, dtype=torch.uint8, device=Q.device)
-        if keep_workspace is not None:
-            keep_workspace.append(workspace)
-        params.workspace, params.workspace_bytes = workspace.data_ptr(), need
     with _lib.on_device(Q.device):
+        if need > 0 and not (cos is not None and os.environ.get("ATTNFUSE_ROPE_IN_KERNEL", "0") == "1"):
+            if keep_workspace is not None:
+                workspace = torch.empty(need, dtype=torch.uint8, device=Q.device)
+                keep_workspace.append(workspace)
+            else:
+                workspace = _inference_workspace(Q.device, stream, need)
+            params.workspace, params.workspace_bytes = workspace.data_ptr(), need
         rc = lib.af_fwd(C.byref(params), stream)
     _lib.check(rc, "af_fwd")
     return out
@@ -219,7 +247,6 @@ def run_attention(graph: Graph, Q: torch.Tensor, K: torch.Tensor, V: torch.Tenso
     if q_offset is not None and (not isinstance(q_offset, int) or q_offset < 0):
         raise ValueError(f"q_offset must be a non-negative int or an int32 tensor (B,); got {q_offset!r}")
 
-    from .flash_decode import can_use_flash_decode, run_flash_decode
     positioned = q_offset is not None or q_positions is not None
     if save_lse is None and can_use_flash_decode(graph, Q, K, positioned):
         if out is None:

@@ -1,5 +1,6 @@
-"""The workspace of a forward call (rotated Q and K, partials of shared keys) belongs to that call: calls of
-two threads whose launches interleave on one stream, a captured graph and later, larger calls do not meet in it."""
+"""Nobody else writes the workspace of a forward call (rotated Q and K, partials of shared keys) before its
+kernels have run: calls of two threads whose launches interleave on one stream, a captured graph and
+later calls do not meet in it."""
 import threading
 
 import pytest
@@ -19,8 +20,10 @@ class FakeLibrary:
     def __init__(self):
         self.seen, self.inside, self.go_on = [], threading.Event(), threading.Event()
 
+    need = 4096
+
     def af_fwd_workspace_bytes(self, params):
-        return 4096
+        return self.need
 
     def af_fwd(self, params, stream):
         p = params._obj
@@ -31,26 +34,58 @@ class FakeLibrary:
         return 0
 
 
-def test_two_threads_on_one_stream_have_a_workspace_each(monkeypatch):
+@pytest.fixture
+def lib(monkeypatch):
     lib = FakeLibrary()
     monkeypatch.setattr(_lib, "load", lambda: lib)
-    monkeypatch.setattr(_lib, "current_stream", lambda device: 7)
+    monkeypatch.setattr(_lib, "current_stream", lambda device: lib.stream)
     monkeypatch.setattr(_lib, "on_device", lambda device: _lib._NO_SWITCH)
-    Q, K, V = qkv(8500, 1, 2, 1, 640, 640, 64, torch.bfloat16)
-    cos, sin = orc.build_rope_cache(640, 64, 10000.0, torch.bfloat16)
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: lib.capturing)
+    monkeypatch.setattr(dispatch, "_KEPT", dispatch._KeptWorkspaces())
+    monkeypatch.setattr(dispatch, "_FWD_TEMPLATES", {})
+    lib.stream, lib.capturing = 7, False
+    return lib
 
-    def call():
-        dispatch.launch_forward(Q, K, V, torch.empty_like(Q), sm_scale=0.125, mask_kind=1, cos=cos, sin=sin)
 
-    first = threading.Thread(target=call)
+def rope_call(n=640):
+    Q, K, V = (torch.zeros(1, h, n, 64, dtype=torch.bfloat16) for h in (2, 1, 1))
+    cos, sin = orc.build_rope_cache(n, 64, 10000.0, torch.bfloat16)
+    dispatch.launch_forward(Q, K, V, torch.empty_like(Q), sm_scale=0.125, mask_kind=1, cos=cos, sin=sin)
+
+
+def test_two_threads_on_one_stream_have_a_workspace_each(lib):
+    first = threading.Thread(target=rope_call)
     first.start()
     assert lib.inside.wait(30)
-    call()                                             # while the first call is between its launches
+    rope_call()                                        # while the first call is between its launches
     lib.go_on.set()
     first.join()
     (ws_a, n_a), (ws_b, n_b) = lib.seen
     assert n_a == n_b == 4096
     assert abs(ws_a - ws_b) >= 4096
+
+
+def test_what_is_kept_is_bounded_and_never_a_graphs(lib):
+    lib.go_on.set()
+    rope_call()
+    rope_call()
+    assert lib.seen[0] == lib.seen[1]                  # a stream's calls follow one another
+    lib.capturing = True
+    rope_call()
+    lib.capturing = False
+    kept = dispatch._KEPT.by_stream
+    assert lib.seen[2][0] != lib.seen[0][0] and len(kept) == 1 and kept[None, 7].data_ptr() == lib.seen[0][0]
+    for lib.stream in range(20):
+        rope_call()
+        assert len(kept) <= 4
+    lib.need, lib.stream = dispatch._KEPT_MAX_BYTES + 1, 100
+    rope_call(700)
+    assert all(t.numel() <= dispatch._KEPT_MAX_BYTES for t in kept.values()) and (None, 100) not in kept
+    others = []
+    thread = threading.Thread(target=lambda: others.append(len(dispatch._KEPT.by_stream)))
+    thread.start()
+    thread.join()
+    assert others == [0]
 
 
 @pytest.mark.gpu

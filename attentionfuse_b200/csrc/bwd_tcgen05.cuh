@@ -77,7 +77,12 @@ template <int D, int MODE = MODE_DKV> struct BCfg {
   static constexpr int SHARES = BT / COLS;                  // element-wise threads per stationary row
   static constexpr int EW_THREADS = BS * SHARES;
   static constexpr int DRAIN_THREADS = FUSED ? BS : 0;      // fused: threads that add dQ^T to its accumulator
-  static constexpr int THREADS = EW_THREADS + DRAIN_THREADS + 96;   // and the producer and two MMA issuers
+  // and the producer and two MMA issuers.  352 threads (head dim 64, and the single pass) leave 168 registers each: a
+  // thread that holds 64 columns of S and 64 of dP at once spills, up to 160 bytes in the key-stationary
+  // instances (causal: 108 at head dim 64, 124 in the single pass; two-pass dQ up to 20).  With 224
+  // threads nothing spilled (216 - 238 registers) and the pass was slower: dK/dV at head dim 64,
+  // [4,12,4096] causal, 341 us against 247, the Llama training step 2534 against 2467.
+  static constexpr int THREADS = EW_THREADS + DRAIN_THREADS + 96;
   static constexpr int STAGES = FUSED ? 3 : 4;
   static constexpr int STRM_PANEL = BT * 128;
   static constexpr int STRM_TILE = PANELS * STRM_PANEL;

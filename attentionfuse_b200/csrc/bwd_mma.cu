@@ -148,11 +148,13 @@ int launch_bwd_mma(const AfBwdParams& a, cudaStream_t st) {
   if ((rc = tc_make_map(&q_strm, p.dtype, q_ptr, p.B, p.H_q, p.N_q, p.D, qs, strm_rows)) != AF_OK) return rc;
   if ((rc = tc_make_map(&do_strm, p.dtype, a.d_o, p.B, p.H_q, p.N_q, p.D, a.do_stride, strm_rows)) != AF_OK) return rc;
 
+  const float key_stationary_scale = p.sm_scale > 0x1p-110f ? p.sm_scale : 0x1p-110f;
   const int64_t acc_bytes = bwd_mma_dq_accum_bytes(a);
   if (acc_bytes > 0 && a.dq_accum != nullptr && a.dq_accum_bytes >= acc_bytes && ((uintptr_t)a.dq_accum & 255) == 0) {
     // ---- single fused pass: dK, dV and dQ from one recompute of S and dP ----
     tcb::BwdArgs f{};
     f.a = a;
+    f.score_scale = key_stationary_scale;
     const bool blk = p.mask_kind == AF_MASK_BLOCKS;
     f.tiles = (p.N_kv + 127) / 128;
     f.stat_per_block = blk ? p.block_n / 128 : 1;
@@ -190,11 +192,13 @@ int launch_bwd_mma(const AfBwdParams& a, cudaStream_t st) {
   const bool blocks = p.mask_kind == AF_MASK_BLOCKS;
   tcb::BwdArgs dkv{};
   dkv.a = a;
+  dkv.score_scale = key_stationary_scale;
   dkv.tiles = (p.N_kv + 127) / 128;
   dkv.stat_per_block = blocks ? p.block_n / 128 : 1;
   dkv.steps_per_block = blocks ? p.block_m / strm_rows : 1;
   tcb::BwdArgs dq{};
   dq.a = a;
+  dq.score_scale = p.sm_scale;
   dq.tiles = (p.N_q + 127) / 128;
   dq.stat_per_block = blocks ? p.block_m / 128 : 1;
   dq.steps_per_block = blocks ? p.block_n / strm_rows : 1;

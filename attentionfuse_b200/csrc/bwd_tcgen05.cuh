@@ -56,11 +56,6 @@ enum { EMASK_NONE = 0, EMASK_CAUSAL = 1, EMASK_WINDOW = 2, EMASK_BITS = 3 };   /
 
 constexpr int BS = 128;   // rows of the stationary operands (TMEM lanes)
 
-// Scale of the scores in the key-stationary passes, which divide L by it (BCfg::KEY_STAT): not below 2^-110, where
-// L / scale leaves fp32.  What a smaller scale would make of a score differs from this one's by under
-// 2^-10 as long as |S| < 2^100.  dK and dQ are multiplied by the caller's scale.
-__device__ __forceinline__ float score_scale(const AfProblem& p) { return fmaxf(p.sm_scale, 0x1p-110f); }
-
 template <int D, int MODE = MODE_DKV> struct BCfg {
   static constexpr bool FUSED = MODE == MODE_FUSED;
   static constexpr int PANELS = D / 64;
@@ -136,6 +131,10 @@ struct BBarriers {
 
 struct BwdArgs {
   AfBwdParams a;
+  // Scale of the scores.  Not below 2^-110 in the key-stationary passes, which divide L by it (BCfg::KEY_STAT) and where
+  // L / scale would leave fp32: what a smaller scale would make of a score differs from this one's by under
+  // 2^-10 as long as |S| < 2^100.  dK and dQ are multiplied by the caller's scale.
+  float score_scale;
   int tiles;            // stationary tiles along the sequence
   int steps_per_block;  // block lists: streamed steps (BCfg::BT rows) per listed block
   int stat_per_block;   // block lists: stationary 128-row tiles per block
@@ -359,7 +358,7 @@ bwd_tcgen05_kernel(const BwdArgs args, const __grid_constant__ CUtensorMap map_a
     // L2 hints: the stationary tiles are read once per item, the streamed rows once per stationary
     // tile of their unit
     const uint64_t pol_once = l2_policy_evict_first(), pol_keep = l2_policy_evict_last();
-    const float inv_scale = 1.f / score_scale(p);
+    const float inv_scale = 1.f / args.score_scale;
     BItem bi;
     int it0 = 0, qi = 0;
     bool ok = true;
@@ -604,7 +603,7 @@ bwd_tcgen05_kernel(const BwdArgs args, const __grid_constant__ CUtensorMap map_a
     // ============================== element-wise group / epilogue ==============================
     const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
     const int lrow = tid & (BS - 1), share = tid / BS, col_first = share * COLS;   // row of the stationary tile, first column of a step
-    const float scale2 = (KVS ? score_scale(p) : p.sm_scale) * kLog2e;
+    const float scale2 = args.score_scale * kLog2e;
     BItem bi;
     int it0 = 0;
     bool alive = true;

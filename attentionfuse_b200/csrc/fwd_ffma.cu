@@ -20,6 +20,7 @@
 // scalar FMAs, 70 us with 16-byte reads (30 % of the issue slots: 1.9 warps per scheduler on average,
 // the longest CTA's eight tiles one after the other), 47 us with two groups and packed FMAs.
 #include "common.cuh"
+#include "ptx_sm100.cuh"
 
 namespace af {
 namespace {
@@ -30,26 +31,8 @@ constexpr int NT = 128;       // threads of a group
 constexpr int PAD = 4;        // row pitch D + 4 floats: 16-byte rows, 8 consecutive rows on distinct banks
 constexpr int LDP = 2 * TN + PAD;   // P is stored twice over, (p, p): the broadcast operand of a packed FMA
 
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ float2 unpack2(uint64_t v) {
-  float2 r;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-  return r;
-}
+using namespace ptx;          // packed fp32 pairs
+
 // Barrier of one group's 128 threads (group 0 or 1; number 0 is __syncthreads).
 __device__ __forceinline__ void group_sync(int group) { asm volatile("bar.sync %0, %1;" ::"r"(group + 1), "r"(NT) : "memory"); }
 
@@ -258,18 +241,19 @@ __global__ void __launch_bounds__(NT * Groups<DMAX>::value, DMAX == 64 ? 2 : 1) 
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) s2[i][j] = fma2(qv[i].x, kv[j].x, s2[i][j]);
+        for (int j = 0; j < 4; ++j) s2[i][j] = f32x2_fma(qv[i].x, kv[j].x, s2[i][j]);
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) s2[i][j] = fma2(qv[i].y, kv[j].y, s2[i][j]);
+        for (int j = 0; j < 4; ++j) s2[i][j] = f32x2_fma(qv[i].y, kv[j].y, s2[i][j]);
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        const float2 h = unpack2(s2[i][j]);
-        s[i][j] = h.x + h.y;
+        float even, odd;
+        f32x2_unpack(s2[i][j], even, odd);
+        s[i][j] = even + odd;
       }
 
     // Tile-level decision: only edge tiles pay for element masking.
@@ -321,7 +305,7 @@ __global__ void __launch_bounds__(NT * Groups<DMAX>::value, DMAX == 64 ? 2 : 1) 
         l_i[i] = alpha * l_i[i] + rs;
         m_i[i] = m_new;
 #pragma unroll
-        for (int c = 0; c < NCH * 2; ++c) acc[i][c] = mul2(acc[i][c], pack2(alpha, alpha));
+        for (int c = 0; c < NCH * 2; ++c) acc[i][c] = f32x2_mul(acc[i][c], f32x2_pack(alpha, alpha));
       } else {
         float rs = 0.f;
 #pragma unroll
@@ -358,8 +342,8 @@ __global__ void __launch_bounds__(NT * Groups<DMAX>::value, DMAX == 64 ? 2 : 1) 
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             const uint64_t w = u == 0 ? pv[i].x : pv[i].y;
-            acc[i][c * 2] = fma2(w, vv.x, acc[i][c * 2]);
-            acc[i][c * 2 + 1] = fma2(w, vv.y, acc[i][c * 2 + 1]);
+            acc[i][c * 2] = f32x2_fma(w, vv.x, acc[i][c * 2]);
+            acc[i][c * 2 + 1] = f32x2_fma(w, vv.y, acc[i][c * 2 + 1]);
           }
         }
       }
@@ -400,8 +384,8 @@ __global__ void __launch_bounds__(NT * Groups<DMAX>::value, DMAX == 64 ? 2 : 1) 
 #pragma unroll
       for (int c = 0; c < NCH; ++c) {
         const ulonglong2 o = *reinterpret_cast<const ulonglong2*>(xo + r * DMAX + c * 64 + tx * 4);
-        acc[i][c * 2] = fma2(o.x, pack2(w_o, w_o), mul2(acc[i][c * 2], pack2(w, w)));
-        acc[i][c * 2 + 1] = fma2(o.y, pack2(w_o, w_o), mul2(acc[i][c * 2 + 1], pack2(w, w)));
+        acc[i][c * 2] = f32x2_fma(o.x, f32x2_pack(w_o, w_o), f32x2_mul(acc[i][c * 2], f32x2_pack(w, w)));
+        acc[i][c * 2 + 1] = f32x2_fma(o.y, f32x2_pack(w_o, w_o), f32x2_mul(acc[i][c * 2 + 1], f32x2_pack(w, w)));
       }
     }
   }
@@ -416,8 +400,11 @@ __global__ void __launch_bounds__(NT * Groups<DMAX>::value, DMAX == 64 ? 2 : 1) 
 #pragma unroll
     for (int c = 0; c < NCH; ++c) {
       const int d0 = c * 64 + tx * 4;
-      const float2 lo2 = unpack2(acc[i][c * 2]), hi2 = unpack2(acc[i][c * 2 + 1]);
-      const float ov[4] = {lo2.x * inv, lo2.y * inv, hi2.x * inv, hi2.y * inv};
+      float ov[4];
+      f32x2_unpack(acc[i][c * 2], ov[0], ov[1]);
+      f32x2_unpack(acc[i][c * 2 + 1], ov[2], ov[3]);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) ov[e] *= inv;
       if (VEC) {
         if (d0 < D)
           *reinterpret_cast<float4*>(reinterpret_cast<float*>(a.o) + o_off + (int64_t)row * a.o_stride[2] + d0) =

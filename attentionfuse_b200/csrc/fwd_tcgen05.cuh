@@ -412,34 +412,8 @@ __device__ __forceinline__ float row_max(const uint32_t (&xr)[NC]) {
 //   EXP_SCALE      y = x * scale2 + shift
 //   EXP_AFFINE     y = x * scale2 + slope_c * c + shift     (ALiBi folded in, c = column index)
 //   EXP_PRESCALED  y = x + shift                            (scores already scaled and biased)
+// on packed fp32 pairs.
 enum { EXP_SCALE = 0, EXP_AFFINE = 1, EXP_PRESCALED = 2 };
-// Packed fp32 pairs (sm_100: fma / add on two fp32 values in one 64-bit register pair, one issue
-// slot): the scale-and-shift and the row sum of the exponent pass take half the instructions.
-__device__ __forceinline__ uint64_t f32x2_pack(float lo, float hi) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ void f32x2_unpack(uint64_t v, float& lo, float& hi) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ uint64_t f32x2_fma(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ uint64_t f32x2_add(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-
-__device__ __forceinline__ uint64_t f32x2_mul(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-
 template <typename T, int KIND, int NC>
 __device__ __forceinline__ void exp_pass(const uint32_t (&xr)[NC], uint32_t (&pk)[NC / 2], float scale2, float shift,
                                          float slope_c, float& rsum) {

@@ -136,9 +136,10 @@ def _inference_workspace(device, stream: int, need: int) -> torch.Tensor:
     same thread on the same stream, whose kernels come after this one's: an allocation costs a short
     prefill 2 of its 23 us ([4,12,512,64] with RoPE, bound by the host).  Of a thread's own, because calls of
     two threads may interleave their launches on one stream; not while a graph is captured, which keeps
-    the addresses and replays when it likes; not above 16 MB, where the kernels take longer than the
-    call.  At most four per thread; they go back when a fifth stream comes or the thread ends."""
-    if need > _KEPT_MAX_BYTES or torch.cuda.is_current_stream_capturing():
+    the addresses and replays when it likes (the default stream, 0, cannot be captured); not above
+    16 MB, where the kernels take longer than the call.  At most four per thread; they go back when
+    a fifth stream comes or the thread ends."""
+    if need > _KEPT_MAX_BYTES or (stream != 0 and torch.cuda.is_current_stream_capturing()):
         return torch.empty(need, dtype=torch.uint8, device=device)
     kept = _KEPT.by_stream
     workspace = kept.get((device.index, stream))

@@ -1,0 +1,630 @@
+// Forward attention for head dim 64 on the tensor cores: two CTAs per SM.
+//
+// Same arithmetic and roles as fwd_tcgen05.cuh (reference: attnfuse/compiler/codegen.py:67-381 and
+// attnfuse/compiler/codegen_blocksparse.py:34-171) on a schedule of its own.  The exponentials bound
+// head dim 64: 1024 clocks per 128 x 128 tile at 16 per clock and SM, against 512 of products.  With
+// two softmax warps per scheduler the unit stood still whenever both waited, loaded or stored.  Half
+// the shared memory and half the tensor memory are enough for a tile of this head dim, so two CTAs
+// share an SM: four independent softmax warps per scheduler, and one CTA's item boundary runs under
+// the other's tiles.  That leaves 96 registers per thread: a thread's 64 key columns go through the
+// exponent pass as two runs of 32, and S has one buffer.  What it waits for now is the chain P -> P.V ->
+// next S of a half (600 - 700 clocks) and issue in the exponent pass; the MUFU is busy 67 % of the time
+// (56 % before).  [4,12,4096,64] f16 back to back, before -> now: causal 188 -> 151 us, with ALiBi 188 -> 160,
+// dense 338 -> 286, window 256 93 -> 66.
+#pragma once
+#include "fwd_tcgen05.cuh"
+
+namespace af {
+namespace tc {
+
+struct Cfg64 {
+  static constexpr int D = 64;
+  static constexpr int TILE_BYTES = PANEL_BYTES;               // 128 rows x 64 elements x 2 bytes
+  static constexpr int STAGES = 2;                             // K ring and V ring
+  static constexpr int O_STAGE_BYTES = 8 * 32 * 64;            // per softmax warp: 32 rows x 64 bytes (64-byte swizzle)
+  static constexpr int BARRIER_BYTES = 2048;
+  static constexpr int SMEM_BYTES = TILE_BYTES * (1 + 2 * STAGES) + O_STAGE_BYTES + 1024 /*align*/ + BARRIER_BYTES;
+  static constexpr int TMEM_COLS = 256;
+  static constexpr int COL_S = 0;                              // 128 columns, the half of a thread over its own 64
+  static constexpr int COL_O0 = 128, COL_O1 = 192;             // one O per half of the key columns
+};
+static_assert(2 * (Cfg64::SMEM_BYTES + 1024) <= 228 * 1024, "two CTAs share an SM");
+
+enum { WARP_MMA64 = 9, WARP_ROTATE64 = 10 };   // behind the softmax warps and WARP_PRODUCER
+constexpr int threads64(int rope) { return rope == ROPE_FUSED ? 352 : 320; }
+
+struct Barriers64 {
+  uint64_t q_full, q_ready;
+  uint64_t k_full[2], k_ready[2], v_full[2];
+  // Group t of products, S of tile t and P.V of tile t - 1, has run (slot t & 1): K slot t & 1, V slot
+  // (t - 1) & 1 and, behind an item's last S, the Q buffer are free.
+  uint64_t ring_free[2];
+  uint64_t s_full[2], p_full[2];   // [half of the key columns]
+  uint64_t o_done, o_free;
+  uint32_t tmem_base;
+  int abort_flag;
+  uint32_t pair_flag[2][8];
+  float xchg[SOFTMAX_THREADS];
+};
+static_assert(sizeof(Barriers64) <= Cfg64::BARRIER_BYTES, "the barriers and the exchange have room");
+
+// Bits [lo, hi] of a 32-bit word (none when the range is empty or outside).
+__device__ __forceinline__ uint32_t bit_range(int lo, int hi) {
+  const uint32_t up = hi >= 31 ? 0xffffffffu : hi < 0 ? 0u : (2u << hi) - 1u;
+  const uint32_t down = lo <= 0 ? 0xffffffffu : lo > 31 ? 0u : 0xffffffffu << lo;
+  return up & down;
+}
+
+template <typename T, int ROPE, int EMASK, bool ALIBI, int SPLIT>
+__global__ void __launch_bounds__(threads64(ROPE), 2)
+fwd_d64_kernel(const TcArgs args, const __grid_constant__ CUtensorMap tmap_q,
+               const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
+               const __grid_constant__ CUtensorMap tmap_o) {
+  using C = Cfg64;
+  constexpr int D = C::D, STAGES = C::STAGES;
+  constexpr bool ROT_K = (ROPE == ROPE_FUSED);
+  constexpr int AB_FMT = (Elem<T>::code == AF_BF16) ? 1 : 0;
+  // One S product per half of the key columns, each with barriers of its own: the two softmax
+  // streams of a row never wait for each other.
+  constexpr uint32_t IDESC_QK = umma_idesc_f16(AB_FMT, BM, HALF_COLS, 0, 0);
+  constexpr uint32_t IDESC_PV = umma_idesc_f16(AB_FMT, BM, D, 0, 1);
+
+  const AfFwdParams& a = args.a;
+  const AfProblem& p = a.p;
+
+  extern __shared__ unsigned char smem_raw[];
+  const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  unsigned char* smem = smem_raw + (smem_base - smem_u32(smem_raw));
+  const uint32_t sQ = smem_base;
+  const uint32_t sK0 = sQ + C::TILE_BYTES;
+  const uint32_t sV0 = sK0 + STAGES * C::TILE_BYTES;
+  const uint32_t sO = sV0 + STAGES * C::TILE_BYTES;
+  Barriers64* bars = reinterpret_cast<Barriers64*>(smem + C::TILE_BYTES * (1 + 2 * STAGES) + C::O_STAGE_BYTES);
+  volatile int* abort_flag = &bars->abort_flag;
+
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+
+  if (tid == 0) {
+    mbar_init(&bars->q_full, 1);
+    mbar_init(&bars->q_ready, 128);
+    mbar_init(&bars->o_done, 1);
+    mbar_init(&bars->o_free, SOFTMAX_THREADS);
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(&bars->k_full[s], 1);
+      mbar_init(&bars->k_ready[s], 32);
+      mbar_init(&bars->v_full[s], 1);
+      mbar_init(&bars->ring_free[s], 1);
+    }
+    for (int hh = 0; hh < 2; ++hh) {
+      mbar_init(&bars->s_full[hh], 1);
+      mbar_init(&bars->p_full[hh], SOFTMAX_THREADS / 2);
+    }
+    bars->abort_flag = 0;
+    for (int i = 0; i < 16; ++i) (&bars->pair_flag[0][0])[i] = 0u;
+    mbar_fence_init();
+  }
+  if (warp == WARP_PRODUCER) {
+    tmem_alloc(&bars->tmem_base, C::TMEM_COLS);
+    tmem_relinquish();
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem = __shfl_sync(0xffffffffu, bars->tmem_base, 0);
+
+  // Running counts as in fwd_tcgen05.cuh: gg = key tiles so far (ring stage gg & 1, ring phase
+  // (gg >> 1) & 1; the S / P barriers complete once per tile, phase gg & 1), qi = items so far.
+  if (warp == WARP_PRODUCER) {
+    // ============================== TMA producer ==============================
+    if (lane == 0) {
+      tma_prefetch_desc(&tmap_q);
+      tma_prefetch_desc(&tmap_k);
+      tma_prefetch_desc(&tmap_v);
+      tma_prefetch_desc(&tmap_o);
+      const uint64_t stream = l2_policy_evict_first(), keep = SPLIT == SPLIT_DECODE ? stream : l2_policy_evict_last();
+      TileCursor ck, cv;   // K runs one tile ahead of V
+      cursor_init(ck);
+      cursor_init(cv);
+      auto load_k = [&]() -> bool {
+        if (ck.j == 0) {
+          // the single Q buffer is free once the last S product of the previous item has run
+          if (ck.qi > 0 && !mbar_wait(&bars->ring_free[(ck.gg - 1) & 1], ((ck.gg - 1) >> 1) & 1, abort_flag)) return false;
+          mbar_arrive_expect_tx(&bars->q_full, C::TILE_BYTES);
+          tma_load_4d_hint(smem, &tmap_q, &bars->q_full, 0, ck.it.m0, ck.it.h, ck.it.b, stream);
+        }
+        const int s = ck.gg & 1;
+        if (ck.gg >= 2 && !mbar_wait(&bars->ring_free[s], ((ck.gg - 2) >> 1) & 1, abort_flag)) return false;
+        mbar_arrive_expect_tx(&bars->k_full[s], C::TILE_BYTES);
+        tma_load_4d_hint(smem + C::TILE_BYTES * (1 + s), &tmap_k, &bars->k_full[s], 0, ck.it.walk.key0(ck.j), ck.it.h_kv,
+                         ck.it.b, keep);
+        return true;
+      };
+      auto load_v = [&]() -> bool {
+        const int s = cv.gg & 1;
+        if (cv.gg >= 2 && !mbar_wait(&bars->ring_free[(cv.gg - 1) & 1], ((cv.gg - 1) >> 1) & 1, abort_flag)) return false;
+        mbar_arrive_expect_tx(&bars->v_full[s], C::TILE_BYTES);
+        tma_load_4d_hint(smem + C::TILE_BYTES * (1 + STAGES + s), &tmap_v, &bars->v_full[s], 0, cv.it.walk.key0(cv.j),
+                         cv.it.h_kv, cv.it.b, keep);
+        return true;
+      };
+      bool more_k = cursor_next<EMASK, SPLIT>(args, ck);
+      bool more_v = cursor_next<EMASK, SPLIT>(args, cv);
+      // K runs one tile ahead of V (a wait for a V slot never holds up a K load) -- except across
+      // an item boundary: the first K load of an item starts with a wait for the Q buffer (the
+      // previous item's last S product), so every V tile of the previous item goes out before it.
+      while (more_k || more_v) {
+        const bool at_boundary = more_k && ck.j == 0 && ck.qi > 0 && more_v && cv.gg < ck.gg;
+        if (more_k && !at_boundary && (!more_v || ck.gg <= cv.gg + 1)) {
+          if (!load_k()) break;
+          more_k = cursor_next<EMASK, SPLIT>(args, ck);
+        } else {
+          if (!load_v()) break;
+          more_v = cursor_next<EMASK, SPLIT>(args, cv);
+        }
+      }
+    }
+  } else if (warp == WARP_MMA64) {
+    // ============================== MMA issuer ==============================
+    // The whole warp walks the tiles and one elected lane issues: the descriptors are then uniform
+    // values, which the products take without a move per operand (a lane that walks alone paid about
+    // 60 clocks per product and 150 per barrier wait, and P -> P.V -> next S is the chain that the
+    // softmax warps wait for).  One thread issues both products: products of one thread run in
+    // order, so S of the next tile follows P.V of its half into the pipe without a wait.
+    {
+      const bool leader = elect_one();
+      const uint64_t desc_q = umma_desc_sw128(sQ, 16, 1024);
+      const uint64_t desc_k0 = umma_desc_sw128(sK0, 16, 1024);
+      const uint64_t desc_v0 = umma_desc_sw128(sV0, PANEL_BYTES, 1024);
+      TileCursor cu;               // the tile whose S comes next
+      cursor_init(cu);
+      auto operands_ready = [&]() -> bool {
+        if (cu.j == 0 && !mbar_wait(ROPE != ROPE_NONE ? &bars->q_ready : &bars->q_full, cu.qi & 1, abort_flag)) return false;
+        return mbar_wait(ROT_K ? &bars->k_ready[cu.gg & 1] : &bars->k_full[cu.gg & 1], (cu.gg >> 1) & 1, abort_flag);
+      };
+      auto issue_s = [&](int hh) {
+        const uint64_t kdesc = desc_k0 + (uint64_t)(((cu.gg & 1) * C::TILE_BYTES + hh * HALF_COLS * 128) >> 4);
+        if (leader) {
+#pragma unroll
+          for (int kk = 0; kk < D / 16; ++kk)
+            umma_ss(tmem + C::COL_S + hh * HALF_COLS, desc_q + (uint64_t)(kk * 2), kdesc + (uint64_t)(kk * 2), IDESC_QK,
+                    kk > 0 ? 1u : 0u);
+          umma_commit(&bars->s_full[hh]);
+        }
+      };
+      bool more = cursor_next<EMASK, SPLIT>(args, cu);
+      if (more && operands_ready()) {
+        issue_s(0);
+        issue_s(1);
+        if (leader) umma_commit(&bars->ring_free[0]);
+        while (more) {
+          const int gg = cu.gg, j = cu.j, qi = cu.qi, s = gg & 1;
+          const bool last = j + 1 == cu.it.walk.n_tiles;
+          more = cursor_next<EMASK, SPLIT>(args, cu);
+          if (!mbar_wait(&bars->v_full[s], (gg >> 1) & 1, abort_flag)) break;
+          // the first P.V product of an item overwrites O: the previous item's rows must be read out
+          if (j == 0 && qi > 0 && !mbar_wait(&bars->o_free, (qi - 1) & 1, abort_flag)) break;
+          if (!last && !operands_ready()) break;
+          bool ok = true;
+          for (int hh = 0; hh < 2; ++hh) {
+            if (!mbar_wait(&bars->p_full[hh], gg & 1, abort_flag)) { ok = false; break; }
+            tc_fence_after_sync();
+            if (leader) {
+#pragma unroll
+              for (int kk = 0; kk < HALF_COLS / 16; ++kk)
+                umma_ts(tmem + (hh ? C::COL_O1 : C::COL_O0), tmem + C::COL_S + hh * HALF_COLS + kk * 8,
+                        desc_v0 + (uint64_t)((s * C::TILE_BYTES + (hh * 4 + kk) * 2048) >> 4), IDESC_PV,
+                        (j > 0 || kk > 0) ? 1u : 0u);
+            }
+            if (!last) issue_s(hh);
+          }
+          if (!ok) break;
+          if (last) {
+            if (leader) umma_commit(&bars->o_done);
+            if (more) {
+              // the next item's Q comes after this item's last S product: its S products follow
+              // both halves of P.V, so that a late Q holds nothing up
+              if (!operands_ready()) break;
+              issue_s(0);
+              issue_s(1);
+            }
+          }
+          if (leader) umma_commit(&bars->ring_free[(gg + 1) & 1]);
+        }
+      }
+    }
+  } else if (warp < SOFTMAX_THREADS / 32) {
+    // ============================== softmax / epilogue ==============================
+    // Two threads per query row, each with an online softmax of its own over 64 of a tile's key
+    // columns (own reference maximum, row sum and accumulator O_h); see fwd_tcgen05.cuh.
+    const int half = warp >> 2, rtid = tid & (BM - 1);
+    const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
+    const uint32_t s_tmem = tmem + lane_base + C::COL_S + half * HALF_COLS;
+    const uint32_t o_tmem = tmem + lane_base + (half ? C::COL_O1 : C::COL_O0);
+    const float scale2 = p.sm_scale * kLog2e;     // > 0 (checked on the host)
+    Item it;
+    int g = 0, qi = 0;
+    uint32_t pair_count = 0;
+    bool alive = true;
+    for (int round = 0; alive && get_item<EMASK, SPLIT>(args, round, it); ++round) {
+      const TileWalk& walk = it.walk;
+      const int n_tiles = walk.n_tiles;
+      const int m0 = it.m0, b = it.b, h = it.h;
+      const int row = m0 + rtid;
+      if (ROPE != ROPE_NONE && n_tiles > 0 && half == 0) {
+        if (mbar_wait(&bars->q_full, qi & 1, abort_flag)) {
+          if (row < p.N_q)
+            rope_row<T, D>(sQ, rtid, reinterpret_cast<const T*>(p.cos) + (int64_t)(row + p.q_offset) * p.rope_stride_n,
+                           reinterpret_cast<const T*>(p.sin) + (int64_t)(row + p.q_offset) * p.rope_stride_n);
+          fence_proxy_async_smem();
+          mbar_arrive(&bars->q_ready);
+        }
+      }
+      const float slope2 = ALIBI ? load_slope<T>(p.slopes, h) * kLog2e : 0.f;
+      const int n_kv = SPLIT == SPLIT_DECODE ? it.n_kv : p.N_kv;
+      const int pos0 = m0 + p.q_offset;             // position of the item's first row on the key axis
+      float m_ref = -INFINITY, l_part = 0.f;        // m_ref in log2 units of the scaled score
+      bool ref_ok = false;   // warp-uniform: every row of the warp has a finite reference (it never becomes -inf again)
+
+      for (int j = 0; j < n_tiles; ++j) {
+        const int gg = g + j;                       // the CTA's running key-tile count
+        const int key0 = walk.key0(j);
+        const int rel = row + p.q_offset - key0 - half * HALF_COLS;   // this row's position on the thread's columns
+        // Tile-level decision: only edge / diagonal tiles look at single columns.
+        bool need_mask = key0 + BN > n_kv;
+        if (EMASK == EMASK_CAUSAL) need_mask = need_mask || (key0 + BN - 1 > pos0);
+        if (EMASK == EMASK_WINDOW)
+          need_mask = need_mask || (pos0 + BM - 1 - key0 >= p.window) || (key0 + BN - 1 - pos0 >= p.window);
+        uint64_t tile_bits = ~0ull;                 // EMASK_BITS: this thread's 64 columns of the tile's bit matrix
+        if (EMASK == EMASK_BITS && walk.slots != nullptr) {
+          const int bs = walk.slots[j / walk.per_block];
+          if (bs >= 0) {
+            const int words = p.block_n >> 6;
+            tile_bits = p.kv_bits[((int64_t)bs * p.block_m + (m0 % p.block_m) + rtid) * words + (j % walk.per_block) * 2 + half];
+            need_mask = true;
+          }
+        }
+        // The visible ones of the thread's columns [32 u, 32 u + 32), one bit each.
+        auto visible = [&](int u) -> uint32_t {
+          if (!need_mask) return 0xffffffffu;
+          const int c0 = half * HALF_COLS + 32 * u, r = rel - 32 * u;
+          int lo = 0, hi = n_kv - 1 - key0 - c0;
+          if (EMASK == EMASK_CAUSAL) hi = min(hi, r);
+          if (EMASK == EMASK_WINDOW) {
+            hi = min(hi, r + (p.window - 1));
+            lo = r - (p.window - 1);
+          }
+          uint32_t v = bit_range(lo, hi);
+          if (EMASK == EMASK_BITS) v &= (uint32_t)(tile_bits >> (32 * u));
+          return v;
+        };
+        // Raw scores of those columns (fp32 bit patterns), the invisible ones at -inf.
+        auto scores = [&](int u, uint32_t vis, uint32_t (&xr)[32]) {
+          tmem_ld32(s_tmem + 32 * u, &xr[0]);
+          tmem_wait_ld32(xr);
+          if (need_mask && __any_sync(0xffffffffu, vis != 0xffffffffu)) {
+#pragma unroll
+            for (int c = 0; c < 32; ++c) xr[c] = (vis >> c) & 1u ? xr[c] : 0xff800000u;
+          }
+        };
+        // ALiBi: affine in the column wherever the sign of rel - c is the same for all of the
+        // thread's visible columns (always under a causal mask).
+        float slope_c = 0.f, bias0 = 0.f;
+        bool affine = true;
+        if (ALIBI) {
+          const bool below = (EMASK == EMASK_CAUSAL) || rel >= HALF_COLS - 1;
+          affine = (EMASK == EMASK_CAUSAL) || __all_sync(0xffffffffu, below || rel <= 0);
+          slope_c = below ? slope2 : -slope2;
+          bias0 = -slope_c * (float)rel;
+        }
+        if (!mbar_wait(&bars->s_full[half], gg & 1, abort_flag)) { alive = false; break; }
+        tc_fence_after_sync();
+        // Usual case: P against the standing reference right away, the row sum verifies it (kRowSumBound).
+        float rsum = 0.f;
+        bool fast = ref_ok && affine;
+        if (fast) {
+          constexpr int KIND = ALIBI ? EXP_AFFINE : EXP_SCALE;
+          uint32_t pk[HALF_COLS / 2];
+          uint32_t (&p0)[16] = *reinterpret_cast<uint32_t (*)[16]>(&pk[0]);
+          uint32_t (&p1)[16] = *reinterpret_cast<uint32_t (*)[16]>(&pk[16]);
+          float rs1;
+          if (__builtin_expect(!need_mask, 1)) {
+            // kept free of the mask's code: four warps of a scheduler are at different places of it
+            uint32_t x0[32], x1[32];
+            tmem_ld32(s_tmem, x0);
+            tmem_wait_ld32(x0);
+            tmem_ld32(s_tmem + 32, x1);
+            exp_pass<T, KIND, 32, 0>(x0, p0, scale2, bias0 - m_ref, slope_c, rsum);
+            tmem_wait_ld32(x1);
+            exp_pass<T, KIND, 32, 32>(x1, p1, scale2, bias0 - m_ref, slope_c, rs1);
+            rsum += rs1;
+          } else {
+            // a run of 32 columns that no row of the warp sees costs nothing
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+              const uint32_t vis = visible(u);
+              if (__any_sync(0xffffffffu, vis != 0u)) {
+                uint32_t xr[32];
+                scores(u, vis, xr);
+                if (u == 0) exp_pass<T, KIND, 32, 0>(xr, p0, scale2, bias0 - m_ref, slope_c, rs1);
+                else exp_pass<T, KIND, 32, 32>(xr, p1, scale2, bias0 - m_ref, slope_c, rs1);
+                rsum += rs1;
+              } else {
+#pragma unroll
+                for (int i = 0; i < 16; ++i) pk[16 * u + i] = 0u;
+              }
+            }
+          }
+          fast = __all_sync(0xffffffffu, rsum <= kRowSumBound);
+          if (fast) {
+            l_part += rsum;
+            tmem_st32(s_tmem, pk);                  // P_h over the first half of the thread's own S columns
+          }
+        }
+        if (__builtin_expect(!fast, 0)) {
+          // First tile of an item, no visible key so far, or a sum past the bound: maximum first,
+          // reference update, accumulator rescale, then P (the scores are read once more).
+          auto biased = [&](int u, uint32_t (&xr)[32]) {
+            if (ALIBI) {
+              const float relf = (float)(rel - 32 * u);
+#pragma unroll
+              for (int c = 0; c < 32; ++c)
+                xr[c] = __float_as_uint(fmaf(__uint_as_float(xr[c]), scale2, -slope2 * fabsf(relf - (float)c)));
+            }
+          };
+          float mx = -INFINITY;
+#pragma unroll 1
+          for (int u = 0; u < 2; ++u) {
+            const uint32_t vis = visible(u);
+            if (need_mask && !__any_sync(0xffffffffu, vis != 0u)) continue;
+            uint32_t xr[32];
+            scores(u, vis, xr);
+            biased(u, xr);
+            mx = fmaxf(mx, row_max(xr));
+          }
+          if (!ALIBI) mx *= scale2;                   // the maximum commutes with the positive scale
+          const bool bump = mx > m_ref + kRescaleThreshold;   // also true for the first finite max
+          const float m_next = bump ? mx : m_ref;
+          const float alpha = bump ? ex2_approx(m_ref - m_next) : 1.f;
+          m_ref = m_next;
+          ref_ok = __all_sync(0xffffffffu, m_ref != -INFINITY);
+          const float neg_m = (m_next == -INFINITY) ? 0.f : -m_next;
+          if (j > 0 && __any_sync(0xffffffffu, bump)) {
+            // The accumulator is expressed relative to the old reference: rescale it in TMEM (the
+            // previous tile's P.V product was issued before this tile's S and is covered by its commit).
+#pragma unroll
+            for (int c = 0; c < D / 32; ++c) {
+              uint32_t o[32];
+              tmem_ld32(o_tmem + c * 32, o);
+              tmem_wait_ld();
+#pragma unroll
+              for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+              tmem_st32(o_tmem + c * 32, o);
+            }
+          }
+          rsum = 0.f;
+#pragma unroll 1
+          for (int u = 0; u < 2; ++u) {
+            const uint32_t vis = visible(u);
+            uint32_t pu[16];
+            if (!need_mask || __any_sync(0xffffffffu, vis != 0u)) {
+              uint32_t xr[32];
+              float rs;
+              scores(u, vis, xr);
+              biased(u, xr);
+              exp_pass<T, ALIBI ? EXP_PRESCALED : EXP_SCALE, 32, 0>(xr, pu, scale2, neg_m, 0.f, rs);
+              rsum += rs;
+            } else {
+#pragma unroll
+              for (int i = 0; i < 16; ++i) pu[i] = 0u;
+            }
+            // columns [0, 16) or [16, 32) of the thread's S: read by the first pass of this loop already
+            tmem_st16(s_tmem + 16 * u, pu);
+          }
+          l_part = l_part * alpha + rsum;
+        }
+        if (SPLIT == SPLIT_DECODE && key0 + BN > n_kv) {
+          // Split-K decode: cache rows past the valid length hold whatever the allocation held
+          // (TMA zero-fills only past the tensor's extent) and 0 * NaN would poison O, so the
+          // softmax threads clear those V rows of the stage before they release P.
+          const int s = gg & 1;
+          if (!mbar_wait(&bars->v_full[s], (gg >> 1) & 1, abort_flag)) { alive = false; break; }
+          // each half clears the rows its own P.V product reads (keys [64 half, 64 half + 64))
+          const int first = max(n_kv - key0, half * HALF_COLS), last = (half + 1) * HALF_COLS;
+          const uint32_t v_tile = sV0 + s * C::TILE_BYTES;
+          for (int idx = rtid; idx < (last - first) * 8; idx += BM)
+            sts128(v_tile + (first + (idx >> 3)) * 128 + ((idx & 7) << 4), make_uint4(0u, 0u, 0u, 0u));
+          fence_proxy_async_smem();
+        }
+        tmem_wait_st();
+        tc_fence_before_sync();
+        mbar_arrive(&bars->p_full[half]);
+      }
+
+      // Epilogue: the two halves of a row meet and each merges its half of the output columns from
+      // both accumulators (two hand-shakes under the last P.V product; see fwd_tcgen05.cuh).
+      if (!alive) break;
+      constexpr bool partial = SPLIT != SPLIT_NONE;
+      if (!partial && lane == 0) bulk_wait_read_all();   // previous item's staged rows: long gone by now
+      float c0 = 0.f, c1 = 0.f, m_all = 0.f, l_sum = 0.f;
+      if (half == 1) {
+        bars->xchg[rtid] = m_ref;
+        bars->xchg[BM + rtid] = l_part;
+      }
+      if (!pair_sync(bars, warp, lane, pair_count, abort_flag)) { alive = false; break; }
+      if (half == 0) {
+        const float m_other = bars->xchg[rtid], l_other = bars->xchg[BM + rtid];
+        m_all = fmaxf(m_ref, m_other);
+        const float w_mine = (m_ref == -INFINITY) ? 0.f : ex2_approx(m_ref - m_all);
+        const float w_other = (m_other == -INFINITY) ? 0.f : ex2_approx(m_other - m_all);
+        l_sum = l_part * w_mine + l_other * w_other;
+        // a share of the keys keeps its partial un-normalised for the merge
+        const float inv = partial ? 1.f : 1.f / ((l_sum == 0.f) ? 1.f : l_sum);
+        c0 = w_mine * inv;
+        c1 = w_other * inv;
+        bars->xchg[rtid] = c0;
+        bars->xchg[BM + rtid] = c1;
+      }
+      if (!pair_sync(bars, warp, lane, pair_count, abort_flag)) { alive = false; break; }
+      if (half == 1) {
+        c0 = bars->xchg[rtid];
+        c1 = bars->xchg[BM + rtid];
+      }
+      float o[32];                                   // output columns [32 half, 32 half + 32)
+      if (n_tiles > 0) {
+        if (!mbar_wait(&bars->o_done, qi & 1, abort_flag)) { alive = false; break; }
+        tc_fence_after_sync();
+        uint32_t o0[32], o1[32];
+        tmem_ld32(tmem + lane_base + C::COL_O0 + half * 32, o0);
+        tmem_ld32(tmem + lane_base + C::COL_O1 + half * 32, o1);
+        tmem_wait_ld();
+        tc_fence_before_sync();
+        mbar_arrive(&bars->o_free);
+#pragma unroll
+        for (int i = 0; i < 32; ++i) o[i] = __uint_as_float(o0[i]) * c0 + __uint_as_float(o1[i]) * c1;
+      } else {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) o[i] = 0.f;
+      }
+      // The rows leave through the warp's staging region, 32 rows x 64 bytes in the 64-byte
+      // swizzle (16-byte chunk c of row r at c ^ ((r >> 1) & 3)): conflict-free.
+      const uint32_t stage = sO + (uint32_t)(warp * 32 * 64);
+      const uint32_t swz = (uint32_t)((lane >> 1) & 3);
+      if (partial) {
+        // un-normalised fp32 partial of this (split, batch, head) for the combine, 16 columns a time
+        const int64_t wr0 = ((int64_t)it.split * p.B + b) * ((int64_t)p.H_q * p.N_q) + (int64_t)h * p.N_q + m0 + (warp & 3) * 32;
+        const int rows_valid = min(32, p.N_q - (m0 + (warp & 3) * 32));   // rows of this warp that exist
+#pragma unroll
+        for (int part = 0; part < 2; ++part) {
+          __syncwarp();
+#pragma unroll
+          for (uint32_t c4 = 0; c4 < 4; ++c4)
+            sts128(stage + (uint32_t)lane * 64 + ((c4 ^ swz) << 4),
+                   make_uint4(__float_as_uint(o[part * 16 + c4 * 4]), __float_as_uint(o[part * 16 + c4 * 4 + 1]),
+                              __float_as_uint(o[part * 16 + c4 * 4 + 2]), __float_as_uint(o[part * 16 + c4 * 4 + 3])));
+          __syncwarp();
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int r = i * 8 + (lane >> 2), c4 = lane & 3;
+            if (r < rows_valid) {
+              const uint4 v = lds128(stage + (uint32_t)(r * 64 + ((c4 ^ ((r >> 1) & 3)) << 4)));
+              *reinterpret_cast<uint4*>(args.ws_acc + (wr0 + r) * D + half * 32 + part * 16 + c4 * 4) = v;
+            }
+          }
+        }
+        if (half == 0 && row < p.N_q) {
+          const int64_t wr = wr0 + lane;
+          args.ws_m[wr] = m_all * kLn2;      // -inf when the split saw no key
+          args.ws_l[wr] = l_sum;
+        }
+      } else {
+        __syncwarp();   // lane 0 has seen the previous store off (above, before the exchange)
+#pragma unroll
+        for (uint32_t c4 = 0; c4 < 4; ++c4) {
+          uint4 v;
+          v.x = Pack2<T>::run(o[c4 * 8 + 0], o[c4 * 8 + 1]);
+          v.y = Pack2<T>::run(o[c4 * 8 + 2], o[c4 * 8 + 3]);
+          v.z = Pack2<T>::run(o[c4 * 8 + 4], o[c4 * 8 + 5]);
+          v.w = Pack2<T>::run(o[c4 * 8 + 6], o[c4 * 8 + 7]);
+          sts128(stage + (uint32_t)lane * 64 + ((c4 ^ swz) << 4), v);
+        }
+        fence_proxy_async_smem();
+        __syncwarp();
+        const int row0 = m0 + (warp & 3) * 32;
+        if (lane == 0 && row0 < p.N_q) {
+          tma_store_4d_hint(&tmap_o, stage, half * 32, row0, h, b, l2_policy_evict_first());
+          bulk_commit_group();
+        }
+        if (a.lse != nullptr && half == 0 && row < p.N_q)
+          a.lse[(int64_t)b * a.lse_stride[0] + (int64_t)h * a.lse_stride[1] + (int64_t)row * a.lse_stride[2]] =
+              m_all * kLn2 + logf((l_sum == 0.f) ? 1.f : l_sum);
+      }
+      if (n_tiles > 0) {
+        g += n_tiles;
+        ++qi;
+      }
+    }
+    if (lane == 0) bulk_wait_all();   // the staged rows must have left shared memory before the CTA exits
+  } else if (ROT_K && warp == WARP_ROTATE64) {
+    // ============================== K rotation warp ==============================
+    TileCursor cu;
+    cursor_init(cu);
+    while (cursor_next<EMASK, SPLIT>(args, cu)) {
+      const int s = cu.gg & 1;
+      if (!mbar_wait(&bars->k_full[s], (cu.gg >> 1) & 1, abort_flag)) break;
+      const int key0 = cu.it.walk.key0(cu.j);
+#pragma unroll 1
+      for (int r = lane; r < BN; r += 32) {
+        const int pos = key0 + r;
+        if (pos < p.N_kv)
+          rope_row<T, D>(sK0 + s * C::TILE_BYTES, r, reinterpret_cast<const T*>(p.cos) + (int64_t)pos * p.rope_stride_n,
+                         reinterpret_cast<const T*>(p.sin) + (int64_t)pos * p.rope_stride_n);
+      }
+      fence_proxy_async_smem();
+      mbar_arrive(&bars->k_ready[s]);
+    }
+  }
+
+  tc_fence_before_sync();
+  __syncthreads();
+  if (tid == 0 && *abort_flag && p.status != nullptr) atomicExch(p.status, AF_STATUS_WAIT_TIMEOUT);
+  if (warp == WARP_PRODUCER) {
+    __syncwarp();
+    tc_fence_after_sync();
+    tmem_dealloc(tmem, C::TMEM_COLS);
+  }
+}
+
+template <typename T, int ROPE, int EMASK, bool ALIBI, int SPLIT = SPLIT_NONE>
+int launch_d64_instance(const TcArgs& args, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
+                        const CUtensorMap& mo, cudaStream_t st) {
+  auto kern = fwd_d64_kernel<T, ROPE, EMASK, ALIBI, SPLIT>;
+  constexpr int smem = Cfg64::SMEM_BYTES;
+  static bool configured = false;   // benign race: the attribute call is idempotent
+  if (!configured) {
+    AF_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    // all of the SM's storage as shared memory, or the second CTA may not fit
+    AF_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+    configured = true;
+  }
+  kern<<<(unsigned)args.grid_ctas, threads64(ROPE), smem, st>>>(args, mq, mk, mv, mo);
+  count_launch();
+  return check_cuda(cudaGetLastError(), "fwd_d64 launch");
+}
+
+// Composition -> instantiation table for one (dtype, RoPE mode).
+template <typename T, int ROPE>
+int launch_d64_composition(const TcArgs& args, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
+                           const CUtensorMap& mo, cudaStream_t st) {
+  const AfProblem& p = args.a.p;
+  const bool alibi = p.bias_kind == AF_BIAS_ALIBI;
+  if constexpr (ROPE == ROPE_NONE) {
+    if (args.num_splits > 0) return launch_d64_instance<T, ROPE, EMASK_NONE, false, SPLIT_DECODE>(args, mq, mk, mv, mo, st);
+    if (p.mask_kind == AF_MASK_BLOCKS && p.kv_slot != nullptr)
+      return alibi ? launch_d64_instance<T, ROPE, EMASK_BITS, true>(args, mq, mk, mv, mo, st)
+                   : launch_d64_instance<T, ROPE, EMASK_BITS, false>(args, mq, mk, mv, mo, st);
+  } else {
+    // split-K decode takes no rotation, and the block-sparse call has no cos / sin
+    if (args.num_splits > 0 || p.mask_kind == AF_MASK_BLOCKS)
+      return fail(AF_ERR_UNSUPPORTED, "split-K decode and block lists take no rotation");
+  }
+  const int em = p.mask_kind == AF_MASK_CAUSAL ? EMASK_CAUSAL : p.mask_kind == AF_MASK_WINDOW ? EMASK_WINDOW : EMASK_NONE;
+  switch (em * 2 + (alibi ? 1 : 0)) {
+    case 0: return launch_d64_instance<T, ROPE, EMASK_NONE, false>(args, mq, mk, mv, mo, st);
+    case 1: return launch_d64_instance<T, ROPE, EMASK_NONE, true>(args, mq, mk, mv, mo, st);
+    case 2: return launch_d64_instance<T, ROPE, EMASK_CAUSAL, false>(args, mq, mk, mv, mo, st);
+    case 3: return launch_d64_instance<T, ROPE, EMASK_CAUSAL, true>(args, mq, mk, mv, mo, st);
+    case 4: return launch_d64_instance<T, ROPE, EMASK_WINDOW, false>(args, mq, mk, mv, mo, st);
+    default: return launch_d64_instance<T, ROPE, EMASK_WINDOW, true>(args, mq, mk, mv, mo, st);
+  }
+}
+
+#define AF_DEFINE_D64_UNIT(NAME, ROPE_MODE)                                                                  \
+  int NAME(int dtype, const TcArgs& args, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, \
+           const CUtensorMap& mo, cudaStream_t st) {                                                         \
+    if (dtype == AF_F16) return launch_d64_composition<__half, ROPE_MODE>(args, mq, mk, mv, mo, st);         \
+    return launch_d64_composition<__nv_bfloat16, ROPE_MODE>(args, mq, mk, mv, mo, st);                       \
+  }
+
+}  // namespace tc
+}  // namespace af

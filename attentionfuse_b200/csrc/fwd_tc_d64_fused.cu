@@ -1,9 +1,9 @@
 // Instantiations of the tcgen05 forward kernel: head_dim 64, RoPE mode ROPE_FUSED, both half
 // precision element types, every (element mask, ALiBi) composition.
-#include "fwd_tcgen05.cuh"
+#include "fwd_d64_tcgen05.cuh"
 
 namespace af {
 namespace tc {
-AF_DEFINE_TC_UNIT(launch_d64_fused, 64, ROPE_FUSED)
+AF_DEFINE_D64_UNIT(launch_d64_fused, ROPE_FUSED)
 }  // namespace tc
 }  // namespace af

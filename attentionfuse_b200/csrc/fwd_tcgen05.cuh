@@ -2,7 +2,8 @@
 //
 // Replaces the reference forward kernel (attnfuse/compiler/codegen.py:67-381) and its
 // block-sparse sibling (attnfuse/compiler/codegen_blocksparse.py:34-171) for f16/bf16 inputs
-// with head_dim 64 or 128 and softmax normalisation.
+// with head_dim 128 and softmax normalisation (head_dim 64: fwd_d64_tcgen05.cuh, which shares the
+// item order, the softmax step and the rotation of this file).
 //
 // A work item is 128 query rows of one (batch, query head) against its 128-key tiles.  The kernel
 // is persistent: one CTA per SM takes items in a zig-zag over the heaviest-first item list, and
@@ -72,10 +73,10 @@ template <int D> struct Cfg {
   // (after the tile's softmax), so a V slot freed by P.V of tile j is not needed before tile j+2
   // has gone through the softmax group: two V stages suffice at head dim 128, and the tile they
   // leave free stages the output rows for a TMA store.
-  static constexpr int STAGES = (D == 128) ? 3 : 4;            // K ring
-  static constexpr int STAGES_V = (D == 128) ? 2 : 4;          // V ring
-  // 8 regions [half][row quadrant] of 32 rows; a row of a region holds D/2 elements and sits on
-  // the 128-byte pitch of the swizzle whether it fills it (D = 128) or not (D = 64)
+  static_assert(D == 128, "head dim 64 has a kernel of its own (fwd_d64_tcgen05.cuh)");
+  static constexpr int STAGES = 3;                             // K ring
+  static constexpr int STAGES_V = 2;                           // V ring
+  // 8 regions [half][row quadrant] of 32 rows of D/2 elements
   static constexpr int O_STAGE_BYTES = 8 * 32 * 128;
   static constexpr int SMEM_BYTES = TILE_BYTES * (1 + STAGES + STAGES_V) + O_STAGE_BYTES + 1024 /*align*/ +
                                     1536 /*barriers, exchange*/;
@@ -93,7 +94,7 @@ struct Barriers {
   uint64_t q_full, q_ready, q_empty;
   uint64_t k_full[4], k_ready[4], k_empty[4];
   uint64_t v_full[4], v_empty[4];
-  uint64_t s_full[2][2], p_full[2][2], pv_done[2][2];   // [S buffer][half of the key columns]; head dim 128 uses [.][0] of s_full / pv_done
+  uint64_t s_full[2], p_full[2][2], pv_done[2];   // [S buffer], p_full also [half of the key columns]
   uint64_t o_free;
   uint32_t tmem_base;
   int abort_flag;
@@ -371,7 +372,8 @@ __device__ __forceinline__ float ex2_approx(float x) {
 // cannot overwrite a word its partner has not read yet.  The wait is bounded like the mbarrier
 // waits (a hardware named barrier would hang if the partner left after a time-out).  It orders
 // shared-memory traffic only: the two warps never touch each other's TMEM columns.
-__device__ __forceinline__ bool pair_sync(Barriers* bars, int warp, int lane, uint32_t& count,
+template <typename BARS>
+__device__ __forceinline__ bool pair_sync(BARS* bars, int warp, int lane, uint32_t& count,
                                           volatile int* abort_flag) {
   ++count;
   __syncwarp();
@@ -410,11 +412,11 @@ __device__ __forceinline__ float row_max(const uint32_t (&xr)[NC]) {
 
 // P = 2^y packed to T and the row sum of the unrounded values, with
 //   EXP_SCALE      y = x * scale2 + shift
-//   EXP_AFFINE     y = x * scale2 + slope_c * c + shift     (ALiBi folded in, c = column index)
+//   EXP_AFFINE     y = x * scale2 + slope_c * (c + OFF) + shift     (ALiBi folded in, c = column index)
 //   EXP_PRESCALED  y = x + shift                            (scores already scaled and biased)
 // on packed fp32 pairs.
 enum { EXP_SCALE = 0, EXP_AFFINE = 1, EXP_PRESCALED = 2 };
-template <typename T, int KIND, int NC>
+template <typename T, int KIND, int NC, int OFF = 0>
 __device__ __forceinline__ void exp_pass(const uint32_t (&xr)[NC], uint32_t (&pk)[NC / 2], float scale2, float shift,
                                          float slope_c, float& rsum) {
   if (KIND == EXP_AFFINE) {
@@ -425,7 +427,7 @@ __device__ __forceinline__ void exp_pass(const uint32_t (&xr)[NC], uint32_t (&pk
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         const float x = __uint_as_float(xr[c + u]);
-        e[u] = ex2_approx(fmaf(x, scale2, fmaf(slope_c, (float)(c + u), shift)));
+        e[u] = ex2_approx(fmaf(x, scale2, fmaf(slope_c, (float)(OFF + c + u), shift)));
         rs4[u] += e[u];
       }
       pk[c >> 1] = Pack2<T>::run(e[0], e[1]);
@@ -467,13 +469,7 @@ fwd_tcgen05_kernel(const TcArgs args, const __grid_constant__ CUtensorMap tmap_q
   constexpr int STAGES = C::STAGES, STAGES_V = C::STAGES_V;
   constexpr bool ROT_K = (ROPE == ROPE_FUSED);
   constexpr int AB_FMT = (Elem<T>::code == AF_BF16) ? 1 : 0;
-  // Head dim 64: one S product per half of the key columns, each with barriers of its own, so the
-  // two softmax streams of a row never wait for each other (the operands are small enough that
-  // reading Q twice per tile does not load the shared-memory port; at head dim 128 it does, and
-  // the whole-tile product is faster there).
-  constexpr bool SPLIT_S = (D == 64);
-  constexpr int S_PARTS = SPLIT_S ? 2 : 1;
-  constexpr uint32_t IDESC_QK = umma_idesc_f16(AB_FMT, BM, SPLIT_S ? HALF_COLS : BN, 0, 0);
+  constexpr uint32_t IDESC_QK = umma_idesc_f16(AB_FMT, BM, BN, 0, 0);
   constexpr uint32_t IDESC_PV = umma_idesc_f16(AB_FMT, BM, D, 0, 1);
 
   const AfFwdParams& a = args.a;
@@ -509,11 +505,9 @@ fwd_tcgen05_kernel(const TcArgs args, const __grid_constant__ CUtensorMap tmap_q
       mbar_init(&bars->v_empty[s], 1);
     }
     for (int t = 0; t < 2; ++t) {
-      for (int hh = 0; hh < 2; ++hh) {
-        mbar_init(&bars->s_full[t][hh], 1);
-        mbar_init(&bars->p_full[t][hh], SOFTMAX_THREADS / 2);
-        mbar_init(&bars->pv_done[t][hh], 1);
-      }
+      mbar_init(&bars->s_full[t], 1);
+      mbar_init(&bars->pv_done[t], 1);
+      for (int hh = 0; hh < 2; ++hh) mbar_init(&bars->p_full[t][hh], SOFTMAX_THREADS / 2);
     }
     bars->abort_flag = 0;
     for (int i = 0; i < 16; ++i) (&bars->pair_flag[0][0])[i] = 0u;
@@ -612,20 +606,16 @@ fwd_tcgen05_kernel(const TcArgs args, const __grid_constant__ CUtensorMap tmap_q
           // Descriptors are built once; a k-step, a ring stage or a half only moves the
           // start-address field (address >> 4), so the issuing thread spends one add per operand.
           const uint64_t kdesc = desc_k0 + (uint64_t)((s * C::TILE_BYTES) >> 4);
-          for (int hh = 0; hh < S_PARTS && ok; ++hh) {
-            // S buffer t (the half's columns of it) still holds P of tile gg-2 until its P.V product has run
-            if (gg >= 2 && !mbar_wait(&bars->pv_done[t][hh], ((gg >> 1) - 1) & 1, abort_flag)) { ok = false; break; }
-            tc_fence_after_sync();
-            const uint32_t d_tmem = tmem + (t ? C::COL_S1 : C::COL_S0) + hh * HALF_COLS;
-            const uint64_t kh = kdesc + (uint64_t)((hh * HALF_COLS * 128) >> 4);   // keys 64 hh .. : rows of the K tile
+          // S buffer t still holds P of tile gg-2 until its P.V product has run
+          if (gg >= 2 && !mbar_wait(&bars->pv_done[t], ((gg >> 1) - 1) & 1, abort_flag)) { ok = false; break; }
+          tc_fence_after_sync();
+          const uint32_t d_tmem = tmem + (t ? C::COL_S1 : C::COL_S0);
 #pragma unroll
-            for (int kk = 0; kk < D / 16; ++kk) {
-              const uint64_t off = (uint64_t)(((kk >> 2) * PANEL_BYTES + (kk & 3) * 32) >> 4);
-              umma_ss(d_tmem, desc_q0 + off, kh + off, IDESC_QK, kk > 0 ? 1u : 0u);
-            }
-            umma_commit(&bars->s_full[t][hh]);
+          for (int kk = 0; kk < D / 16; ++kk) {
+            const uint64_t off = (uint64_t)(((kk >> 2) * PANEL_BYTES + (kk & 3) * 32) >> 4);
+            umma_ss(d_tmem, desc_q0 + off, kdesc + off, IDESC_QK, kk > 0 ? 1u : 0u);
           }
-          if (!ok) break;
+          umma_commit(&bars->s_full[t]);
           umma_commit(&bars->k_empty[s]);
           // the item's last S product: the Q buffer may be refilled when it has run
           if (j + 1 == n_tiles) umma_commit(&bars->q_empty);
@@ -666,11 +656,10 @@ fwd_tcgen05_kernel(const TcArgs args, const __grid_constant__ CUtensorMap tmap_q
               umma_ts(o_tmem, p_tmem + kk * 8, vdesc + (uint64_t)(((hh * 4 + kk) * 2048) >> 4), IDESC_PV,
                       (j > 0 || kk > 0) ? 1u : 0u);
             }
-            if (SPLIT_S) umma_commit(&bars->pv_done[t][hh]);
           }
           if (!ok) break;
           umma_commit(&bars->v_empty[s]);
-          if (!SPLIT_S) umma_commit(&bars->pv_done[t][0]);
+          umma_commit(&bars->pv_done[t]);
         }
         g += n_tiles;
         ++qi;
@@ -713,7 +702,7 @@ fwd_tcgen05_kernel(const TcArgs args, const __grid_constant__ CUtensorMap tmap_q
         const int gg = g + j;                       // the CTA's running key-tile count
         const int t = gg & 1;
         const int key0 = walk.key0(j);
-        if (!mbar_wait(&bars->s_full[t][SPLIT_S ? half : 0], (gg >> 1) & 1, abort_flag)) { alive = false; break; }
+        if (!mbar_wait(&bars->s_full[t], (gg >> 1) & 1, abort_flag)) { alive = false; break; }
         tc_fence_after_sync();
         const uint32_t s_tmem = tmem + lane_base + (t ? C::COL_S1 : C::COL_S0);
         const uint32_t o_tmem = tmem + lane_base + (half ? C::COL_O1 : C::COL_O0);
@@ -795,7 +784,7 @@ fwd_tcgen05_kernel(const TcArgs args, const __grid_constant__ CUtensorMap tmap_q
           if (j > 0 && __any_sync(0xffffffffu, bump)) {
             // The accumulator is expressed relative to the old reference: rescale it in TMEM once
             // the previous P.V product has landed.
-            if (!mbar_wait(&bars->pv_done[(gg - 1) & 1][SPLIT_S ? half : 0], ((gg - 1) >> 1) & 1, abort_flag)) { alive = false; break; }
+            if (!mbar_wait(&bars->pv_done[(gg - 1) & 1], ((gg - 1) >> 1) & 1, abort_flag)) { alive = false; break; }
             tc_fence_after_sync();
 #pragma unroll
             for (int c = 0; c < D / 32; ++c) {
@@ -868,8 +857,7 @@ fwd_tcgen05_kernel(const TcArgs args, const __grid_constant__ CUtensorMap tmap_q
       }
       if (n_tiles > 0) {
         const int gl = g + n_tiles - 1;
-        if (!mbar_wait(&bars->pv_done[gl & 1][0], (gl >> 1) & 1, abort_flag) ||
-            (SPLIT_S && !mbar_wait(&bars->pv_done[gl & 1][1], (gl >> 1) & 1, abort_flag))) { alive = false; break; }
+        if (!mbar_wait(&bars->pv_done[gl & 1], (gl >> 1) & 1, abort_flag)) { alive = false; break; }
         tc_fence_after_sync();
       }
       float o[D / 2];

@@ -55,7 +55,7 @@ int encode_map(CUtensorMap* out, int dtype, const void* ptr, int B, int H, int N
                int box_cols);
 
 // (B, H, N, D) tensor with element strides -> 4-D tiled map {D, N, H, B}, box box_cols x box_rows x 1 x 1
-// (box_cols * 2 bytes <= 128, the swizzle span).
+// (box_cols * 2 bytes <= 128; the swizzle spans 64 bytes for boxes of up to 32 columns, else 128).
 int make_map(CUtensorMap* out, int dtype, const void* ptr, int B, int H, int N, int D, const int64_t* st,
              int box_rows = 128, int box_cols = 64) {
   const MapKey key{ptr, st[0], st[1], st[2], dtype, B, H, N, D, box_rows + (box_cols << 16)};
@@ -92,7 +92,7 @@ int encode_map(CUtensorMap* out, int dtype, const void* ptr, int B, int H, int N
   cuuint32_t estr[4] = {1, 1, 1, 1};
   CUresult r = fn(out, dtype == AF_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4,
                   const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                  box_cols * 2 <= 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(AF_ERR_CUDA, "cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
   return AF_OK;
 }
@@ -516,7 +516,8 @@ int launch_fwd_tcgen05(const AfFwdParams& a, cudaStream_t st) {
   { const int rc_sm = tc_sm_count(&sms); if (rc_sm != AF_OK) return rc_sm; }
   const FwdSetup setup = set_up(a, sms);
   const FwdPlan& plan = setup.plan;
-  auto set_grid = [&]() { args.grid_ctas = (sms > 0 && sms < args.total_items) ? sms : args.total_items; };
+  const int ctas = p.D == 64 ? 2 * sms : sms;   // resident at once
+  auto set_grid = [&]() { args.grid_ctas = (ctas > 0 && ctas < args.total_items) ? ctas : args.total_items; };
   args.key_shares = 1;
   {
     // One CTA fits per SM (shared memory), so the kernel runs persistently: one CTA per SM walks
@@ -630,7 +631,8 @@ int launch_decode_split_tc(const AfDecodeParams& a, cudaStream_t st) {
   set_item_order(args, p.B * p.H_q, p.B * p.H_q, a.num_splits);   // splits x (batch, pseudo-head), plain order
   int sms = 0;
   { const int rc_sm = tc_sm_count(&sms); if (rc_sm != AF_OK) return rc_sm; }
-  args.grid_ctas = (sms > 0 && sms < args.total_items) ? sms : args.total_items;
+  const int ctas = a.D == 64 ? 2 * sms : sms;
+  args.grid_ctas = (ctas > 0 && ctas < args.total_items) ? ctas : args.total_items;
   CUtensorMap mq, mk, mv;
   int rc;
   if ((rc = make_map(&mq, a.dtype, a.q, a.B, a.H_kv, group, a.D, qs)) != AF_OK) return rc;

@@ -1,0 +1,77 @@
+"""The head_dim 64 forward (two CTAs per SM, a thread's 64 key columns in two runs of 32) where its
+branches change: runs that are fully, partly or not masked, maxima that jump inside a run, more
+items than are resident at once.  Against the CPU oracle on the same inputs."""
+import pytest
+import torch
+
+import attentionfuse_b200 as af
+from attentionfuse_b200.runtime.dispatch import _alibi_slopes
+from oracle import attention_oracle as orc
+from tests._util import assert_close, qkv
+
+pytestmark = pytest.mark.gpu
+DEV, D = "cuda", 64
+
+
+def graph(mask, window, alibi_heads):
+    @af.attention
+    def fn(Q, K, V):
+        s = af.scaled_dot_product(Q, K)
+        if alibi_heads:
+            s = af.alibi(s, alibi_heads)
+        s = af.causal(s) if mask == "causal" else af.sliding_window(s, window) if mask == "window" else s
+        return af.softmax(s) @ V
+    return fn
+
+
+def check(Q, K, V, mask, window=0, alibi=False, off=0):
+    H, dt = Q.shape[1], Q.dtype
+    fn = graph(mask, window, H if alibi else 0)
+    got = fn(Q.to(DEV), K.to(DEV), V.to(DEV), **(dict(q_offset=off) if Q.shape[2] != K.shape[2] else {}))
+    slopes = _alibi_slopes(H, DEV, str(dt)).cpu() if alibi else None
+    want = orc.attention(Q, K, V, causal=mask == "causal", window=window if mask == "window" else None, slopes=slopes, q_offset=off)
+    assert_close(got, want, dt, what=f"d64 {mask} w{window} {tuple(Q.shape)} off {off}")
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("alibi", [False, True])
+@pytest.mark.parametrize("mask,window", [("none", 0), ("causal", 0), ("window", 1), ("window", 31), ("window", 33), ("window", 97), ("window", 256)])
+@pytest.mark.parametrize("N_q,N_kv,off", [(2, 33, 31), (33, 34, 1), (129, 161, 0), (200, 351, 151), (384, 384, 0), (100, 800, 613)])
+def test_masks_at_run_edges(N_q, N_kv, off, mask, window, alibi, dtype):
+    Q, K, V = qkv(9100 + N_q + window, 2, 4, 2, N_q, N_kv, D, dtype)
+    check(Q, K, V, mask, window, alibi, off)
+
+
+@pytest.mark.parametrize("mask", ["none", "causal"])
+@pytest.mark.parametrize("where", [5, 40, 70, 127, 200, 255])
+def test_maximum_jumps_inside_a_run(where, mask):
+    """One key far larger than the rest: its run fails the row-sum check of the standing reference and
+    the tile is done again, the other three runs of the tile are not touched."""
+    Q, K, V = qkv(9200 + where, 1, 2, 2, 300, 300, D, torch.bfloat16)
+    Q = Q.abs()
+    K[:, :, where] = 6.0 + 0.1 * K[:, :, where].abs()
+    check(Q, K, V, mask)
+
+
+@pytest.mark.parametrize("shape", [(5, 16, 16, 601), (2, 320, 320, 120)], ids=str)
+@pytest.mark.parametrize("mask,window", [("none", 0), ("causal", 0), ("window", 130)])
+def test_more_items_than_resident_ctas(shape, mask, window):
+    B, H, H_kv, N = shape
+    Q, K, V = qkv(9300 + N, B, H, H_kv, N, N, D, torch.float16)
+    check(Q, K, V, mask, window)
+
+
+def test_infinite_and_lowest_scores():
+    """Scores of -inf and of fp16's lowest value are probabilities of zero; a row of NaN stays NaN and its
+    neighbours do not see it."""
+    Q, K, V = qkv(9400, 1, 2, 2, 160, 160, D, torch.float16)
+    Q[0, 0, 7] = float("nan")
+    K[0, 1, 3] = -60000.0
+    Q[0, 1] = Q[0, 1].abs() + 0.5
+    got = graph("none", 0, 0)(Q.to(DEV), K.to(DEV), V.to(DEV))
+    assert torch.isnan(got[0, 0, 7]).all()
+    keep = torch.ones(160, dtype=torch.bool)
+    keep[7] = False
+    want = orc.attention(Q.nan_to_num(0.0), K, V)
+    assert_close(got[0, 0, keep], want[0, 0, keep], torch.float16, what="rows beside NaN")
+    assert_close(got[0, 1], want[0, 1], torch.float16, what="key at the lowest values")

@@ -62,9 +62,9 @@ template <int D, int MODE = MODE_DKV> struct BCfg {
   static constexpr int STAT_PANEL = BS * 128;               // bytes of a 128-row, 64-element panel
   static constexpr int STAT_TILE = PANELS * STAT_PANEL;
   // Rows of a streamed tile = columns of S per step.  What bounds a step is as much the two issuing
-  // threads as the tensor pipe: every barrier wait that is already over costs them 130 - 180 clocks, an
-  // MMA about 60, a commit 70 (timeline of a head dim 64 dQ step of 64 columns: 1030 clocks, all of it
-  // the first issuing thread's, for 512 clocks of products).  Head dim 64 takes 128 columns a step --
+  // threads as the tensor pipe: before they walked as whole warps, every barrier wait that was already over
+  // cost them 130 - 180 clocks, an MMA about 60, a commit 70 (timeline of a head dim 64 dQ step of 64
+  // columns: 1030 clocks, all of it the first issuing thread's, for 512 clocks of products).  Head dim 64 takes 128 columns a step --
   // N = 128 products also read the stationary operand half as often -- head dim 128 has no TMEM
   // columns left for that.
   static constexpr int BT = (D == 64) ? 128 : 64;
@@ -303,7 +303,8 @@ bwd_tcgen05_kernel(const BwdArgs args, const __grid_constant__ CUtensorMap map_a
   BBarriers* bars = reinterpret_cast<BBarriers*>(smem + STAGE0_OFF + STAGES * STAGE_BYTES);
   volatile int* abort_flag = &bars->abort_flag;
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);   // uniform
   const int group = p.H_q / p.H_kv;
   const int n_heads = KVS ? group : 1;
 
@@ -317,7 +318,7 @@ bwd_tcgen05_kernel(const BwdArgs args, const __grid_constant__ CUtensorMap map_a
       mbar_init(&bars->strm_full[s], 1);
       mbar_init(&bars->strm_empty[s], 1);
       mbar_init(&bars->sched_full[s], 1);
-      mbar_init(&bars->sched_empty[s], 2 + C::EW_THREADS + C::DRAIN_THREADS);   // every role but the producer
+      mbar_init(&bars->sched_empty[s], 2 * 32 + C::EW_THREADS + C::DRAIN_THREADS);   // every role but the producer
     }
     for (int t = 0; t < 2; ++t) {
       mbar_init(&bars->xy_full[t], 1);
@@ -343,7 +344,7 @@ bwd_tcgen05_kernel(const BwdArgs args, const __grid_constant__ CUtensorMap map_a
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
-  const uint32_t tmem = bars->tmem_base;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, bars->tmem_base, 0);
 
   // Every role walks the same item sequence.  `it0` counts the steps of the items before the
   // current one: ring stages, X/Y buffers and barrier phases run on the running count, so that the
@@ -459,8 +460,12 @@ bwd_tcgen05_kernel(const BwdArgs args, const __grid_constant__ CUtensorMap map_a
     // ============================== MMA issuer 1: S / dP products ==============================
     // Two issuing threads feed the tensor pipe: a tcgen05.mma issue blocks while the pipe's short
     // queue is full, so one thread issuing both kinds leaves the pipe idle during its own barrier
-    // waits and commits (measured: 1800 - 2100 cycles per step for 1000 - 1300 cycles of MMA).
-    if (lane == 0) {
+    // waits and commits (measured: 1800 - 2100 cycles per step for 1000 - 1300 cycles of MMA).  Both walk as
+    // whole warps with one elected lane that issues: the operands are then uniform values, which the
+    // products take without a move each.  Training step, forward included: [4,12,4096,64] causal 648 -> 613 us,
+    // Llama layer 2440 -> 2354.
+    {
+      const bool leader = elect_one();
       const uint64_t desc_a1 = umma_desc_sw128(sA1, 16, 1024), desc_a2 = umma_desc_sw128(sA2, 16, 1024);
       const uint64_t desc_b1k = umma_desc_sw128(sStage0, 16, 1024);              // streamed tile, K-major
       const uint64_t desc_ones = umma_desc_sw128(smem_base + C::ONES_OFF, 16, 1024);
@@ -486,31 +491,32 @@ bwd_tcgen05_kernel(const BwdArgs args, const __grid_constant__ CUtensorMap map_a
         const uint64_t b1 = desc_b1k + (uint64_t)((st * STAGE_BYTES) >> 4), b2 = b1 + (uint64_t)(C::STRM_TILE >> 4);
         const uint32_t xt = tmem + C::col_x(t), yt = tmem + C::col_y(t);
         const uint64_t bs = desc_stats + (uint64_t)(((st >> 1) * C::STATS_TILE + (st & 1) * 64) >> 4);   // L terms; delta: 32 bytes on
-        if (KVS) umma_ss(xt, desc_ones, bs, IDESC_STATS, 0u);
+        if (KVS && leader) umma_ss(xt, desc_ones, bs, IDESC_STATS, 0u);
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk)
-          umma_ss(xt, desc_a1 + (uint64_t)(((kk >> 2) * C::STAT_PANEL + (kk & 3) * 32) >> 4),
+          if (leader) umma_ss(xt, desc_a1 + (uint64_t)(((kk >> 2) * C::STAT_PANEL + (kk & 3) * 32) >> 4),
                   b1 + (uint64_t)(((kk >> 2) * C::STRM_PANEL + (kk & 3) * 32) >> 4), IDESC_XY, (KVS || kk > 0) ? 1u : 0u);
         if (C::Y_SINGLE && it >= 1) {
           // the single dP buffer: the element-wise threads have loaded the previous step's values
           if (!mbar_wait(&bars->y_free, (it - 1) & 1, abort_flag)) { ok = false; break; }
           tc_fence_after_sync();
         }
-        if (KVS) umma_ss(yt, desc_ones, bs + 2, IDESC_STATS, 0u);
+        if (KVS && leader) umma_ss(yt, desc_ones, bs + 2, IDESC_STATS, 0u);
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk)
-          umma_ss(yt, desc_a2 + (uint64_t)(((kk >> 2) * C::STAT_PANEL + (kk & 3) * 32) >> 4),
+          if (leader) umma_ss(yt, desc_a2 + (uint64_t)(((kk >> 2) * C::STAT_PANEL + (kk & 3) * 32) >> 4),
                   b2 + (uint64_t)(((kk >> 2) * C::STRM_PANEL + (kk & 3) * 32) >> 4), IDESC_XY, (KVS || kk > 0) ? 1u : 0u);
-        umma_commit(&bars->xy_full[t]);
+        if (leader) umma_commit(&bars->xy_full[t]);
       }
-      if (ok) umma_commit(&bars->stat_empty);   // the item's last products: the stationary tiles may be refilled
+      if (ok && leader) umma_commit(&bars->stat_empty);   // the item's last products: the stationary tiles may be refilled
       it0 += bi.total_steps;
       ++qi;
       }
     }
   } else if (warp == WARP_MMA2) {
     // ============================== MMA issuer 2: gradient accumulation ==============================
-    if (lane == 0) {
+    {
+      const bool leader = elect_one();
       const uint64_t desc_b1n = umma_desc_sw128(sStage0, C::STRM_PANEL, 1024);   // streamed tile, N-major
       // fused mode: dS^T (128 keys x 64 queries, query-contiguous) as N-major B;
       // the stationary K tile (128 keys x D) as M-major A (M = d: 64-element panels LBO apart)
@@ -534,12 +540,12 @@ bwd_tcgen05_kernel(const BwdArgs args, const __grid_constant__ CUtensorMap map_a
         if (KVS) {
 #pragma unroll
           for (int kk = 0; kk < BT / 16; ++kk)      // dV += P^T dO
-            umma_ts(tmem + C::COL_ACC1, tmem + C::col_p(t, kk), b2 + (uint64_t)((kk * 2048) >> 4), IDESC_ACC,
+            if (leader) umma_ts(tmem + C::COL_ACC1, tmem + C::col_p(t, kk), b2 + (uint64_t)((kk * 2048) >> 4), IDESC_ACC,
                     (!first || kk > 0) ? 1u : 0u);
         }
 #pragma unroll
         for (int kk = 0; kk < BT / 16; ++kk)        // dK += dS^T Q, or dQ += dS K
-          umma_ts(tmem + (KVS ? C::COL_ACC2 : C::COL_ACC1), tmem + C::col_ds(t, kk), b1 + (uint64_t)((kk * 2048) >> 4),
+          if (leader) umma_ts(tmem + (KVS ? C::COL_ACC2 : C::COL_ACC1), tmem + C::col_ds(t, kk), b1 + (uint64_t)((kk * 2048) >> 4),
                   IDESC_ACC, (!first || kk > 0) ? 1u : 0u);
         if (FUSED) {
           const uint64_t ds_n = desc_ds_n + (uint64_t)((t * C::DS_TILE) >> 4);
@@ -550,13 +556,13 @@ bwd_tcgen05_kernel(const BwdArgs args, const __grid_constant__ CUtensorMap map_a
           }
 #pragma unroll
           for (int kk = 0; kk < BS / 16; ++kk)      // dQ^T = K^T dS^T over the 128 keys
-            umma_ss(tmem + C::COL_Z, desc_k_m + (uint64_t)((kk * 2048) >> 4), ds_n + (uint64_t)((kk * 2048) >> 4),
+            if (leader) umma_ss(tmem + C::COL_Z, desc_k_m + (uint64_t)((kk * 2048) >> 4), ds_n + (uint64_t)((kk * 2048) >> 4),
                     IDESC_DQT, kk > 0 ? 1u : 0u);
         }
-        umma_commit(&bars->acc_done[t]);
-        umma_commit(&bars->strm_empty[st]);
+        if (leader) umma_commit(&bars->acc_done[t]);
+        if (leader) umma_commit(&bars->strm_empty[st]);
       }
-      if (FUSED && ok) umma_commit(&bars->stat_empty);   // dQ^T reads the stationary K tile too
+      if (FUSED && ok && leader) umma_commit(&bars->stat_empty);   // dQ^T reads the stationary K tile too
       it0 += bi.total_steps;
       ++qi;
       }

@@ -485,7 +485,8 @@ fwd_tcgen05_kernel(const TcArgs args, const __grid_constant__ CUtensorMap tmap_q
   Barriers* bars = reinterpret_cast<Barriers*>(smem + C::TILE_BYTES * (1 + STAGES + STAGES_V) + C::O_STAGE_BYTES);
   volatile int* abort_flag = &bars->abort_flag;
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);   // uniform
 
   // Every role walks the same item sequence (get_item) and keeps two running counts: `g`, key
   // tiles processed so far by this CTA (ring stage g % STAGES, S buffer g & 1, barrier phases
@@ -520,7 +521,7 @@ fwd_tcgen05_kernel(const TcArgs args, const __grid_constant__ CUtensorMap tmap_q
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
-  const uint32_t tmem = bars->tmem_base;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, bars->tmem_base, 0);
 
   if (warp == WARP_PRODUCER) {
     // ============================== TMA producer ==============================
@@ -588,8 +589,11 @@ fwd_tcgen05_kernel(const TcArgs args, const __grid_constant__ CUtensorMap tmap_q
     // ============================== MMA issuer 1: S = Q K^T ==============================
     // The two products are issued by two threads.  A tcgen05.mma issue blocks while the pipe's
     // short queue is full, so a single issuing thread leaves the pipe idle during its own barrier
-    // waits and commits (measured: about 800 of 2000 cycles per key tile).
-    if (lane == 0) {
+    // waits and commits (measured: about 800 of 2000 cycles per key tile).  The whole warp walks the tiles
+    // and one elected lane issues: the operands are then uniform values (500 rows against 8011 keys: 70
+    // us, 73 with a lane that walks alone; fwd_d64_tcgen05.cuh says what such a lane paid).
+    {
+      const bool leader = elect_one();
       const uint64_t desc_q0 = umma_desc_sw128(sQ, 16, 1024);
       const uint64_t desc_k0 = umma_desc_sw128(sK0, 16, 1024);
       Item it;
@@ -613,12 +617,12 @@ fwd_tcgen05_kernel(const TcArgs args, const __grid_constant__ CUtensorMap tmap_q
 #pragma unroll
           for (int kk = 0; kk < D / 16; ++kk) {
             const uint64_t off = (uint64_t)(((kk >> 2) * PANEL_BYTES + (kk & 3) * 32) >> 4);
-            umma_ss(d_tmem, desc_q0 + off, kdesc + off, IDESC_QK, kk > 0 ? 1u : 0u);
+            if (leader) umma_ss(d_tmem, desc_q0 + off, kdesc + off, IDESC_QK, kk > 0 ? 1u : 0u);
           }
-          umma_commit(&bars->s_full[t]);
-          umma_commit(&bars->k_empty[s]);
+          if (leader) umma_commit(&bars->s_full[t]);
+          if (leader) umma_commit(&bars->k_empty[s]);
           // the item's last S product: the Q buffer may be refilled when it has run
-          if (j + 1 == n_tiles) umma_commit(&bars->q_empty);
+          if (leader && j + 1 == n_tiles) umma_commit(&bars->q_empty);
         }
         g += n_tiles;
         ++qi;
@@ -626,7 +630,8 @@ fwd_tcgen05_kernel(const TcArgs args, const __grid_constant__ CUtensorMap tmap_q
     }
   } else if (warp == WARP_PV) {
     // ============================== MMA issuer 2: O += P V ==============================
-    if (lane == 0) {
+    {
+      const bool leader = elect_one();
       const uint64_t desc_v0 = umma_desc_sw128(sV0, PANEL_BYTES, 1024);
       Item it;
       int g = 0, qi = 0;
@@ -653,13 +658,13 @@ fwd_tcgen05_kernel(const TcArgs args, const __grid_constant__ CUtensorMap tmap_q
             for (int kk = 0; kk < HALF_COLS / 16; ++kk) {
               // V tile is N-major: 16 keys = two 8-row groups (SBO 1024 B); the second 64 columns
               // of D live one panel further (LBO).  16 keys further = 2048 bytes.
-              umma_ts(o_tmem, p_tmem + kk * 8, vdesc + (uint64_t)(((hh * 4 + kk) * 2048) >> 4), IDESC_PV,
+              if (leader) umma_ts(o_tmem, p_tmem + kk * 8, vdesc + (uint64_t)(((hh * 4 + kk) * 2048) >> 4), IDESC_PV,
                       (j > 0 || kk > 0) ? 1u : 0u);
             }
           }
           if (!ok) break;
-          umma_commit(&bars->v_empty[s]);
-          umma_commit(&bars->pv_done[t]);
+          if (leader) umma_commit(&bars->v_empty[s]);
+          if (leader) umma_commit(&bars->pv_done[t]);
         }
         g += n_tiles;
         ++qi;

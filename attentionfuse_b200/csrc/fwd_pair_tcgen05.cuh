@@ -15,10 +15,9 @@
 // to the MMA thread on its own, so the P.V product of the first chunk runs under the exponent
 // pass of the second.
 //
-// Roles (384 threads): warps 0-3 softmax of slot 0, warps 4-7 softmax of slot 1, warp 8 TMA
-// producer (Q of both heads per item, K ring and V ring of two stages each), one thread each of
-// warps 9 and 11 issues S_0 / S_1 = Q_q K^T, one thread of warp 10 issues O_q += P_q V.  Every
-// wait is bounded.
+// Roles (352 threads): warps 0-3 softmax of slot 0, warps 4-7 softmax of slot 1, warp 8 TMA
+// producer (Q of both heads per item, K ring and V ring of two stages each), warps 9 and 10 issue the
+// products of slot 0 and 1.  Every wait is bounded.
 #pragma once
 #include "fwd_tcgen05.cuh"
 
@@ -37,11 +36,15 @@ struct PairCfg {
 };
 
 struct PairBarriers {
-  uint64_t q_full, q_empty;
-  uint64_t k_full[2], k_empty[2], v_full[2], v_empty[2];
+  uint64_t q_full;
+  uint64_t k_full[2], v_full[2];
+  // Group t of products of both slots, S of tile t and P.V of tile t - 1, has run (slot t & 1): K slot t & 1,
+  // V slot (t - 1) & 1 and, behind an item's last S, the Q buffers are free.
+  uint64_t ring_free[2];
   uint64_t s_full[2][2];     // [slot][chunk]: the chunk's 64 columns of S_q are in TMEM
   uint64_t p_full[2][2];     // [slot][chunk]: P of the chunk is in TMEM
-  uint64_t pv_done[2][2];    // [slot][chunk]: the chunk's P.V product has run
+  uint64_t pv_first[2];      // [slot]: the first chunk's P.V product of a tile has run
+  uint64_t o_done[2];        // [slot]: the item's last P.V product has run
   uint64_t o_free[2];        // [slot]: the item's accumulator has been read out
   uint32_t tmem_base;
   int abort_flag;
@@ -83,7 +86,7 @@ __device__ __forceinline__ bool pair_cursor_next(const TcArgs& args, TileCursor&
 }
 
 template <typename T, int EMASK, bool ALIBI>
-__global__ void __launch_bounds__(384, 1)
+__global__ void __launch_bounds__(352, 1)
 fwd_pair_kernel(const TcArgs args, const __grid_constant__ CUtensorMap tmap_q,
                 const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
                 const __grid_constant__ CUtensorMap tmap_o) {
@@ -111,19 +114,18 @@ fwd_pair_kernel(const TcArgs args, const __grid_constant__ CUtensorMap tmap_q,
 
   if (tid == 0) {
     mbar_init(&bars->q_full, 1);
-    mbar_init(&bars->q_empty, 2);      // one S-issuing thread per slot
     for (int s = 0; s < 2; ++s) {
       mbar_init(&bars->k_full[s], 1);
-      mbar_init(&bars->k_empty[s], 2);
       mbar_init(&bars->v_full[s], 1);
-      mbar_init(&bars->v_empty[s], 1);
+      mbar_init(&bars->ring_free[s], 2);   // one issuing thread per slot
     }
     for (int q = 0; q < 2; ++q) {
       mbar_init(&bars->o_free[q], BM);
+      mbar_init(&bars->o_done[q], 1);
+      mbar_init(&bars->pv_first[q], 1);
       for (int c = 0; c < 2; ++c) {
         mbar_init(&bars->s_full[q][c], 1);
         mbar_init(&bars->p_full[q][c], BM);
-        mbar_init(&bars->pv_done[q][c], 1);
       }
     }
     bars->abort_flag = 0;
@@ -154,7 +156,7 @@ fwd_pair_kernel(const TcArgs args, const __grid_constant__ CUtensorMap tmap_q,
       auto load_k = [&]() -> bool {
         if (ck.j == 0) {
           // both Q buffers are free once the last S product of the previous item has run
-          if (ck.qi > 0 && !mbar_wait(&bars->q_empty, (ck.qi - 1) & 1, abort_flag)) return false;
+          if (ck.qi > 0 && !mbar_wait(&bars->ring_free[(ck.gg - 1) & 1], ((ck.gg - 1) >> 1) & 1, abort_flag)) return false;
           mbar_arrive_expect_tx(&bars->q_full, 2 * C::TILE_BYTES);
 #pragma unroll
           for (int q = 0; q < 2; ++q)
@@ -164,7 +166,7 @@ fwd_pair_kernel(const TcArgs args, const __grid_constant__ CUtensorMap tmap_q,
                                ck.it.h + q, ck.it.b, stream);
         }
         const int s = ck.gg & 1;
-        if (ck.gg >= 2 && !mbar_wait(&bars->k_empty[s], ((ck.gg >> 1) & 1) ^ 1, abort_flag)) return false;
+        if (ck.gg >= 2 && !mbar_wait(&bars->ring_free[s], ((ck.gg - 2) >> 1) & 1, abort_flag)) return false;
         mbar_arrive_expect_tx(&bars->k_full[s], C::TILE_BYTES);
         const int key0 = ck.it.walk.key0(ck.j);
         unsigned char* dk = smem + C::TILE_BYTES * (2 + s);
@@ -175,7 +177,7 @@ fwd_pair_kernel(const TcArgs args, const __grid_constant__ CUtensorMap tmap_q,
       };
       auto load_v = [&]() -> bool {
         const int s = cv.gg & 1;
-        if (cv.gg >= 2 && !mbar_wait(&bars->v_empty[s], ((cv.gg >> 1) & 1) ^ 1, abort_flag)) return false;
+        if (cv.gg >= 2 && !mbar_wait(&bars->ring_free[(cv.gg - 1) & 1], ((cv.gg - 1) >> 1) & 1, abort_flag)) return false;
         mbar_arrive_expect_tx(&bars->v_full[s], C::TILE_BYTES);
         const int key0 = cv.it.walk.key0(cv.j);
         unsigned char* dv = smem + C::TILE_BYTES * (2 + C::STAGES + s);
@@ -200,75 +202,76 @@ fwd_pair_kernel(const TcArgs args, const __grid_constant__ CUtensorMap tmap_q,
         }
       }
     }
-  } else if (warp == WARP_QK || warp == WARP_ROTATE) {
-    // ============================== MMA issuers 1a / 1b: S_q = Q_q K^T ==============================
-    // One issuing thread per slot, in warps of different schedulers: the issuing threads take
-    // issue slots from the softmax warps they share a scheduler with, and the slowest of a slot's
-    // four softmax warps sets the slot's pace.  The whole warp walks the tiles and one elected lane issues,
-    // so that the operands are uniform values (headline step 609 -> 583 us).
+  } else if (warp == WARP_QK || warp == WARP_PV) {
+    // ============================== MMA issuers: O_q += P_q V, S_q = Q_q K^T ==============================
+    // One issuing warp per slot, on different schedulers: the issuing warps take issue slots from
+    // the softmax warps next to them, and the slowest of a slot's four softmax warps sets the slot's
+    // pace.  The whole warp walks the tiles and one elected lane issues, so that the operands are
+    // uniform values.  Products of one thread run in order: S of the next tile's chunk, over the
+    // columns that P of this one held, follows the chunk's P.V product into the pipe without a wait.
     {
       const bool leader = elect_one();
       const int q = (warp == WARP_QK) ? 0 : 1;
       const uint64_t qdesc = umma_desc_sw128(sQ + q * C::TILE_BYTES, 16, 1024);
       const uint64_t desc_k0 = umma_desc_sw128(sK0, 16, 1024);
-      TileCursor cu;
+      const uint64_t desc_v0 = umma_desc_sw128(sV0, PANEL_BYTES, 1024);
+      TileCursor cu;               // the tile whose S comes next
       cursor_init(cu);
-      bool ok = true;
-      while (ok && pair_cursor_next<EMASK>(args, cu)) {
-        const int gg = cu.gg, s = gg & 1;
-        if (cu.j == 0 && !mbar_wait(&bars->q_full, cu.qi & 1, abort_flag)) break;
-        if (!mbar_wait(&bars->k_full[s], (gg >> 1) & 1, abort_flag)) break;
-        const uint64_t kdesc = desc_k0 + (uint64_t)((s * C::TILE_BYTES) >> 4);
-        for (int c = 0; c < 2 && ok; ++c) {
-          // One product per chunk of 64 key columns (rows 64 c .. 64 c + 63 of the K tile): the
-          // chunk's S columns hold P of the previous tile's chunk until its P.V product has run,
-          // so the first chunk of the next tile is under way while the softmax group is still
-          // in the second chunk of this one.
-          if (gg >= 1 && !mbar_wait(&bars->pv_done[q][c], (gg - 1) & 1, abort_flag)) { ok = false; break; }
-          tc_fence_after_sync();
-          const uint32_t d_tmem = tmem + C::col_s(q) + c * 64;
-          const uint64_t kh = kdesc + (uint64_t)((c * 64 * 128) >> 4);
+      auto operands_ready = [&]() -> bool {
+        if (cu.j == 0 && !mbar_wait(&bars->q_full, cu.qi & 1, abort_flag)) return false;
+        return mbar_wait(&bars->k_full[cu.gg & 1], (cu.gg >> 1) & 1, abort_flag);
+      };
+      auto issue_s = [&](int c) {
+        const uint64_t kh = desc_k0 + (uint64_t)(((cu.gg & 1) * C::TILE_BYTES + c * 64 * 128) >> 4);
+        if (leader) {
 #pragma unroll
           for (int kk = 0; kk < D / 16; ++kk) {
             const uint64_t off = (uint64_t)(((kk >> 2) * PANEL_BYTES + (kk & 3) * 32) >> 4);
-            if (leader) umma_ss(d_tmem, qdesc + off, kh + off, IDESC_QK, kk > 0 ? 1u : 0u);
+            umma_ss(tmem + C::col_s(q) + c * 64, qdesc + off, kh + off, IDESC_QK, kk > 0 ? 1u : 0u);
           }
-          if (leader) umma_commit(&bars->s_full[q][c]);
+          umma_commit(&bars->s_full[q][c]);
         }
-        if (!ok) break;
-        if (leader) umma_commit(&bars->k_empty[s]);        // both slots' products have to be through before the stage is refilled
-        if (leader && cu.j + 1 == cu.it.walk.n_tiles) umma_commit(&bars->q_empty);
-      }
-    }
-  } else if (warp == WARP_PV) {
-    // ============================== MMA issuer 2: O_q += P_q V ==============================
-    {
-      const bool leader = elect_one();
-      const uint64_t desc_v0 = umma_desc_sw128(sV0, PANEL_BYTES, 1024);
-      TileCursor cu;
-      cursor_init(cu);
-      bool ok = true;
-      while (ok && pair_cursor_next<EMASK>(args, cu)) {
-        const int gg = cu.gg, s = gg & 1;
-        if (!mbar_wait(&bars->v_full[s], (gg >> 1) & 1, abort_flag)) break;
-        const uint64_t vdesc = desc_v0 + (uint64_t)((s * C::TILE_BYTES) >> 4);
-        for (int q = 0; q < 2 && ok; ++q) {
-          for (int c = 0; c < 2 && ok; ++c) {
+      };
+      bool more = pair_cursor_next<EMASK>(args, cu);
+      if (more && operands_ready()) {
+        issue_s(0);
+        issue_s(1);
+        if (leader) umma_commit(&bars->ring_free[0]);
+        while (more) {
+          const int gg = cu.gg, j = cu.j, qi = cu.qi, s = gg & 1;
+          const bool last = j + 1 == cu.it.walk.n_tiles;
+          more = pair_cursor_next<EMASK>(args, cu);
+          if (!mbar_wait(&bars->v_full[s], (gg >> 1) & 1, abort_flag)) break;
+          // the item's first product overwrites O_q: the previous item's rows must be read out
+          if (j == 0 && qi > 0 && !mbar_wait(&bars->o_free[q], (qi - 1) & 1, abort_flag)) break;
+          if (!last && !operands_ready()) break;
+          bool ok = true;
+          for (int c = 0; c < 2; ++c) {
             if (!mbar_wait(&bars->p_full[q][c], gg & 1, abort_flag)) { ok = false; break; }
-            // the item's first product overwrites O_q: the previous item's rows must be read out
-            if (cu.j == 0 && c == 0 && cu.qi > 0 && !mbar_wait(&bars->o_free[q], (cu.qi - 1) & 1, abort_flag)) { ok = false; break; }
             tc_fence_after_sync();
-            const uint32_t p_tmem = tmem + C::col_s(q) + c * 64;   // P of a chunk sits in the first 32 of its 64 S columns
-            const uint32_t o_tmem = tmem + C::col_o(q);
+            if (leader) {
 #pragma unroll
-            for (int kk = 0; kk < 4; ++kk)
-              if (leader) umma_ts(o_tmem, p_tmem + kk * 8, vdesc + (uint64_t)(((c * 4 + kk) * 2048) >> 4), IDESC_PV,
-                      (cu.j > 0 || c > 0 || kk > 0) ? 1u : 0u);
-            if (leader) umma_commit(&bars->pv_done[q][c]);
+              for (int kk = 0; kk < 4; ++kk)      // P of a chunk sits in the first 32 of its 64 S columns
+                umma_ts(tmem + C::col_o(q), tmem + C::col_s(q) + c * 64 + kk * 8,
+                        desc_v0 + (uint64_t)((s * C::TILE_BYTES + (c * 4 + kk) * 2048) >> 4), IDESC_PV,
+                        (j > 0 || c > 0 || kk > 0) ? 1u : 0u);
+              if (c == 0) umma_commit(&bars->pv_first[q]);
+            }
+            if (!last) issue_s(c);
           }
+          if (!ok) break;
+          if (last) {
+            if (leader) umma_commit(&bars->o_done[q]);
+            if (more) {
+              // the next item's Q comes after this item's last S products: its S follows both
+              // chunks of P.V, so that a late Q holds nothing up
+              if (!operands_ready()) break;
+              issue_s(0);
+              issue_s(1);
+            }
+          }
+          if (leader) umma_commit(&bars->ring_free[(gg + 1) & 1]);
         }
-        if (!ok) break;
-        if (leader) umma_commit(&bars->v_empty[s]);
       }
     }
   } else if (warp < 8) {
@@ -282,7 +285,7 @@ fwd_pair_kernel(const TcArgs args, const __grid_constant__ CUtensorMap tmap_q,
     const uint32_t o_tmem = tmem + lane_base + C::col_o(q);
     const float scale2 = p.sm_scale * kLog2e;     // > 0 (checked on the host)
     Item it, it_next;
-    int g = 0;
+    int g = 0, qi = 0;
     bool alive = true;
     bool have = get_pair_item<EMASK>(args, 0, it);
     for (int round = 0; alive && have; ++round) {
@@ -355,9 +358,9 @@ fwd_pair_kernel(const TcArgs args, const __grid_constant__ CUtensorMap tmap_q,
             const float neg_m = (m_next == -INFINITY) ? 0.f : -m_next;
             if ((j > 0 || c > 0) && __any_sync(0xffffffffu, bump)) {
               // The accumulator is expressed relative to the old reference: rescale it in TMEM once
-              // the previous chunk's P.V product has landed.
-              const bool prev_ok = (c == 1) ? mbar_wait(&bars->pv_done[q][0], gg & 1, abort_flag)
-                                            : mbar_wait(&bars->pv_done[q][1], (gg - 1) & 1, abort_flag);
+              // the previous chunk's P.V product has landed (the previous tile's second chunk: before
+              // this tile's second S, which the same thread issued after it).
+              const bool prev_ok = mbar_wait(c == 1 ? &bars->pv_first[q] : &bars->s_full[q][1], gg & 1, abort_flag);
               if (!prev_ok) { alive = false; break; }
               tc_fence_after_sync();
 #pragma unroll
@@ -388,8 +391,7 @@ fwd_pair_kernel(const TcArgs args, const __grid_constant__ CUtensorMap tmap_q,
       // the next item is decoded here, under the wait for the last P.V product
       const bool have_next = get_pair_item<EMASK>(args, round + 1, it_next);
       if (n_tiles > 0) {
-        const int gl = g + n_tiles - 1;
-        if (!mbar_wait(&bars->pv_done[q][1], gl & 1, abort_flag)) { alive = false; break; }
+        if (!mbar_wait(&bars->o_done[q], qi & 1, abort_flag)) { alive = false; break; }
         tc_fence_after_sync();
       }
       const float safe_l = (l_row == 0.f) ? 1.f : l_row;
@@ -433,6 +435,7 @@ fwd_pair_kernel(const TcArgs args, const __grid_constant__ CUtensorMap tmap_q,
         a.lse[(int64_t)b * a.lse_stride[0] + (int64_t)h * a.lse_stride[1] + (int64_t)row * a.lse_stride[2]] =
             m_ref * kLn2 + logf(safe_l);
       g += n_tiles;
+      if (n_tiles > 0) ++qi;
       it = it_next;
       have = have_next;
     }
@@ -459,7 +462,7 @@ int launch_pair_instance(const TcArgs& args, const CUtensorMap& mq, const CUtens
     AF_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     configured = true;
   }
-  kern<<<(unsigned)args.grid_ctas, 384, smem, st>>>(args, mq, mk, mv, mo);
+  kern<<<(unsigned)args.grid_ctas, 352, smem, st>>>(args, mq, mk, mv, mo);
   count_launch();
   return check_cuda(cudaGetLastError(), "fwd_pair launch");
 }

@@ -1,6 +1,6 @@
 // Host side of the tcgen05 backward: support predicate, workspace, TMA descriptors, and the
-// launches: delta, then either the two passes (dK/dV, dQ) or -- head_dim 128 with a dQ
-// accumulator from the caller -- the single fused pass followed by the dQ finishing kernel.
+// launches: delta, then either the two passes (dK/dV, dQ) or -- with a dQ accumulator from the
+// caller -- the single fused pass followed by the dQ finishing kernel.
 #include <cstdlib>
 
 #include "bwd_tcgen05.cuh"
@@ -10,8 +10,12 @@ namespace af {
 namespace {
 int64_t align256(int64_t x) { return (x + 255) & ~(int64_t)255; }
 
-// dQ accumulator of the fused pass: fp32 (B, H_q, N_q, D), then 256 bytes holding the item counter.
-int64_t dq_accum_floats(const AfProblem& p) { return (int64_t)p.B * p.H_q * p.N_q * p.D; }
+// dQ accumulator of the fused pass: fp32, (B, H_q, N_q, D) at head dim 128 and (B, H_q, tiles, D, 128) at 64
+// (BwdArgs::dq_acc), then 256 bytes holding the item counter.
+int64_t dq_accum_floats(const AfProblem& p) {
+  const int64_t rows = p.D == 64 ? ((int64_t)p.N_q + 127) / 128 * 128 : p.N_q;
+  return (int64_t)p.B * p.H_q * rows * p.D;
+}
 
 // dq = T(scale * R^T(acc)): the fused pass leaves scale-free, still-rotated sums in `acc`.  One
 // thread per pair of 8-element chunks (d, d + D/2) of one row.
@@ -62,21 +66,79 @@ __global__ void bwd_dq_finish_kernel(const float* __restrict__ acc, const AfBwdP
   *reinterpret_cast<uint4*>(dst + D / 2 + c * 8) = vh;
 }
 
+// The same for head dim 64, whose accumulator keeps 128 query rows contiguous: one block per tile of them, a thread
+// takes 16 columns of a row and their rotation partners (32-byte pieces of the output row).
+template <typename T, bool ROPE>
+__global__ void __launch_bounds__(256) bwd_dq_finish64_kernel(const float* __restrict__ acc, const AfBwdParams a, int q_tiles) {
+  constexpr int D = 64, ROWS = 128;
+  const AfProblem& p = a.p;
+  const int tile = (int)(blockIdx.x % q_tiles), bh = (int)(blockIdx.x / q_tiles);
+  const int h = bh % p.H_q, b = bh / p.H_q;
+  const int r = (int)threadIdx.x & (ROWS - 1), d0 = ((int)threadIdx.x / ROWS) * 16;
+  const int n = tile * ROWS + r;
+  if (n >= p.N_q) return;
+  const float* src = acc + ((int64_t)blockIdx.x * D + d0) * ROWS + r;
+  float gl[16], gh[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    gl[i] = src[i * ROWS] * p.sm_scale;
+    gh[i] = src[(D / 2 + i) * ROWS] * p.sm_scale;
+  }
+  if (ROPE) {
+    const T* cos_row = reinterpret_cast<const T*>(p.cos) + (int64_t)n * p.rope_stride_n + d0;
+    const T* sin_row = reinterpret_cast<const T*>(p.sin) + (int64_t)n * p.rope_stride_n + d0;
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const uint4 cl = __ldg(reinterpret_cast<const uint4*>(cos_row + c * 8));
+      const uint4 ch = __ldg(reinterpret_cast<const uint4*>(cos_row + D / 2 + c * 8));
+      const uint4 sl = __ldg(reinterpret_cast<const uint4*>(sin_row + c * 8));
+      const uint4 sh = __ldg(reinterpret_cast<const uint4*>(sin_row + D / 2 + c * 8));
+      const uint32_t clw[4] = {cl.x, cl.y, cl.z, cl.w}, chw[4] = {ch.x, ch.y, ch.z, ch.w};
+      const uint32_t slw[4] = {sl.x, sl.y, sl.z, sl.w}, shw[4] = {sh.x, sh.y, sh.z, sh.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float2 c1 = tc::Pack2<T>::unpack(clw[i]), c2 = tc::Pack2<T>::unpack(chw[i]);
+        const float2 s1 = tc::Pack2<T>::unpack(slw[i]), s2 = tc::Pack2<T>::unpack(shw[i]);
+        float &l0 = gl[c * 8 + 2 * i], &l1 = gl[c * 8 + 2 * i + 1], &h0 = gh[c * 8 + 2 * i], &h1 = gh[c * 8 + 2 * i + 1];
+        const float a0 = l0, a1 = l1, b0 = h0, b1 = h1;
+        l0 = a0 * c1.x + b0 * s2.x;     l1 = a1 * c1.y + b1 * s2.y;
+        h0 = b0 * c2.x - a0 * s1.x;     h1 = b1 * c2.y - a1 * s1.y;
+      }
+    }
+  }
+  T* dst = reinterpret_cast<T*>(a.dq) + (int64_t)b * a.dq_stride[0] + (int64_t)h * a.dq_stride[1] + (int64_t)n * a.dq_stride[2] + d0;
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+    uint4 vl, vh;
+    vl.x = tc::Pack2<T>::run(gl[c * 8 + 0], gl[c * 8 + 1]); vl.y = tc::Pack2<T>::run(gl[c * 8 + 2], gl[c * 8 + 3]);
+    vl.z = tc::Pack2<T>::run(gl[c * 8 + 4], gl[c * 8 + 5]); vl.w = tc::Pack2<T>::run(gl[c * 8 + 6], gl[c * 8 + 7]);
+    vh.x = tc::Pack2<T>::run(gh[c * 8 + 0], gh[c * 8 + 1]); vh.y = tc::Pack2<T>::run(gh[c * 8 + 2], gh[c * 8 + 3]);
+    vh.z = tc::Pack2<T>::run(gh[c * 8 + 4], gh[c * 8 + 5]); vh.w = tc::Pack2<T>::run(gh[c * 8 + 6], gh[c * 8 + 7]);
+    *reinterpret_cast<uint4*>(dst + c * 8) = vl;
+    *reinterpret_cast<uint4*>(dst + D / 2 + c * 8) = vh;
+  }
+}
+
 template <typename T>
-int launch_dq_finish(const float* acc, const AfBwdParams& a, cudaStream_t st) {
-  constexpr int D = 128;
-  const int64_t rows = (int64_t)a.p.B * a.p.H_q * a.p.N_q;
-  const unsigned blocks = (unsigned)((rows * (D / 16) + 255) / 256);
-  if (a.p.rope) bwd_dq_finish_kernel<T, D, true><<<blocks, 256, 0, st>>>(acc, a, rows);
-  else bwd_dq_finish_kernel<T, D, false><<<blocks, 256, 0, st>>>(acc, a, rows);
+int launch_dq_finish(const float* acc, const AfBwdParams& a, int q_tiles, cudaStream_t st) {
+  if (a.p.D == 64) {
+    const unsigned blocks = (unsigned)((int64_t)a.p.B * a.p.H_q * q_tiles);
+    if (a.p.rope) bwd_dq_finish64_kernel<T, true><<<blocks, 256, 0, st>>>(acc, a, q_tiles);
+    else bwd_dq_finish64_kernel<T, false><<<blocks, 256, 0, st>>>(acc, a, q_tiles);
+  } else {
+    constexpr int D = 128;
+    const int64_t rows = (int64_t)a.p.B * a.p.H_q * a.p.N_q;
+    const unsigned blocks = (unsigned)((rows * (D / 16) + 255) / 256);
+    if (a.p.rope) bwd_dq_finish_kernel<T, D, true><<<blocks, 256, 0, st>>>(acc, a, rows);
+    else bwd_dq_finish_kernel<T, D, false><<<blocks, 256, 0, st>>>(acc, a, rows);
+  }
   count_launch();
   return check_cuda(cudaGetLastError(), "bwd_dq_finish launch");
 }
 }  // namespace
 
-// The fused single-pass kernel exists for head_dim 128 (dQ^T is produced with M = head_dim).
 int64_t bwd_mma_dq_accum_bytes(const AfBwdParams& a) {
-  if (a.p.D != 128 || !bwd_mma_supports(a, nullptr)) return 0;
+  if (!bwd_mma_supports(a, nullptr)) return 0;
   return align256(dq_accum_floats(a.p) * 4) + 256;
 }
 
@@ -175,10 +237,15 @@ int launch_bwd_mma(const AfBwdParams& a, cudaStream_t st) {
     if (chunk > units) chunk = units;
     f.chunk_units = (int)chunk;
     f.dq_acc = static_cast<float*>(a.dq_accum);
+    f.q_tiles = (p.N_q + 127) / 128;
+    AF_REQUIRE((int64_t)p.B * p.H_q * f.q_tiles <= 0x7fffffff, "too many tiles for one launch");
     f.sched_counter = reinterpret_cast<int32_t*>(static_cast<char*>(a.dq_accum) + align256(dq_accum_floats(p) * 4));
     AF_CUDA_OK(cudaMemsetAsync(a.dq_accum, 0, (size_t)acc_bytes, st));
-    if ((rc = tcb::launch_fused_d128(p.dtype, f, k_stat, v_stat, q_strm, do_strm, st)) != AF_OK) return rc;
-    return p.dtype == AF_F16 ? launch_dq_finish<__half>(f.dq_acc, a, st) : launch_dq_finish<__nv_bfloat16>(f.dq_acc, a, st);
+    rc = p.D == 64 ? tcb::launch_fused_d64(p.dtype, f, k_stat, v_stat, q_strm, do_strm, st)
+                   : tcb::launch_fused_d128(p.dtype, f, k_stat, v_stat, q_strm, do_strm, st);
+    if (rc != AF_OK) return rc;
+    return p.dtype == AF_F16 ? launch_dq_finish<__half>(f.dq_acc, a, f.q_tiles, st)
+                             : launch_dq_finish<__nv_bfloat16>(f.dq_acc, a, f.q_tiles, st);
   }
   // the dQ pass keeps what streamed and streams what stayed: the same maps where a step has 128 rows
   CUtensorMap q_stat = q_strm, do_stat = do_strm, k_strm = k_stat, v_strm = v_stat;

@@ -22,8 +22,8 @@
 // threads work on step i; the products and the accumulations are issued by two
 // different threads.  All waits are bounded.
 //
-//   MODE_FUSED  (head_dim 128) the key-stationary pass also produces dQ, so that S and dP are
-//             computed once: 5 products per step instead of 7 over the two passes.  dS^T goes
+//   MODE_FUSED  the key-stationary pass also produces dQ, so that S and dP are
+//             computed once: 5 products per step instead of 7 over the two passes.  At head dim 128 dS^T goes
 //             both to TMEM, next to P^T in the step's S^T columns, as the A operand of
 //             dK_j += dS^T Q_i, and to shared memory (128 keys x 64 queries, query-contiguous,
 //             128-byte swizzle) as the N-major B operand of  dQ_i^T = K_j^T dS^T  (A = the stationary K tile
@@ -35,7 +35,9 @@
 //             as soon as the element-wise threads have loaded it), dQ^T single, dV, dK = 512
 //             columns.  Summation order of dQ over key tiles depends on scheduling, so dQ is
 //             reproducible only to fp32 rounding; the two-pass kernels remain the deterministic
-//             option.  Work items are handed out dynamically (one atomic counter, published to
+//             option.  At head dim 64 a step has 128 queries and dQ_i = dS K_j comes out as it is
+//             (A = dS^T in shared memory read M-major, B = the stationary K tile; TMEM lane = query), over the first
+//             columns of the step's S^T.  Work items are handed out dynamically (one atomic counter, published to
 //             the roles through a 4-deep shared-memory ring) in an order that keeps the dQ
 //             accumulator rows of the (batch, kv head) units in flight inside the L2.
 #pragma once
@@ -72,11 +74,9 @@ template <int D, int MODE = MODE_DKV> struct BCfg {
   static constexpr int SHARES = BT / COLS;                  // element-wise threads per stationary row
   static constexpr int EW_THREADS = BS * SHARES;
   static constexpr int DRAIN_THREADS = FUSED ? BS : 0;      // fused: threads that add dQ^T to its accumulator
-  // and the producer and two MMA issuers.  352 threads (head dim 64, and the single pass) leave 168 registers each: a
-  // thread that holds 64 columns of S and 64 of dP at once spills, up to 160 bytes in the key-stationary
-  // instances (causal: 108 at head dim 64, 124 in the single pass; two-pass dQ up to 20).  With 224
-  // threads nothing spilled (216 - 238 registers) and the pass was slower: dK/dV at head dim 64,
-  // [4,12,4096] causal, 341 us against 247, the Llama training step 2534 against 2467.
+  // and the producer and two MMA issuers: 352 threads with 168 registers each, or 480 with 128 (the single
+  // pass at head dim 64).  An element-wise thread takes its 64 columns of S and dP 32 at a time: with all of them
+  // in registers it spilled 120 - 160 bytes at 168 (Llama training step 2328 us, 2270 so).
   static constexpr int THREADS = EW_THREADS + DRAIN_THREADS + 96;
   static constexpr int STAGES = FUSED ? 3 : 4;
   static constexpr int STRM_PANEL = BT * 128;
@@ -92,29 +92,39 @@ template <int D, int MODE = MODE_DKV> struct BCfg {
   static constexpr int ONES_BYTES = KEY_STAT ? BS * 128 : 0;
   static constexpr int STATS_TILE = BT * 128;
   static constexpr int STATS_BYTES = KEY_STAT ? (STAGES + 1) / 2 * STATS_TILE : 0;
-  static constexpr int DS_TILE = BS * BT * 2;               // dS^T of one step (fused mode): 128 keys x 64 queries
-  static constexpr int DS_BYTES = FUSED ? 2 * DS_TILE : 0;  // two buffers, right after the stationary tiles
+  static constexpr int DS_PANEL = BS * 128;                 // dS^T in shared memory (fused mode): 128 keys x 64 queries
+  static constexpr int DS_TILE = SHARES * DS_PANEL;         // of one step
+  static constexpr int DS_BUFFERS = D == 64 ? 1 : 2;        // right after the stationary tiles
+  static constexpr int DS_BYTES = FUSED ? DS_BUFFERS * DS_TILE : 0;
   static constexpr int ONES_OFF = 2 * STAT_TILE + DS_BYTES, STATS_OFF = ONES_OFF + ONES_BYTES;
   static constexpr int STAGE0_OFF = STATS_OFF + STATS_BYTES, STAGE_BYTES = 2 * STRM_TILE;
   static constexpr int SMEM_BYTES = STAGE0_OFF + STAGES * STAGE_BYTES + 1024 + 512;
   static_assert(SMEM_BYTES <= 232448, "shared memory of one CTA");
   static constexpr int TMEM_COLS = 512;
   // X = S, Y = dP of a step, BT columns each; P and dS as half-precision A operands take half the columns.
-  // fused:            X0 X1 Y Z (Z = dQ^T): P^T and dS^T of a step share its X columns; Y and Z are single,
+  // fused, D = 128:   X0 X1 Y Z (Z = dQ^T): P^T and dS^T of a step share its X columns; Y and Z are single,
   //                   free again as soon as the threads that want them have loaded them.
-  // head dim 64:      X0 X1 Y: the same, a share's P and dS over the share's own 64 columns of X.
+  // head dim 64:      X0 X1 Y: the same, a share's P and dS over the share's own 64 columns of X; the
+  //                   single pass puts Z = dQ over the first 64 columns of its step's X: the product that
+  //                   makes it follows, in the same thread, those that read P and dS.
   // head dim 128:     X0 Y0 X1 Y1: P^T over X, dS^T over Y; MODE_DQ has one accumulator only, dS gets
   //                   columns of its own there (two buffers of 32), so that the next S / dP product does
   //                   not have to wait until dQ += dS K has consumed the previous dS.
   static constexpr bool DS_IN_X = FUSED || D == 64;
   static constexpr bool Y_SINGLE = FUSED || D == 64;
   __host__ __device__ static constexpr int col_x(int t) { return DS_IN_X ? t * BT : t * 128; }
-  __host__ __device__ static constexpr int col_y(int t) { return FUSED ? 128 : D == 64 ? 256 : 64 + t * 128; }
-  static constexpr int COL_Z = 192, COL_ACC1 = (D == 64) ? 384 : 256, COL_ACC2 = COL_ACC1 + D;
-  // k-step kk (16 columns of the step) of the A operands
-  __host__ __device__ static constexpr int col_p(int t, int kk) { return col_x(t) + (kk >> 2) * COLS + (kk & 3) * 8; }
+  __host__ __device__ static constexpr int col_y(int t) { return D == 64 ? 256 : FUSED ? 128 : 64 + t * 128; }
+  __host__ __device__ static constexpr int col_z(int t) { return D == 64 ? col_x(t) : 192; }
+  static constexpr int COL_ACC1 = (D == 64) ? 384 : 256, COL_ACC2 = COL_ACC1 + D;
+  // k-step kk (16 columns of the step) of the A operands.  The element-wise threads write two k-steps at a
+  // time, when they have read the 32 columns of X (and Y) that these come from: where P and dS are
+  // both in X, those of 32 columns lie over these columns.
+  static constexpr bool P_DS_IN_X = DS_IN_X && KEY_STAT;
+  __host__ __device__ static constexpr int col_p(int t, int kk) {
+    return col_x(t) + (kk >> 2) * COLS + (P_DS_IN_X ? ((kk >> 1) & 1) * 32 + (kk & 1) * 8 : (kk & 3) * 8);
+  }
   __host__ __device__ static constexpr int col_ds(int t, int kk) {
-    return DS_IN_X ? col_p(t, kk) + (MODE == MODE_DQ ? 0 : 32) : MODE == MODE_DQ ? 384 + t * 32 + kk * 8 : col_y(t) + kk * 8;
+    return DS_IN_X ? col_p(t, kk) + (P_DS_IN_X ? 16 : 0) : MODE == MODE_DQ ? 384 + t * 32 + kk * 8 : col_y(t) + kk * 8;
   }
 };
 
@@ -122,7 +132,7 @@ struct BBarriers {
   uint64_t stat_full, stat_empty, acc_free;
   uint64_t strm_full[4], strm_empty[4];
   uint64_t xy_full[2], p_full[2], acc_done[2];
-  uint64_t y_free, z_free;                      // single dP / dQ^T columns: loaded by the threads that want them
+  uint64_t y_free, z_free[2];                   // dP / dQ columns: loaded by the threads that want them (z: [step & 1], or [0])
   uint64_t sched_full[4], sched_empty[4];       // fused mode: ring of dynamically fetched item numbers
   int32_t sched_item[4];
   uint32_t tmem_base;
@@ -141,7 +151,10 @@ struct BwdArgs {
   int total_items;      // tiles * B * heads: stationary tiles to process
   int grid_ctas;        // one persistent CTA per SM (or one per item when there are fewer)
   // fused mode
-  float* dq_acc;        // fp32 (B, H_q, N_q, D) accumulator, zeroed before the launch
+  // dQ accumulator, zeroed before the launch.  Head dim 128: fp32 (B, H_q, N_q, D).  Head dim 64: fp32 (B, H_q,
+  // q_tiles, D, 128), 128 query rows contiguous: a warp's lanes are 32 consecutive rows there.
+  float* dq_acc;
+  int q_tiles;          // 128-row tiles of the queries
   int32_t* sched_counter;   // zeroed before the launch
   int chunk_units;      // (batch, kv head) units per scheduling chunk
 };
@@ -281,13 +294,13 @@ bwd_tcgen05_kernel(const BwdArgs args, const __grid_constant__ CUtensorMap map_a
   using C = BCfg<D, MODE>;
   constexpr bool FUSED = MODE == MODE_FUSED;
   constexpr bool KVS = MODE != MODE_DQ;          // key-stationary: MODE_DKV and MODE_FUSED
-  static_assert(!FUSED || D == 128, "the fused pass computes dQ^T with M = head_dim = 128");
   constexpr int STAGES = C::STAGES, BT = C::BT, COLS = C::COLS, SHARES = C::SHARES;
   constexpr int WARP_LOAD = (C::EW_THREADS + C::DRAIN_THREADS) / 32, WARP_MMA1 = WARP_LOAD + 1, WARP_MMA2 = WARP_LOAD + 2;
   constexpr int AB_FMT = (Elem<T>::code == AF_BF16) ? 1 : 0;
   constexpr uint32_t IDESC_XY = umma_idesc_f16(AB_FMT, BS, BT, 0, 0);
   constexpr uint32_t IDESC_ACC = umma_idesc_f16(AB_FMT, BS, D, 0, 1);
-  constexpr uint32_t IDESC_DQT = umma_idesc_f16(AB_FMT, D, BT, 1, 1);   // dQ^T = K^T dS^T: A M-major, B N-major
+  // dQ^T = K^T dS^T at head dim 128 (M = d), dQ = dS K at 64 (M = query): A M-major, B N-major
+  constexpr uint32_t IDESC_DQ = umma_idesc_f16(AB_FMT, 128, 64, 1, 1);
   constexpr int STAGE_BYTES = C::STAGE_BYTES, STAGE0_OFF = C::STAGE0_OFF;
   constexpr uint32_t IDESC_STATS = umma_idesc_f16(1, BS, BT, 0, 0);      // bf16 terms, whatever T is
 
@@ -313,7 +326,8 @@ bwd_tcgen05_kernel(const BwdArgs args, const __grid_constant__ CUtensorMap map_a
     mbar_init(&bars->stat_empty, FUSED ? 2 : 1);   // fused: both issuing threads read the stationary K tile
     mbar_init(&bars->acc_free, C::EW_THREADS);
     mbar_init(&bars->y_free, C::EW_THREADS);
-    mbar_init(&bars->z_free, 128);
+    mbar_init(&bars->z_free[0], BS);
+    mbar_init(&bars->z_free[1], BS);
     for (int s = 0; s < 4; ++s) {
       mbar_init(&bars->strm_full[s], 1);
       mbar_init(&bars->strm_empty[s], 1);
@@ -480,10 +494,10 @@ bwd_tcgen05_kernel(const BwdArgs args, const __grid_constant__ CUtensorMap map_a
         const int st = it % STAGES, t = it & 1;
         if (!mbar_wait(&bars->strm_full[st], (it / STAGES) & 1, abort_flag)) { ok = false; break; }
         // The step's X columns were last used by step it-2.  Where P and dS overwrite them (or Y), the
-        // accumulate MMAs of that step must have run; otherwise the element-wise group must have read
-        // them (its arrival on p_full).
+        // accumulate MMAs of that step must have run, and where dQ does, it must have been loaded;
+        // otherwise the element-wise group must have read them (its arrival on p_full).
         if (it >= 2) {
-          uint64_t* free_bar = (KVS || C::DS_IN_X) ? &bars->acc_done[t] : &bars->p_full[t];
+          uint64_t* free_bar = (FUSED && D == 64) ? &bars->z_free[t] : (KVS || C::DS_IN_X) ? &bars->acc_done[t] : &bars->p_full[t];
           if (!mbar_wait(free_bar, ((it >> 1) - 1) & 1, abort_flag)) { ok = false; break; }
         }
         tc_fence_after_sync();
@@ -518,10 +532,10 @@ bwd_tcgen05_kernel(const BwdArgs args, const __grid_constant__ CUtensorMap map_a
     {
       const bool leader = elect_one();
       const uint64_t desc_b1n = umma_desc_sw128(sStage0, C::STRM_PANEL, 1024);   // streamed tile, N-major
-      // fused mode: dS^T (128 keys x 64 queries, query-contiguous) as N-major B;
-      // the stationary K tile (128 keys x D) as M-major A (M = d: 64-element panels LBO apart)
-      const uint64_t desc_ds_n = umma_desc_sw128(sDS0, C::DS_TILE, 1024);
-      const uint64_t desc_k_m = umma_desc_sw128(sA1, C::STAT_PANEL, 1024);
+      // fused mode: dS^T (128 keys x queries, query-contiguous) and the stationary K tile (128 keys x D) as
+      // the operands of dQ, contracted over the keys: one M-major, the other N-major (64-element panels LBO apart)
+      const uint64_t desc_ds = umma_desc_sw128(sDS0, C::DS_PANEL, 1024);
+      const uint64_t desc_k = umma_desc_sw128(sA1, C::STAT_PANEL, 1024);
       BItem bi;
       int it0 = 0, qi = 0;
       bool ok = true;
@@ -548,16 +562,17 @@ bwd_tcgen05_kernel(const BwdArgs args, const __grid_constant__ CUtensorMap map_a
           if (leader) umma_ts(tmem + (KVS ? C::COL_ACC2 : C::COL_ACC1), tmem + C::col_ds(t, kk), b1 + (uint64_t)((kk * 2048) >> 4),
                   IDESC_ACC, (!first || kk > 0) ? 1u : 0u);
         if (FUSED) {
-          const uint64_t ds_n = desc_ds_n + (uint64_t)((t * C::DS_TILE) >> 4);
-          // the single dQ^T buffer: the previous step's tile has been loaded
-          if (it >= 1) {
-            if (!mbar_wait(&bars->z_free, (it - 1) & 1, abort_flag)) { ok = false; break; }
+          const uint64_t ds = desc_ds + (uint64_t)(((t % C::DS_BUFFERS) * C::DS_TILE) >> 4);
+          // head dim 128, the single dQ^T buffer: the previous step's tile has been loaded
+          if (D == 128 && it >= 1) {
+            if (!mbar_wait(&bars->z_free[0], (it - 1) & 1, abort_flag)) { ok = false; break; }
             tc_fence_after_sync();
           }
+          const uint64_t za = D == 128 ? desc_k : ds, zb = D == 128 ? ds : desc_k;
 #pragma unroll
-          for (int kk = 0; kk < BS / 16; ++kk)      // dQ^T = K^T dS^T over the 128 keys
-            if (leader) umma_ss(tmem + C::COL_Z, desc_k_m + (uint64_t)((kk * 2048) >> 4), ds_n + (uint64_t)((kk * 2048) >> 4),
-                    IDESC_DQT, kk > 0 ? 1u : 0u);
+          for (int kk = 0; kk < BS / 16; ++kk)      // over the 128 keys
+            if (leader) umma_ss(tmem + C::col_z(t), za + (uint64_t)((kk * 2048) >> 4), zb + (uint64_t)((kk * 2048) >> 4),
+                    IDESC_DQ, kk > 0 ? 1u : 0u);
         }
         if (leader) umma_commit(&bars->acc_done[t]);
         if (leader) umma_commit(&bars->strm_empty[st]);
@@ -573,8 +588,10 @@ bwd_tcgen05_kernel(const BwdArgs args, const __grid_constant__ CUtensorMap map_a
     // the load / store pipe, which the element-wise threads spent between two steps (2700 clocks a step,
     // half of them here) while the products waited.  TMEM lane = d, column = query; a warp's 32 lanes
     // cover 32 consecutive d of one query row.
-    const uint32_t z_tmem = tmem + ((uint32_t)((warp & 3) * 32) << 16) + C::COL_Z;
-    const int d = tid & (BS - 1);
+    // Head dim 64: TMEM lane = query, column = d; the accumulator keeps 128 query rows contiguous.
+    const uint32_t z_lanes = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+    const int zlane = tid & (BS - 1);                // d, or the query row of a tile
+    constexpr int ROW = D == 128 ? D : BS;           // accumulator elements from one TMEM column to the next
     BItem bi;
     int it = 0;                                      // running step count
     bool alive = true;
@@ -582,25 +599,26 @@ bwd_tcgen05_kernel(const BwdArgs args, const __grid_constant__ CUtensorMap map_a
       for (int g = 0; g < n_heads && alive; ++g) {
         const int h = bi.h_kv * group + g;
         const StepWalk<BT> w = make_steps<MODE, BT>(p, args, bi.tile, h);
-        float* head_rows = args.dq_acc + ((int64_t)bi.b * p.H_q + h) * p.N_q * D + d;
+        float* head_rows = args.dq_acc + ((int64_t)bi.b * p.H_q + h) * (D == 128 ? p.N_q : args.q_tiles * BS) * D + zlane;
         for (int s = 0; s < w.cnt; ++s, ++it) {
           const int r0 = w.row0(s), n_valid = p.N_q - r0;
           if (!mbar_wait(&bars->acc_done[it & 1], (it >> 1) & 1, abort_flag)) { alive = false; break; }
           tc_fence_after_sync();
+          const uint32_t z_tmem = z_lanes + C::col_z(it & 1);
           uint32_t zr[64];
           tmem_ld32(z_tmem, &zr[0]);
           tmem_ld32(z_tmem + 32, &zr[32]);
           tmem_wait_ld();
           tc_fence_before_sync();
-          mbar_arrive(&bars->z_free);
-          float* acc_rows = head_rows + (int64_t)r0 * D;
-          if (n_valid >= 64) {
+          mbar_arrive(&bars->z_free[D == 128 ? 0 : it & 1]);
+          float* acc_rows = head_rows + (int64_t)r0 * D;         // r0 is a multiple of 128 at head dim 64
+          if (D == 64 || n_valid >= 64) {
 #pragma unroll
-            for (int c = 0; c < 64; ++c) atomicAdd(acc_rows + c * D, __uint_as_float(zr[c]));
+            for (int c = 0; c < 64; ++c) atomicAdd(acc_rows + c * ROW, __uint_as_float(zr[c]));
           } else {
 #pragma unroll
             for (int c = 0; c < 64; ++c)
-              if (c < n_valid) atomicAdd(acc_rows + c * D, __uint_as_float(zr[c]));
+              if (c < n_valid) atomicAdd(acc_rows + c * ROW, __uint_as_float(zr[c]));
           }
         }
       }
@@ -638,16 +656,6 @@ bwd_tcgen05_kernel(const BwdArgs args, const __grid_constant__ CUtensorMap map_a
         tc_fence_after_sync();
         const uint32_t xt = tmem + lane_base + C::col_x(t) + col_first;
         const uint32_t yt = tmem + lane_base + C::col_y(t) + col_first;
-        uint32_t xr[COLS], yr[COLS];
-        tmem_ld32(xt, &xr[0]); tmem_ld32(xt + 32, &xr[32]);
-        tmem_ld32(yt, &yr[0]); tmem_ld32(yt + 32, &yr[32]);
-        tmem_wait_ld();
-        if (C::Y_SINGLE) {
-          // dP is in registers: the next step's dP product may overwrite the buffer
-          tc_fence_before_sync();
-          mbar_arrive(&bars->y_free);
-        }
-
         // Does any element of these 128 x 64 columns need masking?
         //   key-stationary: lane = key srow, column c = query c0 + c;  DQ: lane = query srow, column c = key c0 + c.
         const int c0 = r0 + col_first;
@@ -674,15 +682,28 @@ bwd_tcgen05_kernel(const BwdArgs args, const __grid_constant__ CUtensorMap map_a
           }
         }
 
-        uint32_t pk[COLS / 2], dk[COLS / 2];
-        const float relf = (float)rel;
-        // The masking decision is taken once per tile: the element loop exists in a masked and an
-        // unmasked copy.  The arithmetic runs on packed fp32 pairs (half the issue slots).
-        auto element_pass = [&](auto masked_tag) {
-          constexpr bool MASKED = decltype(masked_tag)::value;
+        // 32 columns at a time (BCfg::THREADS).
+#pragma unroll 1
+        for (int u = 0; u < COLS; u += 32) {
+          uint32_t xr[32], yr[32], pk[16], dk[16];
+          tmem_ld32(xt + u, xr);
+          tmem_ld32(yt + u, yr);
+          tmem_wait_ld32(xr);
+          tmem_wait_ld32(yr);
+          if (C::Y_SINGLE && u + 32 == COLS) {
+            // dP is in registers: the next step's dP product may overwrite the buffer
+            tc_fence_before_sync();
+            mbar_arrive(&bars->y_free);
+          }
+          const int rel_u = rel - u, limit_u = col_limit - u;
+          const uint32_t bits_u = (uint32_t)(tile_bits >> u);
+          const float relf = (float)rel_u;
+          // The masking decision is taken once per tile: the element loop exists in a masked and an
+          // unmasked copy.  The arithmetic runs on packed fp32 pairs (half the issue slots).
+          auto element_pass = [&](auto masked_tag) {
+            constexpr bool MASKED = decltype(masked_tag)::value;
 #pragma unroll
-          for (int cc = 0; cc < COLS; cc += 2) {
-            {
+            for (int cc = 0; cc < 32; cc += 2) {
               float e0, e1, d0, d1;
               // key-stationary: S^T and dP^T come with -L / scale and -delta in them
               const uint64_t x2 = tc::f32x2_pack(__uint_as_float(xr[cc]), __uint_as_float(xr[cc + 1]));
@@ -695,10 +716,10 @@ bwd_tcgen05_kernel(const BwdArgs args, const __grid_constant__ CUtensorMap map_a
               float p0 = ex2_approx(e0), p1 = ex2_approx(e1);
               if (MASKED) {
                 auto kept = [&](int x) {
-                  bool keep = x < col_limit;
-                  if (EMASK == EMASK_CAUSAL) keep = keep && (KVS ? (x >= rel) : (x <= rel));
-                  if (EMASK == EMASK_WINDOW) keep = keep && (x - rel < p.window) && (rel - x < p.window);
-                  if (EMASK == EMASK_BITS) keep = keep && ((tile_bits >> x) & 1ull);
+                  bool keep = x < limit_u;
+                  if (EMASK == EMASK_CAUSAL) keep = keep && (KVS ? (x >= rel_u) : (x <= rel_u));
+                  if (EMASK == EMASK_WINDOW) keep = keep && (x - rel_u < p.window) && (rel_u - x < p.window);
+                  if (EMASK == EMASK_BITS) keep = keep && ((bits_u >> x) & 1u);
                   return keep;
                 };
                 p0 = kept(cc) ? p0 : 0.f;
@@ -709,25 +730,32 @@ bwd_tcgen05_kernel(const BwdArgs args, const __grid_constant__ CUtensorMap map_a
               pk[cc >> 1] = Pack2<T>::run(p0, p1);
               dk[cc >> 1] = Pack2<T>::run(d0, d1);
             }
-          }
-        };
-        if (need_mask) element_pass(std::true_type{});
-        else element_pass(std::false_type{});
-        if (FUSED) {
-          // dS^T row of this key: 64 queries = 128 bytes = eight 16-byte chunks, chunk c stored at
-          // c ^ (row & 7) (the 128-byte swizzle the MMA descriptor expects).  Buffer t was last read
-          // by the products of step it-2, which ran before this step's S^T was issued.
-          const uint32_t row_addr = sDS0 + t * C::DS_TILE + lrow * 128;
+          };
+          if (need_mask) element_pass(std::true_type{});
+          else element_pass(std::false_type{});
+          if (FUSED) {
+            // dS^T row of this key: 64 queries = 128 bytes = eight 16-byte chunks, chunk c stored at
+            // c ^ (row & 7) (the 128-byte swizzle the MMA descriptor expects).  Two buffers: buffer t was
+            // last read by the products of step it-2, which ran before this step's S^T was issued.
+            // One: by those of step it-1.
+            if (C::DS_BUFFERS == 1 && u == 0 && it >= 1 &&
+                !mbar_wait(&bars->acc_done[t ^ 1], ((it - 1) >> 1) & 1, abort_flag)) { alive = false; break; }
+            const uint32_t row_addr = sDS0 + (t % C::DS_BUFFERS) * C::DS_TILE + share * C::DS_PANEL + lrow * 128;
+            const int c0u = u >> 3;
 #pragma unroll
-          for (int c8 = 0; c8 < 8; ++c8)
-            tc::sts128(row_addr + ((c8 ^ (lrow & 7)) << 4),
-                       make_uint4(dk[c8 * 4], dk[c8 * 4 + 1], dk[c8 * 4 + 2], dk[c8 * 4 + 3]));
-          fence_proxy_async_smem();
+            for (int c8 = 0; c8 < 4; ++c8)
+              tc::sts128(row_addr + (((c0u + c8) ^ (lrow & 7)) << 4),
+                         make_uint4(dk[c8 * 4], dk[c8 * 4 + 1], dk[c8 * 4 + 2], dk[c8 * 4 + 3]));
+          }
+          // two-pass dQ at head dim 128: the dS buffer was last read by the accumulate MMAs of step it-2
+          if (MODE == MODE_DQ && !C::DS_IN_X && u == 0 && it >= 2 &&
+              !mbar_wait(&bars->acc_done[t], ((it >> 1) - 1) & 1, abort_flag)) { alive = false; break; }
+          const uint32_t half = (uint32_t)(u >> 5);
+          if (KVS) tmem_st16(tmem + lane_base + C::col_p(t, share * (COLS / 16)) + half * (C::P_DS_IN_X ? 32 : 16), pk);
+          tmem_st16(tmem + lane_base + C::col_ds(t, share * (COLS / 16)) + half * (C::P_DS_IN_X ? 32 : 16), dk);
         }
-        // two-pass dQ at head dim 128: the dS buffer was last read by the accumulate MMAs of step it-2
-        if (MODE == MODE_DQ && !C::DS_IN_X && it >= 2 && !mbar_wait(&bars->acc_done[t], ((it >> 1) - 1) & 1, abort_flag)) { alive = false; break; }
-        if (KVS) tmem_st32(xt, pk);
-        tmem_st32(tmem + lane_base + C::col_ds(t, share * (COLS / 16)), dk);
+        if (!alive) break;
+        if (FUSED) fence_proxy_async_smem();
         tmem_wait_st();
         tc_fence_before_sync();
         mbar_arrive(&bars->p_full[t]);
@@ -896,6 +924,7 @@ int launch_dkv_d64(int dtype, const BwdArgs&, const CUtensorMap&, const CUtensor
 int launch_dkv_d128(int dtype, const BwdArgs&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, cudaStream_t);
 int launch_dq_d64(int dtype, const BwdArgs&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, cudaStream_t);
 int launch_dq_d128(int dtype, const BwdArgs&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, cudaStream_t);
+int launch_fused_d64(int dtype, const BwdArgs&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, cudaStream_t);
 int launch_fused_d128(int dtype, const BwdArgs&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, cudaStream_t);
 
 #define AF_DEFINE_BWD_UNIT(NAME, DIM, MODE)                                                                   \

@@ -122,11 +122,11 @@ typedef struct AfBwdParams {
                                          this problem, as af_fwd left them in its own workspace
                                          (same layout); the RoPE pre-pass is then skipped      */
   void*   dq_accum;                   /* optional scratch of af_bwd_dq_accum_bytes() bytes, 256-byte
-                                         aligned: an fp32 (B, H_q, N_q, D) accumulator for dQ.  With
-                                         it af_bwd runs the single-pass kernel (S and dP computed
-                                         once, dQ summed over key tiles with fp32 atomic adds, so
-                                         its last bits depend on scheduling); without it the
-                                         deterministic two-pass kernels run                    */
+                                         aligned: an fp32 accumulator for dQ.  With it af_bwd
+                                         runs the single-pass kernel (S and dP computed once, dQ
+                                         summed over key tiles with fp32 atomic adds, so its last
+                                         bits depend on scheduling); without it the deterministic
+                                         two-pass kernels run                                  */
   int64_t dq_accum_bytes;
 } AfBwdParams;
 
@@ -220,7 +220,7 @@ AF_API int af_bwd(const AfBwdParams* params, af_stream_t stream);
 AF_API int64_t af_bwd_workspace_bytes(const AfBwdParams* params);
 
 /* Bytes of the optional dQ accumulator (AfBwdParams.dq_accum) with which af_bwd runs its
- * single-pass kernel for this problem; 0 when only the two-pass kernels apply (head_dim other than
+ * single-pass kernel for this problem; 0 when only other kernels apply (head_dim other than 64 and
  * 128, fp32, additive bias, ...).  af_bwd clears the accumulator itself.  No counterpart in the
  * reference, whose backward always recomputes S and dP in both of its kernels
  * (attnfuse/compiler/codegen_backward.py:75-302).  Host only. */

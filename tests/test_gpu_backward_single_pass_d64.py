@@ -1,0 +1,95 @@
+"""The single-pass backward at head_dim 64: dQ of 128-query steps summed over the key tiles in an fp32
+accumulator of padded 128-row tiles.  Every mask and bias, rotation, GQA, odd lengths and block
+lists with partly covered tiles, against the oracle and against the two-pass kernels."""
+import ctypes as C
+
+import pytest
+import torch
+
+import attentionfuse_b200 as af
+from attentionfuse_b200.runtime import _lib
+from attentionfuse_b200.runtime.dispatch import _alibi_slopes, fill_problem
+from oracle import attention_oracle as orc
+from tests._util import assert_close, qkv
+
+pytestmark = pytest.mark.gpu
+DEV, D = "cuda", 64
+
+
+def graph(variant, heads, window=0):
+    @af.attention
+    def fn(Q, K, V):
+        s = af.rope(Q, K) if "rope" in variant else af.scaled_dot_product(Q, K)
+        if "alibi" in variant:
+            s = af.alibi(s, heads)
+        if "causal" in variant:
+            s = af.causal(s)
+        if "window" in variant:
+            s = af.sliding_window(s, window)
+        if "blocks" in variant:
+            s = af.block_sparse(s)
+        return af.softmax(s) @ V
+    return fn
+
+
+def grads(fn, Q, K, V, dO, **kw):
+    q, k, v = (t.to(DEV).requires_grad_(True) for t in (Q, K, V))
+    before = _lib.launch_count()
+    out = fn(q, k, v, **kw)
+    got = torch.autograd.grad(out, (q, k, v), dO.to(DEV))
+    return got, _lib.launch_count() - before
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("variant", ["dense", "causal", "causal rope", "causal alibi", "dense alibi", "window", "window rope"])
+@pytest.mark.parametrize("shape", [(1, 4, 4, 1), (2, 4, 2, 129), (1, 6, 1, 333), (1, 20, 20, 640)], ids=str)
+def test_against_oracle_and_two_pass(shape, variant, dtype, monkeypatch):
+    B, H, H_kv, N = shape
+    Q, K, V = qkv(9500 + N, B, H, H_kv, N, N, D, dtype)
+    dO = orc.randn(9501 + N, Q.shape, dtype)
+    kw, okw = {}, dict(causal="causal" in variant, window=150 if "window" in variant else None)
+    if "rope" in variant:
+        cos, sin = orc.build_rope_cache(N, D, 10000.0, dtype)
+        kw, okw = dict(cos=cos.to(DEV), sin=sin.to(DEV)), dict(okw, cos=cos, sin=sin)
+    if "alibi" in variant:
+        okw["slopes"] = _alibi_slopes(H, "cpu", str(dtype))
+    fn = graph(variant, H, 150)
+    _, *want = orc.attention_grads(Q, K, V, dO, **okw)
+    one, launches = grads(fn, Q, K, V, dO, **kw)
+    assert launches == 4 + ("rope" in variant)      # forward, delta, the pass, dQ; the rotation
+    monkeypatch.setenv("ATTNFUSE_BWD_DETERMINISTIC", "1")
+    two, _ = grads(fn, Q, K, V, dO, **kw)
+    again, _ = grads(fn, Q, K, V, dO, **kw)
+    for name, g1, g2, g3, w in zip(("dQ", "dK", "dV"), one, two, again, want):
+        assert torch.equal(g2, g3)
+        if N == 1 and name != "dV":            # one key: P = 1, dQ = dK = 0 up to the rounding of O in delta
+            assert g1.float().abs().max().item() < 2e-2
+            continue
+        assert_close(g1, w, dtype, grad=True, what=f"single pass d64 {variant} N{N} {name}")
+        assert_close(g2, w, dtype, grad=True, what=f"two passes d64 {variant} N{N} {name}")
+
+
+@pytest.mark.parametrize("block", [64, 128, 256])
+def test_block_lists(block):
+    """Lists of uneven length, tiles that are partly covered (blocks of 64) and queries without any key."""
+    B, H, N, dtype = 2, 4, 700, torch.float16
+    n = (N + block - 1) // block
+    gen = torch.Generator().manual_seed(9600 + block)
+    grids = torch.rand(H, n, n, generator=gen) < 0.4
+    grids[:, :, 0] = True
+    grids[1, 1] = False
+    Q, K, V = qkv(9601, B, H, H, N, N, D, dtype)
+    dO = orc.randn(9602, Q.shape, dtype)
+    got, _ = grads(graph("blocks", H), Q, K, V, dO, block_mask=af.create_block_mask_per_head(grids, block, block, device=DEV))
+    elem = grids.repeat_interleave(block, 1).repeat_interleave(block, 2)[:, :N, :N]
+    _, *want = orc.attention_grads(Q, K, V, dO, elem_mask=elem)
+    for name, g, w in zip(("dQ", "dK", "dV"), got, want):
+        assert_close(g, w, dtype, grad=True, what=f"single pass d64 blocks {block} {name}")
+
+
+def test_accumulator_is_padded_to_whole_tiles():
+    N = 200
+    q, k, v = (t.to(DEV) for t in qkv(9700, 1, 2, 2, N, N, D, torch.bfloat16))
+    p = _lib.AfBwdParams()
+    fill_problem(p.p, q, k, v, sm_scale=D ** -0.5, mask_kind=1)
+    assert int(_lib.load().af_bwd_dq_accum_bytes(C.byref(p))) >= 2 * 256 * D * 4      # two heads, rows padded to 256

@@ -10,8 +10,8 @@ namespace af {
 namespace {
 int64_t align256(int64_t x) { return (x + 255) & ~(int64_t)255; }
 
-// dQ accumulator of the fused pass: fp32, (B, H_q, N_q, D) at head dim 128 and (B, H_q, tiles, D, 128) at 64
-// (BwdArgs::dq_acc), then 256 bytes holding the item counter.
+// dQ accumulator of the fused pass: fp32, (B, H_q, N_q, D) at head dim 128 and (B, H_q, 32-row tiles, D / 4, 32, 4)
+// at 64 (BwdArgs::dq_acc), then 256 bytes holding the item counter.
 int64_t dq_accum_floats(const AfProblem& p) {
   const int64_t rows = p.D == 64 ? ((int64_t)p.N_q + 127) / 128 * 128 : p.N_q;
   return (int64_t)p.B * p.H_q * rows * p.D;
@@ -66,8 +66,8 @@ __global__ void bwd_dq_finish_kernel(const float* __restrict__ acc, const AfBwdP
   *reinterpret_cast<uint4*>(dst + D / 2 + c * 8) = vh;
 }
 
-// The same for head dim 64, whose accumulator keeps 128 query rows contiguous: one block per tile of them, a thread
-// takes 16 columns of a row and their rotation partners (32-byte pieces of the output row).
+// The same for head dim 64: one block per 128 rows of the accumulator, a thread takes 16 columns of a row and their
+// rotation partners (32-byte pieces of the output row).
 template <typename T, bool ROPE>
 __global__ void __launch_bounds__(256) bwd_dq_finish64_kernel(const float* __restrict__ acc, const AfBwdParams a, int q_tiles) {
   constexpr int D = 64, ROWS = 128;
@@ -77,12 +77,13 @@ __global__ void __launch_bounds__(256) bwd_dq_finish64_kernel(const float* __res
   const int r = (int)threadIdx.x & (ROWS - 1), d0 = ((int)threadIdx.x / ROWS) * 16;
   const int n = tile * ROWS + r;
   if (n >= p.N_q) return;
-  const float* src = acc + ((int64_t)blockIdx.x * D + d0) * ROWS + r;
+  const float4* src = reinterpret_cast<const float4*>(acc + (int64_t)blockIdx.x * D * ROWS) + ((r >> 5) * (D / 4) + d0 / 4) * 32 + (r & 31);
   float gl[16], gh[16];
 #pragma unroll
-  for (int i = 0; i < 16; ++i) {
-    gl[i] = src[i * ROWS] * p.sm_scale;
-    gh[i] = src[(D / 2 + i) * ROWS] * p.sm_scale;
+  for (int i = 0; i < 4; ++i) {
+    const float4 l = src[i * 32], u = src[(D / 8 + i) * 32];
+    gl[4 * i] = l.x * p.sm_scale; gl[4 * i + 1] = l.y * p.sm_scale; gl[4 * i + 2] = l.z * p.sm_scale; gl[4 * i + 3] = l.w * p.sm_scale;
+    gh[4 * i] = u.x * p.sm_scale; gh[4 * i + 1] = u.y * p.sm_scale; gh[4 * i + 2] = u.z * p.sm_scale; gh[4 * i + 3] = u.w * p.sm_scale;
   }
   if (ROPE) {
     const T* cos_row = reinterpret_cast<const T*>(p.cos) + (int64_t)n * p.rope_stride_n + d0;

@@ -89,14 +89,16 @@ template <int D, int MODE = MODE_DKV> struct BCfg {
   // steps read 12 KB (BT = 64).  A tile of BT rows x 128 bytes holds the steps of two ring stages: 32 bytes
   // of L terms and 32 bytes of delta terms each.
   static constexpr bool KEY_STAT = MODE != MODE_DQ;
-  static constexpr int ONES_BYTES = KEY_STAT ? BS * 128 : 0;
   static constexpr int STATS_TILE = BT * 128;
   static constexpr int STATS_BYTES = KEY_STAT ? (STAGES + 1) / 2 * STATS_TILE : 0;
   static constexpr int DS_PANEL = BS * 128;                 // dS^T in shared memory (fused mode): 128 keys x 64 queries
   static constexpr int DS_TILE = SHARES * DS_PANEL;         // of one step
-  static constexpr int DS_BUFFERS = D == 64 ? 1 : 2;        // right after the stationary tiles
-  static constexpr int DS_BYTES = FUSED ? DS_BUFFERS * DS_TILE : 0;
-  static constexpr int ONES_OFF = 2 * STAT_TILE + DS_BYTES, STATS_OFF = ONES_OFF + ONES_BYTES;
+  static constexpr int DS_BYTES = FUSED ? 2 * DS_TILE : 0;  // two buffers, right after the stationary tiles
+  // An odd number of stages leaves half of the last statistics tile free; at 128 rows a step the ones fit there.
+  static constexpr bool ONES_IN_STATS = FUSED && D == 64;
+  static constexpr int ONES_BYTES = KEY_STAT && !ONES_IN_STATS ? BS * 128 : 0;
+  static constexpr int STATS_OFF = 2 * STAT_TILE + DS_BYTES + ONES_BYTES;
+  static constexpr int ONES_OFF = ONES_IN_STATS ? STATS_OFF + STATS_BYTES - STATS_TILE + 64 : STATS_OFF - ONES_BYTES;
   static constexpr int STAGE0_OFF = STATS_OFF + STATS_BYTES, STAGE_BYTES = 2 * STRM_TILE;
   static constexpr int SMEM_BYTES = STAGE0_OFF + STAGES * STAGE_BYTES + 1024 + 512;
   static_assert(SMEM_BYTES <= 232448, "shared memory of one CTA");
@@ -132,6 +134,7 @@ struct BBarriers {
   uint64_t stat_full, stat_empty, acc_free;
   uint64_t strm_full[4], strm_empty[4];
   uint64_t xy_full[2], p_full[2], acc_done[2];
+  uint64_t red_done[2];                         // head dim 64: the reduction of a step's dQ has read its staged tile
   uint64_t y_free, z_free[2];                   // dP / dQ columns: loaded by the threads that want them (z: [step & 1], or [0])
   uint64_t sched_full[4], sched_empty[4];       // fused mode: ring of dynamically fetched item numbers
   int32_t sched_item[4];
@@ -152,7 +155,7 @@ struct BwdArgs {
   int grid_ctas;        // one persistent CTA per SM (or one per item when there are fewer)
   // fused mode
   // dQ accumulator, zeroed before the launch.  Head dim 128: fp32 (B, H_q, N_q, D).  Head dim 64: fp32 (B, H_q,
-  // q_tiles, D, 128), 128 query rows contiguous: a warp's lanes are 32 consecutive rows there.
+  // 4 q_tiles, D / 4, 32, 4): a tile of 32 rows is contiguous, 16 bytes of a row next to those of the next row.
   float* dq_acc;
   int q_tiles;          // 128-row tiles of the queries
   int32_t* sched_counter;   // zeroed before the launch
@@ -326,8 +329,10 @@ bwd_tcgen05_kernel(const BwdArgs args, const __grid_constant__ CUtensorMap map_a
     mbar_init(&bars->stat_empty, FUSED ? 2 : 1);   // fused: both issuing threads read the stationary K tile
     mbar_init(&bars->acc_free, C::EW_THREADS);
     mbar_init(&bars->y_free, C::EW_THREADS);
-    mbar_init(&bars->z_free[0], BS);
-    mbar_init(&bars->z_free[1], BS);
+    for (int t = 0; t < 2; ++t) {
+      mbar_init(&bars->z_free[t], BS);
+      mbar_init(&bars->red_done[t], BS / 32);
+    }
     for (int s = 0; s < 4; ++s) {
       mbar_init(&bars->strm_full[s], 1);
       mbar_init(&bars->strm_empty[s], 1);
@@ -344,10 +349,11 @@ bwd_tcgen05_kernel(const BwdArgs args, const __grid_constant__ CUtensorMap map_a
   }
   if (KVS) {
     // the ones (bf16 1.0 in the first three of 16 columns), and zeros behind the terms of the statistics
+    constexpr int REGION = C::STATS_OFF - C::ONES_BYTES, ONES_CHUNK = (C::ONES_OFF & 127) / 16, ONES_TILE = (C::ONES_OFF - REGION) / (BS * 128);
     for (int i = tid; i < (C::ONES_BYTES + C::STATS_BYTES) / 16; i += C::THREADS) {
       const int r = (i >> 3) & 7, c = (i & 7) ^ r;       // row within its 8-row group, logical 16-byte chunk
-      const bool ones = i < C::ONES_BYTES / 16 && c == 0;
-      tc::sts128(smem_base + C::ONES_OFF + i * 16, ones ? make_uint4(0x3f803f80u, 0x00003f80u, 0u, 0u) : make_uint4(0u, 0u, 0u, 0u));
+      const bool ones = i / (BS * 8) == ONES_TILE && c == ONES_CHUNK;
+      tc::sts128(smem_base + REGION + i * 16, ones ? make_uint4(0x3f803f80u, 0x00003f80u, 0u, 0u) : make_uint4(0u, 0u, 0u, 0u));
     }
     fence_proxy_async_smem();
   }
@@ -562,7 +568,7 @@ bwd_tcgen05_kernel(const BwdArgs args, const __grid_constant__ CUtensorMap map_a
           if (leader) umma_ts(tmem + (KVS ? C::COL_ACC2 : C::COL_ACC1), tmem + C::col_ds(t, kk), b1 + (uint64_t)((kk * 2048) >> 4),
                   IDESC_ACC, (!first || kk > 0) ? 1u : 0u);
         if (FUSED) {
-          const uint64_t ds = desc_ds + (uint64_t)(((t % C::DS_BUFFERS) * C::DS_TILE) >> 4);
+          const uint64_t ds = desc_ds + (uint64_t)((t * C::DS_TILE) >> 4);
           // head dim 128, the single dQ^T buffer: the previous step's tile has been loaded
           if (D == 128 && it >= 1) {
             if (!mbar_wait(&bars->z_free[0], (it - 1) & 1, abort_flag)) { ok = false; break; }
@@ -588,10 +594,8 @@ bwd_tcgen05_kernel(const BwdArgs args, const __grid_constant__ CUtensorMap map_a
     // the load / store pipe, which the element-wise threads spent between two steps (2700 clocks a step,
     // half of them here) while the products waited.  TMEM lane = d, column = query; a warp's 32 lanes
     // cover 32 consecutive d of one query row.
-    // Head dim 64: TMEM lane = query, column = d; the accumulator keeps 128 query rows contiguous.
+    // Head dim 64: TMEM lane = query, column = d (BwdArgs::dq_acc).
     const uint32_t z_lanes = tmem + ((uint32_t)((warp & 3) * 32) << 16);
-    const int zlane = tid & (BS - 1);                // d, or the query row of a tile
-    constexpr int ROW = D == 128 ? D : BS;           // accumulator elements from one TMEM column to the next
     BItem bi;
     int it = 0;                                      // running step count
     bool alive = true;
@@ -599,30 +603,59 @@ bwd_tcgen05_kernel(const BwdArgs args, const __grid_constant__ CUtensorMap map_a
       for (int g = 0; g < n_heads && alive; ++g) {
         const int h = bi.h_kv * group + g;
         const StepWalk<BT> w = make_steps<MODE, BT>(p, args, bi.tile, h);
-        float* head_rows = args.dq_acc + ((int64_t)bi.b * p.H_q + h) * (D == 128 ? p.N_q : args.q_tiles * BS) * D + zlane;
+        float* head_rows = args.dq_acc + ((int64_t)bi.b * p.H_q + h) * p.N_q * D + (tid & (BS - 1));   // d
+        float* head_tiles = args.dq_acc + ((int64_t)bi.b * p.H_q + h) * args.q_tiles * BS * D;
         for (int s = 0; s < w.cnt; ++s, ++it) {
           const int r0 = w.row0(s), n_valid = p.N_q - r0;
           if (!mbar_wait(&bars->acc_done[it & 1], (it >> 1) & 1, abort_flag)) { alive = false; break; }
           tc_fence_after_sync();
           const uint32_t z_tmem = z_lanes + C::col_z(it & 1);
+          if (D == 64) {
+            // The warp's 32 rows go out as one bulk reduction of 8 KB, staged where the step's dS^T lay, which
+            // the products have read by now: 64 reductions per thread kept the load / store pipe from
+            // the element-wise threads' dS^T.
+            const uint32_t stage = sDS0 + (it & 1) * C::DS_TILE + (warp & 3) * (32 * D * 4);
+#pragma unroll
+            for (int c0 = 0; c0 < 64; c0 += 32) {
+              uint32_t zr[32];
+              tmem_ld32(z_tmem + c0, zr);
+              tmem_wait_ld32(zr);
+#pragma unroll
+              for (int c = 0; c < 32; c += 4)
+                tc::sts128(stage + (c0 + c) * 128 + lane * 16, make_uint4(zr[c], zr[c + 1], zr[c + 2], zr[c + 3]));
+            }
+            tc_fence_before_sync();
+            mbar_arrive(&bars->z_free[it & 1]);
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+              bulk_reduce_add_f32(head_tiles + (int64_t)(r0 + (warp & 3) * 32) * D, stage, 32 * D * 4);   // r0 is a multiple of 128
+              bulk_commit_group();
+              bulk_wait_read_all();
+              mbar_arrive(&bars->red_done[it & 1]);
+            }
+            __syncwarp();
+            continue;
+          }
           uint32_t zr[64];
           tmem_ld32(z_tmem, &zr[0]);
           tmem_ld32(z_tmem + 32, &zr[32]);
           tmem_wait_ld();
           tc_fence_before_sync();
-          mbar_arrive(&bars->z_free[D == 128 ? 0 : it & 1]);
-          float* acc_rows = head_rows + (int64_t)r0 * D;         // r0 is a multiple of 128 at head dim 64
-          if (D == 64 || n_valid >= 64) {
+          mbar_arrive(&bars->z_free[0]);
+          float* acc_rows = head_rows + (int64_t)r0 * D;
+          if (n_valid >= 64) {
 #pragma unroll
-            for (int c = 0; c < 64; ++c) atomicAdd(acc_rows + c * ROW, __uint_as_float(zr[c]));
+            for (int c = 0; c < 64; ++c) atomicAdd(acc_rows + c * D, __uint_as_float(zr[c]));
           } else {
 #pragma unroll
             for (int c = 0; c < 64; ++c)
-              if (c < n_valid) atomicAdd(acc_rows + c * ROW, __uint_as_float(zr[c]));
+              if (c < n_valid) atomicAdd(acc_rows + c * D, __uint_as_float(zr[c]));
           }
         }
       }
     }
+    if (D == 64 && lane == 0) bulk_wait_all();       // complete before the grid ends
   } else {
     // ============================== element-wise group / epilogue ==============================
     const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
@@ -682,9 +715,11 @@ bwd_tcgen05_kernel(const BwdArgs args, const __grid_constant__ CUtensorMap map_a
           }
         }
 
-        // 32 columns at a time (BCfg::THREADS).
+        // 32 columns at a time (BCfg::THREADS)
 #pragma unroll 1
         for (int u = 0; u < COLS; u += 32) {
+          const int rel_u = rel - u, limit_u = col_limit - u;
+          const uint32_t bits_u = (uint32_t)(tile_bits >> u);
           uint32_t xr[32], yr[32], pk[16], dk[16];
           tmem_ld32(xt + u, xr);
           tmem_ld32(yt + u, yr);
@@ -695,8 +730,6 @@ bwd_tcgen05_kernel(const BwdArgs args, const __grid_constant__ CUtensorMap map_a
             tc_fence_before_sync();
             mbar_arrive(&bars->y_free);
           }
-          const int rel_u = rel - u, limit_u = col_limit - u;
-          const uint32_t bits_u = (uint32_t)(tile_bits >> u);
           const float relf = (float)rel_u;
           // The masking decision is taken once per tile: the element loop exists in a masked and an
           // unmasked copy.  The arithmetic runs on packed fp32 pairs (half the issue slots).
@@ -735,12 +768,11 @@ bwd_tcgen05_kernel(const BwdArgs args, const __grid_constant__ CUtensorMap map_a
           else element_pass(std::false_type{});
           if (FUSED) {
             // dS^T row of this key: 64 queries = 128 bytes = eight 16-byte chunks, chunk c stored at
-            // c ^ (row & 7) (the 128-byte swizzle the MMA descriptor expects).  Two buffers: buffer t was
-            // last read by the products of step it-2, which ran before this step's S^T was issued.
-            // One: by those of step it-1.
-            if (C::DS_BUFFERS == 1 && u == 0 && it >= 1 &&
-                !mbar_wait(&bars->acc_done[t ^ 1], ((it - 1) >> 1) & 1, abort_flag)) { alive = false; break; }
-            const uint32_t row_addr = sDS0 + (t % C::DS_BUFFERS) * C::DS_TILE + share * C::DS_PANEL + lrow * 128;
+            // c ^ (row & 7) (the 128-byte swizzle the MMA descriptor expects).  Buffer t was last read by the
+            // products of step it-2, which ran before this step's S^T was issued, and at head dim 64 by the
+            // reduction of their dQ.
+            if (D == 64 && u == 0 && it >= 2 && !mbar_wait(&bars->red_done[t], ((it >> 1) - 1) & 1, abort_flag)) { alive = false; break; }
+            const uint32_t row_addr = sDS0 + t * C::DS_TILE + share * C::DS_PANEL + lrow * 128;
             const int c0u = u >> 3;
 #pragma unroll
             for (int c8 = 0; c8 < 4; ++c8)
@@ -781,21 +813,22 @@ bwd_tcgen05_kernel(const BwdArgs args, const __grid_constant__ CUtensorMap map_a
         const T* cos_row = ROPE ? reinterpret_cast<const T*>(p.cos) + (int64_t)srow * p.rope_stride_n : nullptr;
         const T* sin_row = ROPE ? reinterpret_cast<const T*>(p.sin) + (int64_t)srow * p.rope_stride_n : nullptr;
 #pragma unroll
-        for (int c = 0; c < D / 64; ++c) {
-          // columns [32c, 32c+32) and their partners [32c + D/2, ...)
-          uint32_t lo[32], hi[32];
+        for (int c = 0; c < D / 32; ++c) {
+          if (SHARES == 2 && !KVS && c != share) continue;
+          // columns [16c, 16c+16) and their partners [16c + D/2, ...)
+          uint32_t lo[16], hi[16];
           if (total_steps > 0) {
-            tmem_ld32(acc + c * 32, lo);
-            tmem_ld32(acc + D / 2 + c * 32, hi);
-            tmem_wait_ld();
+            tmem_ld16(acc + c * 16, lo);
+            tmem_ld16(acc + D / 2 + c * 16, hi);
+            tmem_wait_ld16(lo);
+            tmem_wait_ld16(hi);
           } else {
 #pragma unroll
-            for (int i = 0; i < 32; ++i) lo[i] = hi[i] = 0u;
+            for (int i = 0; i < 16; ++i) lo[i] = hi[i] = 0u;
           }
           if (store) {
 #pragma unroll
-            for (int q4 = 0; q4 < 4; ++q4) {
-              if (SHARES == 2 && !KVS && (q4 >> 1) != share) continue;
+            for (int q4 = 0; q4 < 2; ++q4) {
               float gl[8], gh[8];
 #pragma unroll
               for (int i = 0; i < 8; ++i) {
@@ -803,7 +836,7 @@ bwd_tcgen05_kernel(const BwdArgs args, const __grid_constant__ CUtensorMap map_a
                 gh[i] = __uint_as_float(hi[q4 * 8 + i]) * p.sm_scale;
               }
               if (ROPE) {
-                const int d0 = c * 32 + q4 * 8;
+                const int d0 = c * 16 + q4 * 8;
                 const uint4 cl = __ldg(reinterpret_cast<const uint4*>(cos_row + d0));
                 const uint4 ch = __ldg(reinterpret_cast<const uint4*>(cos_row + D / 2 + d0));
                 const uint4 sl = __ldg(reinterpret_cast<const uint4*>(sin_row + d0));
@@ -825,8 +858,8 @@ bwd_tcgen05_kernel(const BwdArgs args, const __grid_constant__ CUtensorMap map_a
               vl.z = Pack2<T>::run(gl[4], gl[5]); vl.w = Pack2<T>::run(gl[6], gl[7]);
               vh.x = Pack2<T>::run(gh[0], gh[1]); vh.y = Pack2<T>::run(gh[2], gh[3]);
               vh.z = Pack2<T>::run(gh[4], gh[5]); vh.w = Pack2<T>::run(gh[6], gh[7]);
-              *reinterpret_cast<uint4*>(dst + c * 32 + q4 * 8) = vl;
-              *reinterpret_cast<uint4*>(dst + D / 2 + c * 32 + q4 * 8) = vh;
+              *reinterpret_cast<uint4*>(dst + c * 16 + q4 * 8) = vl;
+              *reinterpret_cast<uint4*>(dst + D / 2 + c * 16 + q4 * 8) = vh;
             }
           }
         }

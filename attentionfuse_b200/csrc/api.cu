@@ -125,6 +125,15 @@ int64_t af_bwd_dq_accum_bytes(const AfBwdParams* params) {
   return bwd_mma_dq_accum_bytes(*params);
 }
 
+int af_decode(const AfDecodeParams* params, af_stream_t stream) {
+  if (params == nullptr) return fail(AF_ERR_INVALID, "params is NULL");
+  return launch_decode(*params, static_cast<cudaStream_t>(stream));
+}
+
+int32_t af_decode_cluster_size(const AfDecodeParams* params) {
+  return params == nullptr ? 0 : decode_cluster_size(*params);
+}
+
 int af_decode_split(const AfDecodeParams* params, af_stream_t stream) {
   if (params == nullptr) return fail(AF_ERR_INVALID, "params is NULL");
   return launch_decode_split(*params, static_cast<cudaStream_t>(stream));

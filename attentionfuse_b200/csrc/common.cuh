@@ -87,6 +87,8 @@ int launch_bwd_mma(const AfBwdParams& a, cudaStream_t st);
 bool bwd_mma_supports(const AfBwdParams& a, const char** why);
 
 int launch_decode_split(const AfDecodeParams& a, cudaStream_t st);
+int launch_decode(const AfDecodeParams& a, cudaStream_t st);
+int decode_cluster_size(const AfDecodeParams& a);
 // Split-K decode of large head groups (MQA) on the tcgen05 forward kernel: the query heads of a KV
 // group are the rows of one query tile.  Same partials as launch_decode_split.
 bool decode_tc_supports(const AfDecodeParams& a);

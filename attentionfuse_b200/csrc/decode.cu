@@ -15,6 +15,8 @@
 //   * Partial results go to fp32 workspaces; a vectorised combine kernel merges the splits.
 //
 // Per-sequence valid lengths (kv_lens) are an extension: the reference only has a scalar N_KV.
+#include <cooperative_groups.h>
+
 #include <mutex>
 
 #include "common.cuh"
@@ -140,7 +142,12 @@ __device__ __forceinline__ int keys_upto(const AfDecodeParams& a, int pos) {
 // keys [lo, hi) of that head, written as un-normalised partials (m, l, acc) to the rows starting
 // at `ws_rowc` (the row of the chunk's first head).  Ends with a CTA barrier, so that segments
 // can follow one another in one CTA.
-template <typename T, int D, int KPW, bool ROPE>
+// CLUSTER: the partial of the CTA's keys stays in shared memory instead (Local<D>), for the other CTAs of its cluster.
+template <int D> struct Local {            // rows of one unit: m, l (base 2), acc
+  float m[16], l[16], acc[16 * D];
+  static constexpr int OFFSET = 64 * 1024;  // behind the merge of the warps' partials, inside the ring
+};
+template <typename T, int D, int KPW, bool ROPE, bool CLUSTER = false>
 __device__ __forceinline__ void decode_segment(const AfDecodeParams& a, unsigned char* smem_raw, const int b, const int h_kv,
                                                const int chunk, const int lo, const int hi, const int q_pos,
                                                const int64_t ws_rowc) {
@@ -383,6 +390,12 @@ __device__ __forceinline__ void decode_segment(const AfDecodeParams& a, unsigned
         acc += sc * sm_o[(w * 16 + r) * D + d];
         lsum += sc * sm_l[w * 16 + r];
       }
+      if (CLUSTER) {
+        Local<D>* part = reinterpret_cast<Local<D>*>(smem_raw + Local<D>::OFFSET * D / 128);
+        part->acc[idx] = acc;
+        if (d == 0) { part->m[r] = mstar; part->l[r] = lsum; }
+        continue;
+      }
       const int64_t row = ws_row0 + head0 + r;
       a.ws_acc[row * D + d] = acc;
       if (d == 0) {
@@ -429,6 +442,46 @@ __device__ __forceinline__ KeyRange key_range(const AfDecodeParams& a, int b) {
   r.lo = k_lo;
   r.span = max(k_hi - k_lo, 0);
   return r;
+}
+
+// Decode in one launch: the CTAs of a cluster share the keys of one (batch, kv head), keep their partials in shared
+// memory and each merge a part of the unit's output from all of them.  What bounds a short cache is not
+// bytes but launches and trips to memory: the split and its combine take 9 + 7 us for the 4 MB of 8
+// heads x 1024 keys, two launches and the partials' way through the L2 among them (21.5 us per eager call; 15.5 in
+// one launch).
+template <typename T, int D, bool ROPE>
+__global__ void __launch_bounds__(DEC_THREADS) decode_cluster_kernel(const AfDecodeParams a) {
+  extern __shared__ unsigned char smem_raw[];
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int n = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+  const int unit = (int)(blockIdx.x / n), b = unit / a.H_kv, h_kv = unit - b * a.H_kv;
+  const int group = a.H_q / a.H_kv;
+  const KeyRange range = key_range(a, b);
+  const int tiles = (range.span + DEC_BN - 1) / DEC_BN;
+  const int t0 = (int)((int64_t)rank * tiles / n), t1 = (int)((int64_t)(rank + 1) * tiles / n);
+  decode_segment<T, D, 16, ROPE, true>(a, smem_raw, b, h_kv, 0, range.lo + t0 * DEC_BN,
+                                       range.lo + min(t1 * DEC_BN, range.span), range.q_pos, 0);
+  Local<D>* part = reinterpret_cast<Local<D>*>(smem_raw + Local<D>::OFFSET * D / 128);
+  cluster.sync();
+  for (int idx = rank * DEC_THREADS + (int)threadIdx.x; idx < group * D; idx += n * DEC_THREADS) {
+    const int r = idx / D, d = idx - r * D;
+    float m = -INFINITY;
+    for (int i = 0; i < n; ++i) m = fmaxf(m, cluster.map_shared_rank(part, i)->m[r]);
+    const float m_use = (m == -INFINITY) ? 0.f : m;
+    float acc = 0.f, l = 0.f;
+#pragma unroll 8
+    for (int i = 0; i < n; ++i) {
+      const Local<D>* p = cluster.map_shared_rank(part, i);
+      const float w = exp2f(p->m[r] - m_use);
+      l += w * p->l[r];
+      acc += w * p->acc[idx];
+    }
+    const int h = h_kv * group + r;
+    reinterpret_cast<T*>(a.o)[(int64_t)b * a.o_stride[0] + (int64_t)h * a.o_stride[1] + (int64_t)d * a.o_stride[3]] =
+        Elem<T>::from_f32(l == 0.f ? 0.f : acc / l);
+  }
+  cluster.sync();        // the partials stay until every CTA has read them
 }
 
 // Balanced scheduling (balanced_ctas = C > 0): the 64-key tiles of all (batch, kv head, head
@@ -837,13 +890,47 @@ int launch_combine_impl(const AfDecodeParams& a, cudaStream_t st) {
   return check_cuda(cudaGetLastError(), "decode_combine launch");
 }
 
-int validate_decode(const AfDecodeParams& a) {
+template <typename T, int D>
+int launch_cluster_impl(const AfDecodeParams& a, int size, cudaStream_t st) {
+  constexpr size_t smem = (size_t)2 * DEC_STAGES * DEC_BN * D * 2;
+  static_assert((size_t)Local<D>::OFFSET * D / 128 + sizeof(Local<D>) <= smem && 4 * (2 * 16 + 16 * D) * 4 <= Local<D>::OFFSET * D / 128,
+                "the CTA's partial lies behind the merge of its warps, inside the ring");
+  auto kern = a.rope ? decode_cluster_kernel<T, D, true> : decode_cluster_kernel<T, D, false>;
+  static bool configured[2] = {};       // benign race: the attribute calls are idempotent
+  if (!configured[a.rope ? 1 : 0]) {
+    AF_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    AF_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    configured[a.rope ? 1 : 0] = true;
+  }
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = (unsigned)size;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)(size * a.B * a.H_kv));
+  cfg.blockDim = dim3(DEC_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  AF_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, a));
+  count_launch();
+  return check_cuda(cudaGetLastError(), "decode_cluster launch");
+}
+
+int validate_problem(const AfDecodeParams& a) {
   AF_REQUIRE(a.dtype == AF_F16 || a.dtype == AF_BF16, "decode kernels take f16/bf16 (got dtype %d)", a.dtype);
   AF_REQUIRE(a.D == 64 || a.D == 128, "decode kernels are instantiated for D in {64,128} (got %d)", a.D);
   AF_REQUIRE(a.B > 0 && a.H_kv > 0 && a.H_q > 0 && a.H_q % a.H_kv == 0, "bad head/batch counts");
   AF_REQUIRE(a.num_splits >= 1 || a.balanced_ctas > 0, "num_splits must be >= 1");
   AF_REQUIRE(a.balanced_ctas >= 0 && a.balanced_ctas <= 65535, "balanced_ctas outside [0, 65535]");
   AF_REQUIRE((int64_t)a.B * a.H_kv * ((a.H_q / a.H_kv + 63) / 64) <= 65535, "B*H_kv too large for one launch");
+  return AF_OK;
+}
+
+int validate_decode(const AfDecodeParams& a) {
+  const int rc = validate_problem(a);
+  if (rc != AF_OK) return rc;
   AF_REQUIRE(a.ws_m && a.ws_l && a.ws_acc, "decode workspaces must be non-NULL");
   // the combine reads ws_acc rows as float4 (D = 128) / float2 (D = 64); the tensor-core split
   // epilogue stores float4
@@ -919,9 +1006,25 @@ int launch_decode_static(const AfDecodeParams& in, cudaStream_t st) {
   return launch_decode_combine(a, st);
 }
 
-int launch_decode_split(const AfDecodeParams& a, cudaStream_t st) {
-  int rc = validate_decode(a);
-  if (rc != AF_OK) return rc;
+// CTAs per cluster with which a problem runs in one launch, or 0 where the split and its combine are in charge.  One
+// launch saves 2 - 4 us on the device and 5 in an eager call, until the split's even share of all SMs is worth
+// more.  us in graph replay, 32 query heads on 8 (split; clusters of 8; of 16), D = 128:
+//   1 sequence of 1024 keys 10.4; 6.9; 7.8, of 4096 13.9; 11.8; 11.1, of 8192 20.8; 18.2; 15.5, of 16384 26.7; 31.2; 24.2
+//   2 of 1024 10.7; 8.3; 14.3, of 4096 17.0; 14.9; 20.8, of 8192 (64 heads) 25.7; 24.6; 29.9
+//   3 of 1024 11.2; 9.1; 15.3, of 4096 20.5; 15.9; 22.3      5 of 1024 13.4; 16.1; 22.6
+// So: clusters of 16 while they have an SM per CTA and long caches, of 8 while all CTAs are resident at once (two
+// per SM), and up to 1024 keys a CTA.  A row that a causal or window mask positions inside its cache keeps the split.
+int decode_cluster_size(const AfDecodeParams& a) {
+  if (a.H_kv < 1 || a.B < 1 || a.H_q % a.H_kv != 0 || a.H_q / a.H_kv > 16) return 0;
+  if (a.mask_kind != AF_MASK_FULL || a.rope == 1 || (a.dtype != AF_F16 && a.dtype != AF_BF16) || (a.D != 64 && a.D != 128)) return 0;
+  int sms = 0;
+  if (tc_sm_count(&sms) != AF_OK) return 0;
+  const int64_t units = (int64_t)a.B * a.H_kv;
+  const int size = units * 16 <= sms && a.N_kv >= 4096 ? 16 : units * 8 <= 2 * (int64_t)sms ? 8 : 0;
+  return a.N_kv <= 1024 * size ? size : 0;
+}
+
+static int check_decode_operands(const AfDecodeParams& a) {
   AF_REQUIRE(a.q && a.k && a.v, "q/k/v must be non-NULL");
   AF_REQUIRE(a.q_stride[3] == 1 && a.k_stride[3] == 1 && a.v_stride[3] == 1, "decode needs unit inner strides");
   AF_REQUIRE(a.k_stride[2] % 8 == 0 && a.v_stride[2] % 8 == 0 && a.k_stride[1] % 8 == 0 && a.v_stride[1] % 8 == 0 &&
@@ -939,6 +1042,26 @@ int launch_decode_split(const AfDecodeParams& a, cudaStream_t st) {
     AF_REQUIRE(a.rope_stride_n % 8 == 0 && ((uintptr_t)a.cos & 15) == 0 && ((uintptr_t)a.sin & 15) == 0,
                "cos/sin rows must be 16-byte aligned");
   }
+  return AF_OK;
+}
+
+int launch_decode(const AfDecodeParams& a, cudaStream_t st) {
+  const int size = decode_cluster_size(a);
+  int rc;
+  if (size == 0 || a.ws_acc != nullptr || a.partial != nullptr) {
+    if ((rc = launch_decode_split(a, st)) != AF_OK) return rc;
+    return launch_decode_combine(a, st);
+  }
+  if ((rc = validate_problem(a)) != AF_OK || (rc = check_decode_operands(a)) != AF_OK) return rc;
+  AF_REQUIRE(a.o != nullptr, "decode needs o");
+  if (a.dtype == AF_F16) return a.D == 64 ? launch_cluster_impl<__half, 64>(a, size, st) : launch_cluster_impl<__half, 128>(a, size, st);
+  return a.D == 64 ? launch_cluster_impl<__nv_bfloat16, 64>(a, size, st) : launch_cluster_impl<__nv_bfloat16, 128>(a, size, st);
+}
+
+int launch_decode_split(const AfDecodeParams& a, cudaStream_t st) {
+  int rc = validate_decode(a);
+  if (rc != AF_OK) return rc;
+  if ((rc = check_decode_operands(a)) != AF_OK) return rc;
   // more than 16 query heads per KV head: tensor-bound on mma.sync, so the tcgen05 kernel takes it
   if (a.balanced_ctas == 0 && decode_tc_supports(a)) return launch_decode_split_tc(a, st);
   if (a.dtype == AF_F16) return a.D == 64 ? launch_split_impl<__half, 64>(a, st) : launch_split_impl<__half, 128>(a, st);

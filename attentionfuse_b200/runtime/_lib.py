@@ -96,7 +96,7 @@ class AfPeerExchange(C.Structure):
                 ("wait_cycles", I64)]
 
 
-EXPORTS = ("af_fwd", "af_fwd_workspace_bytes", "af_fwd_layout", "af_bwd", "af_bwd_workspace_bytes", "af_bwd_dq_accum_bytes", "af_decode_split", "af_decode_combine", "af_decode_static", "af_decode_exchange_bytes", "af_decode_combine_push", "af_decode_wait_merge", "af_decode_sharded_step",
+EXPORTS = ("af_fwd", "af_fwd_workspace_bytes", "af_fwd_layout", "af_bwd", "af_bwd_workspace_bytes", "af_bwd_dq_accum_bytes", "af_decode", "af_decode_cluster_size", "af_decode_split", "af_decode_combine", "af_decode_static", "af_decode_exchange_bytes", "af_decode_combine_push", "af_decode_wait_merge", "af_decode_sharded_step",
            "af_decode_combine_gathered", "af_decode_num_splits", "af_query_family",
            "af_launch_count", "af_last_error", "af_abi_version")
 
@@ -133,6 +133,10 @@ def load() -> C.CDLL:
         lib.af_bwd_dq_accum_bytes.restype = I64
         lib.af_decode_split.argtypes = [C.POINTER(AfDecodeParams), PTR]
         lib.af_decode_combine.argtypes = [C.POINTER(AfDecodeParams), PTR]
+        lib.af_decode.argtypes = [C.POINTER(AfDecodeParams), PTR]
+        lib.af_decode.restype = I32
+        lib.af_decode_cluster_size.argtypes = [C.POINTER(AfDecodeParams)]
+        lib.af_decode_cluster_size.restype = I32
         lib.af_decode_exchange_bytes.argtypes = [I32, I32, I32, I32]
         lib.af_decode_exchange_bytes.restype = I64
         lib.af_decode_combine_push.argtypes = [C.POINTER(AfDecodeParams), C.POINTER(AfPeerExchange), PTR]

@@ -102,7 +102,7 @@ def run_flash_decode(graph: Optional[Graph], Q: torch.Tensor, K: torch.Tensor, V
                      cos: Optional[torch.Tensor] = None, sin: Optional[torch.Tensor] = None,
                      balanced_ctas: int = 0, kv_rotated: bool = False,
                      kv_pos_block: int = 0, kv_pos_stride: int = 0) -> torch.Tensor:
-    """Two launches: split-K partials, then the LSE combine.  Returns `out` (or `partial`
+    """Split-K partials, then the LSE combine (one launch where the cache is short).  Returns `out` (or `partial`
     when only the packed partial is requested)."""
     lib = _lib.load()
     B, H_q, _, D = Q.shape
@@ -113,7 +113,8 @@ def run_flash_decode(graph: Optional[Graph], Q: torch.Tensor, K: torch.Tensor, V
     # A rotated row (cos / sin given) is bound by the rotation of the K tiles, not by bandwidth, and
     # wants the higher occupancy of the split grid (0.60 against 1.2 ms at B16 H32/8 L32768) --
     # unless the cache already holds rotated keys (kv_rotated): then only the query row is rotated.
-    if not balanced_ctas and num_splits is None and workspace is None and (cos is None or kv_rotated):
+    own_schedule = not balanced_ctas and num_splits is None and workspace is None
+    if own_schedule and (cos is None or kv_rotated):
         dev_index = Q.device.index if Q.device.index is not None else torch.cuda.current_device()
         balanced_ctas = default_balanced_ctas(B, H_q, H_kv, N_kv, dev_index)
     if balanced_ctas:
@@ -121,16 +122,6 @@ def run_flash_decode(graph: Optional[Graph], Q: torch.Tensor, K: torch.Tensor, V
     elif num_splits is None:
         dev_index = Q.device.index if Q.device.index is not None else torch.cuda.current_device()
         num_splits = _pick_num_splits(B, H_q, H_kv, N_kv, dev_index, kv_lens is not None)
-    if workspace is not None:
-        m_ptr, l_ptr, acc_ptr = (t.data_ptr() for t in workspace)
-    else:
-        # the layout of decode_workspace, addressed without making tensors of its parts
-        rows = balanced_rows(B, H_q, H_kv, balanced_ctas) if balanced_ctas else num_splits * B * H_q
-        rows_pad = (rows + 3) & ~3
-        partials = torch.empty(2 * rows_pad + rows * D, dtype=torch.float32, device=Q.device)
-        m_ptr = partials.data_ptr()
-        l_ptr, acc_ptr = m_ptr + 4 * rows_pad, m_ptr + 8 * rows_pad
-
     slopes = None
     if bias_kind == 1:
         if alibi_slopes is None:
@@ -150,8 +141,8 @@ def run_flash_decode(graph: Optional[Graph], Q: torch.Tensor, K: torch.Tensor, V
            float(sm_scale), int(bias_kind), int(num_splits), int(kv_offset), int(mask_kind), int(window or 0),
            q_position, cos is not None and cos.stride(0), int(balanced_ctas), bool(kv_rotated),
            int(kv_pos_block), int(kv_pos_stride))
-    template = _DECODE_TEMPLATES.get(key)
-    if template is None:
+    known = _DECODE_TEMPLATES.get(key)
+    if known is None:
         p = _lib.AfDecodeParams()
         p.dtype = _lib.dtype_code(Q.dtype)
         p.B, p.H_q, p.H_kv, p.N_kv, p.D = B, H_q, H_kv, N_kv, D
@@ -169,7 +160,20 @@ def run_flash_decode(graph: Optional[Graph], Q: torch.Tensor, K: torch.Tensor, V
             p.o_stride = _lib.strides(out)
         if len(_DECODE_TEMPLATES) >= 256:
             _DECODE_TEMPLATES.clear()
-        template = _DECODE_TEMPLATES[key] = p
+        known = _DECODE_TEMPLATES[key] = (p, int(lib.af_decode_cluster_size(C.byref(p))) > 0)
+    template, one_launch = known
+    # short caches: one launch whose partials stay on the chip
+    one_launch = one_launch and own_schedule and out is not None and partial is None and exchange is None
+    m_ptr = l_ptr = acc_ptr = None
+    if workspace is not None:
+        m_ptr, l_ptr, acc_ptr = (t.data_ptr() for t in workspace)
+    elif not one_launch:
+        # the layout of decode_workspace, addressed without making tensors of its parts
+        rows = balanced_rows(B, H_q, H_kv, balanced_ctas) if balanced_ctas else num_splits * B * H_q
+        rows_pad = (rows + 3) & ~3
+        partials = torch.empty(2 * rows_pad + rows * D, dtype=torch.float32, device=Q.device)
+        m_ptr = partials.data_ptr()
+        l_ptr, acc_ptr = m_ptr + 4 * rows_pad, m_ptr + 8 * rows_pad
     p = _lib.AfDecodeParams.from_buffer_copy(template)
     p.q, p.k, p.v = Q.data_ptr(), K.data_ptr(), V.data_ptr()
     p.slopes, p.kv_lens, p.q_positions = _lib.ptr(slopes), _lib.ptr(kv_lens), _lib.ptr(q_positions)
@@ -187,13 +191,14 @@ def run_flash_decode(graph: Optional[Graph], Q: torch.Tensor, K: torch.Tensor, V
             _lib.check(lib.af_decode_sharded_step(C.byref(p), C.byref(exchange.c), int(exchange_mode), stream),
                        "af_decode_sharded_step")
             return out
-        _lib.check(lib.af_decode_split(C.byref(p), stream), "af_decode_split")
-        if exchange is not None:
+        if exchange is None:
+            _lib.check(lib.af_decode(C.byref(p), stream), "af_decode")
+        else:
+            _lib.check(lib.af_decode_split(C.byref(p), stream), "af_decode_split")
             # KV-sharded step: the combine pushes this rank's partial to every rank's exchange
             # buffer; the caller follows up with exchange.wait_merge(out)
             _lib.check(lib.af_decode_combine_push(C.byref(p), C.byref(exchange.c), stream), "af_decode_combine_push")
             return None
-        _lib.check(lib.af_decode_combine(C.byref(p), stream), "af_decode_combine")
     return out if out is not None else partial
 
 

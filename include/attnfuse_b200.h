@@ -226,6 +226,14 @@ AF_API int64_t af_bwd_workspace_bytes(const AfBwdParams* params);
  * (attnfuse/compiler/codegen_backward.py:75-302).  Host only. */
 AF_API int64_t af_bwd_dq_accum_bytes(const AfBwdParams* params);
 
+/* One decode step: the split and the combine below in one call.  With ws_acc == NULL and
+ * af_decode_cluster_size() > 0 it is one launch and needs no workspace. */
+AF_API int af_decode(const AfDecodeParams* params, af_stream_t stream);
+
+/* CTAs that share the keys of one (batch, kv head) when af_decode runs as one launch, 0 when the problem needs
+ * the split and its workspaces.  Looks at sizes, mask and rotation; pointers may be NULL.  Host only. */
+AF_API int32_t af_decode_cluster_size(const AfDecodeParams* params);
+
 /* Replaces the split launch of run_flash_decode (attnfuse/runtime/flash_decode.py:149-170). */
 AF_API int af_decode_split(const AfDecodeParams* params, af_stream_t stream);
 

@@ -1,0 +1,98 @@
+"""Decode in one launch (a cluster of CTAs per (batch, kv head), partials in shared memory): short caches
+of few sequences.  Against the oracle and against the split and its combine on the same problem, at
+the edges of the keys' deal and of the rule that chooses it."""
+import ctypes as C
+
+import pytest
+import torch
+
+import attentionfuse_b200 as af
+from attentionfuse_b200.runtime import _lib
+from attentionfuse_b200.runtime.flash_decode import run_flash_decode
+from oracle import attention_oracle as orc
+from tests._util import assert_close, qkv
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def decode(Q, K, V, one_launch, **kw):
+    q, k, v = Q.to(DEV), K.to(DEV), V.to(DEV)
+    out = torch.full_like(q, float("nan"))
+    if not one_launch:                          # a caller's split count keeps the two launches
+        kw["num_splits"] = 3
+    before = _lib.launch_count()
+    run_flash_decode(None, q, k, v, Q.shape[-1] ** -0.5, kw.pop("bias_kind", 0), K.shape[1], out, **kw)
+    assert _lib.launch_count() - before == (1 if one_launch else 2)
+    return out
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("shape", [(1, 32, 8, 256, 128), (1, 8, 8, 300, 64), (2, 16, 1, 1023, 128), (4, 64, 8, 511, 64), (1, 6, 2, 4097, 128)], ids=str)
+def test_matches_oracle_and_split(shape, dtype):
+    B, Hq, Hkv, N, D = shape
+    Q, K, V = qkv(9800 + N, B, Hq, Hkv, 1, N, D, dtype)
+    one, two = decode(Q, K, V, True), decode(Q, K, V, False)
+    want = orc.attention(Q, K, V)
+    assert_close(one, want, dtype, what=f"one launch {shape}")
+    assert_close(two, want, dtype, what=f"split {shape}")
+
+
+@pytest.mark.parametrize("alibi", [False, True])
+@pytest.mark.parametrize("D", [64, 128])
+def test_lengths_and_alibi(D, alibi):
+    """Ragged lengths (one of them empty, one of a single key), more CTAs than tiles, ALiBi from each row's
+    position, NaN behind the valid keys."""
+    B, Hq, Hkv, N, dtype = 4, 8, 2, 600, torch.bfloat16
+    Q, K, V = qkv(9900 + D, B, Hq, Hkv, 1, N, D, dtype)
+    lens = torch.tensor([600, 1, 0, 333], dtype=torch.int32)
+    for b in range(B):
+        K[b, :, lens[b]:] = float("nan")
+        V[b, :, lens[b]:] = float("nan")
+    pos = torch.tensor([599, 0, 0, 500], dtype=torch.int32)
+    slopes = torch.tensor([2.0 ** -(i + 1) for i in range(Hq)], dtype=dtype)
+    kw = dict(kv_lens=lens.to(DEV))
+    if alibi:
+        kw.update(q_positions=pos.to(DEV), bias_kind=1, alibi_slopes=slopes.to(DEV))
+    one, two = decode(Q, K, V, True, **kw), decode(Q, K, V, False, **kw)
+    assert torch.isfinite(one).all() and (one[2] == 0).all()
+    for b in (0, 1, 3):
+        n = int(lens[b])
+        want = orc.attention(Q[b:b + 1], K[b:b + 1, :, :n], V[b:b + 1, :, :n],
+                             **(dict(slopes=slopes, q_positions=pos[b:b + 1]) if alibi else {}))
+        assert_close(one[b:b + 1], want, dtype, what=f"one launch, sequence {b}")
+        assert_close(two[b:b + 1], want, dtype, what=f"split, sequence {b}")
+
+
+def test_rule_and_capture():
+    lib = _lib.load()
+
+    def size(B, Hq, Hkv, N, **kw):
+        p = _lib.AfDecodeParams()
+        p.dtype, p.B, p.H_q, p.H_kv, p.N_kv, p.D = 2, B, Hq, Hkv, N, 128
+        for k, v in kw.items():
+            setattr(p, k, v)
+        return int(lib.af_decode_cluster_size(C.byref(p)))
+    code = _lib.dtype_code(torch.bfloat16)
+    assert size(1, 32, 8, 1024, dtype=code) == 8 and size(1, 32, 8, 4096, dtype=code) == 16
+    assert size(1, 32, 8, 16384, dtype=code) == 16 and size(1, 32, 8, 16385, dtype=code) == 0
+    assert size(3, 32, 8, 8192, dtype=code) == 8 and size(3, 32, 8, 8193, dtype=code) == 0
+    assert size(16, 32, 8, 1024, dtype=code) == 0 and size(1, 64, 2, 1024, dtype=code) == 0
+    assert size(1, 32, 8, 1024, dtype=code, rope=1) == 0 and size(1, 32, 8, 1024, dtype=code, mask_kind=1) == 0
+    assert size(1, 32, 8, 1024, dtype=_lib.dtype_code(torch.float32)) == 0
+
+    @af.attention
+    def fn(Q, K, V):
+        return af.softmax(af.scaled_dot_product(Q, K)) @ V
+    Q, K, V = (t.to(DEV) for t in qkv(9950, 1, 32, 8, 1, 700, 128, torch.bfloat16))
+    want = fn(Q, K, V)
+    torch.cuda.synchronize()
+    side, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    with torch.cuda.stream(side):
+        fn(Q, K, V)
+        torch.cuda.synchronize()
+        with torch.cuda.graph(graph, stream=side):
+            got = fn(Q, K, V)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(got, want)

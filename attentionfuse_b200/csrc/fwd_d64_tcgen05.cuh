@@ -9,8 +9,8 @@
 // the other's tiles.  That leaves 96 registers per thread: a thread's 64 key columns go through the
 // exponent pass as two runs of 32, and S has one buffer.  What it waits for now is the chain P -> P.V ->
 // next S of a half (600 - 700 clocks) and issue in the exponent pass; the MUFU is busy 67 % of the time
-// (56 % before).  [4,12,4096,64] f16 back to back, before -> now: causal 188 -> 151 us, with ALiBi 188 -> 160,
-// dense 338 -> 286, window 256 93 -> 66.
+// (56 % before).  [4,12,4096,64] f16 back to back, one CTA per SM -> now: causal 188 -> 146 us, with ALiBi
+// 188 -> 155, dense 338 -> 258, window 256 93 -> 61.
 #pragma once
 #include "fwd_tcgen05.cuh"
 
@@ -41,12 +41,56 @@ struct Barriers64 {
   uint64_t ring_free[2];
   uint64_t s_full[2], p_full[2];   // [half of the key columns]
   uint64_t o_done, o_free;
+  uint64_t item_full[4], item_free[4];
+  uint4 item[4];               // answers to the requests for further items
   uint32_t tmem_base;
   int abort_flag;
   uint32_t pair_flag[2][8];
   float xchg[SOFTMAX_THREADS];
 };
 static_assert(sizeof(Barriers64) <= Cfg64::BARRIER_BYTES, "the barriers and the exchange have room");
+
+// Items are handed out as the CTAs get to them: the grid has a block per item, in the order of get_item
+// (heaviest first), and a resident CTA asks the hardware for blocks that have not started (cluster launch
+// control).  A static deal left the last round part empty -- 1536 equal items are 5.2 rounds of 296 CTAs -- and
+// cannot balance block lists; a CTA per item pays its prologue every time.  us, static deal / CTA per
+// item / handed out: dense [4,12,4096] 286 / 268 / 258, causal 151 / 151 / 146, band masks of three blocks a row
+// [2,16,8192] 52 / 63 / 48, BigBird masks there 139 / 132 / 118 (blocks of 64: 176 / 160 / 131).  Few items with a
+// few heavy ones among them lose, whose CTAs share their SM to the end: BigBird [1,12,4096] 39 / 39 / 46.
+// Item k of this CTA: its own block, then the answers.  The producer asks for item k + 1 when it takes
+// item k (and so never again after an answer without a block); every reader releases the answer.  The
+// slots are few and items without key tiles take no time, so no role asks for its next item before it has
+// done all that the others need of the present one.
+constexpr int item_readers(int rope) { return 1 + 32 + SOFTMAX_THREADS + (rope == ROPE_FUSED ? 32 : 0); }
+template <int EMASK, int SPLIT, bool PRODUCER>
+__device__ __forceinline__ bool next_item(const TcArgs& args, Barriers64* bars, int k, volatile int* abort_flag, Item& it) {
+  int w = (int)blockIdx.x;
+  if (k > 0) {
+    const int slot = (k - 1) & 3;
+    if (!mbar_wait(&bars->item_full[slot], ((k - 1) >> 2) & 1, abort_flag)) return false;
+    w = clc_block(&bars->item[slot]);
+    fence_proxy_async_smem();
+    mbar_arrive(&bars->item_free[slot]);
+    if (w < 0) return false;
+  }
+  if (PRODUCER) {
+    const int slot = k & 3;
+    if (k >= 4 && !mbar_wait(&bars->item_free[slot], ((k >> 2) - 1) & 1, abort_flag)) return false;
+    mbar_arrive_expect_tx(&bars->item_full[slot], 16);
+    clc_request(&bars->item[slot], &bars->item_full[slot]);
+  }
+  decode_item<EMASK, SPLIT>(args, w, it);
+  return true;
+}
+template <int EMASK, int SPLIT>
+__device__ __forceinline__ bool cursor_next64(const TcArgs& args, Barriers64* bars, volatile int* abort_flag, TileCursor& c) {
+  if (c.j + 1 < c.it.walk.n_tiles) { ++c.j; ++c.gg; return true; }
+  for (;;) {
+    ++c.round;
+    if (!next_item<EMASK, SPLIT, false>(args, bars, c.round, abort_flag, c.it)) return false;
+    if (c.it.walk.n_tiles > 0) { c.j = 0; ++c.gg; ++c.qi; return true; }
+  }
+}
 
 // Bits [lo, hi] of a 32-bit word (none when the range is empty or outside).
 __device__ __forceinline__ uint32_t bit_range(int lo, int hi) {
@@ -100,6 +144,10 @@ fwd_d64_kernel(const TcArgs args, const __grid_constant__ CUtensorMap tmap_q,
       mbar_init(&bars->s_full[hh], 1);
       mbar_init(&bars->p_full[hh], SOFTMAX_THREADS / 2);
     }
+    for (int s = 0; s < 4; ++s) {
+      mbar_init(&bars->item_full[s], 1);
+      mbar_init(&bars->item_free[s], item_readers(ROPE));
+    }
     bars->abort_flag = 0;
     for (int i = 0; i < 16; ++i) (&bars->pair_flag[0][0])[i] = 0u;
     mbar_fence_init();
@@ -123,45 +171,34 @@ fwd_d64_kernel(const TcArgs args, const __grid_constant__ CUtensorMap tmap_q,
       tma_prefetch_desc(&tmap_v);
       tma_prefetch_desc(&tmap_o);
       const uint64_t stream = l2_policy_evict_first(), keep = SPLIT == SPLIT_DECODE ? stream : l2_policy_evict_last();
-      TileCursor ck, cv;   // K runs one tile ahead of V
-      cursor_init(ck);
-      cursor_init(cv);
-      auto load_k = [&]() -> bool {
-        if (ck.j == 0) {
-          // the single Q buffer is free once the last S product of the previous item has run
-          if (ck.qi > 0 && !mbar_wait(&bars->ring_free[(ck.gg - 1) & 1], ((ck.gg - 1) >> 1) & 1, abort_flag)) return false;
-          mbar_arrive_expect_tx(&bars->q_full, C::TILE_BYTES);
-          tma_load_4d_hint(smem, &tmap_q, &bars->q_full, 0, ck.it.m0, ck.it.h, ck.it.b, stream);
+      Item it;
+      int g = 0, qi = 0;           // key tiles and items with tiles so far
+      bool ok = true;
+      for (int k = 0; ok && next_item<EMASK, SPLIT, true>(args, bars, k, abort_flag, it); ++k) {
+        const int n_tiles = it.walk.n_tiles;
+        if (n_tiles == 0) continue;
+        // the single Q buffer is free once the last S product of the previous item has run
+        if (qi > 0 && !mbar_wait(&bars->ring_free[(g - 1) & 1], ((g - 1) >> 1) & 1, abort_flag)) break;
+        mbar_arrive_expect_tx(&bars->q_full, C::TILE_BYTES);
+        tma_load_4d_hint(smem, &tmap_q, &bars->q_full, 0, it.m0, it.h, it.b, stream);
+        // K runs one tile ahead of V: a wait for a V slot never holds up a K load
+        for (int j = 0; j <= n_tiles; ++j) {
+          if (j < n_tiles) {
+            const int gg = g + j, s = gg & 1;
+            if (gg >= 2 && !mbar_wait(&bars->ring_free[s], ((gg - 2) >> 1) & 1, abort_flag)) { ok = false; break; }
+            mbar_arrive_expect_tx(&bars->k_full[s], C::TILE_BYTES);
+            tma_load_4d_hint(smem + C::TILE_BYTES * (1 + s), &tmap_k, &bars->k_full[s], 0, it.walk.key0(j), it.h_kv, it.b, keep);
+          }
+          if (j > 0) {
+            const int gg = g + j - 1, s = gg & 1;
+            if (gg >= 2 && !mbar_wait(&bars->ring_free[s ^ 1], ((gg - 1) >> 1) & 1, abort_flag)) { ok = false; break; }
+            mbar_arrive_expect_tx(&bars->v_full[s], C::TILE_BYTES);
+            tma_load_4d_hint(smem + C::TILE_BYTES * (1 + STAGES + s), &tmap_v, &bars->v_full[s], 0, it.walk.key0(j - 1), it.h_kv,
+                             it.b, keep);
+          }
         }
-        const int s = ck.gg & 1;
-        if (ck.gg >= 2 && !mbar_wait(&bars->ring_free[s], ((ck.gg - 2) >> 1) & 1, abort_flag)) return false;
-        mbar_arrive_expect_tx(&bars->k_full[s], C::TILE_BYTES);
-        tma_load_4d_hint(smem + C::TILE_BYTES * (1 + s), &tmap_k, &bars->k_full[s], 0, ck.it.walk.key0(ck.j), ck.it.h_kv,
-                         ck.it.b, keep);
-        return true;
-      };
-      auto load_v = [&]() -> bool {
-        const int s = cv.gg & 1;
-        if (cv.gg >= 2 && !mbar_wait(&bars->ring_free[(cv.gg - 1) & 1], ((cv.gg - 1) >> 1) & 1, abort_flag)) return false;
-        mbar_arrive_expect_tx(&bars->v_full[s], C::TILE_BYTES);
-        tma_load_4d_hint(smem + C::TILE_BYTES * (1 + STAGES + s), &tmap_v, &bars->v_full[s], 0, cv.it.walk.key0(cv.j),
-                         cv.it.h_kv, cv.it.b, keep);
-        return true;
-      };
-      bool more_k = cursor_next<EMASK, SPLIT>(args, ck);
-      bool more_v = cursor_next<EMASK, SPLIT>(args, cv);
-      // K runs one tile ahead of V (a wait for a V slot never holds up a K load) -- except across
-      // an item boundary: the first K load of an item starts with a wait for the Q buffer (the
-      // previous item's last S product), so every V tile of the previous item goes out before it.
-      while (more_k || more_v) {
-        const bool at_boundary = more_k && ck.j == 0 && ck.qi > 0 && more_v && cv.gg < ck.gg;
-        if (more_k && !at_boundary && (!more_v || ck.gg <= cv.gg + 1)) {
-          if (!load_k()) break;
-          more_k = cursor_next<EMASK, SPLIT>(args, ck);
-        } else {
-          if (!load_v()) break;
-          more_v = cursor_next<EMASK, SPLIT>(args, cv);
-        }
+        g += n_tiles;
+        ++qi;
       }
     }
   } else if (warp == WARP_MMA64) {
@@ -192,7 +229,7 @@ fwd_d64_kernel(const TcArgs args, const __grid_constant__ CUtensorMap tmap_q,
           umma_commit(&bars->s_full[hh]);
         }
       };
-      bool more = cursor_next<EMASK, SPLIT>(args, cu);
+      bool more = cursor_next64<EMASK, SPLIT>(args, bars, abort_flag, cu);
       if (more && operands_ready()) {
         issue_s(0);
         issue_s(1);
@@ -200,7 +237,7 @@ fwd_d64_kernel(const TcArgs args, const __grid_constant__ CUtensorMap tmap_q,
         while (more) {
           const int gg = cu.gg, j = cu.j, qi = cu.qi, s = gg & 1;
           const bool last = j + 1 == cu.it.walk.n_tiles;
-          more = cursor_next<EMASK, SPLIT>(args, cu);
+          if (!last) cursor_next64<EMASK, SPLIT>(args, bars, abort_flag, cu);
           if (!mbar_wait(&bars->v_full[s], (gg >> 1) & 1, abort_flag)) break;
           // the first P.V product of an item overwrites O: the previous item's rows must be read out
           if (j == 0 && qi > 0 && !mbar_wait(&bars->o_free, (qi - 1) & 1, abort_flag)) break;
@@ -221,6 +258,7 @@ fwd_d64_kernel(const TcArgs args, const __grid_constant__ CUtensorMap tmap_q,
           if (!ok) break;
           if (last) {
             if (leader) umma_commit(&bars->o_done);
+            more = cursor_next64<EMASK, SPLIT>(args, bars, abort_flag, cu);
             if (more) {
               // the next item's Q comes after this item's last S product: its S products follow
               // both halves of P.V, so that a late Q holds nothing up
@@ -246,7 +284,7 @@ fwd_d64_kernel(const TcArgs args, const __grid_constant__ CUtensorMap tmap_q,
     int g = 0, qi = 0;
     uint32_t pair_count = 0;
     bool alive = true;
-    for (int round = 0; alive && get_item<EMASK, SPLIT>(args, round, it); ++round) {
+    for (int round = 0; alive && next_item<EMASK, SPLIT, false>(args, bars, round, abort_flag, it); ++round) {
       const TileWalk& walk = it.walk;
       const int n_tiles = walk.n_tiles;
       const int m0 = it.m0, b = it.b, h = it.h;
@@ -549,7 +587,7 @@ fwd_d64_kernel(const TcArgs args, const __grid_constant__ CUtensorMap tmap_q,
     // ============================== K rotation warp ==============================
     TileCursor cu;
     cursor_init(cu);
-    while (cursor_next<EMASK, SPLIT>(args, cu)) {
+    while (cursor_next64<EMASK, SPLIT>(args, bars, abort_flag, cu)) {
       const int s = cu.gg & 1;
       if (!mbar_wait(&bars->k_full[s], (cu.gg >> 1) & 1, abort_flag)) break;
       const int key0 = cu.it.walk.key0(cu.j);

@@ -232,11 +232,19 @@ struct Item {
 // item weights that fall monotonically the zig-zag evens out the key tiles per CTA to within a
 // fraction of a percent.  With G = number of items every CTA runs exactly one item.
 template <int EMASK, int SPLIT>
+__device__ __forceinline__ void decode_item(const TcArgs& args, int w, Item& it);
+template <int EMASK, int SPLIT>
 __device__ __forceinline__ bool get_item(const TcArgs& args, int round, Item& it) {
   const int G = (int)gridDim.x, c = (int)blockIdx.x;
   const int64_t w64 = (int64_t)round * G + ((round & 1) ? G - 1 - c : c);
   if (w64 >= args.total_items) return false;
-  const int w = (int)w64;
+  decode_item<EMASK, SPLIT>(args, (int)w64, it);
+  return true;
+}
+
+// What item number w is.
+template <int EMASK, int SPLIT>
+__device__ __forceinline__ void decode_item(const TcArgs& args, int w, Item& it) {
   const AfProblem& p = args.a.p;
   int w_over_bh, bh;   // row of query tiles in visiting order (split mode: the split), (batch, head) unit
   split_item(args, w, SPLIT == SPLIT_DECODE ? args.num_splits : SPLIT == SPLIT_SHARES ? args.num_m_blocks * args.key_shares
@@ -257,7 +265,7 @@ __device__ __forceinline__ bool get_item(const TcArgs& args, int round, Item& it
     const int tiles = (it.n_kv + BN - 1) / BN;
     wk.first_tile = (int)((int64_t)it.split * tiles / args.num_splits);
     wk.n_tiles = (int)((int64_t)(it.split + 1) * tiles / args.num_splits) - wk.first_tile;
-    return true;
+    return;
   }
   if (SPLIT == SPLIT_SHARES) {
     const int m_idx = args.div_shares.div(w_over_bh);
@@ -272,7 +280,6 @@ __device__ __forceinline__ bool get_item(const TcArgs& args, int round, Item& it
     it.walk.n_tiles = args.div_shares.div((it.split + 1) * it.walk.n_tiles) - lo;
     it.walk.first_tile += lo;
   }
-  return true;
 }
 
 // Position of a role in the CTA's sequence of key tiles (items without key tiles are skipped):

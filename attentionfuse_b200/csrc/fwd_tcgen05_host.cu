@@ -516,12 +516,12 @@ int launch_fwd_tcgen05(const AfFwdParams& a, cudaStream_t st) {
   { const int rc_sm = tc_sm_count(&sms); if (rc_sm != AF_OK) return rc_sm; }
   const FwdSetup setup = set_up(a, sms);
   const FwdPlan& plan = setup.plan;
-  const int ctas = p.D == 64 ? 2 * sms : sms;   // resident at once
+  const int ctas = p.D == 64 ? args.total_items : sms;   // head dim 64: a block per item, handed out to the resident CTAs
   auto set_grid = [&]() { args.grid_ctas = (ctas > 0 && ctas < args.total_items) ? ctas : args.total_items; };
   args.key_shares = 1;
   {
-    // One CTA fits per SM (shared memory), so the kernel runs persistently: one CTA per SM walks
-    // its share of the query tiles with the pipeline kept full across tile boundaries (measured
+    // Head dim 128: one CTA fits per SM (shared memory), so the kernel runs persistently: one CTA per SM
+    // walks its share of the query tiles with the pipeline kept full across tile boundaries (measured
     // faster than one CTA per query tile at every size, 951 vs 851 TFLOP/s on causal 4x32x4096x128).
     set_grid();
   }
@@ -631,7 +631,7 @@ int launch_decode_split_tc(const AfDecodeParams& a, cudaStream_t st) {
   set_item_order(args, p.B * p.H_q, p.B * p.H_q, a.num_splits);   // splits x (batch, pseudo-head), plain order
   int sms = 0;
   { const int rc_sm = tc_sm_count(&sms); if (rc_sm != AF_OK) return rc_sm; }
-  const int ctas = a.D == 64 ? 2 * sms : sms;
+  const int ctas = a.D == 64 ? args.total_items : sms;
   args.grid_ctas = (ctas > 0 && ctas < args.total_items) ? ctas : args.total_items;
   CUtensorMap mq, mk, mv;
   int rc;

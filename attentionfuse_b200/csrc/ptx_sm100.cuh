@@ -176,6 +176,29 @@ __device__ __forceinline__ void bulk_wait_read_all() { asm volatile("cp.async.bu
 // ... and have completed
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
+// ------------------------------------------------------------------ cluster launch control
+// Asks for a block of this grid that has not started: 16 bytes of answer to shared memory, counted by
+// the mbarrier.  Not to be issued again after an answer without a block.
+__device__ __forceinline__ void clc_request(void* answer, uint64_t* bar) {
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];"
+               ::"r"(smem_u32(answer)), "r"(smem_u32(bar))
+               : "memory");
+}
+// blockIdx.x of the block that was handed over, or -1.
+__device__ __forceinline__ int clc_block(const void* answer) {
+  int x;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b128 r;\n\t"
+      "ld.shared.b128 r, [%1];\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, r;\n\t"
+      "mov.b32 %0, -1;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid.v4.b32.b128 {%0, _, _, _}, r;\n\t}"
+      : "=r"(x)
+      : "r"(smem_u32(answer))
+      : "memory");
+  return x;
+}
+
 // ------------------------------------------------------------------ TMEM allocation
 __device__ __forceinline__ void tmem_alloc(uint32_t* smem_result, uint32_t ncols) {
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_result)),

@@ -75,3 +75,29 @@ def test_infinite_and_lowest_scores():
     want = orc.attention(Q.nan_to_num(0.0), K, V)
     assert_close(got[0, 0, keep], want[0, 0, keep], torch.float16, what="rows beside NaN")
     assert_close(got[0, 1], want[0, 1], torch.float16, what="key at the lowest values")
+
+
+@pytest.mark.parametrize("keep", [[0, 29], [7], [], list(range(0, 30, 6))], ids=str)
+def test_long_stretches_of_items_without_keys(keep):
+    """Block lists that leave most query blocks without a key: a CTA is handed many items in a row that have
+    nothing to load (their rows are zero), among others that have."""
+    B, H, n, dtype = 1, 40, 30, torch.float16
+    N = n * 128 - 50
+    grids = torch.zeros(H, n, n, dtype=torch.bool)
+    gen = torch.Generator().manual_seed(3)
+    for r in keep:
+        grids[:, r] = torch.rand(H, n, generator=gen) < 0.2
+        grids[:, r, r] = True
+    Q, K, V = qkv(9450, B, H, H, N, N, D, dtype)
+
+    @af.attention
+    def fn(Q, K, V):
+        return af.softmax(af.block_sparse(af.scaled_dot_product(Q, K))) @ V
+    out = fn(Q.to(DEV), K.to(DEV), V.to(DEV), block_mask=af.create_block_mask_per_head(grids, 128, 128, device=DEV)).cpu()
+    live = torch.zeros(n, dtype=torch.bool)
+    live[keep] = True
+    assert (out[:, :, ~live.repeat_interleave(128)[:N]] == 0).all()
+    for h in (0, 17, 39):
+        elem = grids[h:h + 1].repeat_interleave(128, 1).repeat_interleave(128, 2)[:, :N, :N]
+        want = orc.attention(Q[:, h:h + 1], K[:, h:h + 1], V[:, h:h + 1], elem_mask=elem)
+        assert_close(out[:, h:h + 1], want, dtype, what=f"sparse rows {keep} head {h}")

@@ -90,7 +90,7 @@ __global__ void bwd_delta_kernel(const AfBwdParams a) {
 // 63 us = 4.3 TB/s with one row per thread and 64-bit divisions for its coordinates).
 constexpr int DELTA_ROWS = 4;
 template <typename T, int LPR>
-__global__ void bwd_delta_vec_kernel(const AfBwdParams a) {
+__global__ void bwd_delta_vec_kernel(const AfBwdParams a, uint4* __restrict__ clear, const int64_t clear_chunks) {
   const AfProblem& p = a.p;
   const uint32_t gthread = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t r0 = gthread / LPR * DELTA_ROWS, sub = gthread % LPR;
@@ -105,6 +105,8 @@ __global__ void bwd_delta_vec_kernel(const AfBwdParams a) {
     gv[i] = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(a.d_o) + (int64_t)b * a.do_stride[0] +
                                                  (int64_t)h * a.do_stride[1] + (int64_t)row * a.do_stride[2] + sub * 8));
   }
+  // under the loads: the dQ accumulator of the pass that follows (a memset of its own is one operation more)
+  for (int64_t i = gthread; i < clear_chunks; i += (int64_t)gridDim.x * blockDim.x) clear[i] = make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
   for (int i = 0; i < DELTA_ROWS; ++i) {
     const T* oe = reinterpret_cast<const T*>(&ov[i]);
@@ -486,7 +488,7 @@ int launch_dtype(const AfBwdParams& a, cudaStream_t st) {
 }  // namespace
 
 // delta = rowsum(dO * O), fp32 (B, H_q, N_q); shared by both backward families.
-int launch_bwd_delta(const AfBwdParams& a, cudaStream_t st) {
+int launch_bwd_delta(const AfBwdParams& a, cudaStream_t st, void* clear, int64_t clear_bytes) {
   const int64_t rows = (int64_t)a.p.B * a.p.H_q * a.p.N_q;
   if (rows <= 0) return AF_OK;
   const AfProblem& p = a.p;
@@ -496,15 +498,17 @@ int launch_bwd_delta(const AfBwdParams& a, cudaStream_t st) {
   if (aligned && p.dtype != AF_F32 && (p.D == 64 || p.D == 128 || p.D == 256) && rows * (p.D / 8) < (1ll << 31)) {
     const int lpr = p.D / 8;
     const unsigned vblocks = (unsigned)(((rows + DELTA_ROWS - 1) / DELTA_ROWS * lpr + 255) / 256);
+    uint4* zero = static_cast<uint4*>(clear);
 #define AF_DELTA_VEC(TYPE)                                                                  \
-    if (lpr == 8) bwd_delta_vec_kernel<TYPE, 8><<<vblocks, 256, 0, st>>>(a);                \
-    else if (lpr == 16) bwd_delta_vec_kernel<TYPE, 16><<<vblocks, 256, 0, st>>>(a);         \
-    else bwd_delta_vec_kernel<TYPE, 32><<<vblocks, 256, 0, st>>>(a);
+    if (lpr == 8) bwd_delta_vec_kernel<TYPE, 8><<<vblocks, 256, 0, st>>>(a, zero, clear_bytes / 16);        \
+    else if (lpr == 16) bwd_delta_vec_kernel<TYPE, 16><<<vblocks, 256, 0, st>>>(a, zero, clear_bytes / 16); \
+    else bwd_delta_vec_kernel<TYPE, 32><<<vblocks, 256, 0, st>>>(a, zero, clear_bytes / 16);
     if (p.dtype == AF_F16) { AF_DELTA_VEC(__half) } else { AF_DELTA_VEC(__nv_bfloat16) }
 #undef AF_DELTA_VEC
     count_launch();
     return check_cuda(cudaGetLastError(), "bwd_delta launch");
   }
+  if (clear_bytes > 0) AF_CUDA_OK(cudaMemsetAsync(clear, 0, (size_t)clear_bytes, st));
   const unsigned blocks = (unsigned)((rows * 32 + 255) / 256);
   switch (a.p.dtype) {
     case AF_F16: bwd_delta_kernel<__half><<<blocks, 256, 0, st>>>(a); break;

@@ -1,6 +1,7 @@
 // Host side of the tcgen05 backward: support predicate, workspace, TMA descriptors, and the
 // launches: delta, then either the two passes (dK/dV, dQ) or -- with a dQ accumulator from the
 // caller -- the single fused pass followed by the dQ finishing kernel.
+#include <algorithm>
 #include <cstdlib>
 
 #include "bwd_tcgen05.cuh"
@@ -138,9 +139,29 @@ int launch_dq_finish(const float* acc, const AfBwdParams& a, int q_tiles, cudaSt
 }
 }  // namespace
 
+static int64_t dq_accum_bytes(const AfProblem& p) { return align256(dq_accum_floats(p) * 4) + 256; }
+
+// Whether the single pass is worth its accumulator.  At head dim 128 it always was.  At 64 it saves a quarter of the
+// backward's device time (4.3 against 3.3 clocks per 1000 scores and SM) and costs a call an allocation and a launch
+// more: training steps that wait for the host anyway (below about 170 us on the device: 8000 tiles of
+// 128 x 128 scores) lost 6 % with it, larger ones gain 15 - 25 %.  How many blocks a list visits is not known
+// on the host: eight per query tile are taken.  ATTNFUSE_BWD_SINGLE_PASS=1 in the environment (read at every
+// call) asks for it at every size.
+static bool single_pass_pays(const AfProblem& p) {
+  if (p.D != 64) return true;
+  if (const char* e = getenv("ATTNFUSE_BWD_SINGLE_PASS"))
+    if (e[0] == '1') return true;
+  const int64_t rows = (p.N_q + 127) / 128, cols = (p.N_kv + 127) / 128;
+  int64_t per_row = cols;
+  if (p.mask_kind == AF_MASK_CAUSAL) per_row = (cols + 1) / 2;
+  if (p.mask_kind == AF_MASK_WINDOW) per_row = std::min<int64_t>(cols, 2 * (((int64_t)p.window + 127) / 128) + 1);
+  if (p.mask_kind == AF_MASK_BLOCKS) per_row = std::min<int64_t>(cols, 8);
+  return rows * per_row * p.B * p.H_q >= 8000;
+}
+
 int64_t bwd_mma_dq_accum_bytes(const AfBwdParams& a) {
-  if (!bwd_mma_supports(a, nullptr)) return 0;
-  return align256(dq_accum_floats(a.p) * 4) + 256;
+  if (!bwd_mma_supports(a, nullptr) || !single_pass_pays(a.p)) return 0;
+  return dq_accum_bytes(a.p);
 }
 
 bool bwd_mma_supports(const AfBwdParams& a, const char** why) {
@@ -187,7 +208,10 @@ int launch_bwd_mma(const AfBwdParams& a, cudaStream_t st) {
   const char* why = nullptr;
   if (!bwd_mma_supports(a, &why)) return fail(AF_ERR_UNSUPPORTED, "tensor-core backward: %s", why);
   const AfProblem& p = a.p;
-  int rc = launch_bwd_delta(a, st);
+  // an accumulator that is large enough asks for the single pass, whatever the rule advises
+  const int64_t acc_bytes = dq_accum_bytes(p);
+  const bool single_pass = a.dq_accum != nullptr && a.dq_accum_bytes >= acc_bytes && ((uintptr_t)a.dq_accum & 255) == 0;
+  int rc = single_pass ? launch_bwd_delta(a, st, a.dq_accum, acc_bytes) : launch_bwd_delta(a, st);
   if (rc != AF_OK) return rc;
 
   const void* q_ptr = p.q;
@@ -212,8 +236,7 @@ int launch_bwd_mma(const AfBwdParams& a, cudaStream_t st) {
   if ((rc = tc_make_map(&do_strm, p.dtype, a.d_o, p.B, p.H_q, p.N_q, p.D, a.do_stride, strm_rows)) != AF_OK) return rc;
 
   const float key_stationary_scale = p.sm_scale > 0x1p-110f ? p.sm_scale : 0x1p-110f;
-  const int64_t acc_bytes = bwd_mma_dq_accum_bytes(a);
-  if (acc_bytes > 0 && a.dq_accum != nullptr && a.dq_accum_bytes >= acc_bytes && ((uintptr_t)a.dq_accum & 255) == 0) {
+  if (single_pass) {
     // ---- single fused pass: dK, dV and dQ from one recompute of S and dP ----
     tcb::BwdArgs f{};
     f.a = a;
@@ -241,7 +264,6 @@ int launch_bwd_mma(const AfBwdParams& a, cudaStream_t st) {
     f.q_tiles = (p.N_q + 127) / 128;
     AF_REQUIRE((int64_t)p.B * p.H_q * f.q_tiles <= 0x7fffffff, "too many tiles for one launch");
     f.sched_counter = reinterpret_cast<int32_t*>(static_cast<char*>(a.dq_accum) + align256(dq_accum_floats(p) * 4));
-    AF_CUDA_OK(cudaMemsetAsync(a.dq_accum, 0, (size_t)acc_bytes, st));
     rc = p.D == 64 ? tcb::launch_fused_d64(p.dtype, f, k_stat, v_stat, q_strm, do_strm, st)
                    : tcb::launch_fused_d128(p.dtype, f, k_stat, v_stat, q_strm, do_strm, st);
     if (rc != AF_OK) return rc;

@@ -80,7 +80,8 @@ int tc_sm_count(int* sms);
 int tc_launch_prepass(const AfProblem& p, void* q_out, void* k_out, cudaStream_t st);
 
 int launch_bwd_ffma(const AfBwdParams& a, cudaStream_t st);
-int launch_bwd_delta(const AfBwdParams& a, cudaStream_t st);
+// `clear`: bytes that are zero afterwards too (16-byte aligned and a multiple of 16 long).
+int launch_bwd_delta(const AfBwdParams& a, cudaStream_t st, void* clear = nullptr, int64_t clear_bytes = 0);
 int64_t bwd_mma_workspace_bytes(const AfBwdParams& a);
 int64_t bwd_mma_dq_accum_bytes(const AfBwdParams& a);
 int launch_bwd_mma(const AfBwdParams& a, cudaStream_t st);

@@ -220,8 +220,8 @@ AF_API int af_bwd(const AfBwdParams* params, af_stream_t stream);
 AF_API int64_t af_bwd_workspace_bytes(const AfBwdParams* params);
 
 /* Bytes of the optional dQ accumulator (AfBwdParams.dq_accum) with which af_bwd runs its
- * single-pass kernel for this problem; 0 when only other kernels apply (head_dim other than 64 and
- * 128, fp32, additive bias, ...).  af_bwd clears the accumulator itself.  No counterpart in the
+ * single-pass kernel for this problem; 0 when other kernels apply (head_dim other than 64 and 128,
+ * fp32, additive bias, ...) or are advised (few tiles at head_dim 64).  af_bwd clears the accumulator itself.  No counterpart in the
  * reference, whose backward always recomputes S and dP in both of its kernels
  * (attnfuse/compiler/codegen_backward.py:75-302).  Host only. */
 AF_API int64_t af_bwd_dq_accum_bytes(const AfBwdParams* params);

@@ -16,6 +16,11 @@ pytestmark = pytest.mark.gpu
 DEV, D = "cuda", 64
 
 
+@pytest.fixture(autouse=True)
+def at_every_size(monkeypatch):
+    monkeypatch.setenv("ATTNFUSE_BWD_SINGLE_PASS", "1")
+
+
 def graph(variant, heads, window=0):
     @af.attention
     def fn(Q, K, V):
@@ -93,3 +98,18 @@ def test_accumulator_is_padded_to_whole_tiles():
     p = _lib.AfBwdParams()
     fill_problem(p.p, q, k, v, sm_scale=D ** -0.5, mask_kind=1)
     assert int(_lib.load().af_bwd_dq_accum_bytes(C.byref(p))) >= 2 * 256 * D * 4      # two heads, rows padded to 256
+
+
+def test_rule(monkeypatch):
+    """Few tiles keep the two passes (one launch and one allocation less), many take the single pass."""
+    monkeypatch.delenv("ATTNFUSE_BWD_SINGLE_PASS")
+
+    def asks(B, H, N, dim=D, **mask):
+        q, k, v = (torch.empty(B, H, N, dim, device=DEV, dtype=torch.bfloat16) for _ in range(3))
+        p = _lib.AfBwdParams()
+        fill_problem(p.p, q, k, v, sm_scale=0.1, **mask)
+        return int(_lib.load().af_bwd_dq_accum_bytes(C.byref(p))) > 0
+    assert not asks(1, 12, 2000, mask_kind=1) and asks(4, 12, 4096, mask_kind=1)
+    assert not asks(4, 12, 1280, mask_kind=0) and asks(4, 12, 1700, mask_kind=0)
+    assert not asks(4, 12, 3001, mask_kind=2, window=100) and asks(4, 16, 4096, mask_kind=2, window=256)
+    assert asks(1, 2, 128, dim=128, mask_kind=1)
